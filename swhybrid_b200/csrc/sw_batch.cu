@@ -12,7 +12,7 @@
 //   * per bucket, one persistent launch of sw_batch<T,R> over its stacks
 //     (blocks walk the stacks in order, groups claim record pairs from one
 //     device counter per stack), plus, when a cut-over is set, a concurrent
-//     launch of single-group blocks for the pairs longer than the cut-over, so
+//     launch of single-warp blocks for the pairs longer than the cut-over, so
 //     their inherently serial column steps overlap the bulk;
 //   * one 32-bit re-score launch for every flagged (query, record) and one
 //     top-k round sequence with a grid row per query.
@@ -281,10 +281,8 @@ sw_status enqueue_batch(sw_ctx* ctx, sw_batch_state* b, uint32_t nq, size_t qbyt
             q.nstacks = L.scount;
             q.counters = b->d_counters + L.counter_base;
             q.mat = ctx->d_mat;
-            q.bias2 = (uint32_t)(ctx->params.gap_open + ctx->params.gap_extend);
-            q.bias2 |= q.bias2 << 16;
-            q.neg_e = (uint32_t)(uint16_t)(int16_t)(-ctx->params.gap_extend);
-            q.neg_e |= q.neg_e << 16;
+            q.gap_oe = ctx->params.gap_open + ctx->params.gap_extend;
+            q.gap_e = ctx->params.gap_extend;
             q.bnd = b->d_bnd + b->bnd_cap / 2;
             q.bnd_group = L.bnd_group;
             q.scores = b->d_scores;
@@ -318,10 +316,8 @@ sw_status enqueue_batch(sw_ctx* ctx, sw_batch_state* b, uint32_t nq, size_t qbyt
         a.nstacks = L.scount;
         a.counters = b->d_counters + L.counter_base;
         a.mat = ctx->d_mat;
-        a.bias2 = (uint32_t)(ctx->params.gap_open + ctx->params.gap_extend);
-        a.bias2 |= a.bias2 << 16;
-        a.neg_e = (uint32_t)(uint16_t)(int16_t)(-ctx->params.gap_extend);
-        a.neg_e |= a.neg_e << 16;
+        a.gap_oe = ctx->params.gap_open + ctx->params.gap_extend;
+        a.gap_e = ctx->params.gap_extend;
         a.bnd = L.long_part ? b->d_bnd : b->d_bnd + b->bnd_cap / 2;
         a.bnd_group = L.bnd_group;
         a.scores = b->d_scores;
@@ -598,13 +594,15 @@ extern "C" sw_status sw_search_batch(sw_ctx* ctx, uint32_t nq, const uint8_t* qu
             launches.push_back(L);
         }
         if (n_long > 0) {
-            // long pairs: single-group blocks of the same shape (the stacks'
+            // long pairs: single-warp blocks of the same shape (the stacks'
             // row maps are laid out for it)
             const int occl = shape_occupancy(ctx, *kb, (int)max_rows);
             BatchLaunch L;
             L.k = kb;
-            L.threads = kb->T;
-            L.grid = (int)std::min<int64_t>((int64_t)std::max(occl, 1) * 2 * ctx->num_sms, n_long);
+            const int per_warp = 32 / kb->T;       // pairs a warp claims at a time
+            L.threads = 32;
+            L.grid = (int)std::min<int64_t>((int64_t)std::max(occl, 1) * 2 * ctx->num_sms,
+                                            (n_long + per_warp - 1) / per_warp);
             L.smem = kb->smem((int)max_rows);
             L.sbegin = s0;
             L.scount = sidx - s0;
@@ -613,7 +611,7 @@ extern "C" sw_status sw_search_batch(sw_ctx* ctx, uint32_t nq, const uint8_t* qu
             L.counter_base = nst_total + s0;
             L.long_part = true;
             L.bnd_group = 2 * (size_t)ctx->max_cols;
-            bnd_long = std::max(bnd_long, (size_t)L.grid * L.bnd_group);
+            bnd_long = std::max(bnd_long, (size_t)L.grid * per_warp * L.bnd_group);
             launches.push_back(L);
         }
     }

@@ -38,15 +38,15 @@ struct WfArgs {
     int pass0;                  // query passes scored by earlier launches (row segments)
     int more;                   // != 0: a later launch scores the next row segment
     const int8_t* mat;          // 32x32, [query code][db code]; codes >= 24 score 0
-    uint32_t bias2;             // dup16(open+extend): the biased zero of a lane
-    uint32_t neg_e;             // dup16(-extend)
+    int gap_oe;                 // open + extend
+    int gap_e;                  // extend
     int* counter;               // pairs claimed (zero before the launch)
     uint2* bnd;                 // boundary rows: 16 entries per 16-byte stream unit
     int* scores;                // per sorted record position
     int n_records;
     int* ovf_list;              // sorted positions for the 32-bit pass
     int* ovf_count;
-    int ovf_thresh;             // biased lane value >= this may have wrapped
+    int ovf_thresh;             // biased H of a lane >= this may have wrapped
 };
 
 // Row-block map entry of a stacked batch: the query starts at this block.
@@ -66,8 +66,8 @@ struct BatchArgs {
     int nstacks;
     int* counters;              // one pair counter per stack (zero before)
     const int8_t* mat;
-    uint32_t bias2;
-    uint32_t neg_e;
+    int gap_oe;
+    int gap_e;
     uint2* bnd;                 // per-group boundary rows
     size_t bnd_group;           // entries per group (2 per column of the longest pair)
     int* scores;                // [query][sorted position], zero before (atomicMax)

@@ -33,6 +33,7 @@
 #include "sw_registry.h"
 
 namespace swb {
+int plain_cell(int lo, int hi, int q, int e);
 extern const WfKernel wf_table_t4[];
 extern const int wf_table_t4_n;
 extern const WfKernel wf_table_t8[];
@@ -197,14 +198,17 @@ extern "C" sw_status sw_ctx_create(int device, const sw_params* params, sw_ctx**
         if (cudaEventCreate(&e) != cudaSuccess) return fail(SW_ERR_CUDA);
     // matrix: int8 copy; codes >= 24 (zero code, pads) score 0
     int8_t mat8[1024];
-    int hi = 0;
+    int lo = 0, hi = 0;
     for (int i = 0; i < 32; ++i)
         for (int j = 0; j < 32; ++j) {
             int v = (i >= kZeroCode || j >= kZeroCode) ? 0 : ctx->params.matrix[i * 32 + j];
             mat8[i * 32 + j] = (int8_t)v;
+            lo = std::min(lo, v);
             hi = std::max(hi, v);
         }
     ctx->max_score = hi;
+    ctx->cell = plain_cell(lo, hi, ctx->params.gap_open + ctx->params.gap_extend,
+                           ctx->params.gap_extend);
     if (dev_alloc(&ctx->d_mat, 1024) != cudaSuccess) return fail(SW_ERR_NOMEM);
     if (cudaMemcpy(ctx->d_mat, mat8, 1024, cudaMemcpyHostToDevice) != cudaSuccess)
         return fail(SW_ERR_CUDA);
@@ -220,7 +224,7 @@ extern "C" sw_status sw_ctx_create(int device, const sw_params* params, sw_ctx**
     int nk = 0;
     const WfKernel* ks = wf_kernels(&nk);
     for (int i = 0; i < nk; ++i)
-        if (!allow_smem(ks[i].fn) || !allow_smem(ks[i].batch_fn)) return fail(SW_ERR_CUDA);
+        if (!allow_smem(ks[i].fn[ctx->cell]) || !allow_smem(ks[i].batch_fn)) return fail(SW_ERR_CUDA);
     const QpKernel* qks = qp_kernels(&nk);
     for (int i = 0; i < nk; ++i)
         if (!allow_smem(qks[i].fn)) return fail(SW_ERR_CUDA);
@@ -432,16 +436,38 @@ extern "C" sw_status sw_db_stats_get(const sw_ctx* ctx, sw_db_stats* out) {
 
 namespace swb {
 
-// Blocks per SM for a shape at a query length (0 = does not fit).
-int shape_occupancy(sw_ctx* ctx, const WfKernel& k, int qlen) {
-    const size_t smem = k.smem(qlen);
+// The plain kernel's cell variant for a matrix with entries lo..hi (the zero
+// of unscored codes included) and gap costs q = open+extend, e = extend.
+// CellNarrow's profile bytes are P + q, kept in 0..127 so that PRMT's sign
+// extension leaves them unsigned; any other matrix takes CellWide.
+int plain_cell(int lo, int hi, int q, int e) {
+    if (lo < -q || hi > 127 - q) return kCellWide;
+    if (q == 12 && e == 2) return kCellNarrow12_2;
+    if (q == 12 && e == 1) return kCellNarrow12_1;
+    return kCellNarrow;
+}
+
+// Blocks per SM for a kernel of a shape at a query length (0 = does not fit).
+static int kernel_occupancy(sw_ctx* ctx, const void* fn, int block, size_t smem) {
     if (smem > (size_t)ctx->max_smem) return 0;
     int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k.fn, k.block, smem) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, block, smem) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
     return nb;
+}
+
+int shape_occupancy(sw_ctx* ctx, const WfKernel& k, int qlen) {
+    return kernel_occupancy(ctx, k.batch_fn, k.block, k.smem(qlen));
+}
+
+int plain_block(const sw_ctx* ctx, const WfKernel& k) {
+    return ctx->cell == kCellWide ? k.block : k.narrow_block;
+}
+
+int plain_occupancy(sw_ctx* ctx, const WfKernel& k, int qlen) {
+    return kernel_occupancy(ctx, k.fn[ctx->cell], plain_block(ctx, k), k.smem(qlen));
 }
 
 // Query rows one launch of a shape scores: the whole query when its profile
@@ -449,10 +475,10 @@ int shape_occupancy(sw_ctx* ctx, const WfKernel& k, int qlen) {
 // query is scored in row segments by consecutive launches that hand the
 // boundary row on); 0 when not even one pass fits.
 int launch_rows(sw_ctx* ctx, const WfKernel& k, int qlen) {
-    if (shape_occupancy(ctx, k, qlen) > 0) return qlen;
+    if (plain_occupancy(ctx, k, qlen) > 0) return qlen;
     const int rows_pass = k.T * k.R;
     int p = 0;
-    while ((int64_t)(p + 1) * rows_pass < qlen && shape_occupancy(ctx, k, (p + 1) * rows_pass) > 0)
+    while ((int64_t)(p + 1) * rows_pass < qlen && plain_occupancy(ctx, k, (p + 1) * rows_pass) > 0)
         ++p;
     return p * rows_pass;
 }
@@ -477,13 +503,13 @@ double cols_at_least(const sw_ctx* ctx, int64_t b, int64_t e, uint32_t m) {
 // them: at least 2T + 2 steps for a pass a later pass depends on, 3 otherwise.
 double shape_cost(sw_ctx* ctx, const WfKernel& k, int qlen, int64_t b, int64_t e) {
     const int rows = launch_rows(ctx, k, qlen);
-    const int occ = rows > 0 ? shape_occupancy(ctx, k, rows) : 0;
+    const int occ = rows > 0 ? plain_occupancy(ctx, k, rows) : 0;
     if (occ == 0 || e <= b) return occ == 0 ? 1e300 : 0.0;
     const double P = (qlen + k.T * k.R - 1) / (k.T * k.R);
     const double cols = (P - 1) * cols_at_least(ctx, b, e, 2 * k.T + 2) + cols_at_least(ctx, b, e, 3);
     const double work = cols * (k.T * (k.R + 12.9) + 25.1);
     const double g_width = k.T >= 32 ? 1.0 : k.T >= 16 ? 0.854 : k.T >= 8 ? 0.687 : 0.663;
-    const double warps = (double)occ * k.block / 32.0;
+    const double warps = (double)occ * plain_block(ctx, k) / 32.0;
     const double g_warps = warps < 12 ? 0.912 : warps < 20 ? 1.0 : 1.09;
     return work / (g_width * g_warps);
 }
@@ -496,7 +522,7 @@ const sw_tuning_entry* find_entry(sw_ctx* ctx, int qlen) {
         if ((uint32_t)qlen > e.max_qlen) continue;
         const WfKernel* kl = find_kernel(e.cfg.long_group_width, e.cfg.long_rows_per_thread);
         const WfKernel* ks = find_kernel(e.cfg.short_group_width, e.cfg.short_rows_per_thread);
-        if (kl && ks && shape_occupancy(ctx, *kl, qlen) > 0 && shape_occupancy(ctx, *ks, qlen) > 0)
+        if (kl && ks && plain_occupancy(ctx, *kl, qlen) > 0 && plain_occupancy(ctx, *ks, qlen) > 0)
             return &e;
         return nullptr;   // the tuned shape does not fit this length: the model chooses
     }
@@ -633,9 +659,16 @@ constexpr int kMaxRowSegs = SW_PLAN_STEPS + 1;
 
 // Columns of one pass over the DB that an evenly loaded group of shape k gets.
 double group_share(sw_ctx* ctx, const WfKernel& k, int qlen) {
-    const int occ = std::max(1, shape_occupancy(ctx, k, qlen));
-    const double groups = (double)occ * ctx->num_sms * (k.block / k.T);
+    const int occ = std::max(1, plain_occupancy(ctx, k, qlen));
+    const double groups = (double)occ * ctx->num_sms * (plain_block(ctx, k) / k.T);
     return (double)ctx->pair_cols_total / groups;
+}
+
+// The share a plan's steps are checked against: the one at the shape's nominal
+// block size (sw_get_shapes), which the autotuner plans with.
+double plan_share(sw_ctx* ctx, const WfKernel& k, int qlen) {
+    const int occ = std::max(1, shape_occupancy(ctx, k, qlen));
+    return (double)ctx->pair_cols_total / ((double)occ * ctx->num_sms * (k.block / k.T));
 }
 
 // Cut-over for a configuration without one: a DB whose longest pair needs more
@@ -686,7 +719,7 @@ int build_plan(sw_ctx* ctx, int qlen, const WfKernel* ks, int64_t bulk_begin, Ro
     const double longest = (double)ctx->pair_ncols[bulk_begin];
     for (int i = 0; i < n; ++i)
         if (launch_rows(ctx, *segs[i].k, segs[i].rows) == 0 ||
-            longest > group_share(ctx, *segs[i].k, segs[i].rows))
+            longest > plan_share(ctx, *segs[i].k, segs[i].rows))
             return 1;
     std::copy(segs, segs + n, out);
     return n;
@@ -889,10 +922,8 @@ sw_status enqueue_search(sw_ctx* ctx, const uint8_t* d_query, int qlen, int32_t*
         la.qlen = qlen;
         la.passes = lpasses;
         la.mat = ctx->d_mat;
-        la.bias2 = (uint32_t)(ctx->params.gap_open + ctx->params.gap_extend);
-        la.bias2 |= la.bias2 << 16;
-        la.neg_e = (uint32_t)(uint16_t)(int16_t)(-ctx->params.gap_extend);
-        la.neg_e |= la.neg_e << 16;
+        la.gap_oe = ctx->params.gap_open + ctx->params.gap_extend;
+        la.gap_e = ctx->params.gap_extend;
         la.scores = ctx->d_scores;
         la.n_records = (int)ctx->n_records;
         la.ovf_list = ctx->d_ovf;
@@ -921,7 +952,7 @@ sw_status enqueue_search(sw_ctx* ctx, const uint8_t* d_query, int qlen, int32_t*
         const int seg_rows = launch_rows(ctx, *k, plan[pi].rows);
         for (int s0 = 0; s0 < plan[pi].rows; s0 += seg_rows) {
             const int rows = std::min(seg_rows, plan[pi].rows - s0);
-            const int occ = shape_occupancy(ctx, *k, rows);
+            const int occ = plain_occupancy(ctx, *k, rows);
             if (r0 > 0)   // the previous launch has claimed every pair
                 SW_CUDA(ctx, cudaMemsetAsync(ctx->d_counters + L.bulk_counter, 0, sizeof(int), st));
             WfArgs a;
@@ -934,10 +965,8 @@ sw_status enqueue_search(sw_ctx* ctx, const uint8_t* d_query, int qlen, int32_t*
             a.pass0 = passes_before;
             a.more = r0 + rows < qlen ? 1 : 0;
             a.mat = ctx->d_mat;
-            a.bias2 = (uint32_t)(ctx->params.gap_open + ctx->params.gap_extend);
-            a.bias2 |= a.bias2 << 16;
-            a.neg_e = (uint32_t)(uint16_t)(int16_t)(-ctx->params.gap_extend);
-            a.neg_e |= a.neg_e << 16;
+            a.gap_oe = ctx->params.gap_open + ctx->params.gap_extend;
+            a.gap_e = ctx->params.gap_extend;
             a.counter = ctx->d_counters + L.bulk_counter;
             a.bnd = ctx->d_bnd;
             a.scores = ctx->d_scores;
@@ -947,10 +976,13 @@ sw_status enqueue_search(sw_ctx* ctx, const uint8_t* d_query, int qlen, int32_t*
             a.ovf_thresh = ovf_thresh;
             void* args[] = {&a};
             int64_t grid = (int64_t)occ * (ctx->num_sms - reserved_sms);
-            const int64_t groups_per_block = k->block / k->T;
-            grid = std::min<int64_t>(grid, ((L.bulk_e - L.bulk_b) + groups_per_block - 1) / groups_per_block);
+            const int block = plain_block(ctx, *k);
+            // a warp claims 32 / T pairs at a time: no more blocks than claims
+            // (few pairs spread one warp per SM)
+            const int64_t per_claim = 32 / k->T;
+            grid = std::min<int64_t>(grid, ((L.bulk_e - L.bulk_b) + per_claim - 1) / per_claim);
             grid = std::max<int64_t>(grid, 1);
-            SW_CUDA(ctx, cudaLaunchKernel(k->fn, dim3((unsigned)grid), dim3(k->block), args,
+            SW_CUDA(ctx, cudaLaunchKernel(k->fn[ctx->cell], dim3((unsigned)grid), dim3(block), args,
                                           k->smem(rows), st));
             ++*launches;
             ++mk.fp_launches;

@@ -72,6 +72,7 @@ struct sw_ctx {
     sw_totals totals{};
     sw_params params{};
     int max_score = 0;
+    int cell = 0;                      // PlainCell of the plain kernel's launches
     int8_t* d_mat = nullptr;           // 32x32 int8, codes >= 24 zeroed
     int* d_counters = nullptr;         // [0],[1] pair counters, [2] overflow count
 
@@ -122,7 +123,9 @@ struct sw_ctx {
 namespace swb {
 struct WfKernel;
 const WfKernel* find_kernel(int T, int R);
-int shape_occupancy(sw_ctx* ctx, const WfKernel& k, int qlen);
+int shape_occupancy(sw_ctx* ctx, const WfKernel& k, int qlen);   // stacked kernel
+int plain_occupancy(sw_ctx* ctx, const WfKernel& k, int qlen);   // plain kernel
+int plain_block(const sw_ctx* ctx, const WfKernel& k);
 int launch_rows(sw_ctx* ctx, const WfKernel& k, int qlen);
 // sw_search without the serving check: one plain search with host buffers
 // (the serving scheduler runs requests too long for a stack through it)

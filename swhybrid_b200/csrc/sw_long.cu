@@ -57,18 +57,18 @@ __device__ __forceinline__ void long_step(uint32_t (&H)[R], uint32_t (&E)[R], co
                                           const uint2* t1, const uint2* b0, const uint2* b1,
                                           uint32_t prev_h, uint32_t f_in, uint32_t& mid_h,
                                           uint32_t& mid_f, uint32_t& f_bot_out, uint32_t& S,
-                                          const CellK& K) {
+                                          const CellWide& K) {
     constexpr int HALF = R / 2;
     constexpr int JSTRIDE = kCodes * GroupShape<kLT>::SLOTS;
     const uint32_t bot_diag = mid_h;
     uint32_t f_top = f_in, f_bot = mid_f;
     mid_h = H[HALF - 1];
-    reverse_sweep<R, 0, HALF>(H, E, t0, t1, JSTRIDE, prev_h);
-    reverse_sweep<R, HALF, R>(H, E, b0, b1, JSTRIDE, bot_diag);
+    reverse_sweep<R, 0, HALF>(H, E, t0, t1, JSTRIDE, prev_h, K);
+    reverse_sweep<R, HALF, R>(H, E, b0, b1, JSTRIDE, bot_diag, K);
 #pragma unroll
     for (int i = 0; i < HALF; ++i) {
-        forward_cell(H[i], E[i], f_top, K);
-        forward_cell(H[HALF + i], E[HALF + i], f_bot, K);
+        K.forward(H[i], E[i], f_top);
+        K.forward(H[HALF + i], E[HALF + i], f_bot);
         if (i & 1) S = __vimax3_s16x2(S, H[i - 1], H[i]);
         if (i & 1) S = __vimax3_s16x2(S, H[HALF + i - 1], H[HALF + i]);
         if (!(i & 1) && i == HALF - 1) S = __vimax3_s16x2(S, H[i], H[HALF + i]);
@@ -91,18 +91,15 @@ __global__ void __launch_bounds__(LongBlock<R>::value, 1) sw_long(const LongArgs
     const int P = a.passes;                               // warps per pipeline
     uint2* const prof = smem;
     uint2* const ring = smem + (size_t)P * NJ * JSTRIDE;  // G pipelines x (P-1) links
-    build_profile<T, R>(prof, a.query, a.qlen, a.mat, P);
+    build_profile<T, R>(prof, a.query, a.qlen, a.mat, P, 0);
     const int warp = (int)(threadIdx.x >> 5);
     const int g = warp / P;                               // this warp's pipeline
     const int w = warp - g * P;                           // ... and its pass in it
     const int t = (int)(threadIdx.x & 31);
     const bool leader = (w == 0 && t == 0);
-    CellK K;
-    K.bias2 = a.bias2;
-    K.neg_q2 = 0u - a.bias2;
-    K.neg_e2 = a.neg_e;
-    const uint32_t Z = a.bias2;
-    const int bias = (int)(a.bias2 & 0xffffu);
+    const CellWide K(a.gap_oe, a.gap_e);
+    const uint32_t Z = K.hz();
+    const int bias = (int)(Z & 0xffffu);
     const uint2* const prof_p = prof + (w * NJ) * JSTRIDE + t;
     uint2* const links = ring + (size_t)g * (P > 1 ? P - 1 : 0) * kLRing;
     uint2* const ring_out = links + (size_t)(w + 1 < P ? w : 0) * kLRing;       // link w -> w+1

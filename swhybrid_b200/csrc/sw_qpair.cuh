@@ -44,7 +44,7 @@ struct QpArgs {
     int nstacks;
     int* counters;              // one unit counter per double stack (zero before)
     const int8_t* mat;
-    uint32_t bias2, neg_e;
+    int gap_oe, gap_e;          // open + extend, extend
     uint2* bnd;                 // per-group boundary rows
     size_t bnd_group;
     int* scores;                // [query][sorted position], zero before (atomicMax)
@@ -228,7 +228,7 @@ __device__ __forceinline__ void column_step_qp(uint32_t (&H)[R], uint32_t (&E)[R
                                                uint32_t& mid_h, uint32_t& mid_f,
                                                uint32_t& out_h, uint32_t& out_f,
                                                uint32_t& S_top, uint32_t& S_bot,
-                                               const CellK& K) {
+                                               const CellWide& K) {
     constexpr int HALF = R / 2;
     const uint32_t bot_diag = mid_h;
     uint32_t f_top = f_in, f_bot = mid_f;
@@ -237,8 +237,8 @@ __device__ __forceinline__ void column_step_qp(uint32_t (&H)[R], uint32_t (&E)[R
     reverse_sweep_qp<R, HALF, R>(H, E, pb, JSTRIDE, bot_diag);
 #pragma unroll
     for (int i = 0; i < HALF; ++i) {
-        forward_cell(H[i], E[i], f_top, K);
-        forward_cell(H[HALF + i], E[HALF + i], f_bot, K);
+        K.forward(H[i], E[i], f_top);
+        K.forward(H[HALF + i], E[HALF + i], f_bot);
         if (i & 1) S_top = __vimax3_s16x2(S_top, H[i - 1], H[i]);
         if (i & 1) S_bot = __vimax3_s16x2(S_bot, H[HALF + i - 1], H[HALF + i]);
     }
@@ -275,12 +275,9 @@ __device__ __forceinline__ void run_qpairs(const QpArgs& a, const uint4* prof, i
     const int t = lane & (T - 1);
     const int slot = lane & (SLOTS - 1);
     const unsigned gmask = (T == 32) ? FULL : (((1u << T) - 1u) << (lane & ~(T - 1)));
-    CellK K;
-    K.bias2 = a.bias2;
-    K.neg_q2 = 0u - a.bias2;
-    K.neg_e2 = a.neg_e;
-    const uint32_t Z = a.bias2;
-    const int bias = (int)(a.bias2 & 0xffffu);
+    const CellWide K(a.gap_oe, a.gap_e);
+    const uint32_t Z = K.hz();
+    const int bias = (int)(Z & 0xffffu);
     const int units = units_end;
     const int dep_steps = 2 * T + 2;
     // thread 0 claims the group's units

@@ -454,10 +454,8 @@ sw_status enqueue_round(sw_ctx* ctx, sw_serve_state* s, int chunk, int buf,
         q.nstacks = (int)L.count;
         q.counters = s->d_counters + ns + 1 + L.first;
         q.mat = ctx->d_mat;
-        q.bias2 = (uint32_t)(ctx->params.gap_open + ctx->params.gap_extend);
-        q.bias2 |= q.bias2 << 16;
-        q.neg_e = (uint32_t)(uint16_t)(int16_t)(-ctx->params.gap_extend);
-        q.neg_e |= q.neg_e << 16;
+        q.gap_oe = ctx->params.gap_open + ctx->params.gap_extend;
+        q.gap_e = ctx->params.gap_extend;
         q.bnd = s->d_bnd;
         q.bnd_group = s->bnd_group;
         q.scores = s->d_scores;
@@ -498,10 +496,8 @@ sw_status enqueue_round(sw_ctx* ctx, sw_serve_state* s, int chunk, int buf,
         a.nstacks = (int)ns;
         a.counters = s->d_counters;
         a.mat = ctx->d_mat;
-        a.bias2 = (uint32_t)(ctx->params.gap_open + ctx->params.gap_extend);
-        a.bias2 |= a.bias2 << 16;
-        a.neg_e = (uint32_t)(uint16_t)(int16_t)(-ctx->params.gap_extend);
-        a.neg_e |= a.neg_e << 16;
+        a.gap_oe = ctx->params.gap_open + ctx->params.gap_extend;
+        a.gap_e = ctx->params.gap_extend;
         a.bnd = s->d_bnd;
         a.bnd_group = s->bnd_group;
         a.scores = s->d_scores;

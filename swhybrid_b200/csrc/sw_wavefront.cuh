@@ -29,11 +29,12 @@
 // src/AVXKernel.cpp:196-218, with the floor at 0 made explicit):
 //   h  = max(diag + P, E, F, 0);  S = max(S, h)
 //   hq = h - (open+extend);  E = max(E - extend, hq);  F = max(F - extend, hq)
-// Lanes hold value + (open+extend) (see CellK), so every lane stays in
-// [0, 32767] and the subtraction of open+extend cannot borrow across halves; a
-// lane can only wrap upward after exceeding 32767 - max(matrix), which is the
-// overflow threshold handed to the 32-bit re-score pass.  The residue chunk
-// and the boundary row are prefetched so that no step waits on global memory.
+// in one of two instruction sequences (CellWide, CellNarrow below).  Lanes hold
+// value + a bias of at least open+extend, so every lane stays in [0, 32767] and
+// 32-bit adds cannot borrow across halves; a lane can only wrap upward after
+// exceeding 32767 - max(matrix), which is the overflow threshold handed to the
+// 32-bit re-score pass.  The residue chunk and the boundary row are prefetched
+// so that no step waits on global memory.
 //
 // The query profile lives in shared memory as signed bytes, laid out so that
 // each thread's 8-row chunk for a residue code is one 8-byte word and the 16
@@ -71,13 +72,90 @@ __device__ __forceinline__ uint32_t pack_row(int i, const uint2& A, const uint2&
     }
 }
 
-// Constants of the cell recurrence.  Every H/E/F/S lane holds value + B with
-// B = open+extend (so "score 0" is B): h' >= B keeps h' - (open+extend) >= 0
-// in both halves, which makes the packed subtraction an ordinary 32-bit add.
-struct CellK {
+// The cell recurrence for any matrix with entries in -127..127: 4 DPX + 1
+// 32-bit add per row (the profile PRMT and the running maximum apart).  Every
+// H/E/F/S lane holds value + B with B = open+extend (so "score 0" is B):
+// h' >= B keeps h' - (open+extend) >= 0 in both halves, which makes the packed
+// subtraction an ordinary 32-bit add.
+struct CellWide {
     uint32_t bias2;     // (B, B)
     uint32_t neg_q2;    // -(B << 16 | B) mod 2^32, i.e. subtract open+extend per half
     uint32_t neg_e2;    // (-extend, -extend)
+    __device__ __forceinline__ CellWide(int q, int e)
+        : bias2((uint32_t)q * 0x10001u), neg_q2(0u - (uint32_t)q * 0x10001u), neg_e2(dup16(-e)) {}
+    __device__ __forceinline__ uint32_t hz() const { return bias2; }   // stored H of score 0
+    __device__ __forceinline__ uint32_t fz() const { return bias2; }   // E, F of score 0
+    __device__ __forceinline__ int profile_bias() const { return 0; }  // added to profile scores
+    // biased H minus what a lane of H holds (the threshold's shift)
+    __device__ __forceinline__ int stored_shift() const { return 0; }
+    // whether run_stream's plain steps load their profile words a step ahead
+    template <int T, int R>
+    static constexpr bool prefetch = R >= 40 && !(R == 64 && (T == 8 || T == 16));
+    // row k before its F is known: max(H[k-1] + P, E)
+    __device__ __forceinline__ uint32_t diag(uint32_t up, uint32_t p, uint32_t e) const {
+        return __viaddmax_s16x2(up, p, e);
+    }
+    // the rest of the cell: hk holds diag's result and receives H
+    __device__ __forceinline__ void forward(uint32_t& hk, uint32_t& ek, uint32_t& f) const {
+        const uint32_t h = __vimax3_s16x2(hk, f, bias2);
+        hk = h;
+        const uint32_t hq = h + neg_q2;
+        ek = __viaddmax_s16x2(ek, neg_e2, hq);
+        f = __viaddmax_s16x2(f, neg_e2, hq);
+    }
+};
+
+// Biased zero of CellNarrow's lanes: at least any accepted open+extend (1000),
+// and a compile-time constant, so that the maxima take it as an immediate.
+constexpr int kNarrowZero = 1024;
+
+// The cell recurrence for a matrix whose entries lie in [-q, 127 - q], q =
+// open+extend: 3 DPX + 3 32-bit adds per row.  The ALU pipe that runs DPX
+// (and PRMT) issues 2 warp-instructions per clock and SM, the bound of this
+// kernel, while two-input adds also run on the FMA pipe, which it leaves idle.
+//   x = HQ[k-1] + P'     stored lanes are HQ = h - q and profile words P + q >= 0,
+//                        so the substitution is a plain add: P + q cannot
+//                        borrow, and no separate offset has to be taken off
+//   h = max3(x, E, F);  HQ[k] = h - q
+//   E = max(E - e, HQ);  F = max3(F - e, HQ, Z)
+// F is floored at the biased zero Z, so h >= F >= Z needs no floor of its own
+// (a negative F never reaches an H >= 0; flooring F rather than E measured 6.8
+// against 6.1 TCUPS at 16x64).  Measured as a loop of plain steps at 16x64:
+// CellWide 5.75 TCUPS; CellNarrow with q and e from registers 6.65, with both
+// as immediates (template arguments, 0 = run time) 6.76.  Register operands
+// count because three-operand instructions are also bound by the register
+// file's reads (add and DPX with three registers issue 1:1 at 2.8 per clock,
+// with an immediate among them at 3.2).
+template <int Q, int E>
+struct CellNarrow {
+    uint32_t q2, e2;        // (q, q), (e, e)
+    uint32_t ne16;          // (-e, -e)
+    int q;
+    static constexpr uint32_t Z = (uint32_t)kNarrowZero * 0x10001u;
+    __device__ __forceinline__ CellNarrow(int q_, int e_) {
+        q = Q > 0 ? Q : q_;
+        const int e = Q > 0 ? E : e_;
+        q2 = (uint32_t)q * 0x10001u;
+        e2 = (uint32_t)e * 0x10001u;
+        ne16 = dup16(-e);
+    }
+    __device__ __forceinline__ uint32_t hz() const { return Z - q2; }
+    __device__ __forceinline__ uint32_t fz() const { return Z; }
+    __device__ __forceinline__ int profile_bias() const { return q; }
+    __device__ __forceinline__ int stored_shift() const { return q; }
+    // (no prefetch: it measured within 2 % of the loads inside the step at 40+
+    // rows, either way by shape)
+    template <int T, int R>
+    static constexpr bool prefetch = false;
+    __device__ __forceinline__ uint32_t diag(uint32_t up, uint32_t p, uint32_t) const {
+        return up + p;
+    }
+    __device__ __forceinline__ void forward(uint32_t& hk, uint32_t& ek, uint32_t& f) const {
+        const uint32_t hq = __vimax3_s16x2(hk, ek, f) - q2;
+        hk = hq;
+        ek = __viaddmax_s16x2(ek, ne16, hq);
+        f = __vimax3_s16x2(f - e2, hq, Z);
+    }
 };
 
 // Row k's profile word from a chunk pair (A: record 2p's residue, B: record
@@ -86,12 +164,12 @@ __device__ __forceinline__ uint32_t pack_k(int k, const uint2& A, const uint2& B
     return pack_row(k & 7, A, B);
 }
 
-// Reverse sweep of one half: H[k] <- max(H[k-1] + P_k, E_k) for k = HI-1 down
+// Reverse sweep of one half: H[k] <- K.diag(H[k-1], P_k, E_k) for k = HI-1 down
 // to LO, with H[LO-1] replaced by diag.  p0/p1 point at the residues' chunk 0.
-template <int R, int LO, int HI>
+template <int R, int LO, int HI, class CELL>
 __device__ __forceinline__ void reverse_sweep(uint32_t (&H)[R], const uint32_t (&E)[R],
                                               const uint2* p0, const uint2* p1, int jstride,
-                                              uint32_t diag) {
+                                              uint32_t diag, const CELL& K) {
     constexpr int JLO = LO / 8, JHI = (HI - 1) / 8;
     uint2 A = p0[JHI * jstride];
     uint2 B = p1[JHI * jstride];
@@ -107,23 +185,12 @@ __device__ __forceinline__ void reverse_sweep(uint32_t (&H)[R], const uint32_t (
             const int k = j * 8 + i;
             if (k >= LO && k < HI) {
                 const uint32_t up = (k > LO) ? H[k > LO ? k - 1 : LO] : diag;
-                H[k] = __viaddmax_s16x2(up, pack_k(k, A, B), E[k]);
+                H[k] = K.diag(up, pack_k(k, A, B), E[k]);
             }
         }
         A = An;
         B = Bn;
     }
-}
-
-// One forward cell: h = max(t, F, B); hq = h - (open+extend);
-// E = max(E - extend, hq); F = max(F - extend, hq).
-__device__ __forceinline__ void forward_cell(uint32_t& Hk, uint32_t& Ek, uint32_t& f,
-                                             const CellK& K) {
-    const uint32_t h = __vimax3_s16x2(Hk, f, K.bias2);
-    Hk = h;
-    const uint32_t hq = h + K.neg_q2;
-    Ek = __viaddmax_s16x2(Ek, K.neg_e2, hq);
-    f = __viaddmax_s16x2(f, K.neg_e2, hq);
 }
 
 // One column step of a thread's two halves: the top half (rows [0, R/2)) on
@@ -132,7 +199,7 @@ __device__ __forceinline__ void forward_cell(uint32_t& Hk, uint32_t& Ek, uint32_
 // (handed down by the thread above, or the boundary row); mid_h / mid_f carry
 // the top half's last row from one column to the bottom half's next; out_h /
 // out_f receive the bottom half's last row (what the thread below takes).
-template <int R, int JSTRIDE>
+template <int R, int JSTRIDE, class CELL>
 __device__ __forceinline__ void column_step(uint32_t (&H)[R], uint32_t (&E)[R],
                                             const uint2* t0, const uint2* t1,
                                             const uint2* b0, const uint2* b1,
@@ -140,18 +207,18 @@ __device__ __forceinline__ void column_step(uint32_t (&H)[R], uint32_t (&E)[R],
                                             uint32_t& mid_h, uint32_t& mid_f,
                                             uint32_t& out_h, uint32_t& out_f,
                                             uint32_t& S_top, uint32_t& S_bot,
-                                            const CellK& K) {
+                                            const CELL& K) {
     constexpr int HALF = R / 2;
-    const uint32_t Z = K.bias2;
+    const uint32_t Z = K.hz();
     const uint32_t bot_diag = mid_h;
     uint32_t f_top = f_in, f_bot = mid_f;
     mid_h = H[HALF - 1];     // the top's last row one column back
-    reverse_sweep<R, 0, HALF>(H, E, t0, t1, JSTRIDE, prev_h);
-    reverse_sweep<R, HALF, R>(H, E, b0, b1, JSTRIDE, bot_diag);
+    reverse_sweep<R, 0, HALF>(H, E, t0, t1, JSTRIDE, prev_h, K);
+    reverse_sweep<R, HALF, R>(H, E, b0, b1, JSTRIDE, bot_diag, K);
 #pragma unroll
     for (int i = 0; i < HALF; ++i) {
-        forward_cell(H[i], E[i], f_top, K);
-        forward_cell(H[HALF + i], E[HALF + i], f_bot, K);
+        K.forward(H[i], E[i], f_top);
+        K.forward(H[HALF + i], E[HALF + i], f_bot);
         if (i & 1) S_top = __vimax3_s16x2(S_top, H[i - 1], H[i]);
         if (i & 1) S_bot = __vimax3_s16x2(S_bot, H[HALF + i - 1], H[HALF + i]);
         if (!(i & 1) && i == HALF - 1) {
@@ -184,11 +251,11 @@ __device__ __forceinline__ void load_words(uint2 (&A)[HalfChunks<LO, HI>::N],
 }
 
 // reverse_sweep with the profile words already in registers.
-template <int R, int LO, int HI>
+template <int R, int LO, int HI, class CELL>
 __device__ __forceinline__ void reverse_sweep_w(uint32_t (&H)[R], const uint32_t (&E)[R],
                                                 const uint2 (&A)[HalfChunks<LO, HI>::N],
                                                 const uint2 (&B)[HalfChunks<LO, HI>::N],
-                                                uint32_t diag) {
+                                                uint32_t diag, const CELL& K) {
     constexpr int JLO = HalfChunks<LO, HI>::JLO, JHI = HalfChunks<LO, HI>::JHI;
 #pragma unroll
     for (int j = JHI; j >= JLO; --j) {
@@ -197,31 +264,31 @@ __device__ __forceinline__ void reverse_sweep_w(uint32_t (&H)[R], const uint32_t
             const int k = j * 8 + i;
             if (k >= LO && k < HI) {
                 const uint32_t up = (k > LO) ? H[k > LO ? k - 1 : LO] : diag;
-                H[k] = __viaddmax_s16x2(up, pack_k(k, A[j - JLO], B[j - JLO]), E[k]);
+                H[k] = K.diag(up, pack_k(k, A[j - JLO], B[j - JLO]), E[k]);
             }
         }
     }
 }
 
 // column_step with both halves' profile words already in registers.
-template <int R>
+template <int R, class CELL>
 __device__ __forceinline__ void column_step_w(
     uint32_t (&H)[R], uint32_t (&E)[R], const uint2 (&tA)[HalfChunks<0, R / 2>::N],
     const uint2 (&tB)[HalfChunks<0, R / 2>::N], const uint2 (&bA)[HalfChunks<R / 2, R>::N],
     const uint2 (&bB)[HalfChunks<R / 2, R>::N], uint32_t prev_h, uint32_t f_in, uint32_t& mid_h,
     uint32_t& mid_f, uint32_t& out_h, uint32_t& out_f, uint32_t& S_top, uint32_t& S_bot,
-    const CellK& K) {
+    const CELL& K) {
     constexpr int HALF = R / 2;
-    const uint32_t Z = K.bias2;
+    const uint32_t Z = K.hz();
     const uint32_t bot_diag = mid_h;
     uint32_t f_top = f_in, f_bot = mid_f;
     mid_h = H[HALF - 1];
-    reverse_sweep_w<R, 0, HALF>(H, E, tA, tB, prev_h);
-    reverse_sweep_w<R, HALF, R>(H, E, bA, bB, bot_diag);
+    reverse_sweep_w<R, 0, HALF>(H, E, tA, tB, prev_h, K);
+    reverse_sweep_w<R, HALF, R>(H, E, bA, bB, bot_diag, K);
 #pragma unroll
     for (int i = 0; i < HALF; ++i) {
-        forward_cell(H[i], E[i], f_top, K);
-        forward_cell(H[HALF + i], E[HALF + i], f_bot, K);
+        K.forward(H[i], E[i], f_top);
+        K.forward(H[HALF + i], E[HALF + i], f_bot);
         if (i & 1) S_top = __vimax3_s16x2(S_top, H[i - 1], H[i]);
         if (i & 1) S_bot = __vimax3_s16x2(S_bot, H[HALF + i - 1], H[HALF + i]);
         if (!(i & 1) && i == HALF - 1) {
@@ -236,10 +303,11 @@ __device__ __forceinline__ void column_step_w(
 
 // Query profile of one query -> shared memory (whole block; the caller
 // synchronises).  Layout [pass][chunk][code][slot] of 8-byte words holding the
-// signed scores of 8 consecutive rows of the slot's thread.
+// signed scores (plus pbias, the cell's profile bias) of 8 consecutive rows of
+// the slot's thread.
 template <int T, int R>
 __device__ __forceinline__ void build_profile(uint2* prof, const uint8_t* query, int qlen,
-                                              const int8_t* mat, int P) {
+                                              const int8_t* mat, int P, int pbias) {
     constexpr int NJ = (R + 7) / 8;
     constexpr int SLOTS = GroupShape<T>::SLOTS;
     constexpr int JSTRIDE = kCodes * SLOTS;
@@ -259,12 +327,18 @@ __device__ __forceinline__ void build_profile(uint2* prof, const uint8_t* query,
             const int row = row0 + i;
             int v = 0;
             if (row < qlen) v = mat[(query[row] & 31) * 32 + d];
-            const uint32_t b = (uint32_t)(uint8_t)(int8_t)v << (8 * (i & 3));
+            const uint32_t b = (uint32_t)(uint8_t)(int8_t)(v + pbias) << (8 * (i & 3));
             if (i < 4) w0 |= b; else w1 |= b;
         }
         prof[idx] = make_uint2(w0, w1);
     }
 }
+
+// A compile-time flag passed to a generic lambda.
+template <bool B>
+struct Flag {
+    static constexpr bool value = B;
+};
 
 // What one call of run_stream works on.
 struct RunArgs {
@@ -282,7 +356,6 @@ struct RunArgs {
     // row).  0, 0 for a query that fits one launch.
     int pass0;
     int more;
-    uint32_t bias2, neg_e;      // see CellK
     uint2* bnd;                 // boundary rows between passes
     size_t bnd_group;           // 0: per-pair rows at bnd + 16*off16; else this many
                                 // entries per group at bnd + group * bnd_group
@@ -291,7 +364,7 @@ struct RunArgs {
     int* ovf_list;              // (ovf_base + position) of lanes for the 32-bit pass
     int* ovf_count;
     int ovf_base;
-    int ovf_thresh;             // biased lane value >= this may have wrapped
+    int ovf_thresh;             // biased H of a lane >= this may have wrapped
     int ovf_cap;                // entries the overflow list holds
     const uint32_t* pair_ids;   // optional: global pair of table entry i (a
                                 // permuted table); null = identity
@@ -309,15 +382,16 @@ struct RunArgs {
 // overwrites this value with the exact score.
 constexpr int kListed = 0x7fffffff;
 
-// Plain search: a record's first-pass score (biased lane value s) at its
+// Plain search: a record's first-pass score (lane value s) at its
 // sorted position.  A lane that may have wrapped lists the record for the
 // 32-bit pass.  With the query in row segments (pass0 / more) the score is
 // the maximum over the segments, and a listed record keeps kListed so that a
 // later segment does not list it again.
-__device__ __forceinline__ void put_score(const RunArgs& a, int pos, int s, int bias) {
+__device__ __forceinline__ void put_score(const RunArgs& a, int pos, int s, int bias,
+                                          int ovf_thresh) {
     if (a.pass0 == 0 && !a.more) {
         a.scores[pos] = s - bias;
-        if (s >= a.ovf_thresh) {
+        if (s >= ovf_thresh) {
             const int j = atomicAdd(a.ovf_count, 1);
             if (j < a.ovf_cap) a.ovf_list[j] = a.ovf_base + pos;
         }
@@ -325,7 +399,7 @@ __device__ __forceinline__ void put_score(const RunArgs& a, int pos, int s, int 
     }
     const int prev = a.scores[pos];
     if (prev == kListed) return;
-    if (s >= a.ovf_thresh) {
+    if (s >= ovf_thresh) {
         a.scores[pos] = kListed;
         const int j = atomicAdd(a.ovf_count, 1);
         if (j < a.ovf_cap) a.ovf_list[j] = a.ovf_base + pos;
@@ -334,9 +408,19 @@ __device__ __forceinline__ void put_score(const RunArgs& a, int pos, int s, int 
     }
 }
 
-// The group loop: every group of T threads claims pairs from the range and
-// scores them against the query (or query stack) whose profile is in prof;
-// returns when the range is exhausted (warp-wide).
+// The group loop: the G = 32 / T groups of a warp claim G neighbouring pairs of
+// the range at a time and score them against the query (or query stack) whose
+// profile is in prof; returns when the range is exhausted (warp-wide).
+//
+// The groups of a warp run in lockstep: their segments last as many steps as
+// the longest of the G pairs needs (the table is sorted by length, so that is
+// the same count or one or two more), and every group's thread t meets its
+// segment events at the same step.  Claiming pairs one by one, each group went
+// through its own window of 2T + 9 event steps per segment while the other
+// groups of the warp ran theirs as event steps too.  A group beyond the last
+// pair repeats the last one and writes nothing.  A warp's first claim is fixed
+// (warp w of block b takes the w * gridDim + b'th), so that few pairs spread
+// over all SMs; the later ones come from the counter.
 //
 // The groups stream: each thread moves on to the group's next segment (the
 // next pass of the pair, or the next pair) as soon as its own columns of the
@@ -363,8 +447,8 @@ __device__ __forceinline__ void put_score(const RunArgs& a, int pos, int s, int 
 //     zero-score residues, which cannot raise a score); every other segment
 //     lasts at least 3 steps, which keeps the descriptor and maximum hand-offs
 //     one segment apart.
-template <int T, int R, bool STACKED>
-__device__ __forceinline__ void run_stream(const RunArgs& a, const uint2* prof) {
+template <int T, int R, bool STACKED, class CELL>
+__device__ __forceinline__ void run_stream(const RunArgs& a, const uint2* prof, const CELL& K) {
     static_assert(R % 2 == 0 && R >= 4, "R");
     constexpr int NJ = (R + 7) / 8;    // 8-row profile chunks per thread (last one partial)
     constexpr int HALF = R / 2;
@@ -376,15 +460,15 @@ __device__ __forceinline__ void run_stream(const RunArgs& a, const uint2* prof) 
     const int lane = threadIdx.x & 31;
     const int t = lane & (T - 1);
     const int slot = lane & (SLOTS - 1);
-    const unsigned gmask = (T == 32) ? FULL : (((1u << T) - 1u) << (lane & ~(T - 1)));
-    CellK K;
-    K.bias2 = a.bias2;
-    K.neg_q2 = 0u - a.bias2;
-    K.neg_e2 = a.neg_e;
-    const uint32_t Z = a.bias2;        // biased zero of both lanes
-    const int bias = (int)(a.bias2 & 0xffffu);
+    const uint32_t HZ = K.hz(), FZ = K.fz();   // both lanes of H (and maxima), of E and F, at score 0
+    const int bias = (int)(HZ & 0xffffu);
+    const int ovf_thresh = a.ovf_thresh - K.stored_shift();
     const int pair_count = a.pair_count;
+    constexpr int G = 32 / T;          // groups (pairs) per warp
+    const int grp = lane / T;
     const int dep_steps = 2 * T + 2;
+    // no boundary row is read or written: one pass holds the whole query
+    const bool one_pass = P == 1 && a.pass0 == 0 && !a.more;
     uint2* const grp_bnd =
         a.bnd + (size_t)((blockIdx.x * blockDim.x + threadIdx.x) / T) * a.bnd_group;
 
@@ -393,11 +477,11 @@ __device__ __forceinline__ void run_stream(const RunArgs& a, const uint2* prof) 
     uint32_t H[R], E[R];
 #pragma unroll
     for (int k = 0; k < R; ++k) {
-        H[k] = Z;
-        E[k] = Z;
+        H[k] = HZ;
+        E[k] = FZ;
     }
-    uint32_t S_top = Z, S_bot = Z, S_pend = Z, acc_out = Z;
-    uint32_t out_h = Z, out_f = Z, prev_h = Z, mid_h = Z, mid_f = Z;
+    uint32_t S_top = HZ, S_bot = HZ, S_pend = HZ, acc_out = HZ;
+    uint32_t out_h = HZ, out_f = FZ, prev_h = HZ, mid_h = HZ, mid_f = FZ;
     uint32_t d_bot = kPadPair, d_cur = kPadPair;
     // the top half's profile offsets of the last column it computed: the
     // bottom half takes them one step later (its profile base is then the one
@@ -405,6 +489,7 @@ __device__ __forceinline__ void run_stream(const RunArgs& a, const uint2* prof) 
     int po0 = kZeroCode * SLOTS, po1 = kZeroCode * SLOTS;
     // the top half's segment
     int pair = 0, pass = 0, ncols = 0, nst = 0, c = 0;
+    int wcols = 0;             // columns of the warp's longest pair
     uint32_t off16 = 0u;
     const unsigned short* col = reinterpret_cast<const unsigned short*>(a.db);
     const uint2* prof_t = prof + slot;
@@ -422,12 +507,14 @@ __device__ __forceinline__ void run_stream(const RunArgs& a, const uint2* prof) 
     // a segment whose maximum is being finished
     int fpair = 0, f_q = 0;
     bool fpend = false, f_first = false, f_last = false, fin = false;
-    // thread 0: the next pair (claimed one pair ahead) and the boundary row
-    // read by passes after the first (two columns prefetched)
+    // lane 0: the warp's next pairs (claimed one segment ahead); thread 0: its
+    // group's next pair and the boundary row read by passes after the first
+    // (two columns prefetched)
     int next = 0, nload = -1;   // nload: the step of the first pass that loads its entry
     Pair2 ninfo{0u, 0u};
-    uint2 bq0 = make_uint2(Z, Z), bq1 = bq0;
+    uint2 bq0 = make_uint2(HZ, FZ), bq1 = bq0;
     const uint2* rrow = a.bnd;
+    int claimed;               // pairs the warps' first claims take
 
     // the boundary rows are double-buffered by the parity of the pass's index
     // in the whole query; a launch's last pass writes one only when a later
@@ -436,7 +523,7 @@ __device__ __forceinline__ void run_stream(const RunArgs& a, const uint2* prof) 
 #define SWS_SET_SEG()                                                          \
     {                                                                          \
         const int lo = (pass + 1 < P) ? dep_steps : 3;                         \
-        nst = ncols > lo ? ncols : lo;                                         \
+        nst = wcols > lo ? wcols : lo;                                         \
         col = reinterpret_cast<const unsigned short*>(a.db) + (size_t)off16 * 8; \
         uint2* const pb = a.bnd_group ? grp_bnd : a.bnd + (size_t)off16 * 16;  \
         wrow = pb + ((a.pass0 + pass) & 1);                                    \
@@ -454,18 +541,19 @@ __device__ __forceinline__ void run_stream(const RunArgs& a, const uint2* prof) 
     }
 
     {
-        int v = 0;
-        if (t == 0) v = atomicAdd(a.counter, 1);
-        v = __shfl_sync(gmask, v, 0, T);
-        pair = v;
+        const int warps = (int)(blockDim.x >> 5);
+        const int v = ((int)(threadIdx.x >> 5) * (int)gridDim.x + (int)blockIdx.x) * G;
+        claimed = warps * (int)gridDim.x * G;
+        pair = v + grp;
         if (v < pair_count) {
-            const Pair2 pr = a.pairs[a.pair_begin + v];
+            const Pair2 pr = a.pairs[a.pair_begin + min(pair, pair_count - 1)];
             off16 = pr.off16;
             ncols = (int)pr.ncols;
-            if (t == 0) next = atomicAdd(a.counter, 1);
+            if (lane == 0) next = claimed + atomicAdd(a.counter, G);
         } else {
             fin = true;
         }
+        wcols = (int)__reduce_max_sync(FULL, (unsigned)ncols);
         SWS_SET_SEG()
         prof_b = prof_t;
         b_wrow = wrow;
@@ -485,14 +573,15 @@ __device__ __forceinline__ void run_stream(const RunArgs& a, const uint2* prof) 
         uint32_t h_in = __shfl_up_sync(FULL, out_h, 1, T);
         uint32_t f_in = __shfl_up_sync(FULL, out_f, 1, T);
         const uint32_t acc_in = __shfl_up_sync(FULL, acc_out, 1, T);
+        const int warp_next = (G > 1) ? __shfl_sync(FULL, next, 0) : next;
         const uint32_t d_in = d_cur;
         {
             const int c1 = c + 1;     // this thread's top column next step
             d_cur = (c1 >= 0 && c1 < ncols) ? (uint32_t)__ldg(col + c1) : kPadPair;
         }
         if (t == 0) {
-            h_in = Z;
-            f_in = Z;
+            h_in = HZ;
+            f_in = FZ;
             if (a.pass0 + pass > 0 && c < ncols) {
                 h_in = bq0.x;
                 f_in = bq0.y;
@@ -500,11 +589,12 @@ __device__ __forceinline__ void run_stream(const RunArgs& a, const uint2* prof) 
                 if (c + 2 < ncols) bq1 = rrow[2 * (c + 2)];
             }
             // the next pair's table entry, once its claim has returned
-            if (c == nload && next < pair_count) ninfo = a.pairs[a.pair_begin + next];
+            if (c == nload && warp_next < pair_count)
+                ninfo = a.pairs[a.pair_begin + min(warp_next + grp, pair_count - 1)];
         }
         if (STACKED && my_first) {   // a query starts here: nothing flows in from above
-            h_in = Z;
-            f_in = Z;
+            h_in = HZ;
+            f_in = FZ;
         }
         if (!fin && c >= 0) {
             // a column past the segment's end runs on zero-score residues:
@@ -530,46 +620,46 @@ __device__ __forceinline__ void run_stream(const RunArgs& a, const uint2* prof) 
                 // the bottom has just done the finished segment's last column:
                 // this thread's maximum joins the chain down the group
                 fpend = false;
-                uint32_t m = __vimax3_s16x2(S_pend, S_bot, Z);
+                uint32_t m = __vimax3_s16x2(S_pend, S_bot, HZ);
                 if (STACKED) {
-                    if (t > 0 && !f_first) m = __vimax3_s16x2(m, acc_in, Z);
+                    if (t > 0 && !f_first) m = __vimax3_s16x2(m, acc_in, HZ);
                     acc_out = m;
-                    if (f_q >= 0 && f_last) {
+                    if (f_q >= 0 && f_last && fpair < pair_count) {
                         const int gp = a.pair_ids ? (int)a.pair_ids[a.pair_begin + fpair]
                                                   : a.pair_begin + fpair;
                         const int pos = 2 * gp;
                         const int s0 = lo16(m), s1 = hi16(m);
                         const int qb = f_q * a.n_records;
                         atomicMax(a.scores + qb + pos, s0 - bias);
-                        if (s0 >= a.ovf_thresh) {
+                        if (s0 >= ovf_thresh) {
                             const int j = atomicAdd(a.ovf_count, 1);
                             if (j < a.ovf_cap) a.ovf_list[j] = qb + pos;
                         }
                         if (pos + 1 < a.n_records) {
                             atomicMax(a.scores + qb + pos + 1, s1 - bias);
-                            if (s1 >= a.ovf_thresh) {
+                            if (s1 >= ovf_thresh) {
                                 const int j = atomicAdd(a.ovf_count, 1);
                                 if (j < a.ovf_cap) a.ovf_list[j] = qb + pos + 1;
                             }
                         }
                     }
                 } else {
-                    if (t > 0) m = __vimax3_s16x2(m, acc_in, Z);
+                    if (t > 0) m = __vimax3_s16x2(m, acc_in, HZ);
                     acc_out = m;
-                    if (t == T - 1) {
+                    if (t == T - 1 && fpair < pair_count) {
                         const int pos = 2 * (a.pair_begin + fpair);
-                        put_score(a, pos, lo16(m), bias);
-                        if (pos + 1 < a.n_records) put_score(a, pos + 1, hi16(m), bias);
+                        put_score(a, pos, lo16(m), bias, ovf_thresh);
+                        if (pos + 1 < a.n_records) put_score(a, pos + 1, hi16(m), bias, ovf_thresh);
                     }
                 }
-                S_bot = Z;
-                if (pair >= pair_count) fin = true;
+                S_bot = HZ;
+                if (pair - grp >= pair_count) fin = true;
             }
             if (c == 0) {   // the bottom starts this segment's column 0 next step
 #pragma unroll
                 for (int k = HALF; k < R; ++k) {
-                    H[k] = Z;
-                    E[k] = Z;
+                    H[k] = HZ;
+                    E[k] = FZ;
                 }
                 prof_b = prof_t;
                 b_wrow = wrow;
@@ -580,11 +670,14 @@ __device__ __forceinline__ void run_stream(const RunArgs& a, const uint2* prof) 
             const int up_pair = __shfl_up_sync(FULL, pair, 1, T);
             const uint32_t up_off = __shfl_up_sync(FULL, off16, 1, T);
             const int up_ncols = __shfl_up_sync(FULL, ncols, 1, T);
+            const int up_wcols = (G > 1) ? __shfl_up_sync(FULL, wcols, 1, T) : up_ncols;
+            const int next_wcols = (G > 1) ? (int)__reduce_max_sync(FULL, t == 0 ? ninfo.ncols : 0u)
+                                           : (int)ninfo.ncols;
             if (adv) {
                 const bool last_pass = pass + 1 >= P;
                 if (STACKED || last_pass) {   // the maximum being finished
                     S_pend = S_top;
-                    S_top = Z;
+                    S_top = HZ;
                     fpair = pair;
                     f_q = my_q;
                     f_first = my_first;
@@ -596,25 +689,31 @@ __device__ __forceinline__ void run_stream(const RunArgs& a, const uint2* prof) 
                 } else {
                     pass = 0;
                     if (t == 0) {
-                        pair = next;
+                        pair = warp_next + grp;
                         off16 = ninfo.off16;
                         ncols = (int)ninfo.ncols;
-                        if (pair < pair_count) next = atomicAdd(a.counter, 1);
+                        wcols = next_wcols;
+                        if (lane == 0 && warp_next < pair_count)
+                            next = claimed + atomicAdd(a.counter, G);
                     } else {
                         pair = up_pair;
                         off16 = up_off;
                         ncols = up_ncols;
+                        wcols = up_wcols;
                     }
-                    if (pair >= pair_count) ncols = 0;
+                    if (pair - grp >= pair_count) {
+                        ncols = 0;
+                        wcols = 0;
+                    }
                 }
                 SWS_SET_SEG()
                 c = -1;
 #pragma unroll
                 for (int k = 0; k < HALF; ++k) {
-                    H[k] = Z;
-                    E[k] = Z;
+                    H[k] = HZ;
+                    E[k] = FZ;
                 }
-                prev_h = Z;
+                prev_h = HZ;
                 if (t == 0 && a.pass0 + pass > 0) {
                     if (ncols > 0) bq0 = rrow[0];
                     if (ncols > 1) bq1 = rrow[2];
@@ -642,7 +741,7 @@ __device__ __forceinline__ void run_stream(const RunArgs& a, const uint2* prof) 
             const bool rd0 = t == 0 && a.pass0 + pass > 0;            // boundary row in
             const bool zin = (t == 0 && a.pass0 + pass == 0) || (STACKED && my_first);
             const bool wr = t == T - 1 && wlim > 0;                   // boundary row out
-            if constexpr (R >= 40 && !(R == 64 && (T == 8 || T == 16))) {
+            if constexpr (CELL::template prefetch<T, R>) {
                 // With 40 rows or more per thread there are registers to hold the
                 // next step's profile words: they are loaded at the start of a step
                 // from residues already in registers, so no step waits for its
@@ -675,8 +774,8 @@ __device__ __forceinline__ void run_stream(const RunArgs& a, const uint2* prof) 
                             bq1 = rrow[2 * (c + 2)];
                         }
                         if (zin) {
-                            h_in = Z;
-                            f_in = Z;
+                            h_in = HZ;
+                            f_in = FZ;
                         }
                         const int o0 = (int)(d_in & 0xffu) * SLOTS, o1 = (int)((d_in >> 8) & 0xffu) * SLOTS;
                         // the next step's words: its top takes column c + 1, its
@@ -707,34 +806,45 @@ __device__ __forceinline__ void run_stream(const RunArgs& a, const uint2* prof) 
                     }
                 }
             } else {
-                // two steps per iteration (+0.9 % over the sweep, measured)
+                // two steps per iteration (+0.9 % over the sweep, measured); a
+                // query of one pass runs them without the boundary row's
+                // branches and warp syncs (+1.7 % at 16x40, +4.5 % at 32x40)
+                auto plain_steps = [&](auto with_bnd) {
+                    constexpr bool BND = decltype(with_bnd)::value;
 #pragma unroll 2
-                for (; k > 0; --k) {
-                    if (P > 1) __syncwarp();
-                    uint32_t h_in = __shfl_up_sync(FULL, out_h, 1, T);
-                    uint32_t f_in = __shfl_up_sync(FULL, out_f, 1, T);
-                    const uint32_t d_in = d_cur;
-                    d_cur = (uint32_t)__ldg(col + c + 1);
-                    if (rd0) {
-                        h_in = bq0.x;
-                        f_in = bq0.y;
-                        bq0 = bq1;
-                        bq1 = rrow[2 * (c + 2)];
+                    for (; k > 0; --k) {
+                        if (BND) __syncwarp();
+                        uint32_t h_in = __shfl_up_sync(FULL, out_h, 1, T);
+                        uint32_t f_in = __shfl_up_sync(FULL, out_f, 1, T);
+                        const uint32_t d_in = d_cur;
+                        d_cur = (uint32_t)__ldg(col + c + 1);
+                        if (BND && rd0) {
+                            h_in = bq0.x;
+                            f_in = bq0.y;
+                            bq0 = bq1;
+                            bq1 = rrow[2 * (c + 2)];
+                        }
+                        if (zin) {
+                            h_in = HZ;
+                            f_in = FZ;
+                        }
+                        const int o0 = (int)(d_in & 0xffu) * SLOTS;
+                        const int o1 = (int)((d_in >> 8) & 0xffu) * SLOTS;
+                        column_step<R, JSTRIDE>(H, E, prof_t + o0, prof_t + o1, prof_t + po0,
+                                                prof_t + po1, prev_h, f_in, mid_h, mid_f, out_h,
+                                                out_f, S_top, S_bot, K);
+                        if (BND && wr) wrow[2 * (c - 1)] = make_uint2(out_h, out_f);
+                        po0 = o0;
+                        po1 = o1;
+                        prev_h = h_in;
+                        d_bot = d_in;
+                        ++c;
                     }
-                    if (zin) {
-                        h_in = Z;
-                        f_in = Z;
-                    }
-                    const int o0 = (int)(d_in & 0xffu) * SLOTS, o1 = (int)((d_in >> 8) & 0xffu) * SLOTS;
-                    column_step<R, JSTRIDE>(H, E, prof_t + o0, prof_t + o1, prof_t + po0, prof_t + po1,
-                                            prev_h, f_in, mid_h, mid_f, out_h, out_f, S_top, S_bot, K);
-                    if (wr) wrow[2 * (c - 1)] = make_uint2(out_h, out_f);
-                    po0 = o0;
-                    po1 = o1;
-                    prev_h = h_in;
-                    d_bot = d_in;
-                    b_col = c;
-                    ++c;
+                };
+                if (k > 0) {
+                    if (one_pass) plain_steps(Flag<false>{});
+                    else plain_steps(Flag<true>{});
+                    b_col = c - 1;
                 }
             }
         }
@@ -743,11 +853,12 @@ __device__ __forceinline__ void run_stream(const RunArgs& a, const uint2* prof) 
 }
 
 // Plain search: one query, the pairs of one range.
-template <int T, int R, int BLOCK>
+template <int T, int R, int BLOCK, class CELL>
 __global__ void __launch_bounds__(BLOCK, 1) sw_wavefront(const WfArgs a) {
     extern __shared__ uint2 prof[];
     const int P = (a.qlen + T * R - 1) / (T * R);
-    build_profile<T, R>(prof, a.query, a.qlen, a.mat, P);
+    const CELL K(a.gap_oe, a.gap_e);
+    build_profile<T, R>(prof, a.query, a.qlen, a.mat, P, K.profile_bias());
     __syncthreads();
     RunArgs r;
     r.db = a.db;
@@ -758,8 +869,6 @@ __global__ void __launch_bounds__(BLOCK, 1) sw_wavefront(const WfArgs a) {
     r.P = P;
     r.pass0 = a.pass0;
     r.more = a.more;
-    r.bias2 = a.bias2;
-    r.neg_e = a.neg_e;
     r.bnd = a.bnd;
     r.bnd_group = 0;
     r.scores = a.scores;
@@ -771,7 +880,7 @@ __global__ void __launch_bounds__(BLOCK, 1) sw_wavefront(const WfArgs a) {
     r.ovf_cap = a.n_records + 1;
     r.pair_ids = nullptr;
     r.rb_map = nullptr;
-    run_stream<T, R, false>(r, prof);
+    run_stream<T, R, false>(r, prof, K);
 }
 
 // Batched search: one persistent launch over a list of query stacks (each
@@ -788,7 +897,7 @@ __global__ void __launch_bounds__(BLOCK, 1) sw_batch(const BatchArgs a) {
         const int rows = (int)a.stack_rows[i];
         const int P = (rows + T * R - 1) / (T * R);
         __syncthreads();        // every group is done with the previous profile
-        build_profile<T, R>(prof, a.codes + a.stack_off[i], rows, a.mat, P);
+        build_profile<T, R>(prof, a.codes + a.stack_off[i], rows, a.mat, P, 0);
         __syncthreads();
         RunArgs r;
         r.db = a.db;
@@ -799,8 +908,6 @@ __global__ void __launch_bounds__(BLOCK, 1) sw_batch(const BatchArgs a) {
         r.P = P;
         r.pass0 = 0;
         r.more = 0;
-        r.bias2 = a.bias2;
-        r.neg_e = a.neg_e;
         r.bnd = a.bnd;
         r.bnd_group = a.bnd_group;
         r.scores = a.scores;
@@ -812,7 +919,7 @@ __global__ void __launch_bounds__(BLOCK, 1) sw_batch(const BatchArgs a) {
         r.ovf_cap = a.ovf_cap;
         r.pair_ids = a.pair_ids;
         r.rb_map = a.rb_map + a.rb_off[i];
-        run_stream<T, R, true>(r, prof);
+        run_stream<T, R, true>(r, prof, CellWide(a.gap_oe, a.gap_e));
     }
 }
 
