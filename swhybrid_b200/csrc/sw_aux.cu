@@ -107,6 +107,49 @@ __global__ void __launch_bounds__(64) sw_rescore32(const RescoreArgs a) {
     }
 }
 
+// Windows of long pairs, one block per pair (blockIdx.x < the number of pairs
+// to cut).  A pair's columns are one serial chain in the first pass, so a DB
+// whose longest pairs hold more columns than an evenly loaded group gets would
+// end on them.  No alignment of the query that scores above 0 spans more than
+// W columns (its gap costs stay below the sum of its best match scores), so
+// every one lies inside one of a set of windows that overlap by at least
+// W - 1 columns, and the record's score is the maximum over its windows.
+// Each window gets a table entry and a copy of its columns of its own (and
+// with it a boundary row of its own: rows are addressed by stream position),
+// so the first pass scores it like any pair.  Bound by latency: a few MB
+// copied and a prefix sum over the counts of the pairs before (n_w^2 / 2
+// 8-byte loads in all, n_w in the hundreds).
+__global__ void __launch_bounds__(kWindowThreads) sw_windows(const WindowArgs a) {
+    __shared__ int s_sum;
+    const int p = (int)blockIdx.x;
+    if (threadIdx.x == 0) s_sum = 0;
+    __syncthreads();
+    int before = 0;
+    for (int i = (int)threadIdx.x; i < p; i += kWindowThreads)
+        before += window_count((int)a.pairs[i].ncols, a.len, a.stride);
+    before = __reduce_add_sync(0xffffffffu, before);
+    if ((threadIdx.x & 31) == 0 && before) atomicAdd(&s_sum, before);
+    __syncthreads();
+    const int first = s_sum;
+    const Pair2 pr = a.pairs[p];
+    const int n = (int)pr.ncols;
+    const int count = window_count(n, a.len, a.stride), step = window_step(n, a.len, a.stride);
+    const int units = a.len / 8;
+    const uint4* const src = a.db + pr.off16;
+    uint4* const dst = a.db + a.base + (size_t)first * units;
+    for (int w = (int)threadIdx.x; w < count; w += kWindowThreads) {
+        a.win_pairs[first + w] = Pair2{a.base + (uint32_t)(first + w) * (uint32_t)units,
+                                       (uint32_t)max(min(a.len, n - w * step), 0)};
+        a.win_ids[first + w] = (uint32_t)p;
+    }
+    const int src_units = (n + 7) / 8;
+    for (int i = (int)threadIdx.x; i < count * units; i += kWindowThreads) {
+        const int w = i / units, u = i - w * units;
+        const int from = w * (step / 8) + u;
+        if (from < src_units) dst[i] = src[from];
+    }
+}
+
 // Top-k, one block: sort 4096 64-bit keys in shared memory (bitonic,
 // descending) and keep the first k.  Key = score << 32 | ~record_index, so the
 // order is score descending, then record index ascending.  In the first round

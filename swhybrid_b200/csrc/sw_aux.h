@@ -48,6 +48,29 @@ struct TopkArgs {
     const int* rows;                      // optional: round 0 reads score row rows[y]
 };
 
+// Windows of the pairs longer than `len` columns (sw_windows): pair p of
+// [0, n_pairs) is cut into window_count(ncols, len, stride) windows of `len`
+// columns, window_step(...) columns apart.
+struct WindowArgs {
+    uint4* db;                  // column streams; window v's copy at unit base + v * len / 8
+    const Pair2* pairs;
+    int len, stride;            // multiples of 8 (stride: at most this far apart)
+    uint32_t base;              // first unit of the copies
+    Pair2* win_pairs;
+    uint32_t* win_ids;
+};
+constexpr int kWindowThreads = 256;
+
+__host__ __device__ inline int window_count(int ncols, int len, int stride) {
+    return 1 + (ncols - len + stride - 1) / stride;
+}
+// evenly spread: the last window ends at the pair's end (ncols > len)
+__host__ __device__ inline int window_step(int ncols, int len, int stride) {
+    const int gaps = window_count(ncols, len, stride) - 1;
+    return ((ncols - len + gaps - 1) / gaps + 7) / 8 * 8;
+}
+
+__global__ void sw_windows(const WindowArgs a);
 __global__ void sw_rescore32(const RescoreArgs a);
 __global__ void sw_topk_round(const TopkArgs a);
 

@@ -32,7 +32,10 @@ struct WfArgs {
     const uint4* db;            // pair column streams
     const Pair2* pairs;         // pair table, ncols descending
     int pair_begin;             // first pair handled by this launch
-    int pair_count;             // pairs handled by this launch
+    int pair_count;             // windows and pairs handled by this launch
+    const Pair2* win_pairs;     // windows of long pairs, taken before the pairs ...
+    const uint32_t* win_ids;    // ... and the pair each belongs to
+    int n_win;
     const uint8_t* query;       // device query codes of this launch's rows, qlen entries (< 25)
     int qlen;
     int pass0;                  // query passes scored by earlier launches (row segments)

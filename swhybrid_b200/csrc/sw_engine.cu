@@ -71,6 +71,8 @@ using namespace swb;
 
 namespace {
 
+constexpr int kMinWindow = 256;     // shortest window of a long pair, in columns
+
 double now_ms() {
     return std::chrono::duration<double, std::milli>(
                std::chrono::steady_clock::now().time_since_epoch())
@@ -205,6 +207,7 @@ extern "C" sw_status sw_ctx_create(int device, const sw_params* params, sw_ctx**
             mat8[i * 32 + j] = (int8_t)v;
             lo = std::min(lo, v);
             hi = std::max(hi, v);
+            ctx->row_best[i] = std::max(ctx->row_best[i], v);
         }
     ctx->max_score = hi;
     ctx->cell = plain_cell(lo, hi, ctx->params.gap_open + ctx->params.gap_extend,
@@ -244,6 +247,8 @@ static void free_db(sw_ctx* ctx) {
     dev_free(ctx->d_rs_scratch);
     dev_free(ctx->d_db);
     dev_free(ctx->d_pairs);
+    dev_free(ctx->d_win_pairs);
+    dev_free(ctx->d_win_ids);
     dev_free(ctx->d_perm);
     dev_free(ctx->d_bnd);
     dev_free(ctx->d_scores);
@@ -394,10 +399,17 @@ sw_status swb::db_load(sw_ctx* ctx, const uint8_t* residues, const uint64_t* off
         ctx->err = std::string("device allocation failed: ") + what;
         return SW_ERR_NOMEM;
     };
-    if (dev_alloc(&ctx->d_db, units) != cudaSuccess) return nomem("db");
+    // room for windows of long pairs: an eighth of the DB's columns (half a
+    // million for a small DB, never more than the DB itself)
+    ctx->win_units = std::min<uint64_t>(units, std::max<uint64_t>(units / 8, 65536));
+    if (units + ctx->win_units >= (1ull << 32)) ctx->win_units = 0;
+    ctx->win_cap = (int)(ctx->win_units / (kMinWindow / 8) + 1);
+    if (dev_alloc(&ctx->d_db, units + ctx->win_units) != cudaSuccess) return nomem("db");
+    if (dev_alloc(&ctx->d_win_pairs, ctx->win_cap) != cudaSuccess) return nomem("windows");
+    if (dev_alloc(&ctx->d_win_ids, ctx->win_cap) != cudaSuccess) return nomem("windows");
     if (dev_alloc(&ctx->d_pairs, npairs_all) != cudaSuccess) return nomem("pairs");
     if (dev_alloc(&ctx->d_perm, n) != cudaSuccess) return nomem("perm");
-    if (dev_alloc(&ctx->d_bnd, units * 16) != cudaSuccess) return nomem("boundary rows");
+    if (dev_alloc(&ctx->d_bnd, (units + ctx->win_units) * 16) != cudaSuccess) return nomem("boundary rows");
     ctx->db_units = (uint64_t)units;
     if (dev_alloc(&ctx->d_scores, n + 1) != cudaSuccess) return nomem("scores");
     if (dev_alloc(&ctx->d_scores_rec, n + 1) != cudaSuccess) return nomem("scores");
@@ -415,7 +427,8 @@ sw_status swb::db_load(sw_ctx* ctx, const uint8_t* residues, const uint64_t* off
                                 cudaMemcpyHostToDevice));
     if (n) SW_CUDA(ctx, cudaMemcpy(ctx->d_perm, perm.data(), n * sizeof(uint32_t),
                                    cudaMemcpyHostToDevice));
-    ctx->db_bytes = units * 16 + npairs_all * sizeof(Pair2) + n * 4 + units * 16 * 8;
+    ctx->db_bytes = (units + ctx->win_units) * 16 + npairs_all * sizeof(Pair2) + n * 4 +
+                    (units + ctx->win_units) * 16 * 8;
     ctx->db_loaded = true;
     return SW_OK;
 }
@@ -685,7 +698,8 @@ int auto_cutover(sw_ctx* ctx, const sw_kernel_config& cfg, int qlen) {
     return std::max(1024, (int)(share / 4));
 }
 
-// The row segments a plain search runs on the pairs [bulk_begin, n_pairs):
+// The row segments a plain search runs on its bulk pairs (the longest unit of
+// them, a pair or a window, has `longest` columns; 0: there are none):
 // the table entry's plan when it applies, else the whole query with the bulk
 // shape ks (which also takes the rest of a plan without a rest step).  The
 // plan is dropped (one segment) when a step names an uncompiled shape, when
@@ -694,10 +708,10 @@ int auto_cutover(sw_ctx* ctx, const sw_kernel_config& cfg, int qlen) {
 // enough that one group's even share of the columns is below the longest
 // pair's (its launch would end on that pair's serial column steps: narrow
 // shapes only pay with the long-pair split).
-int build_plan(sw_ctx* ctx, int qlen, const WfKernel* ks, int64_t bulk_begin, RowSeg* out) {
+int build_plan(sw_ctx* ctx, int qlen, const WfKernel* ks, double longest, RowSeg* out) {
     out[0] = RowSeg{ks, qlen};
     const sw_tuning_entry* e = find_entry(ctx, qlen);
-    if (!e || e->plan[0].group_width == 0 || !ks || bulk_begin >= ctx->n_pairs) return 1;
+    if (!e || e->plan[0].group_width == 0 || !ks || longest <= 0) return 1;
     RowSeg segs[kMaxRowSegs];
     int n = 0, left = qlen;
     for (int i = 0; i < SW_PLAN_STEPS && left > 0; ++i) {
@@ -716,7 +730,6 @@ int build_plan(sw_ctx* ctx, int qlen, const WfKernel* ks, int64_t bulk_begin, Ro
         left -= (int)rows;
     }
     if (left > 0) segs[n++] = RowSeg{ks, left};
-    const double longest = (double)ctx->pair_ncols[bulk_begin];
     for (int i = 0; i < n; ++i)
         if (launch_rows(ctx, *segs[i].k, segs[i].rows) == 0 ||
             longest > plan_share(ctx, *segs[i].k, segs[i].rows))
@@ -775,6 +788,61 @@ const LongKernel* choose_long(sw_ctx* ctx, const sw_kernel_config& cfg, int qlen
     return nullptr;
 }
 
+// The columns an alignment that scores above 0 can span: its gap costs stay
+// below best_sum, the sum of its rows' best scores (each run of g residues
+// costs gap_open + g * gap_extend), and at most qlen columns are matched.
+// 0: no bound (free gap extension).
+int64_t span_bound(const sw_ctx* ctx, int64_t qlen, int64_t best_sum) {
+    if (ctx->params.gap_extend == 0) return 0;
+    return qlen + std::max<int64_t>(0, best_sum - 1 - ctx->params.gap_open) / ctx->params.gap_extend;
+}
+
+// Windows of the pairs longer than `len` columns (0 windows: none are cut).
+struct Windows {
+    int len = 0, stride = 0;
+    int64_t n_pairs = 0;     // pairs [0, n_pairs) are cut
+    int n = 0;               // windows
+};
+
+// Windows for a bulk launch whose evenly loaded group gets `share` columns,
+// with alignments spanning at most `span` columns.  A unit's columns are
+// serial, so the launch lasts about max(share, longest unit) plus the tail of
+// the last claims (a quarter of a unit); overlaps add columns to all groups.
+// The window length with the least such estimate is taken, if that comes
+// within 1.6 times the share (beyond that the long-pair kernel's pipelined
+// passes do better: measured on the stress DB, where 43 % of the columns are
+// in long pairs, 18 ms against 40 with windows).
+Windows plan_windows(const sw_ctx* ctx, double share, int64_t span) {
+    Windows best;
+    if (span <= 0 || ctx->n_pairs == 0 || (double)ctx->pair_ncols[0] <= 0.8 * share) return best;
+    const double total = (double)ctx->pair_cols_total;
+    double best_est = 1.6 * share;
+    for (const double f : {1.0, 0.8, 0.65, 0.5, 0.4, 0.3, 0.2, 0.12}) {
+        const int64_t len = (int64_t)(f * share) / 8 * 8;
+        const int64_t stride = (len - span + 1) / 8 * 8;
+        if (len < kMinWindow || stride < 64) break;
+        if (len >= (int64_t)ctx->pair_ncols[0]) continue;
+        const int64_t n_w = std::partition_point(ctx->pair_ncols.begin(), ctx->pair_ncols.end(),
+                                                 [len](uint32_t n) { return (int64_t)n > len; }) -
+                            ctx->pair_ncols.begin();
+        if (n_w > 8192) break;      // shorter windows only cut more pairs
+        int64_t n = 0;
+        for (int64_t p = 0; p < n_w; ++p)
+            n += window_count((int)ctx->pair_ncols[p], (int)len, (int)stride);
+        if (n > ctx->win_cap || (uint64_t)n * (len / 8) > ctx->win_units) continue;
+        const double extra = (double)n * len - (double)ctx->pair_prefix[n_w];
+        const double est = share * (1.0 + extra / total) + 0.25 * len;
+        if (est < best_est) {
+            best_est = est;
+            best.len = (int)len;
+            best.stride = (int)stride;
+            best.n_pairs = n_w;
+            best.n = (int)n;
+        }
+    }
+    return best;
+}
+
 // How a plain search of qlen divides the DB's pairs.  With a cut-over (the
 // configured one, else auto_cutover's), the long-pair kernel takes the pairs
 // above it, [0, n_long), when some but not all pairs are, and a pipelined
@@ -783,6 +851,7 @@ const LongKernel* choose_long(sw_ctx* ctx, const sw_kernel_config& cfg, int qlen
 // the cut-over or all are, the short one when no pipelined shape fits.
 struct SearchLayout {
     sw_kernel_config cfg;
+    Windows win;                       // long pairs cut into windows for the bulk launches
     int cutover = 0;
     bool split = false;
     int64_t n_long = 0;                // pairs of the long-pair kernel (split only)
@@ -790,12 +859,26 @@ struct SearchLayout {
     int lpasses = 0, lpipes = 0;
     size_t lsmem = 0;
     int bulk_T = 0, bulk_R = 0;        // the bulk launches' shape ...
-    int64_t bulk_b = 0, bulk_e = 0;    // ... pairs ...
+    int64_t bulk_b = 0, bulk_e = 0;    // ... pairs (after the windows) ...
+    double longest = 0;                // ... columns of the longest unit ...
     int bulk_counter = 0;              // ... and claim counter
 };
 
-void layout_search(sw_ctx* ctx, int qlen, SearchLayout* L) {
+void layout_search(sw_ctx* ctx, int qlen, int64_t span, SearchLayout* L) {
     const sw_kernel_config& cfg = L->cfg = choose_config(ctx, qlen);
+    // windows, unless the caller's configuration asks for a cut-over
+    const WfKernel* kb = find_kernel(cfg.short_group_width, cfg.short_rows_per_thread);
+    if (kb && !(ctx->has_override && cfg.cutover > 0))
+        L->win = plan_windows(ctx, group_share(ctx, *kb, std::min(qlen, launch_rows(ctx, *kb, qlen))),
+                              span);
+    if (L->win.n > 0) {
+        L->bulk_T = cfg.short_group_width;
+        L->bulk_R = cfg.short_rows_per_thread;
+        L->bulk_b = L->win.n_pairs;
+        L->bulk_e = ctx->n_pairs;
+        L->longest = L->win.len;
+        return;
+    }
     L->cutover = cfg.cutover > 0 ? cfg.cutover : auto_cutover(ctx, cfg, qlen);
     int64_t n_long = ctx->n_pairs;
     if (L->cutover > 0) {
@@ -822,17 +905,30 @@ void layout_search(sw_ctx* ctx, int qlen, SearchLayout* L) {
     }
     L->bulk_e = ctx->n_pairs;
     L->n_long = L->split ? n_long : 0;
+    L->longest = L->bulk_b < L->bulk_e ? (double)ctx->pair_ncols[L->bulk_b] : 0.0;
+}
+
+// span_bound for any query of a length.
+int64_t length_span(const sw_ctx* ctx, int64_t qlen) {
+    return span_bound(ctx, qlen, qlen * ctx->max_score);
+}
+
+// span_bound for a query whose residues the host holds.
+int64_t query_span(const sw_ctx* ctx, const uint8_t* query, int64_t qlen) {
+    int64_t sum = 0;
+    for (int64_t i = 0; i < qlen; ++i) sum += ctx->row_best[query[i] & 31];
+    return span_bound(ctx, qlen, sum);
 }
 
 // sw_get_plan: the row segments enqueue_search would run.
 sw_status describe_plan(sw_ctx* ctx, int qlen, sw_plan_step* steps, uint32_t capacity,
                         uint32_t* n_steps) {
     SearchLayout L;
-    layout_search(ctx, qlen, &L);
+    layout_search(ctx, qlen, length_span(ctx, qlen), &L);
     const WfKernel* k = find_kernel(L.bulk_T, L.bulk_R);
     if (!k) SW_SET(ctx, SW_ERR_INVALID, "no kernel %dx%d", L.bulk_T, L.bulk_R);
     RowSeg plan[kMaxRowSegs];
-    const int n = build_plan(ctx, qlen, k, L.bulk_b, plan);
+    const int n = build_plan(ctx, qlen, k, L.longest, plan);
     *n_steps = (uint32_t)n;
     for (int i = 0; i < n && (uint32_t)i < capacity; ++i) {
         const int rp = plan[i].k->T * plan[i].k->R;
@@ -841,11 +937,12 @@ sw_status describe_plan(sw_ctx* ctx, int qlen, sw_plan_step* steps, uint32_t cap
     return SW_OK;
 }
 
-sw_status enqueue_search(sw_ctx* ctx, const uint8_t* d_query, int qlen, int32_t* d_scores_rec,
-                         unsigned long long** keys_final, uint32_t* launches) {
+sw_status enqueue_search(sw_ctx* ctx, const uint8_t* d_query, int qlen, int64_t span,
+                         int32_t* d_scores_rec, unsigned long long** keys_final,
+                         uint32_t* launches) {
     cudaStream_t st = ctx->stream;
     SearchLayout L;
-    layout_search(ctx, qlen, &L);
+    layout_search(ctx, qlen, span, &L);
     ctx->stats.used = L.cfg;
     ctx->stats.used.cutover = L.cutover;
     *launches = 0;
@@ -869,14 +966,14 @@ sw_status enqueue_search(sw_ctx* ctx, const uint8_t* d_query, int qlen, int32_t*
     int nplan = 0;
     // every shape is checked before anything is launched: a search refused
     // half-way would leave a launch in flight that writes into the next one
-    if (L.bulk_e > L.bulk_b) {
+    if (L.bulk_e > L.bulk_b || L.win.n > 0) {
         const WfKernel* k = find_kernel(L.bulk_T, L.bulk_R);
         if (!k) SW_SET(ctx, SW_ERR_INVALID, "no kernel %dx%d", L.bulk_T, L.bulk_R);
         if (launch_rows(ctx, *k, qlen) == 0)
             SW_SET(ctx, SW_ERR_UNSUPPORTED,
                    "one pass of shape %dx%d does not fit shared memory (profile %zu bytes)",
                    L.bulk_T, L.bulk_R, k->smem(L.bulk_T * L.bulk_R));
-        nplan = build_plan(ctx, qlen, k, L.bulk_b, plan);
+        nplan = build_plan(ctx, qlen, k, L.longest, plan);
         if (nplan > 1) {
             ctx->stats.used.short_group_width = plan[0].k->T;
             ctx->stats.used.short_rows_per_thread = plan[0].k->R;
@@ -940,6 +1037,20 @@ sw_status enqueue_search(sw_ctx* ctx, const uint8_t* d_query, int qlen, int32_t*
         SW_CUDA(ctx, cudaEventRecord(mk.e[6], st));
     }
     mk.split = split;
+    if (L.win.n > 0) {
+        WindowArgs w;
+        w.db = ctx->d_db;
+        w.pairs = ctx->d_pairs;
+        w.len = L.win.len;
+        w.stride = L.win.stride;
+        w.base = (uint32_t)ctx->units;
+        w.win_pairs = ctx->d_win_pairs;
+        w.win_ids = ctx->d_win_ids;
+        void* args[] = {&w};
+        SW_CUDA(ctx, cudaLaunchKernel((const void*)sw_windows, dim3((unsigned)L.win.n_pairs),
+                                      dim3(kWindowThreads), args, 0, st));
+        ++*launches;
+    }
     // Row segments of the plan (one for most lengths), each in launches of
     // whole passes up to what one block's profile holds: every launch but the
     // first reads the boundary row the one before wrote (pass0 counts the
@@ -959,7 +1070,10 @@ sw_status enqueue_search(sw_ctx* ctx, const uint8_t* d_query, int qlen, int32_t*
             a.db = ctx->d_db;
             a.pairs = ctx->d_pairs;
             a.pair_begin = (int)L.bulk_b;
-            a.pair_count = (int)(L.bulk_e - L.bulk_b);
+            a.pair_count = (int)(L.bulk_e - L.bulk_b) + L.win.n;
+            a.win_pairs = ctx->d_win_pairs;
+            a.win_ids = ctx->d_win_ids;
+            a.n_win = L.win.n;
             a.query = d_query + r0;
             a.qlen = rows;
             a.pass0 = passes_before;
@@ -980,7 +1094,7 @@ sw_status enqueue_search(sw_ctx* ctx, const uint8_t* d_query, int qlen, int32_t*
             // a warp claims 32 / T pairs at a time: no more blocks than claims
             // (few pairs spread one warp per SM)
             const int64_t per_claim = 32 / k->T;
-            grid = std::min<int64_t>(grid, ((L.bulk_e - L.bulk_b) + per_claim - 1) / per_claim);
+            grid = std::min<int64_t>(grid, (a.pair_count + per_claim - 1) / per_claim);
             grid = std::max<int64_t>(grid, 1);
             SW_CUDA(ctx, cudaLaunchKernel(k->fn[ctx->cell], dim3((unsigned)grid), dim3(block), args,
                                           k->smem(rows), st));
@@ -1141,8 +1255,8 @@ sw_status search_host(sw_ctx* ctx, const uint8_t* query, uint32_t qlen, sw_hit* 
                                  ctx->stream));
     unsigned long long* keys = nullptr;
     uint32_t launches = 0;
-    st = enqueue_search(ctx, ctx->d_query, (int)qlen, scores ? ctx->d_scores_rec : nullptr, &keys,
-                        &launches);
+    st = enqueue_search(ctx, ctx->d_query, (int)qlen, query_span(ctx, query, qlen),
+                        scores ? ctx->d_scores_rec : nullptr, &keys, &launches);
     if (st != SW_OK) return st;
     SW_CUDA(ctx, cudaMemcpyAsync(ctx->h_keys, keys, (size_t)k * sizeof(unsigned long long),
                                  cudaMemcpyDeviceToHost, ctx->stream));
@@ -1190,7 +1304,8 @@ extern "C" sw_status sw_search_device(sw_ctx* ctx, const uint8_t* d_query, uint3
     ctx->stats = sw_run_stats{};
     unsigned long long* keys = nullptr;
     uint32_t launches = 0;
-    sw_status st = enqueue_search(ctx, d_query, (int)qlen, d_scores, &keys, &launches);
+    sw_status st = enqueue_search(ctx, d_query, (int)qlen, length_span(ctx, qlen), d_scores, &keys,
+                                  &launches);
     if (st != SW_OK) return st;
     ctx->stats.cells = (uint64_t)qlen * ctx->n_residues;
     ctx->stats.launches = launches;

@@ -72,6 +72,7 @@ struct sw_ctx {
     sw_totals totals{};
     sw_params params{};
     int max_score = 0;
+    int row_best[32] = {};             // per query code: its best score (at least 0)
     int cell = 0;                      // PlainCell of the plain kernel's launches
     int8_t* d_mat = nullptr;           // 32x32 int8, codes >= 24 zeroed
     int* d_counters = nullptr;         // [0],[1] pair counters, [2] overflow count
@@ -84,6 +85,8 @@ struct sw_ctx {
     uint64_t max_len = 0;
     uint64_t units = 0;                // 16-byte units of the column stream
     uint64_t db_bytes = 0;
+    uint64_t win_units = 0;            // further units of d_db and d_bnd, for windows of long pairs
+    int win_cap = 0;                   // entries of d_win_pairs and d_win_ids
     std::vector<uint32_t> pair_ncols;  // host copy, for shape selection
     uint64_t pair_cols_total = 0;      // sum of pair_ncols
     std::vector<uint64_t> pair_prefix; // pair_prefix[p] = sum of pair_ncols[0, p)
@@ -91,6 +94,8 @@ struct sw_ctx {
     std::vector<uint32_t> rec_len;     // record -> length (host)
     uint4* d_db = nullptr;
     swb::Pair2* d_pairs = nullptr;
+    swb::Pair2* d_win_pairs = nullptr; // windows of the search in flight
+    uint32_t* d_win_ids = nullptr;     // ... and the pair each belongs to
     uint32_t* d_perm = nullptr;        // sorted position -> record
     uint2* d_bnd = nullptr;            // boundary rows between query passes
     uint64_t db_units = 0;             // 16-byte units of the column streams (d_bnd: 16 each)

@@ -344,8 +344,13 @@ struct Flag {
 struct RunArgs {
     const uint4* db;            // pair column streams
     const Pair2* pairs;         // pair table, ncols descending
-    int pair_begin;             // pairs [pair_begin, pair_begin + pair_count)
-    int pair_count;
+    int pair_begin;             // the range: n_win windows, then the pairs
+    int pair_count;             // [pair_begin, pair_begin + pair_count - n_win)
+    // windows of long pairs (plain search, see sw_windows): table entries of
+    // their own and the pair each belongs to; scores merge by maximum
+    const Pair2* win_pairs;
+    const uint32_t* win_ids;
+    int n_win;
     int* counter;               // pairs of the range claimed so far
     int P;                      // query passes of T*R rows
     // A query too long for one launch's profile is scored in row segments by
@@ -382,29 +387,23 @@ struct RunArgs {
 // overwrites this value with the exact score.
 constexpr int kListed = 0x7fffffff;
 
-// Plain search: a record's first-pass score (lane value s) at its
-// sorted position.  A lane that may have wrapped lists the record for the
-// 32-bit pass.  With the query in row segments (pass0 / more) the score is
-// the maximum over the segments, and a listed record keeps kListed so that a
-// later segment does not list it again.
+// Plain search: a record's first-pass score (lane value s) at its sorted
+// position.  A lane that may have wrapped lists the record for the 32-bit pass.
+// With the query in row segments (pass0 / more) or the record in windows the
+// score is the maximum over them, and a listed record keeps kListed so that
+// it is listed once.
 __device__ __forceinline__ void put_score(const RunArgs& a, int pos, int s, int bias,
-                                          int ovf_thresh) {
-    if (a.pass0 == 0 && !a.more) {
+                                          int ovf_thresh, bool merge) {
+    bool list = s >= ovf_thresh;
+    if (!merge)
         a.scores[pos] = s - bias;
-        if (s >= ovf_thresh) {
-            const int j = atomicAdd(a.ovf_count, 1);
-            if (j < a.ovf_cap) a.ovf_list[j] = a.ovf_base + pos;
-        }
-        return;
-    }
-    const int prev = a.scores[pos];
-    if (prev == kListed) return;
-    if (s >= ovf_thresh) {
-        a.scores[pos] = kListed;
+    else if (list)
+        list = atomicMax(a.scores + pos, kListed) != kListed;
+    else
+        atomicMax(a.scores + pos, s - bias);
+    if (list) {
         const int j = atomicAdd(a.ovf_count, 1);
         if (j < a.ovf_cap) a.ovf_list[j] = a.ovf_base + pos;
-    } else {
-        a.scores[pos] = max(prev, s - bias);
     }
 }
 
@@ -516,6 +515,10 @@ __device__ __forceinline__ void run_stream(const RunArgs& a, const uint2* prof, 
     const uint2* rrow = a.bnd;
     int claimed;               // pairs the warps' first claims take
 
+    auto entry = [&](int i) {
+        return !STACKED && i < a.n_win ? a.win_pairs[i]
+                                       : a.pairs[a.pair_begin + i - (STACKED ? 0 : a.n_win)];
+    };
     // the boundary rows are double-buffered by the parity of the pass's index
     // in the whole query; a launch's last pass writes one only when a later
     // launch reads it (that launch starts after this one has finished, so the
@@ -546,7 +549,7 @@ __device__ __forceinline__ void run_stream(const RunArgs& a, const uint2* prof, 
         claimed = warps * (int)gridDim.x * G;
         pair = v + grp;
         if (v < pair_count) {
-            const Pair2 pr = a.pairs[a.pair_begin + min(pair, pair_count - 1)];
+            const Pair2 pr = entry(min(pair, pair_count - 1));
             off16 = pr.off16;
             ncols = (int)pr.ncols;
             if (lane == 0) next = claimed + atomicAdd(a.counter, G);
@@ -590,7 +593,7 @@ __device__ __forceinline__ void run_stream(const RunArgs& a, const uint2* prof, 
             }
             // the next pair's table entry, once its claim has returned
             if (c == nload && warp_next < pair_count)
-                ninfo = a.pairs[a.pair_begin + min(warp_next + grp, pair_count - 1)];
+                ninfo = entry(min(warp_next + grp, pair_count - 1));
         }
         if (STACKED && my_first) {   // a query starts here: nothing flows in from above
             h_in = HZ;
@@ -647,9 +650,13 @@ __device__ __forceinline__ void run_stream(const RunArgs& a, const uint2* prof, 
                     if (t > 0) m = __vimax3_s16x2(m, acc_in, HZ);
                     acc_out = m;
                     if (t == T - 1 && fpair < pair_count) {
-                        const int pos = 2 * (a.pair_begin + fpair);
-                        put_score(a, pos, lo16(m), bias, ovf_thresh);
-                        if (pos + 1 < a.n_records) put_score(a, pos + 1, hi16(m), bias, ovf_thresh);
+                        const bool win = fpair < a.n_win;
+                        const int pos = 2 * (win ? (int)a.win_ids[fpair]
+                                                 : a.pair_begin + fpair - a.n_win);
+                        const bool merge = win || a.pass0 > 0 || a.more;
+                        put_score(a, pos, lo16(m), bias, ovf_thresh, merge);
+                        if (pos + 1 < a.n_records)
+                            put_score(a, pos + 1, hi16(m), bias, ovf_thresh, merge);
                     }
                 }
                 S_bot = HZ;
@@ -865,6 +872,9 @@ __global__ void __launch_bounds__(BLOCK, 1) sw_wavefront(const WfArgs a) {
     r.pairs = a.pairs;
     r.pair_begin = a.pair_begin;
     r.pair_count = a.pair_count;
+    r.win_pairs = a.win_pairs;
+    r.win_ids = a.win_ids;
+    r.n_win = a.n_win;
     r.counter = a.counter;
     r.P = P;
     r.pass0 = a.pass0;
@@ -904,6 +914,9 @@ __global__ void __launch_bounds__(BLOCK, 1) sw_batch(const BatchArgs a) {
         r.pairs = a.pairs;
         r.pair_begin = a.pair_begin;
         r.pair_count = a.pair_count;
+        r.win_pairs = nullptr;
+        r.win_ids = nullptr;
+        r.n_win = 0;
         r.counter = a.counters + i;
         r.P = P;
         r.pass0 = 0;
