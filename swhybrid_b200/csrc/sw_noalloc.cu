@@ -11,15 +11,32 @@
 // about 16 MiB) is held by every GPU that loads the library until the
 // process exits.
 //
-// The kernel is a variant of the exact 32-bit re-score pass (sw_rescore32,
-// sw_aux.cu): one warp per record, anti-diagonal wavefront over 32 lanes x 16
-// query rows per pass, int32 arithmetic; the boundary row between query
-// passes lives in the warp's slice of the static array instead of the DB's
-// boundary buffer.  Records are claimed through a counter that also lives in
-// the static array.
+// One warp scores one record as an anti-diagonal wavefront in int32: lane t
+// holds R query rows, one column behind lane t-1.  R is the smallest compiled
+// row count whose 32 R rows hold the query (4..64), so queries up to 2,048
+// residues run in one pass with no boundary row, and as many warps as fit; a
+// longer query runs in passes of 2,048 rows that hand their last row on
+// through the warp's slice of the static array (as many warps as there are
+// slices of the longest record's length).
+//
+// Bound: the ALU pipe (64 lanes per clock and SM): 4.5 instructions per cell
+// (the maxima of H before F, of H, E and F, and half a vimax3 for the running
+// one), 5.5 with the byte profile's extraction.  The profile is read from shared memory,
+// one conflict-free 16- or 4-byte word per 4 rows; looking each cell up in the
+// matrix cost a bank-conflicted load per cell.  10,000 records, query 375:
+// 4,400 us a call before (256 warps, 512-row passes, matrix lookups), 586 now.
+//
+// A record is a serial chain of columns, so records longer than an even share
+// of the columns are cut into windows that overlap by the longest span an
+// alignment can have (see sw_windows in sw_aux.cu); their scores merge by
+// atomicMax.  Work is claimed through counters in the static array: first the
+// long records' windows, then the other records.
+#include <algorithm>
 #include <climits>
+#include <cstddef>
 #include <cstdint>
 #include <cstring>
+#include <iterator>
 #include <mutex>
 
 #include <cuda_runtime.h>
@@ -28,15 +45,25 @@
 
 namespace {
 
-constexpr int kNaWarps = 256;          // warps of one launch (64 blocks x 4 warps)
+constexpr int kNaSlices = 256;         // boundary rows of kNaMaxLen in the scratch
 constexpr int kNaMaxLen = 8192;        // longest DB record accepted, in residues
-constexpr int kNaRows = 16;            // query rows per lane and pass
 constexpr int kNaHeader = 32;          // uint2 words before the boundary rows (256 B)
-constexpr size_t kScratchWords = (size_t)kNaHeader + (size_t)kNaWarps * kNaMaxLen;
+constexpr size_t kRowWords = (size_t)kNaSlices * kNaMaxLen;
+constexpr size_t kScratchWords = (size_t)kNaHeader + kRowWords;
+constexpr int kNaThreads = 256;
+constexpr int kNaLookupThreads = 64;
+constexpr int kNaCodes = 25;           // 0..23 and the zero-score code 24
 
-// Word 0: .x = record counter, .y = error flag (a record longer than
-// kNaMaxLen was skipped).  Words kNaHeader.. : one boundary row of kNaMaxLen
-// (H, F) entries per warp.  Host code must not use this name as an address.
+// The header's fields, then one boundary row of (H, F) entries per warp.  Host
+// code must not use this name as an address.
+struct NaHeader {
+    unsigned int record;       // records claimed by the sweep over the short ones
+    unsigned int max_len;      // longest record (up to kNaMaxLen)
+    unsigned long long item;   // items claimed by the sweep over the long ones
+    unsigned long long error;  // a record longer than kNaMaxLen was skipped
+    unsigned long long best;   // sum of the query rows' best scores
+};
+static_assert(sizeof(NaHeader) <= kNaHeader * sizeof(uint2), "header");
 static __device__ __align__(256) uint2 g_noalloc_scratch[kScratchWords];
 
 struct NaArgs {
@@ -49,44 +76,272 @@ struct NaArgs {
     int gap_e;
     int cap;
     uint2* scratch;          // device address of g_noalloc_scratch
-    int32_t* scores;
+    int32_t* scores;         // zero before
+    int8_t row_best[32];     // per query code: its best score (at least 0)
     int8_t mat[1024];
 };
 
-__global__ void __launch_bounds__(128) sw_score_noalloc_kernel(const NaArgs a) {
+// Length of record i; kNaMaxLen + 1 for anything longer.
+__device__ __forceinline__ int na_len(const NaArgs& a, int i) {
+    const uint64_t b = a.offsets[i], e = a.offsets[i + 1];
+    return (e <= b) ? 0 : (e - b > (uint64_t)kNaMaxLen) ? kNaMaxLen + 1 : (int)(e - b);
+}
+
+// The header's max_len and best: what the windows are planned from.
+__global__ void __launch_bounds__(kNaThreads) sw_noalloc_prepare(const NaArgs a) {
+    NaHeader* h = reinterpret_cast<NaHeader*>(a.scratch);
+    const int first = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    const int step = (int)(gridDim.x * blockDim.x);
+    int longest = 0;
+    for (int64_t i = first; i < a.n; i += step) {
+        const int len = na_len(a, (int)i);
+        if (len <= kNaMaxLen) longest = max(longest, len);
+    }
+    long long best = 0;
+    for (int i = first; i < a.qlen; i += step) best += a.row_best[a.query[i] & 31];
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    if ((threadIdx.x & 31) == 0 && longest > 0) atomicMax(&h->max_len, (unsigned)longest);
+    if (best > 0) atomicAdd(&h->best, (unsigned long long)best);
+}
+
+// Profile words of 4 rows: int32 scores, or signed bytes.
+template <bool BYTES>
+struct NaWord {
+    using type = int4;
+    static __device__ __forceinline__ int get(const int4& w, int i) {
+        return i == 0 ? w.x : i == 1 ? w.y : i == 2 ? w.z : w.w;
+    }
+    static __device__ __forceinline__ int4 make(const int* v) {
+        return make_int4(v[0], v[1], v[2], v[3]);
+    }
+};
+template <>
+struct NaWord<true> {
+    using type = uint32_t;
+    static __device__ __forceinline__ int get(uint32_t w, int i) {
+        return (int)(int8_t)(w >> (8 * i));
+    }
+    static __device__ __forceinline__ uint32_t make(const int* v) {
+        return (v[0] & 0xff) | (v[1] & 0xff) << 8 | (v[2] & 0xff) << 16 | (uint32_t)v[3] << 24;
+    }
+};
+
+template <int R, bool BYTES>
+size_t na_smem(int qlen) {
+    const int passes = (qlen + 32 * R - 1) / (32 * R);
+    return (size_t)passes * (R / 4) * kNaCodes * 32 * sizeof(typename NaWord<BYTES>::type);
+}
+
+// One record (or window) against the whole query: the warp's best score.
+// PASSES: the query takes more than one pass (a step of a single pass has no
+// branch: it is mostly latency).
+template <int R, bool BYTES, bool PASSES, class WORD>
+__device__ __forceinline__ int na_score(const NaArgs& a, const WORD* prof, int P, uint2* pb,
+                                        const uint8_t* seq, int len) {
+    constexpr unsigned FULL = 0xffffffffu;
+    constexpr int NJ = R / 4, JSTRIDE = kNaCodes * 32;
+    const int lane = (int)(threadIdx.x & 31);
+    int S = 0;
+    for (int pass = 0; pass < (PASSES ? P : 1); ++pass) {
+        const WORD* const pp = prof + pass * NJ * JSTRIDE + lane;
+        const bool rd = PASSES && pass > 0 && lane == 0;
+        const bool wr = PASSES && pass + 1 < P && lane == 31;
+        int H[R], E[R];
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+            H[k] = 0;
+            E[k] = 0;
+        }
+        int out_h = 0, out_f = 0, prev_h = 0;
+        int c = -lane;
+        auto residue = [&](int i) {
+            return (i >= 0 && i < len) ? (unsigned)__ldg(seq + i) : 24u;
+        };
+        // codes 25..31 (none is documented) score 0 like 24
+        auto words_of = [&](unsigned code) { return pp + min(code & 31u, 24u) * 32; };
+        // the profile words of this step's column and the next column's
+        // residue are loaded a step ahead
+        WORD w[NJ];
+        {
+            const WORD* const pd = words_of(residue(c));
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) w[j] = pd[j * JSTRIDE];
+        }
+        unsigned d = residue(c + 1);
+        uint2 row = make_uint2(0u, 0u);
+        if (rd && len > 0) row = pb[0];
+        // a column outside the record runs on zero-score residues: before it
+        // all cells stay at 0, after it no score can rise
+        for (int s = 0; s < len + 31; ++s, ++c) {
+            if (PASSES) __syncwarp();    // orders the boundary row's stores and loads
+            int h_in = __shfl_up_sync(FULL, out_h, 1);
+            int f_in = __shfl_up_sync(FULL, out_f, 1);
+            h_in = lane == 0 ? (PASSES ? (int)row.x : 0) : h_in;
+            f_in = lane == 0 ? (PASSES ? (int)row.y : 0) : f_in;
+            if (PASSES && rd) row = (c + 1 < len) ? pb[c + 1] : make_uint2(0u, 0u);
+            WORD wn[NJ];
+            const WORD* const pd = words_of(d);
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) wn[j] = pd[j * JSTRIDE];
+            d = residue(c + 2);
+#pragma unroll
+            for (int k = R - 1; k >= 0; --k)
+                H[k] = __vimax3_s32((k > 0 ? H[k > 0 ? k - 1 : 0] : prev_h) +
+                                        NaWord<BYTES>::get(w[k / 4], k % 4),
+                                    E[k], 0);
+            // F of the next row from max(H before F, 0): a later row's F never
+            // gains from an H that F itself made (extending is no dearer than
+            // opening), which leaves one add and one maximum per row in the
+            // serial chain
+            int f = f_in;
+#pragma unroll
+            for (int k = 0; k < R; ++k) {
+                const int t = H[k];
+                const int h = max(t, f);
+                H[k] = h;
+                f = max(f - a.gap_e, t - a.gap_oe);
+                E[k] = max(E[k] - a.gap_e, h - a.gap_oe);
+                if (k & 1) S = __vimax3_s32(S, H[k > 0 ? k - 1 : 0], h);
+            }
+            out_h = H[R - 1];
+            out_f = f;
+            if (PASSES && wr && c >= 0 && c < len) pb[c] = make_uint2((uint32_t)out_h, (uint32_t)out_f);
+            prev_h = h_in;
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) w[j] = wn[j];
+        }
+        if (PASSES) __syncwarp();
+    }
+    return __reduce_max_sync(FULL, S);
+}
+
+template <int R, bool BYTES, int THREADS, int MIN_BLOCKS>
+__global__ void __launch_bounds__(THREADS, MIN_BLOCKS) sw_score_noalloc_kernel(const NaArgs a) {
+    using WORD = typename NaWord<BYTES>::type;
+    extern __shared__ int4 na_prof[];
+    WORD* const prof = reinterpret_cast<WORD*>(na_prof);
+    constexpr unsigned FULL = 0xffffffffu;
+    constexpr int NJ = R / 4;
+    NaHeader* const h = reinterpret_cast<NaHeader*>(a.scratch);
+    const int P = (a.qlen + 32 * R - 1) / (32 * R);
+    for (int idx = (int)threadIdx.x; idx < P * NJ * kNaCodes * 32; idx += THREADS) {
+        const int t = idx & 31;
+        int rest = idx >> 5;
+        const int d = rest % kNaCodes;
+        rest /= kNaCodes;
+        const int row0 = (rest / NJ * 32 + t) * R + rest % NJ * 4;
+        int v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            v[i] = row0 + i < a.qlen ? a.mat[(a.query[row0 + i] & 31) * 32 + d] : 0;
+        prof[idx] = NaWord<BYTES>::make(v);
+    }
+    __syncthreads();
+    const int lane = (int)(threadIdx.x & 31);
+    const int warp = (int)((blockIdx.x * THREADS + threadIdx.x) >> 5);
+    const long long warps = (long long)gridDim.x * (THREADS / 32);
+    // windows: long enough that the overlap costs at most two thirds, and at
+    // least a warp's even share of the columns
+    const long long max_len = h->max_len;
+    const long long share = (long long)((a.offsets[a.n] - a.offsets[0]) / (uint64_t)warps);
+    long long span = 0, wlen = kNaMaxLen;
+    if (a.gap_e > 0) {
+        const long long over = (long long)h->best - 1 - (a.gap_oe - a.gap_e);
+        span = a.qlen + (over > 0 ? over / a.gap_e : 0);
+        const long long w = max(share, span + max(span / 2, 256ll));
+        if (w + w / 4 < max_len) wlen = w;
+    }
+    const int L = (int)wlen, stride = (int)(L - span + 1);
+    uint2* pb = a.scratch + kNaHeader;
+    if (P > 1) {
+        const long long row = max(min(max_len, wlen), 1ll);
+        if (warp >= (long long)kRowWords / row) return;     // no boundary row left
+        pb += warp * row;
+    }
+    auto score = [&](int rec, int start, int len, bool merge) {
+        const uint8_t* seq = a.residues + a.offsets[rec] + start;
+        int s = P > 1 ? na_score<R, BYTES, true>(a, prof, P, pb, seq, len)
+                      : na_score<R, BYTES, false>(a, prof, P, pb, seq, len);
+        if (lane == 0) {
+            if (a.cap) s = min(s, 65535);
+            if (merge) atomicMax(a.scores + rec, s);
+            else a.scores[rec] = s;
+        }
+    };
+    // The long records first, so that a unit claimed last is short.  An item
+    // is window k of 4 neighbouring records, those of them that have one.
+    const int big = (int)min(max(share / 8, 128ll), (long long)L);
+    if (big < max_len) {
+        const long long groups = ((long long)a.n + 3) / 4;
+        // (stride is only meaningful where a record is longer than a window)
+        const long long items =
+            groups * (max_len <= L ? 1 : 1 + (max_len - L + stride - 1) / stride);
+        while (true) {
+            unsigned long long it = 0;
+            if (lane == 0) it = atomicAdd(&h->item, 1ull);
+            it = __shfl_sync(FULL, it, 0);
+            if ((long long)it >= items) break;
+            const int k = (int)((long long)it / groups);
+            const long long rec = ((long long)it - k * groups) * 4 + (lane & 3);
+            const int len = rec < a.n ? na_len(a, (int)rec) : 0;
+            const bool has = len > big && len <= kNaMaxLen &&
+                             (k == 0 || (len > L && k <= (len - L + stride - 1) / stride));
+            unsigned todo = __ballot_sync(FULL, has && lane < 4);
+            while (todo) {
+                const int src = __ffs(todo) - 1;
+                todo &= todo - 1;
+                const int n = __shfl_sync(FULL, len, src);
+                score((int)(rec - (lane & 3)) + src, k > 0 ? k * stride : 0,
+                      k > 0 ? min(L, n - k * stride) : min(L, n), n > L);
+            }
+        }
+    }
+    unsigned next = 0;
+    if (lane == 0) next = atomicAdd(&h->record, 1u);
+    while (true) {
+        const unsigned rec = __shfl_sync(FULL, next, 0);
+        if (rec >= (unsigned)a.n) break;
+        if (lane == 0) next = atomicAdd(&h->record, 1u);
+        const int len = na_len(a, (int)rec);
+        if (len > kNaMaxLen) {
+            if (lane == 0) atomicExch(&h->error, 1ull);
+        } else if (len <= big) {
+            score((int)rec, 0, len, false);
+        }
+    }
+}
+
+// Queries whose byte profile does not fit a block's shared memory (over ~9,000
+// residues): passes of 512 rows, scores looked up in a shared copy of the
+// matrix, one boundary row of kNaMaxLen per warp.
+__global__ void __launch_bounds__(kNaLookupThreads) sw_score_noalloc_lookup(const NaArgs a) {
+    constexpr int kRows = 16;
+    constexpr unsigned FULL = 0xffffffffu;
     __shared__ int smat[1024];
     for (int i = threadIdx.x; i < 1024; i += blockDim.x) smat[i] = a.mat[i];
     __syncthreads();
-    constexpr unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    unsigned int* counter = reinterpret_cast<unsigned int*>(&a.scratch[0].x);
-    unsigned int* error = reinterpret_cast<unsigned int*>(&a.scratch[0].y);
-    uint2* pb = a.scratch + kNaHeader + (size_t)warp * kNaMaxLen;
-    const int rows_per_pass = 32 * kNaRows;
-    const int P = (a.qlen + rows_per_pass - 1) / rows_per_pass;
+    NaHeader* const h = reinterpret_cast<NaHeader*>(a.scratch);
+    const int lane = (int)(threadIdx.x & 31);
+    const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    uint2* const pb = a.scratch + kNaHeader + (size_t)warp * kNaMaxLen;
+    const int P = (a.qlen + 32 * kRows - 1) / (32 * kRows);
     while (true) {
-        int rec = 0;
-        if (lane == 0) rec = (int)atomicAdd(counter, 1u);
+        unsigned rec = 0;
+        if (lane == 0) rec = atomicAdd(&h->record, 1u);
         rec = __shfl_sync(FULL, rec, 0);
-        if (rec >= a.n) break;
-        const uint64_t b = a.offsets[rec];
-        const uint64_t e = a.offsets[rec + 1];
-        const int len = (e <= b) ? 0 : (e - b > (uint64_t)kNaMaxLen) ? kNaMaxLen + 1 : (int)(e - b);
+        if (rec >= (unsigned)a.n) break;
+        const int len = na_len(a, (int)rec);
         if (len > kNaMaxLen) {
-            if (lane == 0) {
-                atomicExch(error, 1u);
-                a.scores[rec] = 0;
-            }
+            if (lane == 0) atomicExch(&h->error, 1ull);
             continue;
         }
-        const uint8_t* seq = a.residues + b;
+        const uint8_t* seq = a.residues + a.offsets[rec];
         int S = 0;
         for (int pass = 0; pass < P; ++pass) {
-            int qc[kNaRows], H[kNaRows], E[kNaRows];
+            int qc[kRows], H[kRows], E[kRows];
 #pragma unroll
-            for (int k = 0; k < kNaRows; ++k) {
-                const int row = pass * rows_per_pass + lane * kNaRows + k;
+            for (int k = 0; k < kRows; ++k) {
+                const int row = (pass * 32 + lane) * kRows + k;
                 qc[k] = (row < a.qlen) ? (int)(a.query[row] & 31) * 32 : 24 * 32;
                 H[k] = 0;
                 E[k] = 0;
@@ -114,31 +369,56 @@ __global__ void __launch_bounds__(128) sw_score_noalloc_kernel(const NaArgs a) {
                 if (c >= 0 && c < len) {
                     int diag = prev_h, f = f_in;
 #pragma unroll
-                    for (int k = 0; k < kNaRows; ++k) {
-                        int h = max(diag + smat[qc[k] + d_in], E[k]);
-                        h = max(max(h, f), 0);
+                    for (int k = 0; k < kRows; ++k) {
+                        int hk = max(diag + smat[qc[k] + d_in], E[k]);
+                        hk = max(max(hk, f), 0);
                         diag = H[k];
-                        H[k] = h;
-                        S = max(S, h);
-                        const int hq = h - a.gap_oe;
+                        H[k] = hk;
+                        S = max(S, hk);
+                        const int hq = hk - a.gap_oe;
                         E[k] = max(E[k] - a.gap_e, hq);
                         f = max(f - a.gap_e, hq);
                     }
-                    out_h = H[kNaRows - 1];
+                    out_h = H[kRows - 1];
                     out_f = f;
-                    if (lane == 31 && pass + 1 < P) pb[c] = make_uint2((uint32_t)out_h, (uint32_t)out_f);
+                    if (lane == 31 && pass + 1 < P)
+                        pb[c] = make_uint2((uint32_t)out_h, (uint32_t)out_f);
                 }
                 prev_h = h_in;
                 myd = d_in;
                 __syncwarp();
             }
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) S = max(S, __shfl_xor_sync(FULL, S, o));
+        S = __reduce_max_sync(FULL, S);
         if (lane == 0) a.scores[rec] = (a.cap && S > 65535) ? 65535 : S;
         __syncwarp();
     }
 }
+
+// The compiled row counts: one pass of 32 R rows up to 2,048 query residues.
+struct NaKernel {
+    int rows;
+    int threads;             // per block
+    int blocks;              // per SM
+    const void* fn;
+    size_t (*smem)(int qlen);
+};
+template <int R, bool BYTES, int THREADS, int MIN_BLOCKS>
+constexpr NaKernel na_inst() {
+    return NaKernel{32 * R, THREADS, MIN_BLOCKS,
+                    (const void*)&sw_score_noalloc_kernel<R, BYTES, THREADS, MIN_BLOCKS>,
+                    &na_smem<R, BYTES>};
+}
+// int32 profile words up to 512 rows (51 KB), bytes above.  One block per SM
+// with as few warps as nearly fill its ALU pipe: a column step takes longer
+// with every further warp on its scheduler, and the longest unit's columns are
+// serial (12 rows, 10,000 records: 586 us with 8 warps, 648 with 12).
+const NaKernel kNaKernels[] = {
+    na_inst<4, false, 512, 1>(),  na_inst<8, false, 512, 1>(),
+    na_inst<12, false, 256, 1>(), na_inst<16, false, 256, 1>(),
+    na_inst<24, true, 256, 1>(),  na_inst<32, true, 256, 1>(),
+    na_inst<48, true, 256, 1>(),  na_inst<64, true, 256, 1>(),
+};
 
 // Device address of the static scratch, looked up once per device.
 std::mutex g_na_mutex;
@@ -198,18 +478,51 @@ extern "C" sw_status sw_score_noalloc(int device, const sw_params* params, const
         a.scores = d_scores;
         for (int i = 0; i < 1024; ++i)
             a.mat[i] = (int8_t)(((i >> 5) >= 24 || (i & 31) >= 24) ? 0 : params->matrix[i]);
-        // the counter and the error flag must start at zero on every call
-        if (cudaMemsetAsync(addr, 0, sizeof(uint2), st) != cudaSuccess) {
+        for (int i = 0; i < 32; ++i) {
+            a.row_best[i] = 0;
+            for (int j = 0; j < 32; ++j) a.row_best[i] = std::max(a.row_best[i], a.mat[i * 32 + j]);
+        }
+        int sms = 0, max_smem = 0;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+        cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+        const NaKernel* k = nullptr;
+        for (const NaKernel& x : kNaKernels)
+            if (!k && (x.rows >= (int)qlen || &x == std::end(kNaKernels) - 1)) k = &x;
+        const bool looked_up = k->smem((int)qlen) > (size_t)max_smem;
+        const void* fn = looked_up ? (const void*)&sw_score_noalloc_lookup : k->fn;
+        const size_t smem = looked_up ? 0 : k->smem((int)qlen);
+        const int threads = looked_up ? kNaLookupThreads : k->threads;
+        int occ = 0;
+        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+                cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, threads, smem) !=
+                cudaSuccess || occ < 1 || sms < 1) {
+            cudaGetLastError();
             rc = SW_ERR_CUDA;
             break;
         }
-        sw_score_noalloc_kernel<<<kNaWarps / 4, 128, 0, st>>>(a);
-        if (cudaGetLastError() != cudaSuccess) {
+        // the header and the scores (merged by maximum) start at zero
+        if (cudaMemsetAsync(addr, 0, sizeof(NaHeader), st) != cudaSuccess ||
+            cudaMemsetAsync(d_scores, 0, (size_t)n_records * sizeof(int32_t), st) != cudaSuccess) {
+            rc = SW_ERR_CUDA;
+            break;
+        }
+        void* args[] = {&a};
+        const unsigned prep = std::min<unsigned>(
+            (unsigned)sms, (std::max(n_records, qlen) + kNaThreads - 1) / kNaThreads);
+        const unsigned grid =
+            looked_up ? (unsigned)(kNaSlices / (kNaLookupThreads / 32))
+                      : std::min<unsigned>((unsigned)(std::min(occ, k->blocks) * sms),
+                                           std::max(n_records, 1u));
+        if (cudaLaunchKernel((const void*)sw_noalloc_prepare, dim3(prep), dim3(kNaThreads), args, 0,
+                             st) != cudaSuccess ||
+            cudaLaunchKernel(fn, dim3(grid), dim3(threads), args, smem, st) != cudaSuccess) {
+            cudaGetLastError();
             rc = SW_ERR_CUDA;
             break;
         }
         uint32_t err = 0;
-        if (cudaMemcpyAsync(&err, (const char*)addr + sizeof(uint32_t), sizeof(err),
+        if (cudaMemcpyAsync(&err, (const char*)addr + offsetof(NaHeader, error), sizeof(err),
                             cudaMemcpyDeviceToHost, st) != cudaSuccess ||
             cudaStreamSynchronize(st) != cudaSuccess) {
             rc = SW_ERR_CUDA;
