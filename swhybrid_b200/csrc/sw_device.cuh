@@ -36,6 +36,8 @@ struct WfArgs {
     const Pair2* win_pairs;     // windows of long pairs, taken before the pairs ...
     const uint32_t* win_ids;    // ... and the pair each belongs to
     int n_win;
+    int first_blocks;           // blocks that run from the start, with a fixed first claim
+    int block0;                 // this launch's first block among all that share the counter
     const uint8_t* query;       // device query codes of this launch's rows, qlen entries (< 25)
     int qlen;
     int pass0;                  // query passes scored by earlier launches (row segments)

@@ -233,7 +233,7 @@ extern "C" sw_status sw_ctx_create(int device, const sw_params* params, sw_ctx**
         if (!allow_smem(qks[i].fn)) return fail(SW_ERR_CUDA);
     const LongKernel* lks = long_kernels(&nk);
     for (int i = 0; i < nk; ++i)
-        if (!allow_smem(lks[i].fn)) return fail(SW_ERR_CUDA);
+        if (!allow_smem(lks[i].fn[ctx->cell])) return fail(SW_ERR_CUDA);
     *out = ctx;
     return SW_OK;
 }
@@ -597,6 +597,7 @@ extern "C" sw_status sw_set_tuning(sw_ctx* ctx, const sw_tuning_entry* entries, 
         if (tab[i].max_qlen < tab[i - 1].max_qlen)
             SW_SET(ctx, SW_ERR_INVALID, "tuning entries not sorted by max_qlen");
     ctx->tuning = std::move(tab);
+    ctx->tuning_builtin = false;
     return SW_OK;
 }
 
@@ -754,7 +755,7 @@ const LongKernel* choose_long(sw_ctx* ctx, const sw_kernel_config& cfg, int qlen
         const int P = (qlen + 32 * k.R - 1) / (32 * k.R);
         if (P > kLongMaxPasses) return false;
         cudaFuncAttributes fa;
-        if (cudaFuncGetAttributes(&fa, k.fn) != cudaSuccess) {
+        if (cudaFuncGetAttributes(&fa, k.fn[ctx->cell]) != cudaSuccess) {
             cudaGetLastError();
             return false;
         }
@@ -764,7 +765,8 @@ const LongKernel* choose_long(sw_ctx* ctx, const sw_kernel_config& cfg, int qlen
         while (G > 0 && k.smem(P, G) > dyn) --G;
         while (G > 0) {
             int nb = 0;
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k.fn, G * P * 32, dyn) ==
+            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k.fn[ctx->cell], G * P * 32,
+                                                              dyn) ==
                     cudaSuccess && nb >= 1)
                 break;
             cudaGetLastError();
@@ -814,7 +816,7 @@ struct Windows {
 // in long pairs, 18 ms against 40 with windows).
 Windows plan_windows(const sw_ctx* ctx, double share, int64_t span) {
     Windows best;
-    if (span <= 0 || ctx->n_pairs == 0 || (double)ctx->pair_ncols[0] <= 0.8 * share) return best;
+    if (span <= 0 || ctx->n_pairs == 0 || (double)ctx->pair_ncols[0] <= 0.9 * share) return best;
     const double total = (double)ctx->pair_cols_total;
     double best_est = 1.6 * share;
     for (const double f : {1.0, 0.8, 0.65, 0.5, 0.4, 0.3, 0.2, 0.12}) {
@@ -843,12 +845,171 @@ Windows plan_windows(const sw_ctx* ctx, double share, int64_t span) {
     return best;
 }
 
-// How a plain search of qlen divides the DB's pairs.  With a cut-over (the
-// configured one, else auto_cutover's), the long-pair kernel takes the pairs
-// above it, [0, n_long), when some but not all pairs are, and a pipelined
-// shape fits the length; the bulk launches take the rest with the short shape.
-// Otherwise one shape takes every pair: the long one when no pair is above
-// the cut-over or all are, the short one when no pipelined shape fits.
+// ---- time model ----------------------------------------------------------
+// Clocks of a first pass, for choosing between bulk shapes, windows and the
+// long-pair kernel.  A column step of a thread's R rows is bound by the ALU
+// pipe when an SM is full and by its own latency when few warps are on it;
+// the constants were fitted to the kernels' measured rates on a B200 (bulk:
+// 4.5 / 5.4 / 6.0 / 6.2 TCUPS at 8 / 16 / 24 / 48 rows on 350-residue records;
+// long-pair kernel: 134 / 176 / 265 / 352 clocks a step at 4 / 8 / 16 / 24 rows
+// and one warp per scheduler, 332 at 4 rows and four, 288 at 8 rows and two).
+
+// Cells an SM full of bulk groups of R rows per thread updates per clock.
+double bulk_rate(int R) { return 22.7 * R / (R + 4.0); }
+
+// Bulk launch over `units` units (pairs or windows, `cols` columns in all, the
+// longest `longest`) in P passes on sms SMs.
+double bulk_clocks(const WfKernel& k, int block, double P, double units, double cols,
+                   double longest, double sms) {
+    if (units <= 0) return 0.0;
+    const double per_warp = 32.0 / k.T;
+    const double warps = std::min(block / 32.0, std::max(1.0, units / per_warp / sms));
+    const double step = std::max(60.0 + 11.7 * k.R, warps * 64.0 * k.R / bulk_rate(k.R));
+    const double switches = units * (0.25 * (2 * k.T + 9));     // event steps per segment
+    const double avg = (cols + switches) / (sms * warps * per_warp);
+    return P * step * (std::max(avg, longest) + 0.15 * std::min(avg, longest)) + 15e3;
+}
+
+// One column step of the long-pair kernel with `warps` warps per SM.
+double long_step_clocks(int R, int warps) {
+    return std::max(90.0 + 10.8 * R, (warps + 3) / 4 * 2.3 * (5.6 * R + 16.0));
+}
+
+double long_clocks(int R, int passes, int pipes, double pairs, double cols, double longest,
+                   double sms) {
+    const double step = long_step_clocks(R, passes * pipes);
+    const double fill = (passes - 1) * 64.0 + 48.0;
+    const double even = (cols + pairs * fill) / (sms * pipes);
+    return step * (std::max(even, longest + fill) + (pairs > sms * pipes ? 0.3 * even * sms * pipes / pairs : 0.0)) +
+           15e3;
+}
+
+// A long-pair split chosen by the model: pairs [0, n_long) to the long-pair
+// kernel on `sms` SMs (`pipes` pipelines of `passes` warps each), the others
+// to the bulk shape kb.
+struct Split {
+    const WfKernel* kb = nullptr;
+    const LongKernel* lk = nullptr;
+    int64_t n_long = 0;
+    int passes = 0, pipes = 0, sms = 0;
+    size_t smem = 0;
+    bool join = false;
+    double clocks = 1e300;
+};
+
+// Pipelines of P warps one block of a long kernel holds (0: none fits).
+int long_pipelines(sw_ctx* ctx, const LongKernel& k, int P, size_t* smem) {
+    if (P > kLongMaxPasses) return 0;
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, k.fn[ctx->cell]) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    const size_t dyn = (size_t)ctx->max_smem - fa.sharedSizeBytes;
+    const int warp_regs = (fa.numRegs + 7) / 8 * 8 * 32;
+    int G = std::min(k.max_threads / 32, ctx->regs_per_sm / std::max(warp_regs, 1)) / P;
+    while (G > 0 && k.smem(P, G) > dyn) --G;
+    *smem = dyn;
+    return G;
+}
+
+// The best split over cut-overs (every 1.4x in columns, down to every pair),
+// row counts, SM shares and bulk shapes: `given`, and the shapes that fit the
+// query's rows in 1..4 passes (a table's shape is tuned for a large DB; a small
+// one wants wider groups, whose steps are fewer).
+Split plan_split(sw_ctx* ctx, int qlen, const WfKernel* given) {
+    Split best;
+    const int64_t np = ctx->n_pairs;
+    if (np == 0) return best;
+    const WfKernel* shapes[16];
+    int n_shapes = 0;
+    auto add = [&](const WfKernel* k) {
+        if (!k || n_shapes == 16 || launch_rows(ctx, *k, qlen) != qlen) return;
+        for (int i = 0; i < n_shapes; ++i)
+            if (shapes[i] == k) return;
+        shapes[n_shapes++] = k;
+    };
+    add(given);
+    const sw_tuning_entry* entry = find_entry(ctx, qlen);
+    // a plan's shapes stay, and so does a shape from a caller's table
+    const bool fixed = entry && (entry->plan[0].group_width != 0 || !ctx->tuning_builtin);
+    int n_all = 0;
+    const WfKernel* all = wf_kernels(&n_all);
+    for (const int T : {32, 16, 8})
+        for (int P = 1; P <= 4 && !fixed; ++P) {
+            const int rows = (qlen + T * P - 1) / (T * P);
+            const WfKernel* k = nullptr;      // the smallest row count that holds them
+            for (int i = 0; i < n_all; ++i)
+                if (all[i].T == T && all[i].R >= rows && (!k || all[i].R < k->R)) k = &all[i];
+            if (k && k->R <= 64) add(k);
+        }
+    struct Long {
+        const LongKernel* k;
+        int P, G;
+        size_t smem;
+    } longs[8];
+    int n_longs = 0, n_lk = 0;
+    const LongKernel* lks = long_kernels(&n_lk);
+    for (int i = 0; i < n_lk; ++i) {
+        Long l{&lks[i], (qlen + 32 * lks[i].R - 1) / (32 * lks[i].R), 0, 0};
+        l.G = long_pipelines(ctx, lks[i], l.P, &l.smem);
+        if (l.G > 0 && n_longs < 8) longs[n_longs++] = l;
+    }
+    if (n_longs == 0) return best;
+    const double total = (double)ctx->pair_cols_total;
+    const int sms = ctx->num_sms;
+    int64_t prev = -1;
+    for (double cut = (double)ctx->pair_ncols[0] * 0.98; ; cut /= 1.4) {
+        const bool last = cut < 100.0;
+        const uint32_t c = last ? 0u : (uint32_t)cut;
+        const int64_t n_long = std::partition_point(ctx->pair_ncols.begin(), ctx->pair_ncols.end(),
+                                                    [c](uint32_t n) { return n > c; }) -
+                               ctx->pair_ncols.begin();
+        if (n_long != prev && n_long > 0) {
+            prev = n_long;
+            const double cols = (double)ctx->pair_prefix[n_long], longest = ctx->pair_ncols[0];
+            for (const int x : {1, 2, 4, 8, 12, 16, 24, 32, 40, 48, 64, 80, 96, 112, 128, 148}) {
+                const int on = n_long == np ? sms : std::min(x, sms - 1);
+                double tl = 1e300;
+                const Long* l = nullptr;
+                int pipes = 0;
+                for (int i = 0; i < n_longs; ++i) {
+                    const int G = (int)std::min<int64_t>(longs[i].G, (n_long + on - 1) / on);
+                    const double t = long_clocks(longs[i].k->R, longs[i].P, G, (double)n_long, cols,
+                                                 longest, on);
+                    if (t < tl) {
+                        tl = t;
+                        l = &longs[i];
+                        pipes = G;
+                    }
+                }
+                if (tl >= best.clocks) continue;
+                double tb = n_long == np ? 0.0 : 1e300;
+                const WfKernel* kb = n_long == np ? shapes[0] : nullptr;
+                for (int i = 0; i < n_shapes && n_long < np; ++i) {
+                    const WfKernel& k = *shapes[i];
+                    const double P = (qlen + k.T * k.R - 1) / (k.T * k.R);
+                    const double t = bulk_clocks(k, plain_block(ctx, k), P, (double)(np - n_long),
+                                                 total - cols, ctx->pair_ncols[n_long], sms - on);
+                    if (t < tb) {
+                        tb = t;
+                        kb = &k;
+                    }
+                }
+                const double t = std::max(tl, tb);
+                if (kb && t < best.clocks)
+                    best = Split{kb, l->k, n_long, l->P, pipes, on, l->smem, tl < 0.8 * tb, t};
+                if (on == sms) break;
+            }
+        }
+        if (last) break;
+    }
+    return best;
+}
+
+// How a plain search of qlen divides the DB's pairs: all to one bulk shape; the
+// long ones cut into windows; or the long ones, [0, n_long), to the long-pair
+// kernel and the rest (if any) to the bulk shape.
 struct SearchLayout {
     sw_kernel_config cfg;
     Windows win;                       // long pairs cut into windows for the bulk launches
@@ -856,7 +1017,8 @@ struct SearchLayout {
     bool split = false;
     int64_t n_long = 0;                // pairs of the long-pair kernel (split only)
     const LongKernel* lk = nullptr;
-    int lpasses = 0, lpipes = 0;
+    int lpasses = 0, lpipes = 0, lsms = 0;
+    bool join = false;                 // the long launch ends well before the bulk one
     size_t lsmem = 0;
     int bulk_T = 0, bulk_R = 0;        // the bulk launches' shape ...
     int64_t bulk_b = 0, bulk_e = 0;    // ... pairs (after the windows) ...
@@ -864,11 +1026,70 @@ struct SearchLayout {
     int bulk_counter = 0;              // ... and claim counter
 };
 
+// Without a configured shape or cut-over: the layout the time model prefers.
+// Returns false when it keeps one bulk shape for every pair.
+bool model_layout(sw_ctx* ctx, int qlen, int64_t span, SearchLayout* L) {
+    const sw_kernel_config& cfg = L->cfg;
+    const WfKernel* kb = find_kernel(cfg.short_group_width, cfg.short_rows_per_thread);
+    if (!kb || ctx->n_pairs == 0) return false;
+    const int rows = std::min(qlen, launch_rows(ctx, *kb, qlen));
+    const double share = group_share(ctx, *kb, rows);
+    if ((double)ctx->pair_ncols[0] <= 0.9 * share) return false;
+    const int block = plain_block(ctx, *kb);
+    const double P = (qlen + kb->T * kb->R - 1) / (kb->T * kb->R);
+    const double np = (double)ctx->n_pairs, total = (double)ctx->pair_cols_total;
+    const double whole = bulk_clocks(*kb, block, P, np, total, ctx->pair_ncols[0], ctx->num_sms);
+    double windowed = 1e300;
+    const Windows win = plan_windows(ctx, share, span);
+    if (win.n > 0)
+        windowed = bulk_clocks(*kb, block, P, np - win.n_pairs + win.n,
+                               total + (double)win.n * win.len - (double)ctx->pair_prefix[win.n_pairs],
+                               win.len, ctx->num_sms) + 15e3;
+    const Split sp = plan_split(ctx, qlen, kb);
+    const double least = std::min({whole, windowed, sp.clocks});
+    if (least == whole) return false;
+    if (least == windowed) {
+        L->win = win;
+        L->bulk_T = kb->T;
+        L->bulk_R = kb->R;
+        L->bulk_b = win.n_pairs;
+        L->longest = win.len;
+    } else {
+        L->split = true;
+        L->n_long = sp.n_long;
+        L->lk = sp.lk;
+        L->lpasses = sp.passes;
+        L->lpipes = sp.pipes;
+        L->lsms = sp.sms;
+        L->lsmem = sp.smem;
+        L->join = sp.join;
+        L->bulk_T = sp.kb->T;
+        L->bulk_R = sp.kb->R;
+        L->bulk_b = sp.n_long;
+        L->cutover = sp.n_long < ctx->n_pairs ? (int)ctx->pair_ncols[sp.n_long] : 1;
+        L->longest = sp.n_long < ctx->n_pairs ? (double)ctx->pair_ncols[sp.n_long] : 0.0;
+    }
+    L->bulk_e = ctx->n_pairs;
+    L->bulk_counter = 1;
+    return true;
+}
+
 void layout_search(sw_ctx* ctx, int qlen, int64_t span, SearchLayout* L) {
     const sw_kernel_config& cfg = L->cfg = choose_config(ctx, qlen);
-    // windows, unless the caller's configuration asks for a cut-over
+    const bool callers_cut = cfg.cutover > 0 && !ctx->tuning_builtin;
+    if (!ctx->has_override && !callers_cut) {
+        if (model_layout(ctx, qlen, span, L)) return;
+        L->bulk_T = cfg.short_group_width;
+        L->bulk_R = cfg.short_rows_per_thread;
+        L->bulk_b = 0;
+        L->bulk_e = ctx->n_pairs;
+        L->longest = ctx->n_pairs > 0 ? (double)ctx->pair_ncols[0] : 0.0;
+        return;
+    }
+    // a shape override, or a caller's table with a cut-over: that cut-over, or
+    // windows or a cut-over for the shape
     const WfKernel* kb = find_kernel(cfg.short_group_width, cfg.short_rows_per_thread);
-    if (kb && !(ctx->has_override && cfg.cutover > 0))
+    if (kb && cfg.cutover == 0)
         L->win = plan_windows(ctx, group_share(ctx, *kb, std::min(qlen, launch_rows(ctx, *kb, qlen))),
                               span);
     if (L->win.n > 0) {
@@ -905,6 +1126,29 @@ void layout_search(sw_ctx* ctx, int qlen, int64_t span, SearchLayout* L) {
     }
     L->bulk_e = ctx->n_pairs;
     L->n_long = L->split ? n_long : 0;
+    if (L->split) {
+        // SMs for the long launch: the best of the model for its pairs and
+        // row count beside this bulk shape
+        double best = 1e300;
+        const double cols = (double)ctx->pair_prefix[n_long];
+        const int G0 = L->lpipes;
+        for (int x = 1; x < ctx->num_sms; x += 1 + x / 8) {
+            const int G = (int)std::min<int64_t>(G0, (n_long + x - 1) / x);
+            const double tl = long_clocks(L->lk->R, L->lpasses, G, (double)n_long, cols,
+                                          ctx->pair_ncols[0], x);
+            const WfKernel* k = find_kernel(L->bulk_T, L->bulk_R);
+            const double P = k ? (qlen + k->T * k->R - 1) / (k->T * k->R) : 1;
+            const double tb = k ? bulk_clocks(*k, plain_block(ctx, *k), P,
+                                              (double)(ctx->n_pairs - n_long),
+                                              (double)ctx->pair_cols_total - cols,
+                                              ctx->pair_ncols[n_long], ctx->num_sms - x) : 0.0;
+            if (std::max(tl, tb) < best) {
+                best = std::max(tl, tb);
+                L->lsms = x;
+                L->lpipes = G;
+            }
+        }
+    }
     L->longest = L->bulk_b < L->bulk_e ? (double)ctx->pair_ncols[L->bulk_b] : 0.0;
 }
 
@@ -950,8 +1194,10 @@ sw_status enqueue_search(sw_ctx* ctx, const uint8_t* d_query, int qlen, int64_t 
     const int64_t n_long = L.n_long;
     const LongKernel* lk = L.lk;
     const int lpasses = L.lpasses;
-    int lpipes = L.lpipes;
+    const int lpipes = L.lpipes;
     if (split) {
+        ctx->stats.used.short_group_width = L.bulk_T;
+        ctx->stats.used.short_rows_per_thread = L.bulk_R;
         ctx->stats.used.long_group_width = 32;
         ctx->stats.used.long_rows_per_thread = lk->R;
     }
@@ -992,21 +1238,7 @@ sw_status enqueue_search(sw_ctx* ctx, const uint8_t* d_query, int qlen, int64_t 
     SW_CUDA(ctx, cudaEventRecord(mk.e[1], st));
     int reserved_sms = 0;
     if (split) {
-        uint64_t long_cols = 0;
-        for (int64_t p = 0; p < n_long; ++p) long_cols += ctx->pair_ncols[p];
-        const double share = (double)long_cols / (double)std::max<uint64_t>(ctx->pair_cols_total, 1);
-        // SMs for the long launch: their share of the columns, or, when there
-        // are few long pairs, enough SMs that each warp scheduler runs about
-        // one of their warps (a pair's column steps are serial, so a crowded
-        // SM would make the longest pair the critical path), at most half
-        reserved_sms = (int)std::lround(share * ctx->num_sms);
-        const int64_t spread = (n_long * lpasses + 3) / 4;
-        reserved_sms = (int)std::max<int64_t>(reserved_sms,
-                                              std::min<int64_t>(spread, ctx->num_sms / 2));
-        reserved_sms = std::max(1, std::min(reserved_sms, ctx->num_sms - 1));
-        reserved_sms = (int)std::min<int64_t>(reserved_sms, (n_long + lpipes - 1) / lpipes);
-        // pipelines per block: the long pairs spread evenly over those SMs
-        lpipes = (int)std::min<int64_t>(lpipes, (n_long + reserved_sms - 1) / reserved_sms);
+        reserved_sms = L.lsms;
         SW_CUDA(ctx, cudaEventRecord(ctx->fork_ev, st));
         SW_CUDA(ctx, cudaStreamWaitEvent(ctx->side_stream, ctx->fork_ev, 0));
         LongArgs la;
@@ -1029,8 +1261,10 @@ sw_status enqueue_search(sw_ctx* ctx, const uint8_t* d_query, int qlen, int64_t 
         la.ovf_cap = (int)ctx->n_records + 1;
         void* args[] = {&la};
         SW_CUDA(ctx, cudaEventRecord(mk.e[4], ctx->side_stream));
-        SW_CUDA(ctx, cudaLaunchKernel(lk->fn, dim3((unsigned)reserved_sms),
-                                      dim3(lpasses * lpipes * 32), args, L.lsmem, ctx->side_stream));
+        SW_CUDA(ctx, cudaLaunchKernel(
+                         lk->fn[ctx->cell],
+                         dim3((unsigned)std::min<int64_t>(reserved_sms, (n_long + lpipes - 1) / lpipes)),
+                         dim3(lpasses * lpipes * 32), args, L.lsmem, ctx->side_stream));
         SW_CUDA(ctx, cudaEventRecord(mk.e[5], ctx->side_stream));
         ++*launches;
         ++mk.fp_launches;
@@ -1089,17 +1323,33 @@ sw_status enqueue_search(sw_ctx* ctx, const uint8_t* d_query, int qlen, int64_t 
             a.ovf_count = ctx->d_counters + 2;
             a.ovf_thresh = ovf_thresh;
             void* args[] = {&a};
-            int64_t grid = (int64_t)occ * (ctx->num_sms - reserved_sms);
+            // The first launch leaves the long launch its SMs (blocks that
+            // found them first would hold them to the end); a later row
+            // segment's blocks wait for theirs.
+            const bool first = r0 == 0;
+            int64_t grid = (int64_t)occ * (ctx->num_sms - (first ? reserved_sms : 0));
             const int block = plain_block(ctx, *k);
             // a warp claims 32 / T pairs at a time: no more blocks than claims
             // (few pairs spread one warp per SM)
             const int64_t per_claim = 32 / k->T;
             grid = std::min<int64_t>(grid, (a.pair_count + per_claim - 1) / per_claim);
             grid = std::max<int64_t>(grid, 1);
+            a.block0 = 0;
+            a.first_blocks = (int)std::min<int64_t>(
+                grid, std::max<int64_t>(1, (int64_t)occ * (ctx->num_sms - reserved_sms)));
             SW_CUDA(ctx, cudaLaunchKernel(k->fn[ctx->cell], dim3((unsigned)grid), dim3(block), args,
                                           k->smem(rows), st));
             ++*launches;
             ++mk.fp_launches;
+            if (L.join && first && rows == qlen) {
+                // the whole query in one launch: once the long pairs are done
+                // their SMs take part in it
+                a.block0 = a.first_blocks;
+                SW_CUDA(ctx, cudaLaunchKernel(k->fn[ctx->cell], dim3((unsigned)(occ * reserved_sms)),
+                                              dim3(block), args, k->smem(rows), ctx->side_stream));
+                ++*launches;
+                ++mk.fp_launches;
+            }
             r0 += rows;
             passes_before += (rows + k->T * k->R - 1) / (k->T * k->R);
         }

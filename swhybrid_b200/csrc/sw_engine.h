@@ -119,6 +119,7 @@ struct sw_ctx {
     unsigned long long* h_keys = nullptr;  // pinned
 
     std::vector<sw_tuning_entry> tuning;
+    bool tuning_builtin = true;        // the compiled-in table (sw_set_tuning replaces it)
     bool has_override = false;
     sw_kernel_config override_cfg{};
     sw_run_stats stats{};

@@ -5,10 +5,11 @@
 #include <cstdint>
 
 #include "sw_device.cuh"
+#include "sw_registry.h"
 
 namespace swb {
 
-constexpr int kLongMaxPasses = 8;        // query passes of 32 x R rows = warps per pipeline
+constexpr int kLongMaxPasses = 16;       // query passes of 32 x R rows = warps per pipeline
 constexpr int kLongMaxWarps = 32;        // pipelines x passes per block
 
 struct LongArgs {
@@ -32,7 +33,7 @@ struct LongArgs {
 
 struct LongKernel {
     int R;                                      // query rows per thread; 32 threads per pass
-    const void* fn;                             // __global__ sw_long<R>
+    const void* fn[kPlainCells];                // __global__ sw_long<R, cell>
     size_t (*smem)(int passes, int pipelines);  // dynamic shared memory of one block
     int max_threads;                            // the kernel's launch bound
 };

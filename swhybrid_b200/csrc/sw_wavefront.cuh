@@ -95,6 +95,19 @@ struct CellWide {
     __device__ __forceinline__ uint32_t diag(uint32_t up, uint32_t p, uint32_t e) const {
         return __viaddmax_s16x2(up, p, e);
     }
+    // The same cell with a short serial chain, for the long-pair kernel: F of
+    // the next row comes from t = max(diag + P, E, 0), H before F, so only one
+    // instruction per row waits for the row above (an H that F made never opens
+    // a better gap than F extended); one maximum more per row.
+    __device__ __forceinline__ uint32_t diag_floor(uint32_t up, uint32_t p, uint32_t e) const {
+        return __vmaxs2(__viaddmax_s16x2(up, p, e), bias2);
+    }
+    __device__ __forceinline__ void forward_short(uint32_t& hk, uint32_t& ek, uint32_t& f) const {
+        const uint32_t h = __vmaxs2(hk, f);
+        f = __viaddmax_s16x2(f, neg_e2, hk + neg_q2);
+        hk = h;
+        ek = __viaddmax_s16x2(ek, neg_e2, h + neg_q2);
+    }
     // the rest of the cell: hk holds diag's result and receives H
     __device__ __forceinline__ void forward(uint32_t& hk, uint32_t& ek, uint32_t& f) const {
         const uint32_t h = __vimax3_s16x2(hk, f, bias2);
@@ -149,6 +162,15 @@ struct CellNarrow {
     static constexpr bool prefetch = false;
     __device__ __forceinline__ uint32_t diag(uint32_t up, uint32_t p, uint32_t) const {
         return up + p;
+    }
+    __device__ __forceinline__ uint32_t diag_floor(uint32_t up, uint32_t p, uint32_t e) const {
+        return __vimax3_s16x2(up + p, e, Z);
+    }
+    __device__ __forceinline__ void forward_short(uint32_t& hk, uint32_t& ek, uint32_t& f) const {
+        const uint32_t hq = __vmaxs2(hk, f) - q2;
+        f = __viaddmax_s16x2(f, ne16, hk - q2);
+        hk = hq;
+        ek = __viaddmax_s16x2(ek, ne16, hq);
     }
     __device__ __forceinline__ void forward(uint32_t& hk, uint32_t& ek, uint32_t& f) const {
         const uint32_t hq = __vimax3_s16x2(hk, ek, f) - q2;
@@ -351,7 +373,8 @@ struct RunArgs {
     const Pair2* win_pairs;
     const uint32_t* win_ids;
     int n_win;
-    int* counter;               // pairs of the range claimed so far
+    int* counter;               // pairs claimed after the first claims
+    int first_blocks, block0;   // blocks with a fixed first claim; number of block 0
     int P;                      // query passes of T*R rows
     // A query too long for one launch's profile is scored in row segments by
     // consecutive launches (plain search only): pass0 = passes of the query
@@ -418,8 +441,9 @@ __device__ __forceinline__ void put_score(const RunArgs& a, int pos, int s, int 
 // through its own window of 2T + 9 event steps per segment while the other
 // groups of the warp ran theirs as event steps too.  A group beyond the last
 // pair repeats the last one and writes nothing.  A warp's first claim is fixed
-// (warp w of block b takes the w * gridDim + b'th), so that few pairs spread
-// over all SMs; the later ones come from the counter.
+// (warp w of block b takes the w * first_blocks + b'th), so that few pairs
+// spread over all SMs; the later ones, and all of a block that may start late
+// (b >= first_blocks), come from the counter.
 //
 // The groups stream: each thread moves on to the group's next segment (the
 // next pass of the pair, or the next pair) as soon as its own columns of the
@@ -544,9 +568,13 @@ __device__ __forceinline__ void run_stream(const RunArgs& a, const uint2* prof, 
     }
 
     {
-        const int warps = (int)(blockDim.x >> 5);
-        const int v = ((int)(threadIdx.x >> 5) * (int)gridDim.x + (int)blockIdx.x) * G;
-        claimed = warps * (int)gridDim.x * G;
+        const int warps = (int)(blockDim.x >> 5), block = a.block0 + (int)blockIdx.x;
+        claimed = warps * a.first_blocks * G;
+        int v = ((int)(threadIdx.x >> 5) * a.first_blocks + block) * G;
+        if (block >= a.first_blocks) {
+            if (lane == 0) v = claimed + atomicAdd(a.counter, G);
+            v = __shfl_sync(FULL, v, 0);
+        }
         pair = v + grp;
         if (v < pair_count) {
             const Pair2 pr = entry(min(pair, pair_count - 1));
@@ -876,6 +904,8 @@ __global__ void __launch_bounds__(BLOCK, 1) sw_wavefront(const WfArgs a) {
     r.win_ids = a.win_ids;
     r.n_win = a.n_win;
     r.counter = a.counter;
+    r.first_blocks = a.first_blocks;
+    r.block0 = a.block0;
     r.P = P;
     r.pass0 = a.pass0;
     r.more = a.more;
@@ -918,6 +948,8 @@ __global__ void __launch_bounds__(BLOCK, 1) sw_batch(const BatchArgs a) {
         r.win_ids = nullptr;
         r.n_win = 0;
         r.counter = a.counters + i;
+        r.first_blocks = (int)gridDim.x;
+        r.block0 = 0;
         r.P = P;
         r.pass0 = 0;
         r.more = 0;

@@ -48,7 +48,7 @@ def test_windowed_records_equal_the_oracle(qlen, gap_open, gap_extend, lengths):
     res, off = with_long(rng, 40_000, 150, 350, longs)
     with capi.Context(0, capi.default_params(gap_open=gap_open, gap_extend=gap_extend)) as c:
         c.load_db(res, off)
-        c.set_tuning([(1 << 30, (16, 64, 16, 64, 0))])      # ~2,100 columns per group
+        c.set_kernel_config((16, 64, 16, 64, 0))            # ~2,100 columns per group
         hits, scores = c.search(q, want_scores=True)
         st = c.run_stats()
         # windows + first pass + re-score + two top-k rounds, no long-pair split
@@ -62,26 +62,33 @@ def test_windowed_records_equal_the_oracle(qlen, gap_open, gap_extend, lengths):
 
 @pytest.mark.parametrize("row_segments", [False, True])
 def test_saturation_in_overlapping_windows(row_segments):
-    """W runs of 3,000 in a 40,000-residue record: the lane wraps in every
-    window that holds one, and the record is listed for the 32-bit pass once."""
+    """W runs of 370 (90 per cell) in a 40,000-residue record: the lane wraps
+    in every window that holds one, and the record is listed for the 32-bit
+    pass once, also when the query's rows run as two segments."""
     rng = np.random.default_rng(9)
-    q = param.encode("W" * 3000).astype(np.uint8)
-    rec = np.concatenate([synth.residues(rng, 5000), q, synth.residues(rng, 14_000), q,
-                          synth.residues(rng, 15_000)]).astype(np.uint8)
+    m = M.copy()
+    w = int(param.encode("W")[0])
+    m[w, w] = 90
+    q = param.encode("W" * 370).astype(np.uint8)
+    rec = np.concatenate([synth.residues(rng, 5000), q, synth.residues(rng, 17_000), q,
+                          synth.residues(rng, 17_000)]).astype(np.uint8)
     res, off = with_long(rng, 60_000, 300, 500, [rec])
-    with capi.Context(0, capi.default_params(gap_open=10, gap_extend=50)) as c:
+    with capi.Context(0, capi.default_params(gap_open=10, gap_extend=20, matrix=m)) as c:
         c.load_db(res, off)
         if row_segments:
-            c.set_tuning([(1 << 30, (16, 64, 16, 64, 0), ((16, 64, 1), (16, 56, 0)))])
+            c.set_tuning([(1 << 30, (32, 8, 32, 8, 0), ((32, 8, 1), (32, 8, 0)))])
         else:
-            c.set_tuning([(1 << 30, (16, 64, 16, 64, 0))])
-        assert len(c.plan(3000)) == (2 if row_segments else 1)
+            c.set_kernel_config((32, 8, 32, 8, 0))
+        assert len(c.plan(370)) == (2 if row_segments else 1)
         hits, scores = c.search(q, want_scores=True)
         st = c.run_stats()
-    assert st.used.cutover == 0 and st.rescored == 1
-    top = oracle.gotoh(q, rec, M, 60, 50)
+    assert st.rescored == 1
+    # (with the table the time model may send the one long pair to the
+    # long-pair kernel instead)
+    assert row_segments or (st.used.cutover == 0 and st.launches == 5)
+    top = oracle.gotoh(q, rec, m, 30, 20)
     assert top >= 33_000 and scores[-1] == top and hits[0] == (top, len(off) - 2)
-    pick = rng.choice(60_000, size=50, replace=False)
+    pick = rng.choice(60_000, size=200, replace=False)
     sub = synth.DB(res, off).subset(pick)
-    np.testing.assert_array_equal(scores[pick], oracle.search(q, sub.residues, sub.offsets, M, 60, 50,
-                                                                mode=0))
+    np.testing.assert_array_equal(scores[pick], oracle.search(q, sub.residues, sub.offsets, m, 30, 20,
+                                                              mode=0))
