@@ -298,7 +298,7 @@ sw_status enqueue_batch(sw_ctx* ctx, sw_batch_state* b, uint32_t nq, size_t qbyt
             q.seg_stride = b->seg_stride;
             q.long_units = L.long_units;
             void* args[] = {&q};
-            SW_CUDA(ctx, cudaLaunchKernel(L.qk->fn, dim3((unsigned)L.grid), dim3(L.threads), args,
+            SW_CUDA(ctx, cudaLaunchKernel(L.qk->fn[ctx->cell], dim3((unsigned)L.grid), dim3(L.threads), args,
                                           L.smem, st));
             ++*n_launch;
             continue;
@@ -713,7 +713,7 @@ extern "C" sw_status sw_search_batch(sw_ctx* ctx, uint32_t nq, const uint8_t* qu
             const size_t smem = qk->smem((int)std::max<uint32_t>(max_rows, 1));
             int occ = 0;
             if (smem <= (size_t)ctx->max_smem &&
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, qk->fn, qk->block, smem) !=
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, qk->fn[ctx->cell], qk->block, smem) !=
                     cudaSuccess) {
                 cudaGetLastError();
                 occ = 0;

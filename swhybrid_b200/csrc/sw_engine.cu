@@ -230,7 +230,7 @@ extern "C" sw_status sw_ctx_create(int device, const sw_params* params, sw_ctx**
         if (!allow_smem(ks[i].fn[ctx->cell]) || !allow_smem(ks[i].batch_fn)) return fail(SW_ERR_CUDA);
     const QpKernel* qks = qp_kernels(&nk);
     for (int i = 0; i < nk; ++i)
-        if (!allow_smem(qks[i].fn)) return fail(SW_ERR_CUDA);
+        if (!allow_smem(qks[i].fn[ctx->cell])) return fail(SW_ERR_CUDA);
     const LongKernel* lks = long_kernels(&nk);
     for (int i = 0; i < nk; ++i)
         if (!allow_smem(lks[i].fn[ctx->cell])) return fail(SW_ERR_CUDA);

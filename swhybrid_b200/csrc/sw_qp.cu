@@ -6,7 +6,12 @@ namespace swb {
 namespace {
 template <int T, int R, int B>
 constexpr QpKernel qinst() {
-    return QpKernel{T, R, B, (const void*)&sw_qpbatch<T, R, B>, &qp_smem_bytes<T, R>};
+    return QpKernel{T, R, B,
+                    {(const void*)&sw_qpbatch<T, R, B, CellNarrow<0, 0>>,
+                     (const void*)&sw_qpbatch<T, R, B, CellNarrow<0, 0>>,
+                     (const void*)&sw_qpbatch<T, R, B, CellNarrow<12, 2>>,
+                     (const void*)&sw_qpbatch<T, R, B, CellNarrow<12, 1>>},
+                    &qp_smem_bytes<T, R>};
 }
 }  // namespace
 

@@ -8,7 +8,10 @@
 // record: both lanes then look up the same residue, and the profile can be
 // stored already packed -- word (code, row) = score of query A's row against
 // the code in the low half, query B's in the high half -- so the per-row
-// work is 4.5 ALU instructions (no PRMT) for the same two cells.
+// work is 3.5 ALU instructions (no PRMT; CellNarrow, sw_wavefront.cuh) for the
+// same two cells.  A profile word is the 32-bit sum of both lanes' biased
+// scores, so that adding it carries and borrows across the halves exactly and
+// any matrix will do (H is at least the biased zero, 1,024).
 //
 // Here a "double stack" is two stacks of short queries (the low lane's and
 // the high lane's, each packed first-fit into R-row blocks as in sw_batch)
@@ -161,11 +164,11 @@ __host__ __device__ constexpr size_t qp_smem_bytes(int rows) {
 // Paired profile -> shared memory (whole block; the caller synchronises).
 // Layout [pass][chunk of 4 rows][code][slot] of 16-byte words; component i of
 // a word is row 4*chunk + i of the slot's thread: low half the low lane's
-// score, high half the high lane's.
+// score, high half the high lane's, each plus pbias (the cell's profile bias).
 template <int T, int R>
 __device__ __forceinline__ void build_profile_qp(uint4* prof, const uint8_t* lo, int rows_lo,
                                                  const uint8_t* hi, int rows_hi,
-                                                 const int8_t* mat, int P) {
+                                                 const int8_t* mat, int P, int pbias) {
     constexpr int NJ = R / 4;
     constexpr int SLOTS = GroupShape<T>::SLOTS;
     constexpr int JSTRIDE = kCodes * SLOTS;
@@ -185,7 +188,7 @@ __device__ __forceinline__ void build_profile_qp(uint4* prof, const uint8_t* lo,
             const int row = row0 + i;
             const int a = row < rows_lo ? mat[(lo[row] & 31) * 32 + d] : 0;
             const int b = row < rows_hi ? mat[(hi[row] & 31) * 32 + d] : 0;
-            w[i] = (uint32_t)(uint16_t)(int16_t)a | ((uint32_t)(uint16_t)(int16_t)b << 16);
+            w[i] = (uint32_t)(a + pbias) + ((uint32_t)(b + pbias) << 16);
         }
         prof[idx] = make_uint4(w[0], w[1], w[2], w[3]);
     }
@@ -195,11 +198,12 @@ __device__ __forceinline__ uint32_t qp_word(const uint4& v, int i) {
     return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w;
 }
 
-// Reverse sweep of one half with pre-packed profile words: H[k] <- max(H[k-1]
-// + P_k, E_k) for k = HI-1 down to LO, H[LO-1] replaced by diag.
-template <int R, int LO, int HI>
+// Reverse sweep of one half with pre-packed profile words: H[k] <-
+// K.diag(H[k-1], P_k, E_k) for k = HI-1 down to LO, H[LO-1] replaced by diag.
+template <int R, int LO, int HI, class CELL>
 __device__ __forceinline__ void reverse_sweep_qp(uint32_t (&H)[R], const uint32_t (&E)[R],
-                                                 const uint4* p, int jstride, uint32_t diag) {
+                                                 const uint4* p, int jstride, uint32_t diag,
+                                                 const CELL& K) {
     constexpr int JLO = LO / 4, JHI = (HI - 1) / 4;
     uint4 A = p[JHI * jstride];
 #pragma unroll
@@ -211,7 +215,7 @@ __device__ __forceinline__ void reverse_sweep_qp(uint32_t (&H)[R], const uint32_
             const int k = j * 4 + i;
             if (k >= LO && k < HI) {
                 const uint32_t up = (k > LO) ? H[k > LO ? k - 1 : LO] : diag;
-                H[k] = __viaddmax_s16x2(up, qp_word(A, i), E[k]);
+                H[k] = K.diag(up, qp_word(A, i), E[k]);
             }
         }
         A = An;
@@ -221,20 +225,20 @@ __device__ __forceinline__ void reverse_sweep_qp(uint32_t (&H)[R], const uint32_
 // One column step of a thread's two halves with packed profile words: the
 // top half (rows [0, R/2)) on column c at pt, the bottom half on column c - 1
 // at pb (see column_step in sw_wavefront.cuh for the carried values).
-template <int R, int JSTRIDE>
+template <int R, int JSTRIDE, class CELL>
 __device__ __forceinline__ void column_step_qp(uint32_t (&H)[R], uint32_t (&E)[R],
                                                const uint4* pt, const uint4* pb,
                                                uint32_t prev_h, uint32_t f_in,
                                                uint32_t& mid_h, uint32_t& mid_f,
                                                uint32_t& out_h, uint32_t& out_f,
                                                uint32_t& S_top, uint32_t& S_bot,
-                                               const CellWide& K) {
+                                               const CELL& K) {
     constexpr int HALF = R / 2;
     const uint32_t bot_diag = mid_h;
     uint32_t f_top = f_in, f_bot = mid_f;
     mid_h = H[HALF - 1];
-    reverse_sweep_qp<R, 0, HALF>(H, E, pt, JSTRIDE, prev_h);
-    reverse_sweep_qp<R, HALF, R>(H, E, pb, JSTRIDE, bot_diag);
+    reverse_sweep_qp<R, 0, HALF>(H, E, pt, JSTRIDE, prev_h, K);
+    reverse_sweep_qp<R, HALF, R>(H, E, pb, JSTRIDE, bot_diag, K);
 #pragma unroll
     for (int i = 0; i < HALF; ++i) {
         K.forward(H[i], E[i], f_top);
@@ -247,9 +251,10 @@ __device__ __forceinline__ void column_step_qp(uint32_t (&H)[R], uint32_t (&E)[R
     out_f = f_bot;
 }
 
-// One double stack: every group claims units (records) and scores them
-// against both lanes' stacks.  Returns when the units are exhausted.  The
-// groups stream from pass to pass and unit to unit without draining, as in
+// One double stack: the warps claim units (records), G = 32 / T neighbouring
+// ones at a time, and each group scores one of them against both lanes' stacks.
+// Returns when the units are exhausted.  The groups of a warp run in lockstep
+// and stream from pass to pass and unit to unit without draining, as in
 // run_stream (sw_wavefront.cuh), with the maximum chain and the last-thread
 // atomicMax done per lane (each lane has its own query map).  Rows above pass
 // 0 come from seg_bnd when the stack continues an earlier segment (bit 0 of
@@ -258,10 +263,11 @@ __device__ __forceinline__ void column_step_qp(uint32_t (&H)[R], uint32_t (&E)[R
 // pass's thread T-1 writes it, so one buffer serves both.
 //
 // Units come from `counter` (unit_first + claims, up to units_end) or, with a
-// null counter, the group scores the one unit `single` (none when single >=
-// units_end).
-template <int T, int R>
-__device__ __forceinline__ void run_qpairs(const QpArgs& a, const uint4* prof, int P, int* counter,
+// null counter, the warp scores the units from `single` on (none when single
+// >= units_end).
+template <int T, int R, class CELL>
+__device__ __forceinline__ void run_qpairs(const QpArgs& a, const uint4* prof, const CELL& K,
+                                           int P, int* counter,
                                            const int2* rb_map, uint32_t seg, size_t seg_base,
                                            int unit_first, int units_end, int single) {
     static_assert(R % 8 == 0, "R");
@@ -274,15 +280,18 @@ __device__ __forceinline__ void run_qpairs(const QpArgs& a, const uint4* prof, i
     const int lane = threadIdx.x & 31;
     const int t = lane & (T - 1);
     const int slot = lane & (SLOTS - 1);
-    const unsigned gmask = (T == 32) ? FULL : (((1u << T) - 1u) << (lane & ~(T - 1)));
-    const CellWide K(a.gap_oe, a.gap_e);
-    const uint32_t Z = K.hz();
-    const int bias = (int)(Z & 0xffffu);
+    const uint32_t HZ = K.hz(), FZ = K.fz();
+    const int bias = (int)(HZ & 0xffffu);
+    const int ovf_thresh = a.ovf_thresh - K.stored_shift();
     const int units = units_end;
+    constexpr int G = 32 / T;
+    const int grp = lane / T;
     const int dep_steps = 2 * T + 2;
-    // thread 0 claims the group's units
+    // no boundary row is read or written: one pass, the whole stack
+    const bool one_pass = P == 1 && seg == 0u;
+    // lane 0 claims the warp's units
     auto claim = [&]() -> int {
-        if (counter) return unit_first + atomicAdd(counter, 1);
+        if (counter) return unit_first + atomicAdd(counter, G);
         const int v = single;
         single = units;
         return v;
@@ -292,14 +301,15 @@ __device__ __forceinline__ void run_qpairs(const QpArgs& a, const uint4* prof, i
     uint32_t H[R], E[R];
 #pragma unroll
     for (int k = 0; k < R; ++k) {
-        H[k] = Z;
-        E[k] = Z;
+        H[k] = HZ;
+        E[k] = FZ;
     }
-    uint32_t S_top = Z, S_bot = Z, S_pend = Z, acc_out = Z;
-    uint32_t out_h = Z, out_f = Z, prev_h = Z, mid_h = Z, mid_f = Z;
+    uint32_t S_top = HZ, S_bot = HZ, S_pend = HZ, acc_out = HZ;
+    uint32_t out_h = HZ, out_f = FZ, prev_h = HZ, mid_h = HZ, mid_f = FZ;
     uint32_t d_bot = kZeroCode, d_cur = kZeroCode;
     // the top half's segment
     int unit = 0, half = 0, pass = 0, ncols = 0, nst = 0, c = 0;
+    int wcols = 0;             // columns of the warp's longest unit
     uint32_t off16 = 0u;
     const unsigned short* col = reinterpret_cast<const unsigned short*>(a.db);
     const uint4* prof_t = prof + slot;
@@ -316,17 +326,18 @@ __device__ __forceinline__ void run_qpairs(const QpArgs& a, const uint4* prof, i
     int f_unit = 0, fq_lo = -1, fq_hi = -1;
     uint32_t f_reset = 0u, f_last = 0u;
     bool fpend = false, fin = false;
-    // thread 0: the next unit (claimed one unit ahead) and the rows above
+    // lane 0: the warp's next units (claimed one segment ahead); thread 0: its
+    // group's next unit and the rows above
     int next = 0;
     Pair2 ninfo{0u, 0u};
-    uint2 bq0 = make_uint2(Z, Z), bq1 = bq0;
+    uint2 bq0 = make_uint2(HZ, FZ), bq1 = bq0;
     bool has_in = false;
     const uint2* rrow = pbnd;
 
 #define SWQ_SET_SEG()                                                          \
     {                                                                          \
         const int lo = (pass + 1 < P) ? dep_steps : 3;                         \
-        nst = ncols > lo ? ncols : lo;                                         \
+        nst = wcols > lo ? wcols : lo;                                         \
         col = reinterpret_cast<const unsigned short*>(a.db) + (size_t)off16 * 8; \
         uint2* const sb = a.seg_bnd + seg_base + (size_t)off16 * 16 + half;    \
         wrow = (pass + 1 < P) ? pbnd + (pass & 1) : sb;                        \
@@ -346,18 +357,20 @@ __device__ __forceinline__ void run_qpairs(const QpArgs& a, const uint4* prof, i
 
     {
         int v = 0;
-        if (t == 0) v = claim();
-        v = __shfl_sync(gmask, v, 0, T);
-        unit = v;
+        if (lane == 0) v = claim();
+        v = __shfl_sync(FULL, v, 0);
+        unit = v + grp;
         if (v < units) {
-            const Pair2 pr = a.pairs[a.pair_begin + (v >> 1)];
+            const int u = min(unit, units - 1);      // past the end: the last one again, unwritten
+            const Pair2 pr = a.pairs[a.pair_begin + (u >> 1)];
             off16 = pr.off16;
             ncols = (int)pr.ncols;
-            half = v & 1;
-            if (t == 0) next = claim();
+            half = u & 1;
+            if (lane == 0) next = claim();
         } else {
             fin = true;
         }
+        wcols = (int)__reduce_max_sync(FULL, (unsigned)ncols);
         SWQ_SET_SEG()
         c = -2 * t;
         d_cur = (t == 0 && ncols > 0) ? (((uint32_t)__ldg(col) >> (8 * half)) & 0xffu)
@@ -373,6 +386,7 @@ __device__ __forceinline__ void run_qpairs(const QpArgs& a, const uint4* prof, i
         uint32_t h_in = __shfl_up_sync(FULL, out_h, 1, T);
         uint32_t f_in = __shfl_up_sync(FULL, out_f, 1, T);
         const uint32_t acc_in = __shfl_up_sync(FULL, acc_out, 1, T);
+        const int warp_next = (G > 1) ? __shfl_sync(FULL, next, 0) : next;
         const uint32_t d_in = d_cur;
         {
             const int c1 = c + 1;
@@ -380,8 +394,8 @@ __device__ __forceinline__ void run_qpairs(const QpArgs& a, const uint4* prof, i
                                              : (uint32_t)kZeroCode;
         }
         if (t == 0) {
-            h_in = Z;
-            f_in = Z;
+            h_in = HZ;
+            f_in = FZ;
             if (has_in && c < ncols) {
                 h_in = bq0.x;
                 f_in = bq0.y;
@@ -389,12 +403,12 @@ __device__ __forceinline__ void run_qpairs(const QpArgs& a, const uint4* prof, i
                 if (c + 2 < ncols) bq1 = rrow[2 * (c + 2)];
             }
             // the next unit's pair entry, once its claim has returned
-            if (pass == 0 && c == (nst < 9 ? nst - 1 : 8) && next < units)
-                ninfo = a.pairs[a.pair_begin + (next >> 1)];
+            if (pass == 0 && c == (nst < 9 ? nst - 1 : 8) && warp_next < units)
+                ninfo = a.pairs[a.pair_begin + (min(warp_next + grp, units - 1) >> 1)];
         }
         // a lane whose query starts here takes nothing from above
-        h_in = (h_in & ~reset) | (Z & reset);
-        f_in = (f_in & ~reset) | (Z & reset);
+        h_in = (h_in & ~reset) | (HZ & reset);
+        f_in = (f_in & ~reset) | (FZ & reset);
         if (!fin && c >= 0) {
             column_step_qp<R, JSTRIDE>(H, E, prof_t + (int)d_in * SLOTS,
                                        prof_b + (int)d_bot * SLOTS, prev_h, f_in, mid_h, mid_f,
@@ -412,19 +426,19 @@ __device__ __forceinline__ void run_qpairs(const QpArgs& a, const uint4* prof, i
             // the bottom has just done the finished segment's last column:
             // per lane, this thread's maximum joins its query's chain
             fpend = false;
-            uint32_t m = __vimax3_s16x2(S_pend, S_bot, Z);
+            uint32_t m = __vimax3_s16x2(S_pend, S_bot, HZ);
             const uint32_t cont = (t > 0) ? ~f_reset : 0u;
-            m = __vimax3_s16x2(m, (acc_in & cont) | (Z & ~cont), Z);
+            m = __vimax3_s16x2(m, (acc_in & cont) | (HZ & ~cont), HZ);
             acc_out = m;
             const int gp = a.pair_ids ? (int)a.pair_ids[a.pair_begin + (f_unit >> 1)]
                                       : a.pair_begin + (f_unit >> 1);
             const int pos = 2 * gp + (f_unit & 1);
-            if (pos < a.n_records) {
+            if (pos < a.n_records && f_unit < units) {
                 if (fq_lo >= 0 && (f_last & 0xffffu)) {
                     const int s0 = lo16(m);
                     const int qb = fq_lo * a.n_records;
                     atomicMax(a.scores + qb + pos, s0 - bias);
-                    if (s0 >= a.ovf_thresh) {
+                    if (s0 >= ovf_thresh) {
                         const int j = atomicAdd(a.ovf_count, 1);
                         if (j < a.ovf_cap) a.ovf_list[j] = qb + pos;
                     }
@@ -433,20 +447,20 @@ __device__ __forceinline__ void run_qpairs(const QpArgs& a, const uint4* prof, i
                     const int s1 = hi16(m);
                     const int qb = fq_hi * a.n_records;
                     atomicMax(a.scores + qb + pos, s1 - bias);
-                    if (s1 >= a.ovf_thresh) {
+                    if (s1 >= ovf_thresh) {
                         const int j = atomicAdd(a.ovf_count, 1);
                         if (j < a.ovf_cap) a.ovf_list[j] = qb + pos;
                     }
                 }
             }
-            S_bot = Z;
-            if (unit >= units) fin = true;
+            S_bot = HZ;
+            if (unit - grp >= units) fin = true;
         }
         if (c == 0) {   // the bottom starts this segment's column 0 next step
 #pragma unroll
             for (int k = HALF; k < R; ++k) {
-                H[k] = Z;
-                E[k] = Z;
+                H[k] = HZ;
+                E[k] = FZ;
             }
         }
         const bool adv = !fin && c == nst - 1;
@@ -454,9 +468,12 @@ __device__ __forceinline__ void run_qpairs(const QpArgs& a, const uint4* prof, i
             const int up_unit = __shfl_up_sync(FULL, unit, 1, T);
             const uint32_t up_off = __shfl_up_sync(FULL, off16, 1, T);
             const int up_ncols = __shfl_up_sync(FULL, ncols, 1, T);
+            const int up_wcols = (G > 1) ? __shfl_up_sync(FULL, wcols, 1, T) : up_ncols;
+            const int next_wcols = (G > 1) ? (int)__reduce_max_sync(FULL, t == 0 ? ninfo.ncols : 0u)
+                                           : (int)ninfo.ncols;
             if (adv) {
                 S_pend = S_top;
-                S_top = Z;
+                S_top = HZ;
                 f_unit = unit;
                 fq_lo = q_lo;
                 fq_hi = q_hi;
@@ -468,29 +485,36 @@ __device__ __forceinline__ void run_qpairs(const QpArgs& a, const uint4* prof, i
                 } else {
                     pass = 0;
                     if (t == 0) {
-                        unit = next;
+                        unit = warp_next + grp;
                         off16 = ninfo.off16;
                         ncols = (int)ninfo.ncols;
-                        if (unit < units) next = claim();
+                        wcols = next_wcols;
+                        if (lane == 0 && warp_next < units) next = claim();
                     } else {
                         unit = up_unit;
                         off16 = up_off;
                         ncols = up_ncols;
+                        wcols = up_wcols;
                     }
-                    if (unit >= units) ncols = 0;
-                    half = unit & 1;
+                    if (unit - grp >= units) {
+                        ncols = 0;
+                        wcols = 0;
+                    }
+                    half = min(unit, units - 1) & 1;
                 }
                 SWQ_SET_SEG()
                 c = -1;
 #pragma unroll
                 for (int k = 0; k < HALF; ++k) {
-                    H[k] = Z;
-                    E[k] = Z;
+                    H[k] = HZ;
+                    E[k] = FZ;
                 }
-                prev_h = Z;
-                if (t == 0 && has_in) {
-                    if (ncols > 0) bq0 = rrow[0];
-                    if (ncols > 1) bq1 = rrow[2];
+                prev_h = HZ;
+                if (t == 0) {
+                    bq0 = make_uint2(HZ, FZ);
+                    bq1 = bq0;
+                    if (has_in && ncols > 0) bq0 = rrow[0];
+                    if (has_in && ncols > 1) bq1 = rrow[2];
                 }
                 d_cur = (ncols > 0) ? (((uint32_t)__ldg(col) >> (8 * half)) & 0xffu)
                                     : (uint32_t)kZeroCode;
@@ -510,36 +534,41 @@ __device__ __forceinline__ void run_qpairs(const QpArgs& a, const uint4* prof, i
             }
             k = (int)__reduce_min_sync(FULL, (unsigned)k);
             const bool rd0 = t == 0 && has_in;
-            const bool z0 = t == 0 && !has_in;
             const bool wr = t == T - 1 && wlim > 0;
-            const uint32_t keep = ~reset, zr = Z & reset;
+            const uint32_t keep = ~reset, zr = HZ & reset, zf = FZ & reset;
             const uint8_t* colb = reinterpret_cast<const uint8_t*>(col) + half;
-            for (; k > 0; --k) {
-                __syncwarp();
-                uint32_t h_in = __shfl_up_sync(FULL, out_h, 1, T);
-                uint32_t f_in = __shfl_up_sync(FULL, out_f, 1, T);
-                const uint32_t d_in = d_cur;
-                d_cur = (uint32_t)__ldg(colb + 2 * (c + 1));
-                if (rd0) {
-                    h_in = bq0.x;
-                    f_in = bq0.y;
-                    bq0 = bq1;
-                    bq1 = rrow[2 * (c + 2)];
+            // thread 0 takes the row above from bq0 (the zero row where there
+            // is none): a branch in this loop costs more than the selects
+            auto plain_steps = [&](auto with_bnd) {
+                constexpr bool BND = decltype(with_bnd)::value;
+#pragma unroll 2
+                for (; k > 0; --k) {
+                    if (BND) __syncwarp();
+                    uint32_t h_in = __shfl_up_sync(FULL, out_h, 1, T);
+                    uint32_t f_in = __shfl_up_sync(FULL, out_f, 1, T);
+                    const uint32_t d_in = d_cur;
+                    d_cur = (uint32_t)__ldg(colb + 2 * (c + 1));
+                    h_in = t == 0 ? (BND ? bq0.x : HZ) : h_in;
+                    f_in = t == 0 ? (BND ? bq0.y : FZ) : f_in;
+                    if (BND) {
+                        bq0 = bq1;
+                        if (rd0) bq1 = rrow[2 * (c + 2)];
+                    }
+                    h_in = (h_in & keep) | zr;
+                    f_in = (f_in & keep) | zf;
+                    column_step_qp<R, JSTRIDE>(H, E, prof_t + (int)d_in * SLOTS,
+                                               prof_t + (int)d_bot * SLOTS, prev_h, f_in, mid_h,
+                                               mid_f, out_h, out_f, S_top, S_bot, K);
+                    if (BND && wr) wrow[2 * (c - 1)] = make_uint2(out_h, out_f);
+                    prev_h = h_in;
+                    d_bot = d_in;
+                    ++c;
                 }
-                if (z0) {
-                    h_in = Z;
-                    f_in = Z;
-                }
-                h_in = (h_in & keep) | zr;
-                f_in = (f_in & keep) | zr;
-                column_step_qp<R, JSTRIDE>(H, E, prof_t + (int)d_in * SLOTS,
-                                           prof_t + (int)d_bot * SLOTS, prev_h, f_in, mid_h,
-                                           mid_f, out_h, out_f, S_top, S_bot, K);
-                if (wr) wrow[2 * (c - 1)] = make_uint2(out_h, out_f);
-                prev_h = h_in;
-                d_bot = d_in;
-                b_col = c;
-                ++c;
+            };
+            if (k > 0) {
+                if (one_pass) plain_steps(Flag<false>{});
+                else plain_steps(Flag<true>{});
+                b_col = c - 1;
             }
         }
     }
@@ -553,10 +582,11 @@ __device__ __forceinline__ void run_qpairs(const QpArgs& a, const uint4* prof, i
 // work starts the rest earlier); then the blocks walk the double stacks in
 // order, claiming the other units.  The kernel holds no static shared memory
 // (the host gives the dynamic profile the whole opt-in maximum).
-template <int T, int R, int BLOCK>
+template <int T, int R, int BLOCK, class CELL>
 __global__ void __launch_bounds__(BLOCK, 1) sw_qpbatch(const QpArgs a) {
     extern __shared__ uint4 prof4[];
     constexpr int G = BLOCK / T;
+    const CELL K(a.gap_oe, a.gap_e);
     const int units = 2 * a.pair_count;
     const int n_long = min(a.long_units, units);
     int cur = -1;               // the double stack whose profile is in shared memory
@@ -565,7 +595,8 @@ __global__ void __launch_bounds__(BLOCK, 1) sw_qpbatch(const QpArgs a) {
         const int P = (rows + T * R - 1) / (T * R);
         if (i != cur) {
             build_profile_qp<T, R>(prof4, a.codes + a.off_lo[i], (int)a.rows_lo[i],
-                                   a.codes + a.off_hi[i], (int)a.rows_hi[i], a.mat, P);
+                                   a.codes + a.off_hi[i], (int)a.rows_hi[i], a.mat, P,
+                                   K.profile_bias());
             cur = i;
         }
         __syncthreads();
@@ -577,9 +608,10 @@ __global__ void __launch_bounds__(BLOCK, 1) sw_qpbatch(const QpArgs a) {
         for (int it = (int)blockIdx.x; it < items; it += (int)gridDim.x) {
             __syncthreads();    // every group is done with the previous item
             const int i = it / per;
-            const int u = (it - i * per) * G + (int)threadIdx.x / T;
+            // (a warp's first unit)
+            const int u = (it - i * per) * G + (int)(threadIdx.x >> 5) * (32 / T);
             const int P = stage(i);
-            run_qpairs<T, R>(a, prof4, P, nullptr, a.rb_map + a.rb_off[i],
+            run_qpairs<T, R>(a, prof4, K, P, nullptr, a.rb_map + a.rb_off[i],
                              a.seg_flags ? a.seg_flags[i] : 0u,
                              a.seg_slot ? (size_t)a.seg_slot[i] * a.seg_stride : (size_t)0, 0,
                              n_long, u);
@@ -588,7 +620,7 @@ __global__ void __launch_bounds__(BLOCK, 1) sw_qpbatch(const QpArgs a) {
     for (int i = 0; i < a.nstacks; ++i) {
         __syncthreads();        // every group is done with the previous profile
         const int P = stage(i);
-        run_qpairs<T, R>(a, prof4, P, a.counters + i, a.rb_map + a.rb_off[i],
+        run_qpairs<T, R>(a, prof4, K, P, a.counters + i, a.rb_map + a.rb_off[i],
                          a.seg_flags ? a.seg_flags[i] : 0u,
                          a.seg_slot ? (size_t)a.seg_slot[i] * a.seg_stride : (size_t)0, n_long,
                          units, 0);

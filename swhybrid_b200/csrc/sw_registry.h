@@ -30,7 +30,7 @@ const WfKernel* wf_kernels(int* n);
 // Paired-query batched kernel shapes (sw_qp.cu).
 struct QpKernel {
     int T, R, block;
-    const void* fn;                // __global__ sw_qpbatch<T, R, block>
+    const void* fn[kPlainCells];   // __global__ sw_qpbatch<T, R, block, cell> (kCellWide: as kCellNarrow)
     size_t (*smem)(int rows);      // shared memory for a double stack of `rows` rows
 };
 const QpKernel* qp_kernels(int* n);

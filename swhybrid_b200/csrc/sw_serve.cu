@@ -429,7 +429,7 @@ sw_status enqueue_round(sw_ctx* ctx, sw_serve_state* s, int chunk, int buf,
         const size_t smem = qk->smem((int)std::max<uint32_t>(L.max_rows, 1));
         int occq = 0;
         if (smem > (size_t)ctx->max_smem ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occq, qk->fn, qk->block, smem) !=
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occq, qk->fn[ctx->cell], qk->block, smem) !=
                 cudaSuccess) {
             cudaGetLastError();
             occq = 0;
@@ -478,7 +478,7 @@ sw_status enqueue_round(sw_ctx* ctx, sw_serve_state* s, int chunk, int buf,
                                      pair_count, s->chunk_cols[(size_t)chunk],
                                      (long long)occq * ctx->num_sms * (qk->block / qk->T));
         void* qargs[] = {&q};
-        SW_CUDA(ctx, cudaLaunchKernel(qk->fn, dim3((unsigned)(occq * ctx->num_sms)),
+        SW_CUDA(ctx, cudaLaunchKernel(qk->fn[ctx->cell], dim3((unsigned)(occq * ctx->num_sms)),
                                       dim3(qk->block), qargs, smem, st));
         ++*launches;
     }
@@ -908,7 +908,7 @@ extern "C" sw_status sw_serve_start(sw_ctx* ctx, const sw_serve_options* opt) {
         int occq = 0;
         const size_t smem_seg = qk->smem((int)s->pair_seg);
         if (smem_seg > (size_t)ctx->max_smem ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occq, qk->fn, qk->block, smem_seg) !=
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occq, qk->fn[ctx->cell], qk->block, smem_seg) !=
                 cudaSuccess ||
             occq <= 0) {
             cudaGetLastError();
@@ -917,7 +917,7 @@ extern "C" sw_status sw_serve_start(sw_ctx* ctx, const sw_serve_options* opt) {
             SW_SET(ctx, SW_ERR_UNSUPPORTED, "paired shape %dx%d cannot hold a lane of %u rows",
                    qk->T, qk->R, seg);
         }
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&s->occ_qp_max, qk->fn, qk->block,
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&s->occ_qp_max, qk->fn[ctx->cell], qk->block,
                                                       qk->smem(qk->T * qk->R));
         s->qk = qk;
     }
