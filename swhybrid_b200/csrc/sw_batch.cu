@@ -14,6 +14,8 @@
 //     device counter per stack), plus, when a cut-over is set, a concurrent
 //     launch of single-warp blocks for the pairs longer than the cut-over, so
 //     their inherently serial column steps overlap the bulk;
+//   * the paired-query launches' too-long records, if any, go to sw_long_items
+//     on the side stream, on SMs the first of those launches leaves free;
 //   * one 32-bit re-score launch for every flagged (query, record) and one
 //     top-k round sequence with a grid row per query.
 // The whole sequence (query upload, launches, result download) is captured
@@ -210,11 +212,11 @@ int seg_regions_for(sw_ctx* ctx, sw_batch_state* b, int want) {
 //   qp_rb_map[...] (16-byte aligned)            int2
 struct MetaLayout {
     size_t qoff, qlen, soff, srows, rboff, rbmap, qp_off_lo, qp_rows_lo, qp_off_hi, qp_rows_hi,
-        qp_rboff, qp_flags, qp_slot, qp_rbmap, codes, total;
+        qp_rboff, qp_flags, qp_slot, qp_rbmap, items, codes, total;
     int nst, nqp;
 };
 
-MetaLayout meta_layout(uint32_t nq, const StackPlan& sp) {
+MetaLayout meta_layout(uint32_t nq, const StackPlan& sp, size_t n_items) {
     MetaLayout m;
     const size_t ns = sp.off.size(), nqp = sp.qp_off_lo.size();
     m.nst = (int)ns;
@@ -233,14 +235,15 @@ MetaLayout meta_layout(uint32_t nq, const StackPlan& sp) {
     m.qp_flags = m.qp_rboff + 4 * nqp;
     m.qp_slot = m.qp_flags + 4 * nqp;
     m.qp_rbmap = (m.qp_slot + 4 * nqp + 15) / 16 * 16;
-    m.codes = m.qp_rbmap + 4 * sp.qp_rb_map.size();
+    m.items = (m.qp_rbmap + 4 * sp.qp_rb_map.size() + 7) / 8 * 8;
+    m.codes = m.items + 8 * n_items;
     m.total = (m.codes + sp.codes.size() + 15) / 16 * 16;
     return m;
 }
 
 sw_status enqueue_batch(sw_ctx* ctx, sw_batch_state* b, uint32_t nq, size_t qbytes,
                         const MetaLayout& ml, const std::vector<BatchLaunch>& launches,
-                        bool want_scores, uint32_t* n_launch) {
+                        const LongItemPlan& lplan, bool want_scores, uint32_t* n_launch) {
     cudaStream_t st = ctx->stream;
     const int n_rec = (int)ctx->n_records;
     const int k = ctx->params.top_k;
@@ -251,7 +254,7 @@ sw_status enqueue_batch(sw_ctx* ctx, sw_batch_state* b, uint32_t nq, size_t qbyt
     SW_CUDA(ctx, cudaMemcpyAsync(b->d_meta, b->h_stage + meta_at, ml.total,
                                  cudaMemcpyHostToDevice, st));
     const int nst = ml.nst;
-    SW_CUDA(ctx, cudaMemsetAsync(b->d_counters, 0, (2 * (size_t)nst + 1 + ml.nqp) * sizeof(int),
+    SW_CUDA(ctx, cudaMemsetAsync(b->d_counters, 0, (2 * (size_t)nst + 1 + ml.nqp + kLongBuckets) * sizeof(int),
                                  st));
     SW_CUDA(ctx, cudaMemsetAsync(b->d_scores, 0, (size_t)nq * n_rec * sizeof(int), st));
     const uint32_t* d_qoff = reinterpret_cast<const uint32_t*>(b->d_meta + ml.qoff);
@@ -264,13 +267,23 @@ sw_status enqueue_batch(sw_ctx* ctx, sw_batch_state* b, uint32_t nq, size_t qbyt
     int* d_ovf_count = b->d_counters + 2 * nst;
     const int ovf_thresh = 32767 - std::max(ctx->max_score, 1) + 1;
     bool forked = false;
+    if (lplan.n_long > 0) {
+        SW_CUDA(ctx, cudaEventRecord(ctx->fork_ev, st));
+        SW_CUDA(ctx, cudaStreamWaitEvent(ctx->side_stream, ctx->fork_ev, 0));
+        forked = true;
+        const sw_status ls = launch_long_items(
+            ctx, ctx->side_stream, lplan, reinterpret_cast<const uint2*>(b->d_meta + ml.items),
+            b->d_counters + 2 * nst + 1 + ml.nqp, b->d_queries, d_qoff, d_qlen, b->d_scores, b->d_ovf,
+            d_ovf_count, (int)std::min<size_t>(b->ovf_cap, (size_t)INT32_MAX), n_launch);
+        if (ls != SW_OK) return ls;
+    }
     for (const BatchLaunch& L : launches) {
         if (L.qk) {      // paired queries: main stream, the bulk half of the boundary rows
             QpArgs q;
             q.db = ctx->d_db;
             q.pairs = ctx->d_pairs;
-            q.pair_begin = 0;
-            q.pair_count = (int)ctx->n_pairs;
+            q.pair_begin = L.pair_begin;
+            q.pair_count = L.pair_count;
             q.codes = d_codes;
             q.off_lo = reinterpret_cast<const uint32_t*>(b->d_meta + ml.qp_off_lo) + L.sbegin;
             q.rows_lo = reinterpret_cast<const uint32_t*>(b->d_meta + ml.qp_rows_lo) + L.sbegin;
@@ -540,6 +553,7 @@ extern "C" sw_status sw_search_batch(sw_ctx* ctx, uint32_t nq, const uint8_t* qu
     }
     // host image of every stack: row codes and the (pass, thread) -> query map
     StackPlan sp;
+    LongItemPlan lplan;
     std::vector<BatchLaunch> launches;
     size_t bnd_long = 0, bnd_bulk = 0;
     int nst_total = 0;
@@ -686,6 +700,24 @@ extern "C" sw_status sw_search_batch(sw_ctx* ctx, uint32_t nq, const uint8_t* qu
                         groups.back().push_back({(uint32_t)tall[i], lv, (uint32_t)(i - w0)});
             }
         }
+        // the records too long for these launches, if any
+        std::vector<QpLoad> loads;
+        for (const auto& grp : groups) {
+            if (grp.empty()) continue;
+            QpLoad load;
+            for (const auto& e : grp) {
+                const Double& D = dbl[e[0]];
+                const uint32_t at = e[1] * seg, h = std::max(D.rows[0], D.rows[1]);
+                const double P = h > at ? (std::min(seg, h - at) + pass_rows - 1) / pass_rows : 1.0;
+                load.sum_passes += P;
+                load.max_passes = std::max(load.max_passes, P);
+            }
+            loads.push_back(load);
+        }
+        std::vector<uint32_t> lq(nq, 0);
+        for (uint32_t i = ip; i < nz; ++i) lq[order[i]] = qlen[order[i]];
+        lplan = plan_long_items(ctx, lq, loads, qk->block / qk->T, (int)pass_rows, 1.0, -1);
+        bool first_launch = true;
         for (const auto& grp : groups) {
             if (grp.empty()) continue;
             const int first = (int)sp.qp_off_lo.size();
@@ -725,16 +757,18 @@ extern "C" sw_status sw_search_batch(sw_ctx* ctx, uint32_t nq, const uint8_t* qu
             L.qk = qk;
             L.k = nullptr;
             L.threads = qk->block;
-            L.grid = occ * ctx->num_sms;
+            // the first launch leaves the long pairs' launches their SMs
+            L.grid = occ * (ctx->num_sms - (first_launch ? lplan.sms : 0));
+            first_launch = false;
             L.smem = smem;
             L.sbegin = first;
             L.scount = (int)sp.qp_off_lo.size() - first;
-            L.pair_begin = 0;
-            L.pair_count = (int)ctx->n_pairs;
+            L.pair_begin = (int)lplan.n_long;
+            L.pair_count = (int)(ctx->n_pairs - lplan.n_long);
             L.counter_base = 2 * nst_total + 1 + first;
             L.long_part = false;
             L.bnd_group = 2 * (size_t)ctx->max_cols;
-            L.long_units = qp_long_units(
+            L.long_units = lplan.n_long > 0 ? 0 : qp_long_units(
                 [&](int p) { return (uint64_t)ctx->pair_ncols[(size_t)p]; },
                 (int)ctx->n_pairs, ctx->pair_cols_total,
                 (long long)L.grid * (L.threads / qk->T));
@@ -743,8 +777,9 @@ extern "C" sw_status sw_search_batch(sw_ctx* ctx, uint32_t nq, const uint8_t* qu
         }
     }
     // counters: bulk of stack i at [i], long at [nst_total + i], overflow count
-    // at [2 nst_total], paired double stack j at [2 nst_total + 1 + j]
-    const MetaLayout ml = meta_layout(nq, sp);
+    // at [2 nst_total], paired double stack j at [2 nst_total + 1 + j], then the
+    // long items' per row count
+    const MetaLayout ml = meta_layout(nq, sp, lplan.count());
 
     // ---- buffers (before any capture) ----
     const long long nblk0 = std::max<long long>(1, ((long long)n_rec + kTopkKeys - 1) / kTopkKeys);
@@ -756,7 +791,7 @@ extern "C" sw_status sw_search_batch(sw_ctx* ctx, uint32_t nq, const uint8_t* qu
         }
         b->graphs.clear();
     };
-    const size_t counters_need = 2 * (size_t)nst_total + 1 + ml.nqp;
+    const size_t counters_need = 2 * (size_t)nst_total + 1 + ml.nqp + kLongBuckets;
     if (std::max<uint64_t>(qbytes, 1) > b->queries_cap || ml.total > b->meta_cap ||
         counters_need > b->counters_cap)
         drop_graphs();
@@ -841,6 +876,11 @@ extern "C" sw_status sw_search_batch(sw_ctx* ctx, uint32_t nq, const uint8_t* qu
         memcpy(m + ml.qp_flags, sp.qp_flags.data(), 4 * nqp);
         memcpy(m + ml.qp_slot, sp.qp_slot.data(), 4 * nqp);
         memcpy(m + ml.qp_rbmap, sp.qp_rb_map.data(), 4 * sp.qp_rb_map.size());
+        uint8_t* at = m + ml.items;
+        for (const auto& v : lplan.items) {
+            memcpy(at, v.data(), 4 * v.size());
+            at += 4 * v.size();
+        }
         memcpy(m + ml.codes, sp.codes.data(), sp.codes.size());
     }
 
@@ -865,7 +905,8 @@ extern "C" sw_status sw_search_batch(sw_ctx* ctx, uint32_t nq, const uint8_t* qu
             BatchGraph g;
             SW_CUDA(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
             sw_status es =
-                enqueue_batch(ctx, b, nq, qbytes, ml, launches, scores != nullptr, &g.launches);
+                enqueue_batch(ctx, b, nq, qbytes, ml, launches, lplan, scores != nullptr,
+                              &g.launches);
             cudaGraph_t graph = nullptr;
             const cudaError_t ce = cudaStreamEndCapture(ctx->stream, &graph);
             if (es != SW_OK) {
@@ -886,7 +927,7 @@ extern "C" sw_status sw_search_batch(sw_ctx* ctx, uint32_t nq, const uint8_t* qu
         SW_CUDA(ctx, cudaGraphLaunch(it->second.exec, ctx->stream));
         n_launch = it->second.launches;
     } else {
-        s = enqueue_batch(ctx, b, nq, qbytes, ml, launches, scores != nullptr, &n_launch);
+        s = enqueue_batch(ctx, b, nq, qbytes, ml, launches, lplan, scores != nullptr, &n_launch);
         if (s != SW_OK) return s;
     }
     SW_CUDA(ctx, cudaEventRecord(ctx->ev[1], ctx->stream));

@@ -234,6 +234,9 @@ extern "C" sw_status sw_ctx_create(int device, const sw_params* params, sw_ctx**
     const LongKernel* lks = long_kernels(&nk);
     for (int i = 0; i < nk; ++i)
         if (!allow_smem(lks[i].fn[ctx->cell])) return fail(SW_ERR_CUDA);
+    const LongItemKernel* liks = long_item_kernels(&nk);
+    for (int i = 0; i < nk; ++i)
+        if (!allow_smem(liks[i].fn[ctx->cell])) return fail(SW_ERR_CUDA);
     *out = ctx;
     return SW_OK;
 }
@@ -1005,6 +1008,155 @@ Split plan_split(sw_ctx* ctx, int qlen, const WfKernel* given) {
         if (last) break;
     }
     return best;
+}
+
+// ---- long pairs of a batch or a serving round -----------------------------
+//
+// A paired-query launch scores every record of every double stack, so a record
+// whose columns exceed a group's share of its smallest launch holds the whole
+// launch, once per segment level of the tall stacks (48 requests against 57,000
+// records with 20 of 10,000..35,000 residues: 100 ms a round, 25 of them work).
+// The pairs above a cut-over go to sw_long_items instead, beside the launches.
+
+// Clocks of the paired launches on `sms` SMs, longest record `longest`: a
+// group's step takes as long as the SM's groups at 23.5 cells per clock.
+static double qp_clocks(const std::vector<QpLoad>& loads, double cols, double longest, double groups,
+                        int rows_per_pass, double sms) {
+    const double step = groups * rows_per_pass * 2.0 / 23.5;
+    double t = 0;
+    for (const QpLoad& l : loads)
+        t += std::max(l.sum_passes * 2.0 * cols / (groups * sms), l.max_passes * longest) * step + 20e3;
+    return t;
+}
+
+static int long_bucket(uint32_t qlen) {
+    int n = 0;
+    const LongItemKernel* k = long_item_kernels(&n);
+    for (int i = 0; i < n; ++i)
+        if (qlen <= (uint32_t)(32 * k[i].R * kLongItemWarps)) return i;
+    return -1;
+}
+
+LongItemPlan plan_long_items(sw_ctx* ctx, const std::vector<uint32_t>& qlen,
+                             const std::vector<QpLoad>& loads, int groups_per_sm, int rows_per_pass,
+                             double chunks, int64_t given) {
+    LongItemPlan plan;
+    const int64_t np = ctx->n_pairs;
+    int nk = 0;
+    const LongItemKernel* lk = long_item_kernels(&nk);
+    if (np == 0 || nk != kLongBuckets) return plan;
+    // per pair column: SM clocks of all queries, and the slowest query's step
+    double per_col = 0, slow = 0;
+    for (const uint32_t q : qlen) {
+        if (q == 0) continue;
+        const int b = long_bucket(q);
+        if (b < 0) return plan;                      // too long for a block's warps
+        const int P = (int)((q + 32 * lk[b].R - 1) / (32 * lk[b].R));
+        const int G = kLongItemWarps / P;
+        const double step = long_step_clocks(lk[b].R, P * G);
+        per_col += step / G;
+        slow = std::max(slow, step);
+    }
+    if (per_col == 0) return plan;
+    const double total = (double)ctx->pair_cols_total / chunks, longest = ctx->pair_ncols[0];
+    const int sms = ctx->num_sms;
+    if (given < 0) {
+        double best = 0.95 * qp_clocks(loads, total, longest, groups_per_sm, rows_per_pass, sms);
+        int64_t prev = 0;
+        for (double cut = longest * 0.95; cut >= 256.0; cut /= 1.4) {
+            const int64_t n = std::partition_point(ctx->pair_ncols.begin(), ctx->pair_ncols.end(),
+                                                   [cut](uint32_t c) { return c > cut; }) -
+                              ctx->pair_ncols.begin();
+            if (n == prev || n == np) continue;
+            prev = n;
+            if (n > 16384) break;
+            const double cols = (double)ctx->pair_prefix[n];
+            for (const int x : {2, 4, 8, 12, 16, 24, 32, 48, 64, 80, 96}) {
+                const double tl = std::max(slow * longest, per_col * cols / x) +
+                                  0.3 * std::min(slow * longest, per_col * cols / x);
+                const double tb = qp_clocks(loads, total - cols / chunks, ctx->pair_ncols[n],
+                                            groups_per_sm, rows_per_pass, sms - x);
+                if (std::max(tl, tb) < best) {
+                    best = std::max(tl, tb);
+                    plan.n_long = n;
+                    plan.sms = x;
+                }
+            }
+        }
+    } else if (given > 0) {
+        // the pairs are given: SMs in proportion to the work
+        plan.n_long = given;
+        const double wl = per_col * (double)ctx->pair_prefix[given];
+        const double wb = qp_clocks(loads, total, 0.0, groups_per_sm, rows_per_pass, 1.0);
+        plan.sms = std::max(1, std::min(sms * 2 / 3, (int)std::lround(sms * wl / (wl + wb))));
+    }
+    if (plan.n_long == 0) return plan;
+    struct Item {
+        uint32_t q, pair;
+        double t;
+    };
+    std::vector<Item> list[kLongBuckets];
+    for (uint32_t q = 0; q < (uint32_t)qlen.size(); ++q) {
+        if (qlen[q] == 0) continue;
+        const int b = long_bucket(qlen[q]);
+        const int P = (int)((qlen[q] + 32 * lk[b].R - 1) / (32 * lk[b].R)), G = kLongItemWarps / P;
+        plan.smem[b] = std::max(plan.smem[b], lk[b].smem(P, G));
+        for (int64_t p = 0; p < plan.n_long; p += G)
+            list[b].push_back(Item{q, (uint32_t)p, ctx->pair_ncols[p] * long_step_clocks(lk[b].R, P * G)});
+    }
+    for (int b = 0; b < kLongBuckets; ++b) {
+        if (plan.smem[b] > (size_t)ctx->max_smem - 1024) return LongItemPlan{};
+        std::stable_sort(list[b].begin(), list[b].end(),
+                         [](const Item& x, const Item& y) { return x.t > y.t; });
+        for (const Item& i : list[b]) {
+            plan.items[b].push_back(i.q);
+            plan.items[b].push_back(i.pair);
+        }
+    }
+    return plan;
+}
+
+// The plan's launches (one per row count, longest queries first), `sms` blocks
+// each; d_items holds the buckets' items back to back.
+sw_status launch_long_items(sw_ctx* ctx, cudaStream_t stream, const LongItemPlan& plan,
+                            const uint2* d_items, int* d_counters, const uint8_t* d_queries,
+                            const uint32_t* d_qoff, const uint32_t* d_qlens, int* d_scores,
+                            int* d_ovf, int* d_ovf_count, int ovf_cap, uint32_t* launches) {
+    int nk = 0;
+    const LongItemKernel* lk = long_item_kernels(&nk);
+    size_t at[kLongBuckets], n_all = 0;
+    for (int b = 0; b < kLongBuckets; ++b) {
+        at[b] = n_all;
+        n_all += plan.items[b].size() / 2;
+    }
+    for (int b = kLongBuckets - 1; b >= 0; --b) {
+        const int n = (int)(plan.items[b].size() / 2);
+        if (n == 0) continue;
+        LongItemArgs a;
+        a.db = ctx->d_db;
+        a.pairs = ctx->d_pairs;
+        a.n_pairs = (int)plan.n_long;
+        a.items = d_items + at[b];
+        a.n_items = n;
+        a.counter = d_counters + b;
+        a.queries = d_queries;
+        a.qoff = d_qoff;
+        a.qlens = d_qlens;
+        a.mat = ctx->d_mat;
+        a.gap_oe = ctx->params.gap_open + ctx->params.gap_extend;
+        a.gap_e = ctx->params.gap_extend;
+        a.scores = d_scores;
+        a.n_records = (int)ctx->n_records;
+        a.ovf_list = d_ovf;
+        a.ovf_count = d_ovf_count;
+        a.ovf_thresh = 32767 - std::max(ctx->max_score, 1) + 1;
+        a.ovf_cap = ovf_cap;
+        void* args[] = {&a};
+        SW_CUDA(ctx, cudaLaunchKernel(lk[b].fn[ctx->cell], dim3((unsigned)std::min(n, plan.sms)),
+                                      dim3(32 * kLongItemWarps), args, plan.smem[b], stream));
+        ++*launches;
+    }
+    return SW_OK;
 }
 
 // How a plain search of qlen divides the DB's pairs: all to one bulk shape; the

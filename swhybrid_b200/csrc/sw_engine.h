@@ -127,6 +127,33 @@ struct sw_ctx {
 };
 
 namespace swb {
+// Long pairs of a batch or a serving round, scored by sw_long_items beside the
+// paired-query launches.
+struct QpLoad {                        // a paired-query launch: passes of its double stacks
+    double sum_passes = 0, max_passes = 0;
+};
+constexpr int kLongBuckets = 3;        // row counts of sw_long_items
+struct LongItemPlan {
+    int64_t n_long = 0;                // pairs [0, n_long); 0: no split
+    int sms = 0;                       // SMs the first paired launch leaves free
+    std::vector<uint32_t> items[kLongBuckets];   // (query, first pair) per row count
+    size_t smem[kLongBuckets] = {};
+    size_t count() const {
+        size_t n = 0;
+        for (const auto& v : items) n += v.size() / 2;
+        return n;
+    }
+};
+// The split of the pairs for queries of the given lengths (0: none), or of
+// `n_long` pairs when that is >= 0.  cols, units: columns and pairs of the
+// paired launches without a split (a serving round sees one chunk of them).
+LongItemPlan plan_long_items(sw_ctx* ctx, const std::vector<uint32_t>& qlen,
+                             const std::vector<QpLoad>& loads, int groups_per_sm, int rows_per_pass,
+                             double chunks, int64_t n_long);
+sw_status launch_long_items(sw_ctx* ctx, cudaStream_t stream, const LongItemPlan& plan,
+                            const uint2* d_items, int* d_counters, const uint8_t* d_queries,
+                            const uint32_t* d_qoff, const uint32_t* d_qlens, int* d_scores,
+                            int* d_ovf, int* d_ovf_count, int ovf_cap, uint32_t* launches);
 struct WfKernel;
 const WfKernel* find_kernel(int T, int R);
 int shape_occupancy(sw_ctx* ctx, const WfKernel& k, int qlen);   // stacked kernel

@@ -59,47 +59,43 @@ struct LongBlock {
     static constexpr int value = R <= 4 ? 768 : R <= 16 ? 512 : R <= 32 ? 384 : 256;
 };
 
+// One warp of a pipeline: query pass w of P against the pipeline's pair.
 template <int R, class CELL>
-__global__ void __launch_bounds__(LongBlock<R>::value, 1) sw_long(const LongArgs a) {
-    constexpr int T = kLT;
-    constexpr int NJ = (R + 7) / 8;
-    constexpr int SLOTS = GroupShape<T>::SLOTS;
-    constexpr int JSTRIDE = kCodes * SLOTS;
-    constexpr unsigned FULL = 0xffffffffu;
-    extern __shared__ uint2 smem[];
-    __shared__ int s_next[kLongMaxWarps];                 // per pipeline: its next pair
-    __shared__ uint32_t s_max[kLongMaxWarps];             // per warp: its pass's max
-    const int P = a.passes;                               // warps per pipeline
-    const CELL K(a.gap_oe, a.gap_e);
-    uint2* const prof = smem;
-    uint2* const ring = smem + (size_t)P * NJ * JSTRIDE;  // G pipelines x (P-1) links
-    build_profile<T, R>(prof, a.query, a.qlen, a.mat, P, K.profile_bias());
-    const int warp = (int)(threadIdx.x >> 5);
-    const int g = warp / P;                               // this warp's pipeline
-    const int w = warp - g * P;                           // ... and its pass in it
-    const int t = (int)(threadIdx.x & 31);
-    const bool leader = (w == 0 && t == 0);
-    const uint32_t HZ = K.hz(), FZ = K.fz();
-    const int bias = (int)(HZ & 0xffffu);
-    const int ovf_thresh = a.ovf_thresh - K.stored_shift();
-    const uint2* const prof_p = prof + (w * NJ) * JSTRIDE + t;
-    uint2* const links = ring + (size_t)g * (P > 1 ? P - 1 : 0) * kLRing;
-    uint2* const ring_out = links + (size_t)(w + 1 < P ? w : 0) * kLRing;       // link w -> w+1
-    const uint2* const ring_in = links + (size_t)(w > 0 ? w - 1 : 0) * kLRing;  // link w-1 -> w
-    const bool ring_wr = t == T - 1 && w + 1 < P;
-    const bool ring_rd = w > 0;
+struct LongWarp {
+    static constexpr int T = kLT;
+    static constexpr int NJ = (R + 7) / 8;
+    static constexpr int SLOTS = GroupShape<T>::SLOTS;
+    static constexpr int JSTRIDE = kCodes * SLOTS;
+    const CELL& K;
+    const int t;                          // lane
+    const uint32_t HZ, FZ;
+    const uint2* prof_p = nullptr;        // the pass's profile at this lane's slot
+    uint2* ring_out = nullptr;            // link w -> w+1
+    const uint2* ring_in = nullptr;       // link w-1 -> w
+    bool ring_wr = false, ring_rd = false;
     uint32_t H[R], E[R];
-    uint32_t S = HZ, out_h = HZ, out_f = FZ, prev_h = HZ;
-    uint2 up = make_uint2(HZ, FZ);                        // lane 0: the row above, next column
-    uint2 wa[NJ], wb[NJ];                                 // this step's profile words
-    uint32_t d = kPadPair;                                // the next step's residue pair
-    const unsigned short* col = reinterpret_cast<const unsigned short*>(a.db);
-    int pair = 0, ncols = 0, span = 0, total = 0, start = 0, c = 0;
-    bool active = false;
-    auto residue = [&](int i) {
+    uint32_t S, out_h, out_f, prev_h;
+    uint2 up;                             // lane 0: the row above, next column
+    uint2 wa[NJ], wb[NJ];                 // this step's profile words
+    uint32_t d;                           // the next step's residue pair
+    const unsigned short* col = nullptr;
+    int ncols = 0, c = 0;
+
+    __device__ __forceinline__ explicit LongWarp(const CELL& cell)
+        : K(cell), t((int)(threadIdx.x & 31)), HZ(cell.hz()), FZ(cell.fz()) {}
+
+    // links: this pipeline's P - 1 rings of kLRing columns
+    __device__ __forceinline__ void place(const uint2* prof, uint2* links, int w, int P) {
+        prof_p = prof + (w * NJ) * JSTRIDE + t;
+        ring_out = links + (size_t)(w + 1 < P ? w : 0) * kLRing;
+        ring_in = links + (size_t)(w > 0 ? w - 1 : 0) * kLRing;
+        ring_wr = t == T - 1 && w + 1 < P;
+        ring_rd = w > 0;
+    }
+    __device__ __forceinline__ uint32_t residue(int i) const {
         return i >= 0 && i < ncols ? (uint32_t)__ldg(col + i) : kPadPair;
-    };
-    auto load = [&](uint2 (&A)[NJ], uint2 (&B)[NJ], uint32_t pr) {
+    }
+    __device__ __forceinline__ void load(uint2 (&A)[NJ], uint2 (&B)[NJ], uint32_t pr) const {
         const uint2* const p0 = prof_p + (int)(pr & 0xffu) * SLOTS;
         const uint2* const p1 = prof_p + (int)((pr >> 8) & 0xffu) * SLOTS;
 #pragma unroll
@@ -107,42 +103,35 @@ __global__ void __launch_bounds__(LongBlock<R>::value, 1) sw_long(const LongArgs
             A[j] = p0[j * JSTRIDE];
             B[j] = p1[j * JSTRIDE];
         }
-    };
-    // a pipeline's pair starts at a barrier (block step `at`, a multiple of K)
-    // and lasts `total` steps, also a multiple of K
-    auto begin_pair = [&](int v, int at) {
-        pair = v;
-        active = pair < a.pair_count;
-        if (active) {
-            const Pair2 pr = a.pairs[a.pair_begin + pair];
-            ncols = (int)pr.ncols;
-            span = (ncols + T - 1 + kLK - 1) / kLK * kLK;
-            total = (P - 1) * kLD + span;
-            start = at;
+    }
+    // steps of a pass over a pair, in whole barrier intervals
+    static __device__ __forceinline__ int span_of(int ncols) {
+        return (ncols + T - 1 + kLK - 1) / kLK * kLK;
+    }
+    __device__ __forceinline__ void begin(const uint4* db, const Pair2& pr) {
+        ncols = (int)pr.ncols;
+        col = reinterpret_cast<const unsigned short*>(db) + (size_t)pr.off16 * 8;
 #pragma unroll
-            for (int k = 0; k < R; ++k) {
-                H[k] = HZ;
-                E[k] = FZ;
-            }
-            S = HZ;
-            out_h = HZ;
-            out_f = FZ;
-            prev_h = HZ;
-            col = reinterpret_cast<const unsigned short*>(a.db) + (size_t)pr.off16 * 8;
-            c = -t;
-            load(wa, wb, residue(c));
-            d = residue(c + 1);
-            up = make_uint2(HZ, FZ);
+        for (int k = 0; k < R; ++k) {
+            H[k] = HZ;
+            E[k] = FZ;
         }
-    };
-    if (leader) s_next[g] = atomicAdd(a.counter, 1);
-    __syncthreads();                                       // profile built, first claims made
-    begin_pair(s_next[g], 0);
-    // K column steps of this warp from its step s0.  INSIDE: every lane's
-    // column and the two loaded ahead lie inside the pair, and so does lane 0's
-    // next ring entry, so nothing is checked.
-    auto interval = [&](auto inside, int s0) {
-        constexpr bool INSIDE = decltype(inside)::value;
+        S = HZ;
+        out_h = HZ;
+        out_f = FZ;
+        prev_h = HZ;
+        up = make_uint2(HZ, FZ);
+        c = -t;
+        load(wa, wb, residue(c));
+        d = residue(c + 1);
+    }
+    // K column steps from step s0.  INSIDE: every lane's column and the two
+    // loaded ahead lie inside the pair, and so does lane 0's next ring entry,
+    // so nothing is checked.
+    template <bool INSIDE>
+    __device__ __forceinline__ void steps(int s0) {
+        constexpr unsigned FULL = 0xffffffffu;
+        if (!INSIDE && ring_rd && s0 == 0) up = ring_in[0];
 #pragma unroll 2
         for (int s = s0; s < s0 + kLK; ++s) {
             uint32_t h_in = __shfl_up_sync(FULL, out_h, 1);
@@ -178,25 +167,85 @@ __global__ void __launch_bounds__(LongBlock<R>::value, 1) sw_long(const LongArgs
             }
             ++c;
         }
+    }
+    // the barrier interval that starts at this warp's step s0
+    __device__ __forceinline__ void interval(int s0) {
+        if (s0 >= T && s0 + kLK + 2 <= ncols) steps<true>(s0);
+        else steps<false>(s0);
+    }
+    // the pass's maximum, in every lane
+    __device__ __forceinline__ uint32_t maximum() const {
+        uint32_t m = S;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            m = __vimax3_s16x2(m, __shfl_xor_sync(0xffffffffu, m, o), HZ);
+        return m;
+    }
+};
+
+// A finished pair's scores (lanes of m) at row + its sorted position.
+__device__ __forceinline__ void long_scores(int* scores, int row, int pos, int n_records, uint32_t m,
+                                            int bias, int thresh, int* ovf_list, int* ovf_count,
+                                            int ovf_cap) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        if (pos + i >= n_records) break;
+        const int s = i ? hi16(m) : lo16(m);
+        scores[row + pos + i] = s - bias;
+        if (s >= thresh) {
+            const int j = atomicAdd(ovf_count, 1);
+            if (j < ovf_cap) ovf_list[j] = row + pos + i;
+        }
+    }
+}
+
+// Plain search: one query, pairs claimed pipeline by pipeline.
+template <int R, class CELL>
+__global__ void __launch_bounds__(LongBlock<R>::value, 1) sw_long(const LongArgs a) {
+    using W = LongWarp<R, CELL>;
+    extern __shared__ uint2 smem[];
+    __shared__ int s_next[kLongMaxWarps];                 // per pipeline: its next pair
+    __shared__ uint32_t s_max[kLongMaxWarps];             // per warp: its pass's max
+    const int P = a.passes;                               // warps per pipeline
+    const CELL K(a.gap_oe, a.gap_e);
+    build_profile<kLT, R>(smem, a.query, a.qlen, a.mat, P, K.profile_bias());
+    const int warp = (int)(threadIdx.x >> 5);
+    const int g = warp / P;                               // this warp's pipeline
+    const int w = warp - g * P;                           // ... and its pass in it
+    W x(K);
+    x.place(smem, smem + (size_t)P * W::NJ * W::JSTRIDE + (size_t)g * (P > 1 ? P - 1 : 0) * kLRing, w,
+            P);
+    const bool leader = w == 0 && x.t == 0;
+    int pair = 0, span = 0, total = 0, start = 0;
+    bool active = false;
+    // a pipeline's pair starts at a barrier (block step `at`, a multiple of K)
+    // and lasts `total` steps, also a multiple of K
+    auto begin_pair = [&](int v, int at) {
+        pair = v;
+        active = pair < a.pair_count;
+        if (active) {
+            x.begin(a.db, a.pairs[a.pair_begin + pair]);
+            span = W::span_of(x.ncols);
+            total = (P - 1) * kLD + span;
+            start = at;
+        }
     };
+    if (leader) s_next[g] = atomicAdd(a.counter, 1);
+    __syncthreads();                                       // profile built, first claims made
+    begin_pair(s_next[g], 0);
     for (int gs = 0;;) {                                   // block step
         const int s0 = gs - start - w * kLD;               // this warp's first step of the interval
-        if (active && s0 >= 0 && s0 < span) {              // warp-uniform, whole intervals
-            if (ring_rd && s0 == 0) up = ring_in[0];
-            if (s0 >= T && s0 + kLK + 2 <= ncols) interval(Flag<true>{}, s0);
-            else interval(Flag<false>{}, s0);
-        }
+        if (active && s0 >= 0 && s0 < span) x.interval(s0);    // warp-uniform, whole intervals
         gs += kLK;
         // barrier: pipelines whose pair ends here publish their passes' maxima
         // and (leader) claim the next pair; the OR says whether any pipeline
         // still has work after this barrier
         const bool ending = active && gs - start >= total;
         bool alive = active && !ending;
+        uint32_t m = x.HZ;
         if (ending) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
-                S = __vimax3_s16x2(S, __shfl_xor_sync(FULL, S, o), HZ);
-            if (t == 0) s_max[warp] = S;
+            m = x.maximum();
+            if (x.t == 0) s_max[warp] = m;
             if (leader) {
                 const int v = atomicAdd(a.counter, 1);
                 s_next[g] = v;
@@ -206,25 +255,73 @@ __global__ void __launch_bounds__(LongBlock<R>::value, 1) sw_long(const LongArgs
         const int any = __syncthreads_or(alive ? 1 : 0);
         if (ending) {
             if (leader) {
-                for (int i = 1; i < P; ++i) S = __vimax3_s16x2(S, s_max[warp + i], HZ);
-                const int pos = 2 * (a.pair_begin + pair);
-                const int s0 = lo16(S), s1 = hi16(S);
-                a.scores[pos] = s0 - bias;
-                if (s0 >= ovf_thresh) {
-                    const int j = atomicAdd(a.ovf_count, 1);
-                    if (j < a.ovf_cap) a.ovf_list[j] = pos;
-                }
-                if (pos + 1 < a.n_records) {
-                    a.scores[pos + 1] = s1 - bias;
-                    if (s1 >= ovf_thresh) {
-                        const int j = atomicAdd(a.ovf_count, 1);
-                        if (j < a.ovf_cap) a.ovf_list[j] = pos + 1;
-                    }
-                }
+                for (int i = 1; i < P; ++i) m = __vimax3_s16x2(m, s_max[warp + i], x.HZ);
+                long_scores(a.scores, 0, 2 * (a.pair_begin + pair), a.n_records, m,
+                            (int)(x.HZ & 0xffffu), a.ovf_thresh - K.stored_shift(), a.ovf_list,
+                            a.ovf_count, a.ovf_cap);
             }
             begin_pair(s_next[g], gs);
         }
         if (!any) break;
+    }
+}
+
+// Batched search and serving: items of one query and as many neighbouring
+// pairs as a block of kLongItemWarps warps holds pipelines for (similar
+// lengths, the table being longest first), claimed longest first.
+template <int R, class CELL>
+__global__ void __launch_bounds__(32 * kLongItemWarps, 1) sw_long_items(const LongItemArgs a) {
+    using W = LongWarp<R, CELL>;
+    extern __shared__ uint2 smem[];
+    __shared__ int s_item;
+    __shared__ uint32_t s_max[kLongItemWarps];
+    const CELL K(a.gap_oe, a.gap_e);
+    const int warp = (int)(threadIdx.x >> 5);
+    int query = -1;
+    while (true) {
+        __syncthreads();                 // the previous item is done
+        if (threadIdx.x == 0) s_item = atomicAdd(a.counter, 1);
+        __syncthreads();
+        if (s_item >= a.n_items) break;
+        const uint2 item = a.items[s_item];
+        const int qlen = (int)a.qlens[item.x];
+        const int P = (qlen + 32 * R - 1) / (32 * R);
+        const int G = kLongItemWarps / P;
+        if ((int)item.x != query) {
+            query = (int)item.x;
+            build_profile<kLT, R>(smem, a.queries + a.qoff[query], qlen, a.mat, P, K.profile_bias());
+        }
+        const int g = warp / P, w = warp - g * P;
+        const int pair = (int)item.y + g;
+        const bool active = g < G && pair < a.n_pairs;
+        W x(K);
+        __syncthreads();                 // profile built
+        int span = 0;
+        if (active) {
+            x.place(smem, smem + (size_t)P * W::NJ * W::JSTRIDE + (size_t)g * (P > 1 ? P - 1 : 0) * kLRing,
+                    w, P);
+            x.begin(a.db, a.pairs[pair]);
+            span = W::span_of(x.ncols);
+        }
+        // the item's first pair is its longest
+        const int total = (P - 1) * kLD + W::span_of((int)a.pairs[item.y].ncols);
+        for (int gs = 0; gs < total; gs += kLK) {
+            const int s0 = gs - w * kLD;
+            if (active && s0 >= 0 && s0 < span) x.interval(s0);
+            __syncthreads();
+        }
+        uint32_t m = x.HZ;
+        if (active) {
+            m = x.maximum();
+            if (x.t == 0) s_max[warp] = m;
+        }
+        __syncthreads();
+        if (active && w == 0 && x.t == 0) {
+            for (int i = 1; i < P; ++i) m = __vimax3_s16x2(m, s_max[warp + i], x.HZ);
+            long_scores(a.scores, query * a.n_records, 2 * pair, a.n_records, m,
+                        (int)(x.HZ & 0xffffu), a.ovf_thresh - K.stored_shift(), a.ovf_list,
+                        a.ovf_count, a.ovf_cap);
+        }
     }
 }
 
@@ -244,11 +341,29 @@ constexpr LongKernel linst() {
                       &long_smem<R>, LongBlock<R>::value};
 }
 
+template <int R>
+constexpr LongItemKernel iinst() {
+    return LongItemKernel{R,
+                          {(const void*)&sw_long_items<R, CellWide>,
+                           (const void*)&sw_long_items<R, CellNarrow<0, 0>>,
+                           (const void*)&sw_long_items<R, CellNarrow<12, 2>>,
+                           (const void*)&sw_long_items<R, CellNarrow<12, 1>>},
+                          &long_smem<R>};
+}
+
+// kLongItemWarps passes of 32 R rows: up to 2,048, 4,096 and 8,192 query rows
+const LongItemKernel kLongItemTable[] = {iinst<4>(), iinst<8>(), iinst<16>()};
+
 const LongKernel kLongTable[] = {
     linst<4>(), linst<8>(), linst<16>(), linst<24>(), linst<32>(), linst<64>(),
 };
 
 }  // namespace
+
+const LongItemKernel* long_item_kernels(int* n) {
+    *n = (int)(sizeof(kLongItemTable) / sizeof(kLongItemTable[0]));
+    return kLongItemTable;
+}
 
 const LongKernel* long_kernels(int* n) {
     *n = (int)(sizeof(kLongTable) / sizeof(kLongTable[0]));

@@ -40,4 +40,35 @@ struct LongKernel {
 
 const LongKernel* long_kernels(int* n);
 
+// Long pairs of several queries (batched search, serving): see sw_long_items.
+constexpr int kLongItemWarps = 16;
+
+struct LongItemArgs {
+    const uint4* db;
+    const Pair2* pairs;         // the long pairs are [0, n_pairs), ncols descending
+    int n_pairs;
+    const uint2* items;         // (query, first pair), longest first
+    int n_items;
+    int* counter;               // items claimed so far
+    const uint8_t* queries;     // query q: codes at queries + qoff[q], qlens[q] of them
+    const uint32_t* qoff;
+    const uint32_t* qlens;
+    const int8_t* mat;
+    int gap_oe, gap_e;
+    int* scores;                // [query][sorted position]
+    int n_records;
+    int* ovf_list;              // query * n_records + position
+    int* ovf_count;
+    int ovf_thresh;
+    int ovf_cap;
+};
+
+struct LongItemKernel {
+    int R;
+    const void* fn[kPlainCells];
+    size_t (*smem)(int passes, int pipelines);
+};
+
+const LongItemKernel* long_item_kernels(int* n);
+
 }  // namespace swb
