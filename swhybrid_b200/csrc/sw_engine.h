@@ -132,7 +132,8 @@ namespace swb {
 struct QpLoad {                        // a paired-query launch: passes of its double stacks
     double sum_passes = 0, max_passes = 0;
 };
-constexpr int kLongBuckets = 3;        // row counts of sw_long_items
+constexpr int kLongBuckets = 3;        // row counts of sw_long_items ...
+constexpr uint32_t kLongItemRows = 8192;   // ... and the query rows the tallest holds
 struct LongItemPlan {
     int64_t n_long = 0;                // pairs [0, n_long); 0: no split
     int sms = 0;                       // SMs the first paired launch leaves free

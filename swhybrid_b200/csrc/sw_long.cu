@@ -351,7 +351,8 @@ constexpr LongItemKernel iinst() {
                           &long_smem<R>};
 }
 
-// kLongItemWarps passes of 32 R rows: up to 2,048, 4,096 and 8,192 query rows
+// kLongItemWarps passes of 32 R rows: up to 2,048, 4,096 and 8,192
+// (kLongItemRows) query rows
 const LongItemKernel kLongItemTable[] = {iinst<4>(), iinst<8>(), iinst<16>()};
 
 const LongKernel kLongTable[] = {

@@ -87,6 +87,9 @@ struct sw_serve_state {
     uint32_t max_stack_rows = 0;          // longer requests run alone (plain path)
     int occ_max = 0;                      // most blocks per SM any stack height gives
     int occ_qp_max = 0;                   // ... and any paired lane height
+    // pairs [0, n_long) are not in the ring: a request scores them in its first
+    // round, beside the paired launches (sw_long_items)
+    int64_t n_long = 0;
     std::vector<int> chunk_begin;         // n_chunks + 1 entries into d_pairs
     std::vector<uint32_t> ring_ncols;     // column count of each entry of d_pairs
     std::vector<uint64_t> chunk_cols;     // sum of ring_ncols per chunk
@@ -348,6 +351,34 @@ sw_status enqueue_round(sw_ctx* ctx, sw_serve_state* s, int chunk, int buf,
         }
     }
     const size_t ne = qp_flags.size();
+    // the long pairs of the requests admitted at this boundary
+    LongItemPlan lplan;
+    if (s->n_long > 0) {
+        std::vector<uint32_t> lq((size_t)s->n_slots, 0);
+        bool any = false;
+        for (int sl : active)
+            if (s->slots[sl].fresh) {
+                lq[(size_t)sl] = (uint32_t)s->slots[sl].req.query.size();
+                any = true;
+            }
+        std::vector<QpLoad> loads;
+        for (const QpLaunch& L : qp_launches) {
+            QpLoad load;
+            for (size_t e = L.first; e < L.first + L.count; ++e) {
+                const double P = std::max<uint32_t>(
+                    1, (std::max(qp_rows[0][e], qp_rows[1][e]) + qT * qR - 1) / (qT * qR));
+                load.sum_passes += P;
+                load.max_passes = std::max(load.max_passes, P);
+            }
+            loads.push_back(load);
+        }
+        if (any) {
+            lplan = plan_long_items(ctx, lq, loads, qk->block / qk->T, (int)(qT * qR),
+                                    (double)s->n_chunks, s->n_long);
+            if (lplan.n_long == 0)
+                SW_SET(ctx, SW_ERR_UNSUPPORTED, "long pairs of a round do not fit shared memory");
+        }
+    }
     // table layout (one upload; the paired block map is read as int2)
     size_t total = 0;
     auto place = [&total](size_t bytes, size_t align) {
@@ -363,6 +394,7 @@ sw_status enqueue_round(sw_ctx* ctx, sw_serve_state* s, int chunk, int buf,
     const size_t o_qpo1 = place(4 * ne, 4), o_qpr1 = place(4 * ne, 4), o_qprb = place(4 * ne, 4);
     const size_t o_qpfl = place(4 * ne, 4), o_qpsl = place(4 * ne, 4);
     const size_t o_qpmap = place(4 * qp_rbmap.size(), 8);
+    const size_t o_items = place(8 * lplan.count(), 8);
     const size_t o_codes = place(codes.size(), 16);
     total = (total + 15) / 16 * 16;
     if (total > s->meta_cap) {
@@ -404,6 +436,13 @@ sw_status enqueue_round(sw_ctx* ctx, sw_serve_state* s, int chunk, int buf,
         memcpy(m + o_qpsl, qp_slot.data(), 4 * ne);
         memcpy(m + o_qpmap, qp_rbmap.data(), 4 * qp_rbmap.size());
     }
+    {
+        uint8_t* at = m + o_items;
+        for (const auto& v : lplan.items) {
+            if (!v.empty()) memcpy(at, v.data(), 4 * v.size());
+            at += 4 * v.size();
+        }
+    }
     if (!codes.empty()) memcpy(m + o_codes, codes.data(), codes.size());
     SW_CUDA(ctx, cudaEventRecord(s->start_ev[buf], st));
     SW_CUDA(ctx, cudaMemcpyAsync(s->d_meta, m, total, cudaMemcpyHostToDevice, st));
@@ -413,8 +452,8 @@ sw_status enqueue_round(sw_ctx* ctx, sw_serve_state* s, int chunk, int buf,
             SW_CUDA(ctx, cudaMemsetAsync(s->d_scores + (size_t)sl * n_rec, 0,
                                          (size_t)n_rec * sizeof(int), st));
     // counters: stack i at [i], the overflow count at [ns], paired entry j at
-    // [ns + 1 + j]
-    const size_t n_counters = ns + 1 + ne;
+    // [ns + 1 + j], then the long items' per row count
+    const size_t n_counters = ns + 1 + ne + kLongBuckets;
     if (n_counters > s->counters_cap)
         SW_SET(ctx, SW_ERR_UNSUPPORTED, "%zu paired launch entries exceed the counters (%zu)", ne,
                s->counters_cap);
@@ -425,6 +464,18 @@ sw_status enqueue_round(sw_ctx* ctx, sw_serve_state* s, int chunk, int buf,
                T, R);
     int* d_ovf_count = s->d_counters + ns;
     const int pair_count = s->chunk_begin[chunk + 1] - s->chunk_begin[chunk];
+    if (lplan.n_long > 0) {
+        SW_CUDA(ctx, cudaEventRecord(ctx->fork_ev, st));
+        SW_CUDA(ctx, cudaStreamWaitEvent(ctx->side_stream, ctx->fork_ev, 0));
+        const sw_status ls = launch_long_items(
+            ctx, ctx->side_stream, lplan, reinterpret_cast<const uint2*>(s->d_meta + o_items),
+            s->d_counters + ns + 1 + ne, s->d_meta + o_codes,
+            reinterpret_cast<const uint32_t*>(s->d_meta + o_qoff),
+            reinterpret_cast<const uint32_t*>(s->d_meta + o_qlen), s->d_scores, s->d_ovf, d_ovf_count,
+            (int)std::min<size_t>(s->ovf_cap, (size_t)INT32_MAX), launches);
+        if (ls != SW_OK) return ls;
+    }
+    bool first_launch = true;
     for (const QpLaunch& L : pair_count > 0 ? qp_launches : std::vector<QpLaunch>()) {
         const size_t smem = qk->smem((int)std::max<uint32_t>(L.max_rows, 1));
         int occq = 0;
@@ -478,7 +529,10 @@ sw_status enqueue_round(sw_ctx* ctx, sw_serve_state* s, int chunk, int buf,
                                      pair_count, s->chunk_cols[(size_t)chunk],
                                      (long long)occq * ctx->num_sms * (qk->block / qk->T));
         void* qargs[] = {&q};
-        SW_CUDA(ctx, cudaLaunchKernel(qk->fn[ctx->cell], dim3((unsigned)(occq * ctx->num_sms)),
+        // (the round's first paired launch leaves the long items their SMs)
+        const int sms = ctx->num_sms - (first_launch ? lplan.sms : 0);
+        first_launch = false;
+        SW_CUDA(ctx, cudaLaunchKernel(qk->fn[ctx->cell], dim3((unsigned)(occq * sms)),
                                       dim3(qk->block), qargs, smem, st));
         ++*launches;
     }
@@ -513,6 +567,10 @@ sw_status enqueue_round(sw_ctx* ctx, sw_serve_state* s, int chunk, int buf,
                                           dim3(s->k->block), args, s->k->smem((int)max_rows), st));
             ++*launches;
         }
+    }
+    if (lplan.n_long > 0) {
+        SW_CUDA(ctx, cudaEventRecord(ctx->join_ev, ctx->side_stream));
+        SW_CUDA(ctx, cudaStreamWaitEvent(st, ctx->join_ev, 0));
     }
     {
         RescoreArgs r;
@@ -922,6 +980,21 @@ extern "C" sw_status sw_serve_start(sw_ctx* ctx, const sw_serve_options* opt) {
         s->qk = qk;
     }
     const int64_t npairs = ctx->n_pairs;
+    // Records longer than a group's share of one double stack over one chunk
+    // would hold every round that has a single tall request: they leave the
+    // ring (at least 1,024 columns, so that few do).  The items' warps score up
+    // to kLongItemRows rows; a longer request then runs alone.
+    if (qk && o.pair_long && npairs > 0) {
+        const double groups = (double)ctx->num_sms * (qk->block / qk->T);
+        const double cut = std::max(1024.0, 2.0 * (double)ctx->pair_cols_total / o.chunks / groups);
+        const int64_t n = std::partition_point(ctx->pair_ncols.begin(), ctx->pair_ncols.end(),
+                                               [cut](uint32_t c) { return c > cut; }) -
+                          ctx->pair_ncols.begin();
+        if (n > 0 && n < npairs && n <= 4096) {
+            s->n_long = n;
+            s->max_stack_rows = std::min(s->max_stack_rows, kLongItemRows);
+        }
+    }
     s->n_chunks = (int)std::max<int64_t>(1, std::min<int64_t>(o.chunks, std::max<int64_t>(npairs, 1)));
     auto fail = [&](const char* what) {
         serve_free(s);
@@ -929,8 +1002,8 @@ extern "C" sw_status sw_serve_start(sw_ctx* ctx, const sw_serve_options* opt) {
         ctx->err = std::string("device allocation failed: serving ") + what;
         return SW_ERR_NOMEM;
     };
-    // the ring: pairs dealt round-robin (every n_chunks-th pair of the
-    // length-sorted order) and stored chunk after chunk
+    // the ring: the other pairs dealt round-robin (every n_chunks-th pair of
+    // the length-sorted order) and stored chunk after chunk
     std::vector<Pair2> host_pairs((size_t)npairs);
     if (npairs && cudaMemcpy(host_pairs.data(), ctx->d_pairs, (size_t)npairs * sizeof(Pair2),
                              cudaMemcpyDeviceToHost) != cudaSuccess)
@@ -942,7 +1015,7 @@ extern "C" sw_status sw_serve_start(sw_ctx* ctx, const sw_serve_options* opt) {
     s->chunk_begin.assign(1, 0);
     for (int c = 0; c < s->n_chunks; ++c) {
         uint64_t cols = 0;
-        for (int64_t p = c; p < npairs; p += s->n_chunks) {
+        for (int64_t p = s->n_long + c; p < npairs; p += s->n_chunks) {
             ring.push_back(host_pairs[(size_t)p]);
             ids.push_back((uint32_t)p);
             s->ring_ncols.push_back(host_pairs[(size_t)p].ncols);
@@ -960,7 +1033,7 @@ extern "C" sw_status sw_serve_start(sw_ctx* ctx, const sw_serve_options* opt) {
          cudaMemcpy(s->d_pair_ids, ids.data(), ids.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess))
         return fail("pair ring");
     if (dev_alloc(&s->d_scores, (size_t)s->n_slots * std::max(n_rec, 1)) != cudaSuccess ||
-        dev_alloc(&s->d_counters, 6 * (size_t)s->n_slots + 16) != cudaSuccess)
+        dev_alloc(&s->d_counters, 6 * (size_t)s->n_slots + 16 + kLongBuckets) != cudaSuccess)
         return fail("slots");
     // overflow entries: one per (request, record) at worst, bounded
     s->ovf_cap = std::min<size_t>((size_t)s->n_slots * std::max(n_rec, 1),
@@ -1008,7 +1081,7 @@ extern "C" sw_status sw_serve_start(sw_ctx* ctx, const sw_serve_options* opt) {
     // stacks (at most one per slot), the overflow count, and paired entries
     // (a lane of at most max_stack_rows rows has at most that / pair_seg
     // segments; two lanes per double stack)
-    s->counters_cap = 6 * (size_t)s->n_slots + 16;
+    s->counters_cap = 6 * (size_t)s->n_slots + 16 + kLongBuckets;
     s->slots.assign((size_t)s->n_slots, Slot());
     s->stats.slots = (uint32_t)s->n_slots;
     s->stats.chunks = (uint32_t)s->n_chunks;

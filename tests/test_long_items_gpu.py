@@ -59,3 +59,25 @@ def test_saturated_long_record_in_a_batch():
         assert c.run_stats().rescored == 1
     assert scores[0][-1] == oracle.gotoh(w, rec, M) >= 34_000
     np.testing.assert_array_equal(scores[1], oracle.search(qs[1], res, off, M, 12, 2))
+
+
+@pytest.mark.parametrize("chunks", [1, 4])
+def test_served_requests_with_long_records(case, chunks):
+    """Requests score the long pairs in their first round, whatever else is in
+    flight; each list equals the plain search's."""
+    db, queries = case
+    with capi.Context(0) as c:
+        c.load_db(db.residues, db.offsets)
+        plain = [c.search(q)[0] for q in queries]
+        c.serve_start(chunks=chunks, max_active=6)
+        got, sent = {}, 0
+        while len(got) < 2 * len(queries):
+            if sent < 2 * len(queries):
+                c.serve_submit(sent, queries[sent % len(queries)])
+                sent += 1
+            for r in c.serve_poll(timeout_ms=0 if sent < 2 * len(queries) else 5000):
+                assert r["status"] == 0
+                got[r["id"]] = r["hits"]
+        c.serve_stop()
+    for i, h in got.items():
+        assert h == plain[i % len(queries)], f"request {i}"
