@@ -150,18 +150,33 @@ __global__ void __launch_bounds__(kWindowThreads) sw_windows(const WindowArgs a)
     }
 }
 
-// Top-k, one block: sort 4096 64-bit keys in shared memory (bitonic,
-// descending) and keep the first k.  Key = score << 32 | ~record_index, so the
-// order is score descending, then record index ascending.  In the first round
-// the keys are made from the per-position scores (clamped when asked) and the
-// position -> record permutation, and the record-order score array is filled.
+// A warp's largest key, in every lane.
+__device__ __forceinline__ unsigned long long warp_max_key(unsigned long long key) {
+    const uint32_t hi = (uint32_t)(key >> 32);
+    const uint32_t top = __reduce_max_sync(0xffffffffu, hi);
+    const uint32_t lo = __reduce_max_sync(0xffffffffu, hi == top ? (uint32_t)key : 0u);
+    return ((unsigned long long)top << 32) | lo;
+}
+
+// Top-k, one block: the first k of 4096 64-bit keys, descending.  Key = score
+// << 32 | ~record_index, so the order is score descending, then record index
+// ascending.  In the first round the keys are made from the per-position
+// scores (clamped when asked) and the position -> record permutation, and the
+// record-order score array is filled.  Bound: latency.  Up to kTopkSelect
+// hits the block takes its maximum k times (4 keys a thread in registers, two
+// warp reductions and one barrier each, about 200 clocks); more hits are
+// sorted in shared memory (bitonic, 78 stages of a barrier each, 32 us).
 __global__ void __launch_bounds__(kTopkThreads) sw_topk_round(const TopkArgs a) {
     __shared__ unsigned long long sk[kTopkKeys];
+    constexpr int kPer = kTopkKeys / kTopkThreads;
     const long long base = (long long)blockIdx.x * kTopkKeys;
     const long long y = blockIdx.y;                 // query of a batch
     const long long ys = (a.rows && !a.keys_in) ? a.rows[y] : y;   // its score row
-    for (int i = threadIdx.x; i < kTopkKeys; i += kTopkThreads) {
-        const long long g = base + i;
+    unsigned long long* const out = a.keys_out + y * a.out_stride + (long long)blockIdx.x * a.k;
+    unsigned long long mine[kPer];
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+        const long long g = base + j * kTopkThreads + threadIdx.x;
         unsigned long long key = 0ull;
         if (g < a.n) {
             if (a.keys_in) {
@@ -174,8 +189,34 @@ __global__ void __launch_bounds__(kTopkThreads) sw_topk_round(const TopkArgs a) 
                 if (s > 0) key = ((unsigned long long)(uint32_t)s << 32) | (0xffffffffu - rec);
             }
         }
-        sk[i] = key;
+        mine[j] = key;
     }
+    if (a.k <= kTopkSelect) {
+        const int lane = (int)(threadIdx.x & 31), warp = (int)(threadIdx.x >> 5);
+        static_assert(kTopkThreads == 1024, "one warp maximum per lane of the second reduction");
+        unsigned long long best = 0ull;
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) best = max(best, mine[j]);
+        for (int i = 0; i < a.k; ++i) {
+            const unsigned long long w = warp_max_key(best);
+            unsigned long long* const s = sk + 32 * (i & 1);   // the other half is still read
+            if (lane == 0) s[warp] = w;
+            __syncthreads();
+            const unsigned long long top = warp_max_key(s[lane]);
+            if (threadIdx.x == 0) out[i] = top;
+            if (best == top && top != 0ull) {      // keys differ: one thread holds it
+                best = 0ull;
+#pragma unroll
+                for (int j = 0; j < kPer; ++j) {
+                    if (mine[j] == top) mine[j] = 0ull;
+                    best = max(best, mine[j]);
+                }
+            }
+        }
+        return;
+    }
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) sk[j * kTopkThreads + threadIdx.x] = mine[j];
     __syncthreads();
     for (int size = 2; size <= kTopkKeys; size <<= 1) {
         for (int stride = size >> 1; stride > 0; stride >>= 1) {
@@ -183,17 +224,16 @@ __global__ void __launch_bounds__(kTopkThreads) sw_topk_round(const TopkArgs a) 
                 const int lo = 2 * i - (i & (stride - 1));
                 const int hi = lo + stride;
                 const bool desc = (lo & size) == 0;
-                const unsigned long long x = sk[lo], y = sk[hi];
-                if (desc ? (x < y) : (x > y)) {
-                    sk[lo] = y;
+                const unsigned long long x = sk[lo], z = sk[hi];
+                if (desc ? (x < z) : (x > z)) {
+                    sk[lo] = z;
                     sk[hi] = x;
                 }
             }
             __syncthreads();
         }
     }
-    for (int i = threadIdx.x; i < a.k; i += kTopkThreads)
-        a.keys_out[y * a.out_stride + (long long)blockIdx.x * a.k + i] = sk[i];
+    for (int i = threadIdx.x; i < a.k; i += kTopkThreads) out[i] = sk[i];
 }
 
 }  // namespace swb
