@@ -303,7 +303,10 @@ sw_status sw_get_kernel_config(struct sw_ctx *ctx, uint32_t qlen, sw_kernel_conf
 /* Row segments a plain search of this length runs on the DB's pairs below the
  * long-pair cut-over, in order: each step's shape and passes (the last step
  * holds the rest of the query, its last pass padded).  Fills up to capacity
- * steps; *n_steps receives the count (1 without a plan). */
+ * steps; *n_steps receives the count (1 without a plan).  On a DB whose longest
+ * records need a layout of their own (windows, or a long-pair split), sw_search
+ * also looks at the query's residues: they bound how far an alignment can span,
+ * and with it the windows, more tightly than the length alone does here. */
 sw_status sw_get_plan(struct sw_ctx *ctx, uint32_t qlen, sw_plan_step *steps, uint32_t capacity,
                       uint32_t *n_steps);
 

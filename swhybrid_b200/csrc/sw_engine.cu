@@ -830,21 +830,22 @@ Windows plan_windows(const sw_ctx* ctx, double share, int64_t span) {
         const int64_t n_w = std::partition_point(ctx->pair_ncols.begin(), ctx->pair_ncols.end(),
                                                  [len](uint32_t n) { return (int64_t)n > len; }) -
                             ctx->pair_ncols.begin();
-        if (n_w > 8192) break;      // shorter windows only cut more pairs
-        int64_t n = 0;
-        for (int64_t p = 0; p < n_w; ++p)
-            n += window_count((int)ctx->pair_ncols[p], (int)len, (int)stride);
-        if (n > ctx->win_cap || (uint64_t)n * (len / 8) > ctx->win_units) continue;
-        const double extra = (double)n * len - (double)ctx->pair_prefix[n_w];
+        if (n_w > 3000) break;      // shorter windows only cut more pairs
+        // (each pair's last partial stride counted as half a window, at most one)
+        const double strides = ((double)ctx->pair_prefix[n_w] - (double)n_w * len) / stride;
+        const double most = 2.0 * n_w + strides;
+        if (most > ctx->win_cap || most * (len / 8) > (double)ctx->win_units) continue;
+        const double extra = (1.5 * n_w + strides) * len - (double)ctx->pair_prefix[n_w];
         const double est = share * (1.0 + extra / total) + 0.25 * len;
         if (est < best_est) {
             best_est = est;
             best.len = (int)len;
             best.stride = (int)stride;
             best.n_pairs = n_w;
-            best.n = (int)n;
         }
     }
+    for (int64_t p = 0; p < best.n_pairs; ++p)
+        best.n += window_count((int)ctx->pair_ncols[p], best.len, best.stride);
     return best;
 }
 
@@ -858,7 +859,7 @@ Windows plan_windows(const sw_ctx* ctx, double share, int64_t span) {
 // and one warp per scheduler, 332 at 4 rows and four, 288 at 8 rows and two).
 
 // Cells an SM full of bulk groups of R rows per thread updates per clock.
-double bulk_rate(int R) { return 22.7 * R / (R + 4.0); }
+double bulk_rate(int R) { return 24.0 * R / (R + 4.3); }
 
 // Bulk launch over `units` units (pairs or windows, `cols` columns in all, the
 // longest `longest`) in P passes on sms SMs.
@@ -880,7 +881,7 @@ double long_step_clocks(int R, int warps) {
 
 double long_clocks(int R, int passes, int pipes, double pairs, double cols, double longest,
                    double sms) {
-    const double step = long_step_clocks(R, passes * pipes);
+    const double step = 1.04 * long_step_clocks(R, passes * pipes);
     const double fill = (passes - 1) * 64.0 + 48.0;
     const double even = (cols + pairs * fill) / (sms * pipes);
     return step * (std::max(even, longest + fill) + (pairs > sms * pipes ? 0.3 * even * sms * pipes / pairs : 0.0)) +
@@ -916,18 +917,15 @@ int long_pipelines(sw_ctx* ctx, const LongKernel& k, int P, size_t* smem) {
     return G;
 }
 
-// The best split over cut-overs (every 1.4x in columns, down to every pair),
-// row counts, SM shares and bulk shapes: `given`, and the shapes that fit the
-// query's rows in 1..4 passes (a table's shape is tuned for a large DB; a small
-// one wants wider groups, whose steps are fewer).
-Split plan_split(sw_ctx* ctx, int qlen, const WfKernel* given) {
-    Split best;
-    const int64_t np = ctx->n_pairs;
-    if (np == 0) return best;
-    const WfKernel* shapes[16];
+// Bulk shapes the model chooses from: `given`, and (unless they are fixed) the
+// two of each group width that suit the query's rows best.  A table's shape is
+// tuned for a large DB; a small one, or one with long records, wants wider
+// groups, whose units are fewer.
+constexpr int kModelShapes = 16;
+int model_shapes(sw_ctx* ctx, int qlen, const WfKernel* given, const WfKernel** shapes) {
     int n_shapes = 0;
     auto add = [&](const WfKernel* k) {
-        if (!k || n_shapes == 16 || launch_rows(ctx, *k, qlen) != qlen) return;
+        if (!k || n_shapes == kModelShapes || launch_rows(ctx, *k, qlen) != qlen) return;
         for (int i = 0; i < n_shapes; ++i)
             if (shapes[i] == k) return;
         shapes[n_shapes++] = k;
@@ -938,14 +936,35 @@ Split plan_split(sw_ctx* ctx, int qlen, const WfKernel* given) {
     const bool fixed = entry && (entry->plan[0].group_width != 0 || !ctx->tuning_builtin);
     int n_all = 0;
     const WfKernel* all = wf_kernels(&n_all);
-    for (const int T : {32, 16, 8})
-        for (int P = 1; P <= 4 && !fixed; ++P) {
-            const int rows = (qlen + T * P - 1) / (T * P);
-            const WfKernel* k = nullptr;      // the smallest row count that holds them
-            for (int i = 0; i < n_all; ++i)
-                if (all[i].T == T && all[i].R >= rows && (!k || all[i].R < k->R)) k = &all[i];
-            if (k && k->R <= 64) add(k);
+    for (const int T : {32, 16, 8, 4}) {
+        // the two row counts with the least time for the rows they compute
+        const WfKernel* k2[2] = {nullptr, nullptr};
+        double t2[2] = {1e300, 1e300};
+        for (int i = 0; i < n_all && !fixed; ++i) {
+            if (all[i].T != T) continue;
+            const int rows = T * all[i].R;
+            const double t = (qlen + rows - 1) / rows * (double)rows / bulk_rate(all[i].R);
+            const int at = t < t2[0] ? 0 : t < t2[1] ? 1 : 2;
+            if (at == 2) continue;
+            if (at == 0) {
+                k2[1] = k2[0];
+                t2[1] = t2[0];
+            }
+            k2[at] = &all[i];
+            t2[at] = t;
         }
+        add(k2[0]);
+        add(k2[1]);
+    }
+    return n_shapes;
+}
+
+// The best split over cut-overs (every 1.5x in columns, down to every pair),
+// row counts, SM shares and bulk shapes.
+Split plan_split(sw_ctx* ctx, int qlen, const WfKernel* const* shapes, int n_shapes) {
+    Split best;
+    const int64_t np = ctx->n_pairs;
+    if (np == 0) return best;
     struct Long {
         const LongKernel* k;
         int P, G;
@@ -962,7 +981,7 @@ Split plan_split(sw_ctx* ctx, int qlen, const WfKernel* given) {
     const double total = (double)ctx->pair_cols_total;
     const int sms = ctx->num_sms;
     int64_t prev = -1;
-    for (double cut = (double)ctx->pair_ncols[0] * 0.98; ; cut /= 1.4) {
+    for (double cut = (double)ctx->pair_ncols[0] * 0.98; ; cut /= 1.5) {
         const bool last = cut < 100.0;
         const uint32_t c = last ? 0u : (uint32_t)cut;
         const int64_t n_long = std::partition_point(ctx->pair_ncols.begin(), ctx->pair_ncols.end(),
@@ -971,21 +990,23 @@ Split plan_split(sw_ctx* ctx, int qlen, const WfKernel* given) {
         if (n_long != prev && n_long > 0) {
             prev = n_long;
             const double cols = (double)ctx->pair_prefix[n_long], longest = ctx->pair_ncols[0];
-            for (const int x : {1, 2, 4, 8, 12, 16, 24, 32, 40, 48, 64, 80, 96, 112, 128, 148}) {
+            for (const int x : {1, 2, 4, 8, 12, 16, 24, 32, 48, 64, 96, 128}) {
                 const int on = n_long == np ? sms : std::min(x, sms - 1);
+                // (no row count's step is shorter than the first's)
+                if (longest * long_step_clocks(longs[0].k->R, 1) >= best.clocks) break;
                 double tl = 1e300;
                 const Long* l = nullptr;
                 int pipes = 0;
-                for (int i = 0; i < n_longs; ++i) {
-                    const int G = (int)std::min<int64_t>(longs[i].G, (n_long + on - 1) / on);
-                    const double t = long_clocks(longs[i].k->R, longs[i].P, G, (double)n_long, cols,
-                                                 longest, on);
-                    if (t < tl) {
-                        tl = t;
-                        l = &longs[i];
-                        pipes = G;
+                for (int i = 0; i < n_longs; ++i)
+                    for (int G = 1; G <= longs[i].G && (int64_t)(G - 1) * on < n_long; G *= 2) {
+                        const double t = long_clocks(longs[i].k->R, longs[i].P, G, (double)n_long,
+                                                     cols, longest, on);
+                        if (t < tl) {
+                            tl = t;
+                            l = &longs[i];
+                            pipes = G;
+                        }
                     }
-                }
                 if (tl >= best.clocks) continue;
                 double tb = n_long == np ? 0.0 : 1e300;
                 const WfKernel* kb = n_long == np ? shapes[0] : nullptr;
@@ -1187,23 +1208,35 @@ bool model_layout(sw_ctx* ctx, int qlen, int64_t span, SearchLayout* L) {
     const int rows = std::min(qlen, launch_rows(ctx, *kb, qlen));
     const double share = group_share(ctx, *kb, rows);
     if ((double)ctx->pair_ncols[0] <= 0.9 * share) return false;
-    const int block = plain_block(ctx, *kb);
-    const double P = (qlen + kb->T * kb->R - 1) / (kb->T * kb->R);
     const double np = (double)ctx->n_pairs, total = (double)ctx->pair_cols_total;
-    const double whole = bulk_clocks(*kb, block, P, np, total, ctx->pair_ncols[0], ctx->num_sms);
+    auto passes = [qlen](const WfKernel& k) { return (double)((qlen + k.T * k.R - 1) / (k.T * k.R)); };
+    const double whole = bulk_clocks(*kb, plain_block(ctx, *kb), passes(*kb), np, total,
+                                     ctx->pair_ncols[0], ctx->num_sms);
+    const WfKernel* shapes[kModelShapes];
+    const int n_shapes = model_shapes(ctx, qlen, kb, shapes);
     double windowed = 1e300;
-    const Windows win = plan_windows(ctx, share, span);
-    if (win.n > 0)
-        windowed = bulk_clocks(*kb, block, P, np - win.n_pairs + win.n,
-                               total + (double)win.n * win.len - (double)ctx->pair_prefix[win.n_pairs],
-                               win.len, ctx->num_sms) + 15e3;
-    const Split sp = plan_split(ctx, qlen, kb);
+    Windows win;
+    const WfKernel* kw = kb;
+    for (int i = 0; i < n_shapes; ++i) {
+        const WfKernel& k = *shapes[i];
+        const Windows w = plan_windows(ctx, group_share(ctx, k, qlen), span);
+        if (w.n == 0) continue;
+        const double t = bulk_clocks(k, plain_block(ctx, k), passes(k), np - w.n_pairs + w.n,
+                                     total + (double)w.n * w.len - (double)ctx->pair_prefix[w.n_pairs],
+                                     w.len, ctx->num_sms) + 15e3;
+        if (t < windowed) {
+            windowed = t;
+            win = w;
+            kw = &k;
+        }
+    }
+    const Split sp = plan_split(ctx, qlen, shapes, n_shapes);
     const double least = std::min({whole, windowed, sp.clocks});
     if (least == whole) return false;
     if (least == windowed) {
         L->win = win;
-        L->bulk_T = kb->T;
-        L->bulk_R = kb->R;
+        L->bulk_T = kw->T;
+        L->bulk_R = kw->R;
         L->bulk_b = win.n_pairs;
         L->longest = win.len;
     } else {
@@ -1341,6 +1374,10 @@ sw_status enqueue_search(sw_ctx* ctx, const uint8_t* d_query, int qlen, int64_t 
     layout_search(ctx, qlen, span, &L);
     ctx->stats.used = L.cfg;
     ctx->stats.used.cutover = L.cutover;
+    if (L.win.n > 0) {
+        ctx->stats.used.short_group_width = ctx->stats.used.long_group_width = L.bulk_T;
+        ctx->stats.used.short_rows_per_thread = ctx->stats.used.long_rows_per_thread = L.bulk_R;
+    }
     *launches = 0;
     const bool split = L.split;
     const int64_t n_long = L.n_long;
@@ -1612,8 +1649,9 @@ sw_status ensure_query_buffers(sw_ctx* ctx, size_t qlen) {
     if (dev_alloc(&ctx->d_query, cap) != cudaSuccess) SW_SET(ctx, SW_ERR_NOMEM, "query buffer");
     if (cudaMallocHost((void**)&ctx->h_query, cap) != cudaSuccess)
         SW_SET(ctx, SW_ERR_NOMEM, "pinned query buffer");
-    if (!ctx->h_keys && cudaMallocHost((void**)&ctx->h_keys, kMaxTopK * sizeof(unsigned long long)) !=
-                            cudaSuccess)
+    // (the keys, then the count of re-scored records)
+    if (!ctx->h_keys && cudaMallocHost((void**)&ctx->h_keys,
+                                       (kMaxTopK + 1) * sizeof(unsigned long long)) != cudaSuccess)
         SW_SET(ctx, SW_ERR_NOMEM, "pinned key buffer");
     ctx->query_cap = cap;
     return SW_OK;
@@ -1662,6 +1700,9 @@ sw_status search_host(sw_ctx* ctx, const uint8_t* query, uint32_t qlen, sw_hit* 
     if (st != SW_OK) return st;
     SW_CUDA(ctx, cudaMemcpyAsync(ctx->h_keys, keys, (size_t)k * sizeof(unsigned long long),
                                  cudaMemcpyDeviceToHost, ctx->stream));
+    int* const rescored = reinterpret_cast<int*>(ctx->h_keys + kMaxTopK);
+    SW_CUDA(ctx, cudaMemcpyAsync(rescored, ctx->d_counters + 2, sizeof(int), cudaMemcpyDeviceToHost,
+                                 ctx->stream));
     if (scores)
         SW_CUDA(ctx, cudaMemcpyAsync(scores, ctx->d_scores_rec,
                                      (size_t)ctx->n_records * sizeof(int32_t),
@@ -1680,12 +1721,10 @@ sw_status search_host(sw_ctx* ctx, const uint8_t* query, uint32_t qlen, sw_hit* 
         ++m;
     }
     *n_hits = m;
-    int rescored = 0;
-    cudaMemcpy(&rescored, ctx->d_counters + 2, sizeof(int), cudaMemcpyDeviceToHost);
     ctx->stats.kernel_ms = kms;
     ctx->stats.first_pass_ms = fpms;
     ctx->stats.cells = (uint64_t)qlen * ctx->n_residues;
-    ctx->stats.rescored = (uint64_t)rescored;
+    ctx->stats.rescored = (uint64_t)*rescored;
     ctx->stats.launches = launches;
     ctx->stats.queries = 1;
     ctx->stats.total_ms = now_ms() - t0;

@@ -749,9 +749,12 @@ __device__ __forceinline__ void run_stream(const RunArgs& a, const uint2* prof, 
                     E[k] = FZ;
                 }
                 prev_h = HZ;
-                if (t == 0 && a.pass0 + pass > 0) {
-                    if (ncols > 0) bq0 = rrow[0];
-                    if (ncols > 1) bq1 = rrow[2];
+                if (t == 0) {
+                    const bool above = a.pass0 + pass > 0;
+                    bq0 = make_uint2(HZ, FZ);
+                    bq1 = bq0;
+                    if (above && ncols > 0) bq0 = rrow[0];
+                    if (above && ncols > 1) bq1 = rrow[2];
                 }
                 d_cur = (ncols > 0) ? (uint32_t)__ldg(col) : kPadPair;
             }
@@ -842,8 +845,10 @@ __device__ __forceinline__ void run_stream(const RunArgs& a, const uint2* prof, 
                 }
             } else {
                 // two steps per iteration (+0.9 % over the sweep, measured); a
-                // query of one pass runs them without the boundary row's
-                // branches and warp syncs (+1.7 % at 16x40, +4.5 % at 32x40)
+                // query of one pass runs them without the boundary row and the
+                // warp syncs (+1.7 % at 16x40, +4.5 % at 32x40); thread 0 takes
+                // the row above from bq0 (the zero row where there is none),
+                // as a branch in this loop costs more than the selects
                 auto plain_steps = [&](auto with_bnd) {
                     constexpr bool BND = decltype(with_bnd)::value;
 #pragma unroll 2
@@ -853,15 +858,15 @@ __device__ __forceinline__ void run_stream(const RunArgs& a, const uint2* prof, 
                         uint32_t f_in = __shfl_up_sync(FULL, out_f, 1, T);
                         const uint32_t d_in = d_cur;
                         d_cur = (uint32_t)__ldg(col + c + 1);
-                        if (BND && rd0) {
-                            h_in = bq0.x;
-                            f_in = bq0.y;
+                        h_in = t == 0 ? (BND ? bq0.x : HZ) : h_in;
+                        f_in = t == 0 ? (BND ? bq0.y : FZ) : f_in;
+                        if (BND) {
                             bq0 = bq1;
-                            bq1 = rrow[2 * (c + 2)];
+                            if (rd0) bq1 = rrow[2 * (c + 2)];
                         }
-                        if (zin) {
-                            h_in = HZ;
-                            f_in = FZ;
+                        if (STACKED) {
+                            h_in = my_first ? HZ : h_in;
+                            f_in = my_first ? FZ : f_in;
                         }
                         const int o0 = (int)(d_in & 0xffu) * SLOTS;
                         const int o1 = (int)((d_in >> 8) & 0xffu) * SLOTS;
