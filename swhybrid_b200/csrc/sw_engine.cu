@@ -405,9 +405,12 @@ sw_status swb::db_load(sw_ctx* ctx, const uint8_t* residues, const uint64_t* off
     // room for windows of long pairs: an eighth of the DB's columns (half a
     // million for a small DB, never more than the DB itself)
     ctx->win_units = std::min<uint64_t>(units, std::max<uint64_t>(units / 8, 65536));
-    if (units + ctx->win_units >= (1ull << 32)) ctx->win_units = 0;
-    ctx->win_cap = (int)(ctx->win_units / (kMinWindow / 8) + 1);
-    if (dev_alloc(&ctx->d_db, units + ctx->win_units) != cudaSuccess) return nomem("db");
+    // (the long-pair kernel's windows need no boundary rows, eight times as
+    // much memory: twice the room)
+    ctx->long_win_units = std::min<uint64_t>(units, std::max<uint64_t>(units / 4, 131072));
+    if (units + ctx->long_win_units >= (1ull << 32)) ctx->win_units = ctx->long_win_units = 0;
+    ctx->win_cap = (int)(ctx->long_win_units / (kMinWindow / 8) + 1);
+    if (dev_alloc(&ctx->d_db, units + ctx->long_win_units) != cudaSuccess) return nomem("db");
     if (dev_alloc(&ctx->d_win_pairs, ctx->win_cap) != cudaSuccess) return nomem("windows");
     if (dev_alloc(&ctx->d_win_ids, ctx->win_cap) != cudaSuccess) return nomem("windows");
     if (dev_alloc(&ctx->d_pairs, npairs_all) != cudaSuccess) return nomem("pairs");
@@ -430,7 +433,7 @@ sw_status swb::db_load(sw_ctx* ctx, const uint8_t* residues, const uint64_t* off
                                 cudaMemcpyHostToDevice));
     if (n) SW_CUDA(ctx, cudaMemcpy(ctx->d_perm, perm.data(), n * sizeof(uint32_t),
                                    cudaMemcpyHostToDevice));
-    ctx->db_bytes = (units + ctx->win_units) * 16 + npairs_all * sizeof(Pair2) + n * 4 +
+    ctx->db_bytes = (units + ctx->long_win_units) * 16 + npairs_all * sizeof(Pair2) + n * 4 +
                     (units + ctx->win_units) * 16 * 8;
     ctx->db_loaded = true;
     return SW_OK;
@@ -809,6 +812,30 @@ struct Windows {
     int n = 0;               // windows
 };
 
+// Pairs of more than `cols` columns: [0, pairs_above).
+int64_t pairs_above(const sw_ctx* ctx, int64_t cols) {
+    return std::partition_point(ctx->pair_ncols.begin(), ctx->pair_ncols.end(),
+                                [cols](uint32_t n) { return (int64_t)n > cols; }) -
+           ctx->pair_ncols.begin();
+}
+
+// Whether the windows of pairs [0, n_w) fit `units` of room; *windows: about
+// how many there are (each pair's last partial stride as half a window, at
+// most one).
+bool windows_fit(const sw_ctx* ctx, int64_t n_w, int64_t len, int64_t stride, uint64_t units,
+                 double* windows) {
+    const double strides = ((double)ctx->pair_prefix[n_w] - (double)n_w * len) / stride;
+    const double most = 2.0 * n_w + strides;
+    *windows = 1.5 * n_w + strides;
+    return most <= ctx->win_cap && most * (len / 8) <= (double)units;
+}
+
+void count_windows(const sw_ctx* ctx, Windows* w) {
+    w->n = 0;
+    for (int64_t p = 0; p < w->n_pairs; ++p)
+        w->n += window_count((int)ctx->pair_ncols[p], w->len, w->stride);
+}
+
 // Windows for a bulk launch whose evenly loaded group gets `share` columns,
 // with alignments spanning at most `span` columns.  A unit's columns are
 // serial, so the launch lasts about max(share, longest unit) plus the tail of
@@ -827,15 +854,11 @@ Windows plan_windows(const sw_ctx* ctx, double share, int64_t span) {
         const int64_t stride = (len - span + 1) / 8 * 8;
         if (len < kMinWindow || stride < 64) break;
         if (len >= (int64_t)ctx->pair_ncols[0]) continue;
-        const int64_t n_w = std::partition_point(ctx->pair_ncols.begin(), ctx->pair_ncols.end(),
-                                                 [len](uint32_t n) { return (int64_t)n > len; }) -
-                            ctx->pair_ncols.begin();
+        const int64_t n_w = pairs_above(ctx, len);
         if (n_w > 3000) break;      // shorter windows only cut more pairs
-        // (each pair's last partial stride counted as half a window, at most one)
-        const double strides = ((double)ctx->pair_prefix[n_w] - (double)n_w * len) / stride;
-        const double most = 2.0 * n_w + strides;
-        if (most > ctx->win_cap || most * (len / 8) > (double)ctx->win_units) continue;
-        const double extra = (1.5 * n_w + strides) * len - (double)ctx->pair_prefix[n_w];
+        double windows = 0;
+        if (!windows_fit(ctx, n_w, len, stride, ctx->win_units, &windows)) continue;
+        const double extra = windows * len - (double)ctx->pair_prefix[n_w];
         const double est = share * (1.0 + extra / total) + 0.25 * len;
         if (est < best_est) {
             best_est = est;
@@ -844,8 +867,7 @@ Windows plan_windows(const sw_ctx* ctx, double share, int64_t span) {
             best.n_pairs = n_w;
         }
     }
-    for (int64_t p = 0; p < best.n_pairs; ++p)
-        best.n += window_count((int)ctx->pair_ncols[p], best.len, best.stride);
+    count_windows(ctx, &best);
     return best;
 }
 
@@ -855,8 +877,11 @@ Windows plan_windows(const sw_ctx* ctx, double share, int64_t span) {
 // pipe when an SM is full and by its own latency when few warps are on it;
 // the constants were fitted to the kernels' measured rates on a B200 (bulk:
 // 4.5 / 5.4 / 6.0 / 6.2 TCUPS at 8 / 16 / 24 / 48 rows on 350-residue records;
-// long-pair kernel: 134 / 176 / 265 / 352 clocks a step at 4 / 8 / 16 / 24 rows
-// and one warp per scheduler, 332 at 4 rows and four, 288 at 8 rows and two).
+// long-pair kernel, clocks a step at 4 / 8 / 12 / 16 / 24 rows: 133 / 171 / 220 /
+// 251 / 347 with one warp per scheduler, 185 / 263 / 356 / 422 / 612 with two,
+// 306 / 494 / 653 / 815 / - with four).  Over 25 queries of 43..5,478 residues and
+// DBs of 190..150,000 records the time it gives for the layout it picks came
+// within 10 % of the measured one for all but a few launches under 0.15 ms.
 
 // Cells an SM full of bulk groups of R rows per thread updates per clock.
 double bulk_rate(int R) { return 24.0 * R / (R + 4.3); }
@@ -871,12 +896,18 @@ double bulk_clocks(const WfKernel& k, int block, double P, double units, double 
     const double step = std::max(60.0 + 11.7 * k.R, warps * 64.0 * k.R / bulk_rate(k.R));
     const double switches = units * (0.25 * (2 * k.T + 9));     // event steps per segment
     const double avg = (cols + switches) / (sms * warps * per_warp);
-    return P * step * (std::max(avg, longest) + 0.15 * std::min(avg, longest)) + 15e3;
+    // Units are claimed longest first, so the launch ends on short ones; but
+    // warps of an SM differ in speed, so a unit as long as the even share ends
+    // late (query 1,434 against 570,000 records, 4x40: 44.7 ms with units of up
+    // to 0.56 of the share, 47.1 with 0.90, 48.1 with 0.95).
+    const double tail = 0.15 * std::min({avg, longest, 2.0 * cols / units});
+    return P * step * (std::max(avg, 1.18 * longest) + tail) + 15e3;
 }
 
 // One column step of the long-pair kernel with `warps` warps per SM.
 double long_step_clocks(int R, int warps) {
-    return std::max(90.0 + 10.8 * R, (warps + 3) / 4 * 2.3 * (5.6 * R + 16.0));
+    const int n = (warps + 3) / 4;      // warps per scheduler
+    return std::max(90.0 + 10.8 * R, n * (36.0 + 10.6 * R) + (n == 2 ? 20.0 : 0.0));
 }
 
 double long_clocks(int R, int passes, int pipes, double pairs, double cols, double longest,
@@ -898,6 +929,7 @@ struct Split {
     int passes = 0, pipes = 0, sms = 0;
     size_t smem = 0;
     bool join = false;
+    Windows win;                // of the longest of those pairs (n 0: none)
     double clocks = 1e300;
 };
 
@@ -959,9 +991,13 @@ int model_shapes(sw_ctx* ctx, int qlen, const WfKernel* given, const WfKernel** 
     return n_shapes;
 }
 
+constexpr int kModelLongs = 12;     // >= the compiled long-pair row counts
+
 // The best split over cut-overs (every 1.5x in columns, down to every pair),
-// row counts, SM shares and bulk shapes.
-Split plan_split(sw_ctx* ctx, int qlen, const WfKernel* const* shapes, int n_shapes) {
+// row counts, SM shares, bulk shapes and windows of the longest pairs
+// (alignments span at most `span` columns).
+Split plan_split(sw_ctx* ctx, int qlen, int64_t span, const WfKernel* const* shapes,
+                 int n_shapes) {
     Split best;
     const int64_t np = ctx->n_pairs;
     if (np == 0) return best;
@@ -969,65 +1005,108 @@ Split plan_split(sw_ctx* ctx, int qlen, const WfKernel* const* shapes, int n_sha
         const LongKernel* k;
         int P, G;
         size_t smem;
-    } longs[8];
+    } longs[kModelLongs];
     int n_longs = 0, n_lk = 0;
     const LongKernel* lks = long_kernels(&n_lk);
     for (int i = 0; i < n_lk; ++i) {
         Long l{&lks[i], (qlen + 32 * lks[i].R - 1) / (32 * lks[i].R), 0, 0};
         l.G = long_pipelines(ctx, lks[i], l.P, &l.smem);
-        if (l.G > 0 && n_longs < 8) longs[n_longs++] = l;
+        if (l.G > 0 && n_longs < kModelLongs) longs[n_longs++] = l;
     }
     if (n_longs == 0) return best;
     const double total = (double)ctx->pair_cols_total;
     const int sms = ctx->num_sms;
-    int64_t prev = -1;
-    for (double cut = (double)ctx->pair_ncols[0] * 0.98; ; cut /= 1.5) {
-        const bool last = cut < 100.0;
-        const uint32_t c = last ? 0u : (uint32_t)cut;
-        const int64_t n_long = std::partition_point(ctx->pair_ncols.begin(), ctx->pair_ncols.end(),
-                                                    [c](uint32_t n) { return n > c; }) -
-                               ctx->pair_ncols.begin();
-        if (n_long != prev && n_long > 0) {
-            prev = n_long;
-            const double cols = (double)ctx->pair_prefix[n_long], longest = ctx->pair_ncols[0];
-            for (const int x : {1, 2, 4, 8, 12, 16, 24, 32, 48, 64, 96, 128}) {
-                const int on = n_long == np ? sms : std::min(x, sms - 1);
-                // (no row count's step is shorter than the first's)
-                if (longest * long_step_clocks(longs[0].k->R, 1) >= best.clocks) break;
-                double tl = 1e300;
-                const Long* l = nullptr;
-                int pipes = 0;
-                for (int i = 0; i < n_longs; ++i)
-                    for (int G = 1; G <= longs[i].G && (int64_t)(G - 1) * on < n_long; G *= 2) {
-                        const double t = long_clocks(longs[i].k->R, longs[i].P, G, (double)n_long,
-                                                     cols, longest, on);
-                        if (t < tl) {
-                            tl = t;
-                            l = &longs[i];
-                            pipes = G;
-                        }
-                    }
-                if (tl >= best.clocks) continue;
-                double tb = n_long == np ? 0.0 : 1e300;
-                const WfKernel* kb = n_long == np ? shapes[0] : nullptr;
-                for (int i = 0; i < n_shapes && n_long < np; ++i) {
-                    const WfKernel& k = *shapes[i];
-                    const double P = (qlen + k.T * k.R - 1) / (k.T * k.R);
-                    const double t = bulk_clocks(k, plain_block(ctx, k), P, (double)(np - n_long),
-                                                 total - cols, ctx->pair_ncols[n_long], sms - on);
-                    if (t < tb) {
-                        tb = t;
-                        kb = &k;
+    // Pairs [0, n_long) to the long-pair kernel as `units` units of `cols`
+    // columns in all, the longest `longest`: more SMs for them end their launch
+    // earlier and the bulk one later, so the best number of SMs is the first at
+    // which theirs is done first, or the one before it.
+    static constexpr int kSms[] = {1, 2, 4, 8, 12, 16, 24, 32, 48, 64, 96, 128};
+    constexpr int kNumSms = sizeof(kSms) / sizeof(kSms[0]);
+    auto consider = [&](int64_t n_long, double units, double cols, double longest,
+                        const Windows* win) {
+        // (no row count's step is shorter than the first's)
+        if (longest * long_step_clocks(longs[0].k->R, 1) >= best.clocks) return;
+        const double bulk_cols = total - (double)ctx->pair_prefix[n_long];
+        auto at = [&](int on) {
+            double tl = 1e300;
+            const Long* l = nullptr;
+            int pipes = 0;
+            for (int i = 0; i < n_longs; ++i)
+                for (int G = 1; G <= longs[i].G && (G - 1.0) * on < units; G *= 2) {
+                    const double t = long_clocks(longs[i].k->R, longs[i].P, G, units, cols, longest, on);
+                    if (t < tl) {
+                        tl = t;
+                        l = &longs[i];
+                        pipes = G;
                     }
                 }
-                const double t = std::max(tl, tb);
-                if (kb && t < best.clocks)
-                    best = Split{kb, l->k, n_long, l->P, pipes, on, l->smem, tl < 0.8 * tb, t};
-                if (on == sms) break;
+            double tb = n_long == np ? 0.0 : 1e300;
+            const WfKernel* kb = n_long == np ? shapes[0] : nullptr;
+            for (int i = 0; i < n_shapes && n_long < np; ++i) {
+                const WfKernel& k = *shapes[i];
+                const double P = (qlen + k.T * k.R - 1) / (k.T * k.R);
+                const double t = bulk_clocks(k, plain_block(ctx, k), P, (double)(np - n_long), bulk_cols,
+                                             ctx->pair_ncols[n_long], sms - on);
+                if (t < tb) {
+                    tb = t;
+                    kb = &k;
+                }
             }
+            const double t = std::max(tl, tb) + (win ? 10e3 : 0.0);
+            if (kb && t < best.clocks) {
+                best = Split{kb, l->k, n_long, l->P, pipes, on, l->smem, tl < 0.8 * tb, Windows{}, t};
+                if (win) best.win = *win;
+            }
+            return tl <= tb;
+        };
+        if (n_long == np) {
+            at(sms);
+            return;
         }
-        if (last) break;
+        int lo = 0, hi = kNumSms - 1;
+        while (hi > 0 && kSms[hi] >= sms) --hi;
+        while (lo < hi) {
+            const int mid = (lo + hi) / 2;
+            if (at(kSms[mid])) hi = mid;
+            else lo = mid + 1;
+        }
+        at(kSms[lo]);
+    };
+    const int64_t longest = ctx->pair_ncols[0];
+    int64_t prev = -1;
+    for (double cut = (double)longest * 0.98;; cut /= 1.5) {
+        const int64_t n_long = pairs_above(ctx, cut < 100.0 ? 0 : (int64_t)cut);
+        if (n_long != prev && n_long > 0)
+            consider(n_long, (double)n_long, (double)ctx->pair_prefix[n_long], (double)longest, nullptr);
+        prev = n_long;
+        if (cut < 100.0) break;
     }
+    // Windows of the longest pairs, where the split's long launch waits on the
+    // serial columns of a few of them: query 43 against 45,000 records and 90 of
+    // 10,000..35,000 residues 2,426 -> 442 us, query 198 against 6,200 and 12 of
+    // them 2,300 -> 371, query 1,875 against 984 and one 3,883 -> 1,059 (plain
+    // split -> windows), query 144 against 200 records of up to 1,400 179 -> 122.
+    if (span <= 0 || !best.lk) return best;
+    for (const double f : {0.7, 0.5, 0.35, 0.25, 0.17, 0.12, 0.08, 0.05, 0.035}) {
+        Windows w;
+        w.len = (int)(f * longest) / 8 * 8;
+        w.stride = (int)std::max<int64_t>((w.len - span + 1) / 8 * 8, 0);
+        if (w.len < kMinWindow || w.stride < std::max(64, w.len / 8)) break;
+        w.n_pairs = pairs_above(ctx, w.len);
+        if (w.n_pairs > 3000) break;
+        double n = 0;
+        if (!windows_fit(ctx, w.n_pairs, w.len, w.stride, ctx->long_win_units, &n)) continue;
+        prev = -1;
+        for (double cut = w.len; cut > 100.0 && cut > 0.2 * w.len; cut /= 1.5) {
+            const int64_t n_long = pairs_above(ctx, (int64_t)cut);
+            if (n_long != prev)
+                consider(n_long, n + (double)(n_long - w.n_pairs),
+                         n * w.len + (double)(ctx->pair_prefix[n_long] - ctx->pair_prefix[w.n_pairs]),
+                         w.len, &w);
+            prev = n_long;
+        }
+    }
+    count_windows(ctx, &best.win);
     return best;
 }
 
@@ -1185,10 +1264,12 @@ sw_status launch_long_items(sw_ctx* ctx, cudaStream_t stream, const LongItemPlan
 // kernel and the rest (if any) to the bulk shape.
 struct SearchLayout {
     sw_kernel_config cfg;
-    Windows win;                       // long pairs cut into windows for the bulk launches
+    Windows win;                       // long pairs cut into windows, for the long-pair
+                                       // kernel with a split, else for the bulk launches
     int cutover = 0;
     bool split = false;
-    int64_t n_long = 0;                // pairs of the long-pair kernel (split only)
+    int64_t n_long = 0;                // pairs of the long-pair kernel (split only), the
+                                       // first win.n_pairs of them as windows
     const LongKernel* lk = nullptr;
     int lpasses = 0, lpipes = 0, lsms = 0;
     bool join = false;                 // the long launch ends well before the bulk one
@@ -1230,7 +1311,7 @@ bool model_layout(sw_ctx* ctx, int qlen, int64_t span, SearchLayout* L) {
             kw = &k;
         }
     }
-    const Split sp = plan_split(ctx, qlen, shapes, n_shapes);
+    const Split sp = plan_split(ctx, qlen, span, shapes, n_shapes);
     const double least = std::min({whole, windowed, sp.clocks});
     if (least == whole) return false;
     if (least == windowed) {
@@ -1241,6 +1322,7 @@ bool model_layout(sw_ctx* ctx, int qlen, int64_t span, SearchLayout* L) {
         L->longest = win.len;
     } else {
         L->split = true;
+        L->win = sp.win;
         L->n_long = sp.n_long;
         L->lk = sp.lk;
         L->lpasses = sp.passes;
@@ -1374,7 +1456,7 @@ sw_status enqueue_search(sw_ctx* ctx, const uint8_t* d_query, int qlen, int64_t 
     layout_search(ctx, qlen, span, &L);
     ctx->stats.used = L.cfg;
     ctx->stats.used.cutover = L.cutover;
-    if (L.win.n > 0) {
+    if (L.win.n > 0 && !L.split) {
         ctx->stats.used.short_group_width = ctx->stats.used.long_group_width = L.bulk_T;
         ctx->stats.used.short_rows_per_thread = ctx->stats.used.long_rows_per_thread = L.bulk_R;
     }
@@ -1401,7 +1483,8 @@ sw_status enqueue_search(sw_ctx* ctx, const uint8_t* d_query, int qlen, int64_t 
     int nplan = 0;
     // every shape is checked before anything is launched: a search refused
     // half-way would leave a launch in flight that writes into the next one
-    if (L.bulk_e > L.bulk_b || L.win.n > 0) {
+    const int bulk_win = split ? 0 : L.win.n;
+    if (L.bulk_e > L.bulk_b || bulk_win > 0) {
         const WfKernel* k = find_kernel(L.bulk_T, L.bulk_R);
         if (!k) SW_SET(ctx, SW_ERR_INVALID, "no kernel %dx%d", L.bulk_T, L.bulk_R);
         if (launch_rows(ctx, *k, qlen) == 0)
@@ -1425,6 +1508,20 @@ sw_status enqueue_search(sw_ctx* ctx, const uint8_t* d_query, int qlen, int64_t 
     SW_CUDA(ctx, cudaMemsetAsync(ctx->d_counters, 0, 16 * sizeof(int), st));
     SW_CUDA(ctx, cudaMemsetAsync(ctx->d_scores, 0, (size_t)(ctx->n_records + 1) * sizeof(int), st));
     SW_CUDA(ctx, cudaEventRecord(mk.e[1], st));
+    if (L.win.n > 0) {
+        WindowArgs w;
+        w.db = ctx->d_db;
+        w.pairs = ctx->d_pairs;
+        w.len = L.win.len;
+        w.stride = L.win.stride;
+        w.base = (uint32_t)ctx->units;
+        w.win_pairs = ctx->d_win_pairs;
+        w.win_ids = ctx->d_win_ids;
+        void* args[] = {&w};
+        SW_CUDA(ctx, cudaLaunchKernel((const void*)sw_windows, dim3((unsigned)L.win.n_pairs),
+                                      dim3(kWindowThreads), args, 0, st));
+        ++*launches;
+    }
     int reserved_sms = 0;
     if (split) {
         reserved_sms = L.lsms;
@@ -1433,8 +1530,11 @@ sw_status enqueue_search(sw_ctx* ctx, const uint8_t* d_query, int qlen, int64_t 
         LongArgs la;
         la.db = ctx->d_db;
         la.pairs = ctx->d_pairs;
-        la.pair_begin = 0;
-        la.pair_count = (int)n_long;
+        la.n_win = L.win.n;
+        la.win_pairs = ctx->d_win_pairs;
+        la.win_ids = ctx->d_win_ids;
+        la.pair_begin = (int)L.win.n_pairs;
+        la.count = L.win.n + (int)(n_long - L.win.n_pairs);
         la.counter = ctx->d_counters;      // counter 0: the long pairs' claims
         la.query = d_query;
         la.qlen = qlen;
@@ -1452,7 +1552,7 @@ sw_status enqueue_search(sw_ctx* ctx, const uint8_t* d_query, int qlen, int64_t 
         SW_CUDA(ctx, cudaEventRecord(mk.e[4], ctx->side_stream));
         SW_CUDA(ctx, cudaLaunchKernel(
                          lk->fn[ctx->cell],
-                         dim3((unsigned)std::min<int64_t>(reserved_sms, (n_long + lpipes - 1) / lpipes)),
+                         dim3((unsigned)std::min<int64_t>(reserved_sms, (la.count + lpipes - 1) / lpipes)),
                          dim3(lpasses * lpipes * 32), args, L.lsmem, ctx->side_stream));
         SW_CUDA(ctx, cudaEventRecord(mk.e[5], ctx->side_stream));
         ++*launches;
@@ -1460,20 +1560,6 @@ sw_status enqueue_search(sw_ctx* ctx, const uint8_t* d_query, int qlen, int64_t 
         SW_CUDA(ctx, cudaEventRecord(mk.e[6], st));
     }
     mk.split = split;
-    if (L.win.n > 0) {
-        WindowArgs w;
-        w.db = ctx->d_db;
-        w.pairs = ctx->d_pairs;
-        w.len = L.win.len;
-        w.stride = L.win.stride;
-        w.base = (uint32_t)ctx->units;
-        w.win_pairs = ctx->d_win_pairs;
-        w.win_ids = ctx->d_win_ids;
-        void* args[] = {&w};
-        SW_CUDA(ctx, cudaLaunchKernel((const void*)sw_windows, dim3((unsigned)L.win.n_pairs),
-                                      dim3(kWindowThreads), args, 0, st));
-        ++*launches;
-    }
     // Row segments of the plan (one for most lengths), each in launches of
     // whole passes up to what one block's profile holds: every launch but the
     // first reads the boundary row the one before wrote (pass0 counts the
@@ -1493,10 +1579,10 @@ sw_status enqueue_search(sw_ctx* ctx, const uint8_t* d_query, int qlen, int64_t 
             a.db = ctx->d_db;
             a.pairs = ctx->d_pairs;
             a.pair_begin = (int)L.bulk_b;
-            a.pair_count = (int)(L.bulk_e - L.bulk_b) + L.win.n;
+            a.pair_count = (int)(L.bulk_e - L.bulk_b) + bulk_win;
             a.win_pairs = ctx->d_win_pairs;
             a.win_ids = ctx->d_win_ids;
-            a.n_win = L.win.n;
+            a.n_win = bulk_win;
             a.query = d_query + r0;
             a.qlen = rows;
             a.pass0 = passes_before;

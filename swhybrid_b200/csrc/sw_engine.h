@@ -86,6 +86,7 @@ struct sw_ctx {
     uint64_t units = 0;                // 16-byte units of the column stream
     uint64_t db_bytes = 0;
     uint64_t win_units = 0;            // further units of d_db and d_bnd, for windows of long pairs
+    uint64_t long_win_units = 0;       // ... of d_db: windows for the long-pair kernel need no d_bnd
     int win_cap = 0;                   // entries of d_win_pairs and d_win_ids
     std::vector<uint32_t> pair_ncols;  // host copy, for shape selection
     uint64_t pair_cols_total = 0;      // sum of pair_ncols

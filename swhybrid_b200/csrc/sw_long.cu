@@ -30,11 +30,15 @@
 // in its serial chain (forward_short), no branch and no bounds guard: columns
 // outside the pair run on zero-score residues, which raise no score, and the
 // profile words, the residue and the ring entry are read a step ahead.  A step
-// measured 134 / 176 / 265 / 352 clocks at 4 / 8 / 16 / 24 rows with one warp per
+// measured 133 / 171 / 251 / 347 clocks at 4 / 8 / 16 / 24 rows with one warp per
 // scheduler (183 / 187 / 280 / 374 with the columns' checks in every step).
+// Between them, 6, 12 and 20 rows keep a pass's padding small (query 375 in one
+// pass: 251 clocks at 16 rows, 220 at 12).  A record much longer than the others
+// would still hold the launch for its columns times that: it is cut into windows
+// (sw_windows) that are units of their own and merge by maximum.
 // Query 1,900 against 20,200 records of which 200 hold 43 % of the residues:
 // 17.5 ms before (two half-columns per thread, guarded steps, 3 warps of 24 rows
-// per pair, pipelines crowded on few SMs), 6.6 now.
+// per pair, pipelines crowded on few SMs), 5.2 now.
 #include <cstdint>
 
 #include <cuda_runtime.h>
@@ -56,7 +60,7 @@ constexpr int kLRing = 128;              // ring columns per link (>= 3K, power 
 // register file holds at the row count's register need, without spills.
 template <int R>
 struct LongBlock {
-    static constexpr int value = R <= 4 ? 768 : R <= 16 ? 512 : R <= 32 ? 384 : 256;
+    static constexpr int value = R <= 6 ? 768 : R <= 16 ? 512 : R <= 32 ? 384 : 256;
 };
 
 // One warp of a pipeline: query pass w of P against the pipeline's pair.
@@ -183,23 +187,29 @@ struct LongWarp {
     }
 };
 
-// A finished pair's scores (lanes of m) at row + its sorted position.
+// A finished pair's scores (lanes of m) at row + its sorted position; merge: a
+// window's, by maximum (put_score's rule).
 __device__ __forceinline__ void long_scores(int* scores, int row, int pos, int n_records, uint32_t m,
                                             int bias, int thresh, int* ovf_list, int* ovf_count,
-                                            int ovf_cap) {
+                                            int ovf_cap, bool merge) {
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         if (pos + i >= n_records) break;
         const int s = i ? hi16(m) : lo16(m);
-        scores[row + pos + i] = s - bias;
-        if (s >= thresh) {
+        int* const at = scores + row + pos + i;
+        bool list = s >= thresh;
+        if (!merge) *at = s - bias;
+        else if (list) list = atomicMax(at, kListed) != kListed;
+        else atomicMax(at, s - bias);
+        if (list) {
             const int j = atomicAdd(ovf_count, 1);
             if (j < ovf_cap) ovf_list[j] = row + pos + i;
         }
     }
 }
 
-// Plain search: one query, pairs claimed pipeline by pipeline.
+// Plain search: one query, units (windows, then pairs) claimed pipeline by
+// pipeline.
 template <int R, class CELL>
 __global__ void __launch_bounds__(LongBlock<R>::value, 1) sw_long(const LongArgs a) {
     using W = LongWarp<R, CELL>;
@@ -222,9 +232,10 @@ __global__ void __launch_bounds__(LongBlock<R>::value, 1) sw_long(const LongArgs
     // and lasts `total` steps, also a multiple of K
     auto begin_pair = [&](int v, int at) {
         pair = v;
-        active = pair < a.pair_count;
+        active = pair < a.count;
         if (active) {
-            x.begin(a.db, a.pairs[a.pair_begin + pair]);
+            x.begin(a.db, pair < a.n_win ? a.win_pairs[pair]
+                                         : a.pairs[a.pair_begin + pair - a.n_win]);
             span = W::span_of(x.ncols);
             total = (P - 1) * kLD + span;
             start = at;
@@ -249,16 +260,18 @@ __global__ void __launch_bounds__(LongBlock<R>::value, 1) sw_long(const LongArgs
             if (leader) {
                 const int v = atomicAdd(a.counter, 1);
                 s_next[g] = v;
-                alive = v < a.pair_count;
+                alive = v < a.count;
             }
         }
         const int any = __syncthreads_or(alive ? 1 : 0);
         if (ending) {
             if (leader) {
                 for (int i = 1; i < P; ++i) m = __vimax3_s16x2(m, s_max[warp + i], x.HZ);
-                long_scores(a.scores, 0, 2 * (a.pair_begin + pair), a.n_records, m,
-                            (int)(x.HZ & 0xffffu), a.ovf_thresh - K.stored_shift(), a.ovf_list,
-                            a.ovf_count, a.ovf_cap);
+                const bool win = pair < a.n_win;
+                const int at = win ? (int)a.win_ids[pair] : a.pair_begin + pair - a.n_win;
+                long_scores(a.scores, 0, 2 * at, a.n_records, m, (int)(x.HZ & 0xffffu),
+                            a.ovf_thresh - K.stored_shift(), a.ovf_list, a.ovf_count, a.ovf_cap,
+                            win);
             }
             begin_pair(s_next[g], gs);
         }
@@ -320,7 +333,7 @@ __global__ void __launch_bounds__(32 * kLongItemWarps, 1) sw_long_items(const Lo
             for (int i = 1; i < P; ++i) m = __vimax3_s16x2(m, s_max[warp + i], x.HZ);
             long_scores(a.scores, query * a.n_records, 2 * pair, a.n_records, m,
                         (int)(x.HZ & 0xffffu), a.ovf_thresh - K.stored_shift(), a.ovf_list,
-                        a.ovf_count, a.ovf_cap);
+                        a.ovf_count, a.ovf_cap, false);
         }
     }
 }
@@ -356,7 +369,8 @@ constexpr LongItemKernel iinst() {
 const LongItemKernel kLongItemTable[] = {iinst<4>(), iinst<8>(), iinst<16>()};
 
 const LongKernel kLongTable[] = {
-    linst<4>(), linst<8>(), linst<16>(), linst<24>(), linst<32>(), linst<64>(),
+    linst<4>(),  linst<6>(),  linst<8>(),  linst<12>(), linst<16>(),
+    linst<20>(), linst<24>(), linst<32>(), linst<64>(),
 };
 
 }  // namespace

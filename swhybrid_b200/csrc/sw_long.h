@@ -15,9 +15,12 @@ constexpr int kLongMaxWarps = 32;        // pipelines x passes per block
 struct LongArgs {
     const uint4* db;            // pair column streams
     const Pair2* pairs;         // pair table, ncols descending
-    int pair_begin;             // pairs [pair_begin, pair_begin + pair_count)
-    int pair_count;
-    int* counter;               // pairs claimed so far (one pipeline per pair)
+    int n_win;                  // units: n_win windows of long pairs (see sw_windows),
+    const Pair2* win_pairs;     // ... table entries of their own
+    const uint32_t* win_ids;    // ... and the pair each belongs to,
+    int pair_begin;             // then the pairs [pair_begin, pair_begin + count - n_win)
+    int count;
+    int* counter;               // units claimed so far (one pipeline per unit)
     const uint8_t* query;
     int qlen;                   // at most kLongMaxPasses * 32 * R rows
     int passes;                 // ceil(qlen / (32 R)); blockDim.x = 32 * passes * pipelines
