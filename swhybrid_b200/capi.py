@@ -55,6 +55,17 @@ class sw_hit(ctypes.Structure):
                 ("index", ctypes.c_uint64)]
 
 
+_HIT = np.dtype([("score", np.int32), ("reserved", np.uint32), ("index", np.uint64)])
+
+
+def _hit_list(hits, first: int, n: int) -> list:
+    """Entries first..first+n of a sw_hit array as (score, index) tuples."""
+    if n == 0:
+        return []
+    a = np.frombuffer(hits, dtype=_HIT, count=n, offset=first * _HIT.itemsize)
+    return list(zip(a["score"].tolist(), a["index"].tolist()))
+
+
 class sw_kernel_config(ctypes.Structure):
     _fields_ = [("long_group_width", ctypes.c_int32), ("long_rows_per_thread", ctypes.c_int32),
                 ("short_group_width", ctypes.c_int32), ("short_rows_per_thread", ctypes.c_int32),
@@ -437,8 +448,7 @@ class Context:
         scores = np.zeros(max(self.n_records, 1), dtype=np.int32) if want_scores else None
         self._check(self.L.sw_search(self.h, _ptr(q), len(q), hits, ctypes.byref(nh),
                                      _ptr(scores) if want_scores else None), "sw_search")
-        out = [(hits[i].score, hits[i].index) for i in range(nh.value)]
-        return out, (scores[:self.n_records] if want_scores else None)
+        return _hit_list(hits, 0, nh.value), (scores[:self.n_records] if want_scores else None)
 
     def search_device(self, d_query_ptr: int, qlen: int, d_scores_ptr: int | None = None):
         self._check(self.L.sw_search_device(self.h, ctypes.c_void_p(d_query_ptr), qlen,
@@ -475,8 +485,7 @@ class Context:
         self._check(self.L.sw_search_batch(self.h, nq, _ptr(flat), _ptr(off), hits, nh,
                                            _ptr(scores) if want_scores else None),
                     "sw_search_batch")
-        out = [[(hits[q * k + i].score, hits[q * k + i].index) for i in range(nh[q])]
-               for q in range(nq)]
+        out = [_hit_list(hits, q * k, nh[q]) for q in range(nq)]
         return out, (scores[:, :self.n_records] if want_scores else None)
 
     def set_tuning(self, table):
@@ -548,8 +557,8 @@ class Context:
         res = []
         for i in range(n):
             a = out[i]
-            cig = "".join(f"{int(o) >> 4}{'MID'[int(o) & 15]}"
-                          for o in ops[a.ops_offset:a.ops_offset + a.n_ops])
+            cig = "".join([f"{o >> 4}{'MID'[o & 15]}"
+                           for o in ops[a.ops_offset:a.ops_offset + a.n_ops].tolist()])
             res.append(dict(index=int(a.index), score=a.score, q_begin=a.q_begin,
                             q_end=a.q_end, d_begin=a.d_begin, d_end=a.d_end,
                             matches=a.matches, cigar=cig))
@@ -605,8 +614,7 @@ class Context:
         for i in range(n.value):
             r = res[i]
             out.append(dict(id=r.request_id, status=r.status,
-                            hits=[(hits[i * k + j].score, hits[i * k + j].index)
-                                  for j in range(r.n_hits)],
+                            hits=_hit_list(hits, i * k, r.n_hits),
                             submit_ms=r.submit_ms, start_ms=r.start_ms, done_ms=r.done_ms))
         return out
 

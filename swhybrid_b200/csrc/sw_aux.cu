@@ -173,6 +173,7 @@ __global__ void __launch_bounds__(kTopkThreads) sw_topk_round(const TopkArgs a) 
     const long long y = blockIdx.y;                 // query of a batch
     const long long ys = (a.rows && !a.keys_in) ? a.rows[y] : y;   // its score row
     unsigned long long* const out = a.keys_out + y * a.out_stride + (long long)blockIdx.x * a.k;
+    if (a.count && threadIdx.x == 0) out[a.k] = (unsigned long long)(uint32_t)*a.count;
     unsigned long long mine[kPer];
 #pragma unroll
     for (int j = 0; j < kPer; ++j) {

@@ -47,6 +47,8 @@ struct TopkArgs {
     long long rec_stride;                 // per query: scores_by_record
     long long out_stride;                 // per query: keys_out
     const int* rows;                      // optional: round 0 reads score row rows[y]
+    const int* count = nullptr;           // optional (a plain search's last round): its value
+                                          // goes behind the k keys
 };
 
 // Windows of the pairs longer than `len` columns (sw_windows): pair p of

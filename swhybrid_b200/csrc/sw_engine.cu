@@ -215,7 +215,6 @@ extern "C" sw_status sw_ctx_create(int device, const sw_params* params, sw_ctx**
     if (dev_alloc(&ctx->d_mat, 1024) != cudaSuccess) return fail(SW_ERR_NOMEM);
     if (cudaMemcpy(ctx->d_mat, mat8, 1024, cudaMemcpyHostToDevice) != cudaSuccess)
         return fail(SW_ERR_CUDA);
-    if (dev_alloc(&ctx->d_counters, 16) != cudaSuccess) return fail(SW_ERR_NOMEM);
     // every first-pass kernel may use the opt-in shared-memory maximum, less
     // what it holds statically (the long-pair kernels hold a few words)
     auto allow_smem = [&](const void* fn) {
@@ -224,16 +223,35 @@ extern "C" sw_status sw_ctx_create(int device, const sw_params* params, sw_ctx**
                cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     ctx->max_smem - (int)fa.sharedSizeBytes) == cudaSuccess;
     };
+    // what the kernels' registers and static shared memory allow, for the layout
+    // of each search
     int nk = 0;
     const WfKernel* ks = wf_kernels(&nk);
-    for (int i = 0; i < nk; ++i)
-        if (!allow_smem(ks[i].fn[ctx->cell]) || !allow_smem(ks[i].batch_fn)) return fail(SW_ERR_CUDA);
+    for (int i = 0; i < nk; ++i) {
+        sw_ctx::PlainFit f;
+        const void* fns[2] = {ks[i].fn[ctx->cell], ks[i].batch_fn};
+        const int blocks[2] = {plain_block(ctx, ks[i]), ks[i].block};
+        for (int v = 0; v < 2; ++v) {
+            cudaFuncAttributes fa;
+            if (!allow_smem(fns[v]) || cudaFuncGetAttributes(&fa, fns[v]) != cudaSuccess ||
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&f.blocks[v], fns[v], blocks[v], 0) !=
+                    cudaSuccess)
+                return fail(SW_ERR_CUDA);
+            f.max_dyn[v] = ctx->max_smem - (int)fa.sharedSizeBytes;
+        }
+        ctx->plain_fit.push_back(f);
+    }
     const QpKernel* qks = qp_kernels(&nk);
     for (int i = 0; i < nk; ++i)
         if (!allow_smem(qks[i].fn[ctx->cell])) return fail(SW_ERR_CUDA);
     const LongKernel* lks = long_kernels(&nk);
-    for (int i = 0; i < nk; ++i)
-        if (!allow_smem(lks[i].fn[ctx->cell])) return fail(SW_ERR_CUDA);
+    for (int i = 0; i < nk; ++i) {
+        cudaFuncAttributes fa;
+        if (!allow_smem(lks[i].fn[ctx->cell]) ||
+            cudaFuncGetAttributes(&fa, lks[i].fn[ctx->cell]) != cudaSuccess)
+            return fail(SW_ERR_CUDA);
+        ctx->long_fit.push_back({fa.numRegs, ctx->max_smem - (int)fa.sharedSizeBytes});
+    }
     const LongItemKernel* liks = long_item_kernels(&nk);
     for (int i = 0; i < nk; ++i)
         if (!allow_smem(liks[i].fn[ctx->cell])) return fail(SW_ERR_CUDA);
@@ -254,7 +272,8 @@ static void free_db(sw_ctx* ctx) {
     dev_free(ctx->d_win_ids);
     dev_free(ctx->d_perm);
     dev_free(ctx->d_bnd);
-    dev_free(ctx->d_scores);
+    dev_free(ctx->d_counters);
+    ctx->d_scores = nullptr;
     dev_free(ctx->d_scores_rec);
     dev_free(ctx->d_ovf);
     dev_free(ctx->d_keys[0]);
@@ -275,7 +294,6 @@ extern "C" sw_status sw_ctx_destroy(sw_ctx* ctx) {
     if (ctx->side_stream) cudaStreamSynchronize(ctx->side_stream);
     free_db(ctx);
     dev_free(ctx->d_mat);
-    dev_free(ctx->d_counters);
     dev_free(ctx->d_query);
     if (ctx->h_query) cudaFreeHost(ctx->h_query);
     if (ctx->h_keys) cudaFreeHost(ctx->h_keys);
@@ -417,7 +435,8 @@ sw_status swb::db_load(sw_ctx* ctx, const uint8_t* residues, const uint64_t* off
     if (dev_alloc(&ctx->d_perm, n) != cudaSuccess) return nomem("perm");
     if (dev_alloc(&ctx->d_bnd, (units + ctx->win_units) * 16) != cudaSuccess) return nomem("boundary rows");
     ctx->db_units = (uint64_t)units;
-    if (dev_alloc(&ctx->d_scores, n + 1) != cudaSuccess) return nomem("scores");
+    if (dev_alloc(&ctx->d_counters, kCounters + n + 1) != cudaSuccess) return nomem("scores");
+    ctx->d_scores = ctx->d_counters + kCounters;
     if (dev_alloc(&ctx->d_scores_rec, n + 1) != cudaSuccess) return nomem("scores");
     if (dev_alloc(&ctx->d_ovf, n + 1) != cudaSuccess) return nomem("overflow list");
     ctx->max_cols = max_cols;
@@ -466,11 +485,20 @@ int plain_cell(int lo, int hi, int q, int e) {
     return kCellNarrow;
 }
 
-// Blocks per SM for a kernel of a shape at a query length (0 = does not fit).
-static int kernel_occupancy(sw_ctx* ctx, const void* fn, int block, size_t smem) {
-    if (smem > (size_t)ctx->max_smem) return 0;
+// Blocks per SM for a kernel (v: 0 plain, 1 stacked) of a shape at a query
+// length (0 = does not fit).  The runtime is asked only where shared memory
+// can make a difference: it takes about a microsecond, and a layout looks at a
+// dozen shapes.
+static int kernel_occupancy(sw_ctx* ctx, const WfKernel& k, int v, int qlen) {
+    int n = 0;
+    const sw_ctx::PlainFit& f = ctx->plain_fit[&k - wf_kernels(&n)];
+    const size_t smem = k.smem(qlen);
+    if (smem > (size_t)f.max_dyn[v]) return 0;
+    if (f.blocks[v] <= 1) return f.blocks[v];
     int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, block, smem) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+            &nb, v ? k.batch_fn : k.fn[ctx->cell], v ? k.block : plain_block(ctx, k), smem) !=
+        cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
@@ -478,7 +506,7 @@ static int kernel_occupancy(sw_ctx* ctx, const void* fn, int block, size_t smem)
 }
 
 int shape_occupancy(sw_ctx* ctx, const WfKernel& k, int qlen) {
-    return kernel_occupancy(ctx, k.batch_fn, k.block, k.smem(qlen));
+    return kernel_occupancy(ctx, k, 1, qlen);
 }
 
 int plain_block(const sw_ctx* ctx, const WfKernel& k) {
@@ -486,7 +514,7 @@ int plain_block(const sw_ctx* ctx, const WfKernel& k) {
 }
 
 int plain_occupancy(sw_ctx* ctx, const WfKernel& k, int qlen) {
-    return kernel_occupancy(ctx, k.fn[ctx->cell], plain_block(ctx, k), k.smem(qlen));
+    return kernel_occupancy(ctx, k, 0, qlen);
 }
 
 // Query rows one launch of a shape scores: the whole query when its profile
@@ -936,13 +964,10 @@ struct Split {
 // Pipelines of P warps one block of a long kernel holds (0: none fits).
 int long_pipelines(sw_ctx* ctx, const LongKernel& k, int P, size_t* smem) {
     if (P > kLongMaxPasses) return 0;
-    cudaFuncAttributes fa;
-    if (cudaFuncGetAttributes(&fa, k.fn[ctx->cell]) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
-    const size_t dyn = (size_t)ctx->max_smem - fa.sharedSizeBytes;
-    const int warp_regs = (fa.numRegs + 7) / 8 * 8 * 32;
+    int n = 0;
+    const sw_ctx::LongFit& f = ctx->long_fit[&k - long_kernels(&n)];
+    const size_t dyn = (size_t)f.max_dyn;
+    const int warp_regs = (f.regs + 7) / 8 * 8 * 32;
     int G = std::min(k.max_threads / 32, ctx->regs_per_sm / std::max(warp_regs, 1)) / P;
     while (G > 0 && k.smem(P, G) > dyn) --G;
     *smem = dyn;
@@ -1505,8 +1530,8 @@ sw_status enqueue_search(sw_ctx* ctx, const uint8_t* d_query, int qlen, int64_t 
     mk.fp_launches = 0;
     mk.cells = (uint64_t)qlen * ctx->n_residues;
     SW_CUDA(ctx, cudaEventRecord(mk.e[0], st));
-    SW_CUDA(ctx, cudaMemsetAsync(ctx->d_counters, 0, 16 * sizeof(int), st));
-    SW_CUDA(ctx, cudaMemsetAsync(ctx->d_scores, 0, (size_t)(ctx->n_records + 1) * sizeof(int), st));
+    SW_CUDA(ctx, cudaMemsetAsync(ctx->d_counters, 0,
+                                 (size_t)(kCounters + ctx->n_records + 1) * sizeof(int), st));
     SW_CUDA(ctx, cudaEventRecord(mk.e[1], st));
     if (L.win.n > 0) {
         WindowArgs w;
@@ -1680,6 +1705,7 @@ sw_status enqueue_search(sw_ctx* ctx, const uint8_t* d_query, int qlen, int64_t 
         t.rec_stride = 0;
         t.out_stride = 0;
         t.rows = nullptr;
+        t.count = blocks == 1 ? ctx->d_counters + 2 : nullptr;
         void* args[] = {&t};
         SW_CUDA(ctx, cudaLaunchKernel((const void*)sw_topk_round, dim3((unsigned)blocks),
                                       dim3(kTopkThreads), args, 0, st));
@@ -1784,11 +1810,9 @@ sw_status search_host(sw_ctx* ctx, const uint8_t* query, uint32_t qlen, sw_hit* 
     st = enqueue_search(ctx, ctx->d_query, (int)qlen, query_span(ctx, query, qlen),
                         scores ? ctx->d_scores_rec : nullptr, &keys, &launches);
     if (st != SW_OK) return st;
-    SW_CUDA(ctx, cudaMemcpyAsync(ctx->h_keys, keys, (size_t)k * sizeof(unsigned long long),
+    // the hits and, behind them, the count of re-scored records
+    SW_CUDA(ctx, cudaMemcpyAsync(ctx->h_keys, keys, (size_t)(k + 1) * sizeof(unsigned long long),
                                  cudaMemcpyDeviceToHost, ctx->stream));
-    int* const rescored = reinterpret_cast<int*>(ctx->h_keys + kMaxTopK);
-    SW_CUDA(ctx, cudaMemcpyAsync(rescored, ctx->d_counters + 2, sizeof(int), cudaMemcpyDeviceToHost,
-                                 ctx->stream));
     if (scores)
         SW_CUDA(ctx, cudaMemcpyAsync(scores, ctx->d_scores_rec,
                                      (size_t)ctx->n_records * sizeof(int32_t),
@@ -1810,7 +1834,7 @@ sw_status search_host(sw_ctx* ctx, const uint8_t* query, uint32_t qlen, sw_hit* 
     ctx->stats.kernel_ms = kms;
     ctx->stats.first_pass_ms = fpms;
     ctx->stats.cells = (uint64_t)qlen * ctx->n_residues;
-    ctx->stats.rescored = (uint64_t)*rescored;
+    ctx->stats.rescored = ctx->h_keys[k];
     ctx->stats.launches = launches;
     ctx->stats.queries = 1;
     ctx->stats.total_ms = now_ms() - t0;

@@ -47,6 +47,8 @@ struct sw_batch_state;   // batched search buffers and captured graphs (sw_batch
 struct sw_serve_state;   // serving loop: slots, ring of DB chunks, scheduler (sw_serve.cu)
 struct sw_tb_state;      // traceback scratch (sw_traceback.cu)
 
+constexpr int kCounters = 16;
+
 struct sw_ctx {
     int device = 0;
     int num_sms = 0;
@@ -75,7 +77,20 @@ struct sw_ctx {
     int row_best[32] = {};             // per query code: its best score (at least 0)
     int cell = 0;                      // PlainCell of the plain kernel's launches
     int8_t* d_mat = nullptr;           // 32x32 int8, codes >= 24 zeroed
-    int* d_counters = nullptr;         // [0],[1] pair counters, [2] overflow count
+    // the plain kernels' blocks per SM with no dynamic shared memory, by
+    // wf_kernels() index ([0] fn[cell] at plain_block, [1] batch_fn at block), and
+    // the long-pair kernels' attributes by long_kernels() index
+    struct PlainFit {
+        int blocks[2];
+        int max_dyn[2];
+    };
+    struct LongFit {
+        int regs, max_dyn;
+    };
+    std::vector<PlainFit> plain_fit;
+    std::vector<LongFit> long_fit;
+    int* d_counters = nullptr;         // [0],[1] pair counters, [2] overflow count; kCounters
+                                       // entries in front of d_scores (cleared together)
 
     // resident DB
     bool db_loaded = false;
