@@ -24,7 +24,7 @@
 // one), 5.5 with the byte profile's extraction.  The profile is read from shared memory,
 // one conflict-free 16- or 4-byte word per 4 rows; looking each cell up in the
 // matrix cost a bank-conflicted load per cell.  10,000 records, query 375:
-// 4,400 us a call before (256 warps, 512-row passes, matrix lookups), 586 now.
+// 4,400 us a call before (256 warps, 512-row passes, matrix lookups), 559 now.
 //
 // A record is a serial chain of columns, so records longer than an even share
 // of the columns are cut into windows that overlap by the longest span an
@@ -269,29 +269,34 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) sw_score_noalloc_kernel(c
         }
     };
     // The long records first, so that a unit claimed last is short.  An item
-    // is window k of 4 neighbouring records, those of them that have one.
+    // is window k of 4 neighbouring records, those of them that have one; of one
+    // record where the claims are few (up to 16 a warp), since a warp scores an
+    // item's records one after the other while others idle (us with 4 -> with 1:
+    // 181 records, query 444 386 -> 196, 3,000 and 375 430 -> 288, 5,000 and
+    // 1,500 2,047 -> 1,449).
     const int big = (int)min(max(share / 8, 128ll), (long long)L);
     if (big < max_len) {
-        const long long groups = ((long long)a.n + 3) / 4;
         // (stride is only meaningful where a record is longer than a window)
-        const long long items =
-            groups * (max_len <= L ? 1 : 1 + (max_len - L + stride - 1) / stride);
+        const long long windows = max_len <= L ? 1 : 1 + (max_len - L + stride - 1) / stride;
+        const int per = a.n * windows > 16 * warps ? 4 : 1;
+        const long long groups = ((long long)a.n + per - 1) / per;
+        const long long items = groups * windows;
         while (true) {
             unsigned long long it = 0;
             if (lane == 0) it = atomicAdd(&h->item, 1ull);
             it = __shfl_sync(FULL, it, 0);
             if ((long long)it >= items) break;
             const int k = (int)((long long)it / groups);
-            const long long rec = ((long long)it - k * groups) * 4 + (lane & 3);
+            const long long rec = ((long long)it - k * groups) * per + (lane & (per - 1));
             const int len = rec < a.n ? na_len(a, (int)rec) : 0;
             const bool has = len > big && len <= kNaMaxLen &&
                              (k == 0 || (len > L && k <= (len - L + stride - 1) / stride));
-            unsigned todo = __ballot_sync(FULL, has && lane < 4);
+            unsigned todo = __ballot_sync(FULL, has && lane < per);
             while (todo) {
                 const int src = __ffs(todo) - 1;
                 todo &= todo - 1;
                 const int n = __shfl_sync(FULL, len, src);
-                score((int)(rec - (lane & 3)) + src, k > 0 ? k * stride : 0,
+                score((int)(rec - (lane & (per - 1))) + src, k > 0 ? k * stride : 0,
                       k > 0 ? min(L, n - k * stride) : min(L, n), n > L);
             }
         }
