@@ -7,9 +7,9 @@
 namespace swb {
 
 constexpr int kTopkThreads = 1024;
-constexpr int kTopkKeys = 4096;     // keys sorted per block and round
+constexpr int kTopkKeys = 4096;     // keys per block and round
 constexpr int kMaxTopK = 1024;      // so that every round shrinks the key set
-constexpr int kTopkSelect = 128;    // up to this many hits: repeated maxima instead of a sort
+constexpr int kTopkSelect = 128;    // up to this many hits: repeated maxima instead of a search
 
 constexpr int kRescoreBlocks = 148;   // x 64 threads: 296 warps
 constexpr int kRescoreWarps = kRescoreBlocks * 2;
