@@ -280,10 +280,42 @@ def _top_equal(hits, want_scores, k=10) -> bool:
     return [h[0] for h in hits] == ws.tolist() and [h[1] for h in hits] == wi.tolist()
 
 
+def sampled_parity(db, queries, gpu, n=2000):
+    """Without the reference's kernels: the scores of n seeded records against
+    the C restatement of its scoring."""
+    import oracle
+    from swhybrid_b200 import param
+    m = param.blosum62()
+    pick = np.random.default_rng(1).choice(db.n, size=min(n, db.n), replace=False)
+    sub = db.subset(pick)
+    bad, checked = 0, 0
+    for i in range(0, len(queries), 4):
+        want = oracle.search(queries[i], sub.residues, sub.offsets, m, 12, 2)
+        bad += int(np.count_nonzero(gpu["sweep"][i][1][pick] != want))
+        checked += 1
+    return {"sweep": {"queries": checked, "records": len(pick), "mismatches": bad},
+            "reference": "C restatement of the reference's scoring, sampled records"}
+
+
 # ---------------------------------------------------------------------------
+NO_REFERENCE = "the reference's kernels are not built (oracle/_ref needs its source tree)"
+
+
+def have_reference() -> bool:
+    import oracle
+    try:
+        oracle.ref_threads()
+    except FileNotFoundError:
+        return False
+    return True
+
+
 def run_reference(args, rank, world):
     """--impl reference: the reference CPU kernels only, rank 0."""
     if rank != 0:
+        return
+    if not have_reference():
+        print(json.dumps({"impl": "reference", "unavailable": NO_REFERENCE}), flush=True)
         return
     import oracle
     from swhybrid_b200 import param
@@ -929,7 +961,12 @@ def main(argv=None):
     # all ranks meet at the final barrier (with or without one)
     line, db, queries, gpu_scores = run_ours(args, rank, world, local_rank)
     if line is not None and rank == 0 and world == 1 and not args.no_cpu_baseline:
-        cb, _, parity = cpu_baseline(db, queries, args.cpu_seconds, gpu_scores)
+        if have_reference():
+            cb, _, parity = cpu_baseline(db, queries, args.cpu_seconds, gpu_scores)
+        else:
+            cb = {"unavailable": NO_REFERENCE}
+            parity = (sampled_parity(db, queries, gpu_scores)
+                      if gpu_scores and gpu_scores.get("sweep") else None)
         if parity is not None:
             line["parity"] = parity
         line["cpu_baseline"] = {k: (round(v, 3) if isinstance(v, float) else v)
