@@ -69,17 +69,18 @@ typedef struct sw_hit {
  * kept in registers per thread (an even number).  Pairs of records with more
  * than cutover columns run concurrently in the long-pair kernel, whose query
  * passes are pipelined across the warps of a block: the long shape's rows per
- * thread when it is 32 x {8, 16, 24, 32, 64} and differs from the short shape,
- * otherwise chosen automatically (the smallest row count of at most 3 passes).
- * The rest use the short shape.  cutover 0: automatic (a split only when the
- * DB's longest pairs would dominate the bulk launch, else one shape -- the
- * long one -- for the whole DB).  sw_run_stats.used reports what ran. */
+ * thread when it is 32 x {4, 6, 8, 12, 16, 20, 24, 32, 64} and differs from the
+ * short shape, otherwise chosen automatically (the smallest row count of at
+ * most 3 passes).  The rest use the short shape.  cutover 0: automatic (where
+ * the DB's longest pairs would dominate the bulk launch they are cut into
+ * windows or split off, else one shape -- the long one -- for the whole DB).
+ * sw_run_stats.used reports what ran. */
 typedef struct sw_kernel_config {
     int32_t long_group_width;
     int32_t long_rows_per_thread;
     int32_t short_group_width;
     int32_t short_rows_per_thread;
-    int32_t cutover;        /* columns; 0 = one shape for the whole DB */
+    int32_t cutover;        /* columns; 0 = automatic */
 } sw_kernel_config;
 
 typedef struct sw_db_stats {
@@ -266,7 +267,10 @@ typedef struct sw_plan_step {
  * when its shapes fit that length (else the cost model chooses).  A new
  * context starts with the table measured on B200 that is compiled into the
  * library (swhybrid_b200/tuned/b200.json); this call replaces it, and n = 0
- * clears it (the cost model alone chooses).
+ * clears it (the cost model alone chooses).  With the built-in table a time
+ * model may take another bulk shape, windows or a long-pair split where the
+ * DB's longest pairs ask for one; this call's entries keep their shapes and
+ * their cut-overs.
  *
  * plan (optional, plan[0].group_width = 0 for none): the query's rows in
  * consecutive row segments of different shapes, so that only the last
@@ -344,7 +348,8 @@ sw_status sw_get_totals(const struct sw_ctx *ctx, sw_totals *out);
  * query) and scored by one launch of shape group_width x rows_per_thread;
  * longer queries form stacks of their own, grouped by the shape the tuning
  * table gives their length.  Pairs of records longer than cutover columns run
- * in a concurrent launch with the long shape (0 = no split).  use_graph != 0
+ * in a concurrent launch with the long shape (0: those too long for the paired
+ * launches run beside them in the long-pair kernel).  use_graph != 0
  * captures each batch signature (query count and lengths) as a CUDA graph and
  * replays it. */
 typedef struct sw_batch_options {
@@ -486,8 +491,8 @@ sw_status sw_serve_start(struct sw_ctx *ctx, const sw_serve_options *opt);
 
 /* Queues a request (codes 0..24, 1..2^24 residues).  SW_ERR_BUSY when
  * max_pending requests already wait; SW_ERR_STATE when not serving.  A
- * request longer than one stack of the serving shape holds (8,192 rows for
- * the default 16 x 64; its query profile must fit one block's shared memory)
+ * request longer than one stack of the serving shape holds (and than 8,192
+ * residues; its query profile must fit one block's shared memory)
  * is scored alone at a round boundary by the plain path, which splits its
  * rows over consecutive launches, instead of sharing the round's launches. */
 sw_status sw_serve_submit(struct sw_ctx *ctx, uint64_t request_id, const uint8_t *query,

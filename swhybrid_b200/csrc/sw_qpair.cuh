@@ -3,7 +3,7 @@
 // In the plain and stacked kernels (sw_wavefront.cuh) a 32-bit register
 // holds one query row against two DB records, so every row of every column
 // step must assemble its two profile scores (one per record residue) with a
-// PRMT: 1 of the 5.5 ALU-pipe instructions per row.  When a batch has many
+// PRMT: 1 of the 4.5 ALU-pipe instructions per row.  When a batch has many
 // queries, the two 16-bit lanes can instead hold two QUERIES against one
 // record: both lanes then look up the same residue, and the profile can be
 // stored already packed -- word (code, row) = score of query A's row against
