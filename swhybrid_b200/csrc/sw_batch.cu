@@ -897,6 +897,21 @@ extern "C" sw_status sw_search_batch(sw_ctx* ctx, uint32_t nq, const uint8_t* qu
                   (uint64_t)(b->opt.pair_long != 0));
     sig.push_back((uint64_t)b->opt.pair_regions);
     for (uint32_t i = 0; i < nq; ++i) sig.push_back(qlen[i]);
+    // what the graph holds of the plan: the shapes also follow the tuning table
+    // and the shape override, which the caller may change between batches
+    sig.push_back((uint64_t)ml.total);
+    for (const BatchLaunch& L : launches) {
+        sig.push_back((uint64_t)(uintptr_t)(L.qk ? (const void*)L.qk : (const void*)L.k));
+        sig.push_back((uint64_t)L.grid << 32 | (uint32_t)L.threads);
+        sig.push_back((uint64_t)L.smem);
+        sig.push_back((uint64_t)L.sbegin << 32 | (uint32_t)L.scount);
+        sig.push_back((uint64_t)L.pair_begin << 32 | (uint32_t)L.pair_count);
+        sig.push_back((uint64_t)L.counter_base << 32 | (uint32_t)L.long_units);
+        sig.push_back((uint64_t)L.bnd_group << 1 | (L.long_part ? 1u : 0u));
+    }
+    sig.push_back((uint64_t)lplan.n_long << 32 | (uint32_t)lplan.sms);
+    for (int i = 0; i < kLongBuckets; ++i)
+        sig.push_back((uint64_t)lplan.items[i].size() << 32 | (uint32_t)lplan.smem[i]);
     uint32_t n_launch = 0;
     SW_CUDA(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
     if (b->opt.use_graph) {
