@@ -254,7 +254,7 @@ sw_status enqueue_batch(sw_ctx* ctx, sw_batch_state* b, uint32_t nq, size_t qbyt
     SW_CUDA(ctx, cudaMemcpyAsync(b->d_meta, b->h_stage + meta_at, ml.total,
                                  cudaMemcpyHostToDevice, st));
     const int nst = ml.nst;
-    SW_CUDA(ctx, cudaMemsetAsync(b->d_counters, 0, (2 * (size_t)nst + 1 + ml.nqp + kLongBuckets) * sizeof(int),
+    SW_CUDA(ctx, cudaMemsetAsync(b->d_counters, 0, (2 * (size_t)nst + 1 + ml.nqp + 1) * sizeof(int),
                                  st));
     SW_CUDA(ctx, cudaMemsetAsync(b->d_scores, 0, (size_t)nq * n_rec * sizeof(int), st));
     const uint32_t* d_qoff = reinterpret_cast<const uint32_t*>(b->d_meta + ml.qoff);
@@ -778,7 +778,7 @@ extern "C" sw_status sw_search_batch(sw_ctx* ctx, uint32_t nq, const uint8_t* qu
     }
     // counters: bulk of stack i at [i], long at [nst_total + i], overflow count
     // at [2 nst_total], paired double stack j at [2 nst_total + 1 + j], then the
-    // long items' per row count
+    // long items'
     const MetaLayout ml = meta_layout(nq, sp, lplan.count());
 
     // ---- buffers (before any capture) ----
@@ -791,7 +791,7 @@ extern "C" sw_status sw_search_batch(sw_ctx* ctx, uint32_t nq, const uint8_t* qu
         }
         b->graphs.clear();
     };
-    const size_t counters_need = 2 * (size_t)nst_total + 1 + ml.nqp + kLongBuckets;
+    const size_t counters_need = 2 * (size_t)nst_total + 1 + ml.nqp + 1;
     if (std::max<uint64_t>(qbytes, 1) > b->queries_cap || ml.total > b->meta_cap ||
         counters_need > b->counters_cap)
         drop_graphs();
@@ -876,11 +876,7 @@ extern "C" sw_status sw_search_batch(sw_ctx* ctx, uint32_t nq, const uint8_t* qu
         memcpy(m + ml.qp_flags, sp.qp_flags.data(), 4 * nqp);
         memcpy(m + ml.qp_slot, sp.qp_slot.data(), 4 * nqp);
         memcpy(m + ml.qp_rbmap, sp.qp_rb_map.data(), 4 * sp.qp_rb_map.size());
-        uint8_t* at = m + ml.items;
-        for (const auto& v : lplan.items) {
-            memcpy(at, v.data(), 4 * v.size());
-            at += 4 * v.size();
-        }
+        memcpy(m + ml.items, lplan.items.data(), 4 * lplan.items.size());
         memcpy(m + ml.codes, sp.codes.data(), sp.codes.size());
     }
 
@@ -910,8 +906,7 @@ extern "C" sw_status sw_search_batch(sw_ctx* ctx, uint32_t nq, const uint8_t* qu
         sig.push_back((uint64_t)L.bnd_group << 1 | (L.long_part ? 1u : 0u));
     }
     sig.push_back((uint64_t)lplan.n_long << 32 | (uint32_t)lplan.sms);
-    for (int i = 0; i < kLongBuckets; ++i)
-        sig.push_back((uint64_t)lplan.items[i].size() << 32 | (uint32_t)lplan.smem[i]);
+    sig.push_back((uint64_t)lplan.items.size() << 32 | (uint32_t)lplan.smem);
     uint32_t n_launch = 0;
     SW_CUDA(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
     if (b->opt.use_graph) {

@@ -252,9 +252,7 @@ extern "C" sw_status sw_ctx_create(int device, const sw_params* params, sw_ctx**
             return fail(SW_ERR_CUDA);
         ctx->long_fit.push_back({fa.numRegs, ctx->max_smem - (int)fa.sharedSizeBytes});
     }
-    const LongItemKernel* liks = long_item_kernels(&nk);
-    for (int i = 0; i < nk; ++i)
-        if (!allow_smem(liks[i].fn[ctx->cell])) return fail(SW_ERR_CUDA);
+    if (!allow_smem(long_item_kernel().fn[ctx->cell])) return fail(SW_ERR_CUDA);
     *out = ctx;
     return SW_OK;
 }
@@ -1153,31 +1151,24 @@ static double qp_clocks(const std::vector<QpLoad>& loads, double cols, double lo
     return t;
 }
 
-static int long_bucket(uint32_t qlen) {
-    int n = 0;
-    const LongItemKernel* k = long_item_kernels(&n);
-    for (int i = 0; i < n; ++i)
-        if (qlen <= (uint32_t)(32 * k[i].R * kLongItemWarps)) return i;
-    return -1;
-}
-
 LongItemPlan plan_long_items(sw_ctx* ctx, const std::vector<uint32_t>& qlen,
                              const std::vector<QpLoad>& loads, int groups_per_sm, int rows_per_pass,
                              double chunks, int64_t given) {
     LongItemPlan plan;
     const int64_t np = ctx->n_pairs;
-    int nk = 0;
-    const LongItemKernel* lk = long_item_kernels(&nk);
-    if (np == 0 || nk != kLongBuckets) return plan;
+    if (np == 0) return plan;
+    auto step_of = [](uint32_t q, int* pipes) {
+        const int R = long_item_rows((int)q), P = (int)((q + 32 * R - 1) / (32 * R));
+        *pipes = kLongItemWarps / P;
+        return long_step_clocks(R, P * *pipes);
+    };
     // per pair column: SM clocks of all queries, and the slowest query's step
     double per_col = 0, slow = 0;
     for (const uint32_t q : qlen) {
         if (q == 0) continue;
-        const int b = long_bucket(q);
-        if (b < 0) return plan;                      // too long for a block's warps
-        const int P = (int)((q + 32 * lk[b].R - 1) / (32 * lk[b].R));
-        const int G = kLongItemWarps / P;
-        const double step = long_step_clocks(lk[b].R, P * G);
+        if (q > (uint32_t)kLongItemRows) return plan;     // too long for a block's warps
+        int G = 0;
+        const double step = step_of(q, &G);
         per_col += step / G;
         slow = std::max(slow, step);
     }
@@ -1219,67 +1210,56 @@ LongItemPlan plan_long_items(sw_ctx* ctx, const std::vector<uint32_t>& qlen,
         uint32_t q, pair;
         double t;
     };
-    std::vector<Item> list[kLongBuckets];
+    std::vector<Item> list;
     for (uint32_t q = 0; q < (uint32_t)qlen.size(); ++q) {
         if (qlen[q] == 0) continue;
-        const int b = long_bucket(qlen[q]);
-        const int P = (int)((qlen[q] + 32 * lk[b].R - 1) / (32 * lk[b].R)), G = kLongItemWarps / P;
-        plan.smem[b] = std::max(plan.smem[b], lk[b].smem(P, G));
+        int G = 0;
+        const double step = step_of(qlen[q], &G);
+        plan.smem = std::max(plan.smem, long_item_smem((int)qlen[q]));
         for (int64_t p = 0; p < plan.n_long; p += G)
-            list[b].push_back(Item{q, (uint32_t)p, ctx->pair_ncols[p] * long_step_clocks(lk[b].R, P * G)});
+            list.push_back(Item{q, (uint32_t)p, ctx->pair_ncols[p] * step});
     }
-    for (int b = 0; b < kLongBuckets; ++b) {
-        if (plan.smem[b] > (size_t)ctx->max_smem - 1024) return LongItemPlan{};
-        std::stable_sort(list[b].begin(), list[b].end(),
-                         [](const Item& x, const Item& y) { return x.t > y.t; });
-        for (const Item& i : list[b]) {
-            plan.items[b].push_back(i.q);
-            plan.items[b].push_back(i.pair);
-        }
+    if (plan.smem > (size_t)ctx->max_smem - 1024) return LongItemPlan{};
+    std::stable_sort(list.begin(), list.end(),
+                     [](const Item& x, const Item& y) { return x.t > y.t; });
+    for (const Item& i : list) {
+        plan.items.push_back(i.q);
+        plan.items.push_back(i.pair);
     }
     return plan;
 }
 
-// The plan's launches (one per row count, longest queries first), `sms` blocks
-// each; d_items holds the buckets' items back to back.
+// The plan's launch, at most `sms` blocks.
 sw_status launch_long_items(sw_ctx* ctx, cudaStream_t stream, const LongItemPlan& plan,
-                            const uint2* d_items, int* d_counters, const uint8_t* d_queries,
+                            const uint2* d_items, int* d_counter, const uint8_t* d_queries,
                             const uint32_t* d_qoff, const uint32_t* d_qlens, int* d_scores,
                             int* d_ovf, int* d_ovf_count, int ovf_cap, uint32_t* launches) {
-    int nk = 0;
-    const LongItemKernel* lk = long_item_kernels(&nk);
-    size_t at[kLongBuckets], n_all = 0;
-    for (int b = 0; b < kLongBuckets; ++b) {
-        at[b] = n_all;
-        n_all += plan.items[b].size() / 2;
-    }
-    for (int b = kLongBuckets - 1; b >= 0; --b) {
-        const int n = (int)(plan.items[b].size() / 2);
-        if (n == 0) continue;
-        LongItemArgs a;
-        a.db = ctx->d_db;
-        a.pairs = ctx->d_pairs;
-        a.n_pairs = (int)plan.n_long;
-        a.items = d_items + at[b];
-        a.n_items = n;
-        a.counter = d_counters + b;
-        a.queries = d_queries;
-        a.qoff = d_qoff;
-        a.qlens = d_qlens;
-        a.mat = ctx->d_mat;
-        a.gap_oe = ctx->params.gap_open + ctx->params.gap_extend;
-        a.gap_e = ctx->params.gap_extend;
-        a.scores = d_scores;
-        a.n_records = (int)ctx->n_records;
-        a.ovf_list = d_ovf;
-        a.ovf_count = d_ovf_count;
-        a.ovf_thresh = 32767 - std::max(ctx->max_score, 1) + 1;
-        a.ovf_cap = ovf_cap;
-        void* args[] = {&a};
-        SW_CUDA(ctx, cudaLaunchKernel(lk[b].fn[ctx->cell], dim3((unsigned)std::min(n, plan.sms)),
-                                      dim3(32 * kLongItemWarps), args, plan.smem[b], stream));
-        ++*launches;
-    }
+    const int n = (int)plan.count();
+    if (n == 0) return SW_OK;
+    LongItemArgs a;
+    a.db = ctx->d_db;
+    a.pairs = ctx->d_pairs;
+    a.n_pairs = (int)plan.n_long;
+    a.items = d_items;
+    a.n_items = n;
+    a.counter = d_counter;
+    a.queries = d_queries;
+    a.qoff = d_qoff;
+    a.qlens = d_qlens;
+    a.mat = ctx->d_mat;
+    a.gap_oe = ctx->params.gap_open + ctx->params.gap_extend;
+    a.gap_e = ctx->params.gap_extend;
+    a.scores = d_scores;
+    a.n_records = (int)ctx->n_records;
+    a.ovf_list = d_ovf;
+    a.ovf_count = d_ovf_count;
+    a.ovf_thresh = 32767 - std::max(ctx->max_score, 1) + 1;
+    a.ovf_cap = ovf_cap;
+    void* args[] = {&a};
+    SW_CUDA(ctx, cudaLaunchKernel(long_item_kernel().fn[ctx->cell],
+                                  dim3((unsigned)std::min(n, plan.sms)), dim3(32 * kLongItemWarps),
+                                  args, plan.smem, stream));
+    ++*launches;
     return SW_OK;
 }
 

@@ -148,18 +148,12 @@ namespace swb {
 struct QpLoad {                        // a paired-query launch: passes of its double stacks
     double sum_passes = 0, max_passes = 0;
 };
-constexpr int kLongBuckets = 3;        // row counts of sw_long_items ...
-constexpr uint32_t kLongItemRows = 8192;   // ... and the query rows the tallest holds
 struct LongItemPlan {
     int64_t n_long = 0;                // pairs [0, n_long); 0: no split
     int sms = 0;                       // SMs the first paired launch leaves free
-    std::vector<uint32_t> items[kLongBuckets];   // (query, first pair) per row count
-    size_t smem[kLongBuckets] = {};
-    size_t count() const {
-        size_t n = 0;
-        for (const auto& v : items) n += v.size() / 2;
-        return n;
-    }
+    std::vector<uint32_t> items;       // (query, first pair), longest first
+    size_t smem = 0;
+    size_t count() const { return items.size() / 2; }
 };
 // The split of the pairs for queries of the given lengths (0: none), or of
 // `n_long` pairs when that is >= 0.  cols, units: columns and pairs of the
@@ -168,7 +162,7 @@ LongItemPlan plan_long_items(sw_ctx* ctx, const std::vector<uint32_t>& qlen,
                              const std::vector<QpLoad>& loads, int groups_per_sm, int rows_per_pass,
                              double chunks, int64_t n_long);
 sw_status launch_long_items(sw_ctx* ctx, cudaStream_t stream, const LongItemPlan& plan,
-                            const uint2* d_items, int* d_counters, const uint8_t* d_queries,
+                            const uint2* d_items, int* d_counter, const uint8_t* d_queries,
                             const uint32_t* d_qoff, const uint32_t* d_qlens, int* d_scores,
                             int* d_ovf, int* d_ovf_count, int ovf_cap, uint32_t* launches);
 struct WfKernel;

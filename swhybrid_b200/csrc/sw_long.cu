@@ -279,17 +279,64 @@ __global__ void __launch_bounds__(LongBlock<R>::value, 1) sw_long(const LongArgs
     }
 }
 
+// One item of sw_long_items at R rows a lane (whole block).
+template <int R, class CELL>
+__device__ __forceinline__ void long_item(const LongItemArgs& a, const CELL& K, uint2* smem,
+                                          uint32_t* s_max, const uint2 item, int qlen,
+                                          bool new_query) {
+    using W = LongWarp<R, CELL>;
+    const int warp = (int)(threadIdx.x >> 5);
+    const int query = (int)item.x;
+    const int P = (qlen + 32 * R - 1) / (32 * R);
+    const int G = kLongItemWarps / P;
+    if (new_query)
+        build_profile<kLT, R>(smem, a.queries + a.qoff[query], qlen, a.mat, P, K.profile_bias());
+    const int g = warp / P, w = warp - g * P;
+    const int pair = (int)item.y + g;
+    const bool active = g < G && pair < a.n_pairs;
+    W x(K);
+    __syncthreads();                 // profile built
+    int span = 0;
+    if (active) {
+        x.place(smem, smem + (size_t)P * W::NJ * W::JSTRIDE + (size_t)g * (P > 1 ? P - 1 : 0) * kLRing,
+                w, P);
+        x.begin(a.db, a.pairs[pair]);
+        span = W::span_of(x.ncols);
+    }
+    // the item's first pair is its longest
+    const int total = (P - 1) * kLD + W::span_of((int)a.pairs[item.y].ncols);
+    for (int gs = 0; gs < total; gs += kLK) {
+        const int s0 = gs - w * kLD;
+        if (active && s0 >= 0 && s0 < span) x.interval(s0);
+        __syncthreads();
+    }
+    uint32_t m = x.HZ;
+    if (active) {
+        m = x.maximum();
+        if (x.t == 0) s_max[warp] = m;
+    }
+    __syncthreads();
+    if (active && w == 0 && x.t == 0) {
+        for (int i = 1; i < P; ++i) m = __vimax3_s16x2(m, s_max[warp + i], x.HZ);
+        long_scores(a.scores, query * a.n_records, 2 * pair, a.n_records, m, (int)(x.HZ & 0xffffu),
+                    a.ovf_thresh - K.stored_shift(), a.ovf_list, a.ovf_count, a.ovf_cap, false);
+    }
+}
+
 // Batched search and serving: items of one query and as many neighbouring
 // pairs as a block of kLongItemWarps warps holds pipelines for (similar
-// lengths, the table being longest first), claimed longest first.
-template <int R, class CELL>
+// lengths, the table being longest first), claimed longest first.  One launch
+// takes the items of every row count: it has its SMs while the first paired
+// launch leaves them free, and a launch queued behind another one of the side
+// stream met the next paired launch's blocks there and waited for their end (64
+// queries of 50..5,000 residues against 57,000 records, paired shape 16x48: 324
+// ms with a launch per row count, 229 now; 8x64: 289, 225).
+template <class CELL>
 __global__ void __launch_bounds__(32 * kLongItemWarps, 1) sw_long_items(const LongItemArgs a) {
-    using W = LongWarp<R, CELL>;
     extern __shared__ uint2 smem[];
     __shared__ int s_item;
     __shared__ uint32_t s_max[kLongItemWarps];
     const CELL K(a.gap_oe, a.gap_e);
-    const int warp = (int)(threadIdx.x >> 5);
     int query = -1;
     while (true) {
         __syncthreads();                 // the previous item is done
@@ -298,42 +345,12 @@ __global__ void __launch_bounds__(32 * kLongItemWarps, 1) sw_long_items(const Lo
         if (s_item >= a.n_items) break;
         const uint2 item = a.items[s_item];
         const int qlen = (int)a.qlens[item.x];
-        const int P = (qlen + 32 * R - 1) / (32 * R);
-        const int G = kLongItemWarps / P;
-        if ((int)item.x != query) {
-            query = (int)item.x;
-            build_profile<kLT, R>(smem, a.queries + a.qoff[query], qlen, a.mat, P, K.profile_bias());
-        }
-        const int g = warp / P, w = warp - g * P;
-        const int pair = (int)item.y + g;
-        const bool active = g < G && pair < a.n_pairs;
-        W x(K);
-        __syncthreads();                 // profile built
-        int span = 0;
-        if (active) {
-            x.place(smem, smem + (size_t)P * W::NJ * W::JSTRIDE + (size_t)g * (P > 1 ? P - 1 : 0) * kLRing,
-                    w, P);
-            x.begin(a.db, a.pairs[pair]);
-            span = W::span_of(x.ncols);
-        }
-        // the item's first pair is its longest
-        const int total = (P - 1) * kLD + W::span_of((int)a.pairs[item.y].ncols);
-        for (int gs = 0; gs < total; gs += kLK) {
-            const int s0 = gs - w * kLD;
-            if (active && s0 >= 0 && s0 < span) x.interval(s0);
-            __syncthreads();
-        }
-        uint32_t m = x.HZ;
-        if (active) {
-            m = x.maximum();
-            if (x.t == 0) s_max[warp] = m;
-        }
-        __syncthreads();
-        if (active && w == 0 && x.t == 0) {
-            for (int i = 1; i < P; ++i) m = __vimax3_s16x2(m, s_max[warp + i], x.HZ);
-            long_scores(a.scores, query * a.n_records, 2 * pair, a.n_records, m,
-                        (int)(x.HZ & 0xffffu), a.ovf_thresh - K.stored_shift(), a.ovf_list,
-                        a.ovf_count, a.ovf_cap, false);
+        const bool new_query = (int)item.x != query;
+        query = (int)item.x;
+        switch (long_item_rows(qlen)) {
+            case 4: long_item<4>(a, K, smem, s_max, item, qlen, new_query); break;
+            case 8: long_item<8>(a, K, smem, s_max, item, qlen, new_query); break;
+            default: long_item<16>(a, K, smem, s_max, item, qlen, new_query); break;
         }
     }
 }
@@ -354,19 +371,9 @@ constexpr LongKernel linst() {
                       &long_smem<R>, LongBlock<R>::value};
 }
 
-template <int R>
-constexpr LongItemKernel iinst() {
-    return LongItemKernel{R,
-                          {(const void*)&sw_long_items<R, CellWide>,
-                           (const void*)&sw_long_items<R, CellNarrow<0, 0>>,
-                           (const void*)&sw_long_items<R, CellNarrow<12, 2>>,
-                           (const void*)&sw_long_items<R, CellNarrow<12, 1>>},
-                          &long_smem<R>};
-}
-
-// kLongItemWarps passes of 32 R rows: up to 2,048, 4,096 and 8,192
-// (kLongItemRows) query rows
-const LongItemKernel kLongItemTable[] = {iinst<4>(), iinst<8>(), iinst<16>()};
+const LongItemKernel kLongItems{
+    {(const void*)&sw_long_items<CellWide>, (const void*)&sw_long_items<CellNarrow<0, 0>>,
+     (const void*)&sw_long_items<CellNarrow<12, 2>>, (const void*)&sw_long_items<CellNarrow<12, 1>>}};
 
 const LongKernel kLongTable[] = {
     linst<4>(),  linst<6>(),  linst<8>(),  linst<12>(), linst<16>(),
@@ -375,9 +382,11 @@ const LongKernel kLongTable[] = {
 
 }  // namespace
 
-const LongItemKernel* long_item_kernels(int* n) {
-    *n = (int)(sizeof(kLongItemTable) / sizeof(kLongItemTable[0]));
-    return kLongItemTable;
+const LongItemKernel& long_item_kernel() { return kLongItems; }
+
+size_t long_item_smem(int qlen) {
+    const int R = long_item_rows(qlen), P = (qlen + 32 * R - 1) / (32 * R), G = kLongItemWarps / P;
+    return R == 4 ? long_smem<4>(P, G) : R == 8 ? long_smem<8>(P, G) : long_smem<16>(P, G);
 }
 
 const LongKernel* long_kernels(int* n) {

@@ -45,6 +45,12 @@ const LongKernel* long_kernels(int* n);
 
 // Long pairs of several queries (batched search, serving): see sw_long_items.
 constexpr int kLongItemWarps = 16;
+constexpr int kLongItemRows = 32 * 16 * kLongItemWarps;    // longest query
+
+// Query rows per lane: the least whose passes the block's warps hold.
+__host__ __device__ constexpr int long_item_rows(int qlen) {
+    return qlen <= 32 * 4 * kLongItemWarps ? 4 : qlen <= 32 * 8 * kLongItemWarps ? 8 : 16;
+}
 
 struct LongItemArgs {
     const uint4* db;
@@ -67,11 +73,10 @@ struct LongItemArgs {
 };
 
 struct LongItemKernel {
-    int R;
-    const void* fn[kPlainCells];
-    size_t (*smem)(int passes, int pipelines);
+    const void* fn[kPlainCells];                // __global__ sw_long_items<cell>
 };
 
-const LongItemKernel* long_item_kernels(int* n);
+const LongItemKernel& long_item_kernel();
+size_t long_item_smem(int qlen);                // dynamic shared memory of a query's items
 
 }  // namespace swb

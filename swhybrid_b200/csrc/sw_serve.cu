@@ -45,6 +45,7 @@
 #include "sw_aux.h"
 #include "sw_device.cuh"
 #include "sw_engine.h"
+#include "sw_long.h"
 #include "sw_qpair.cuh"
 #include "sw_registry.h"
 
@@ -436,13 +437,7 @@ sw_status enqueue_round(sw_ctx* ctx, sw_serve_state* s, int chunk, int buf,
         memcpy(m + o_qpsl, qp_slot.data(), 4 * ne);
         memcpy(m + o_qpmap, qp_rbmap.data(), 4 * qp_rbmap.size());
     }
-    {
-        uint8_t* at = m + o_items;
-        for (const auto& v : lplan.items) {
-            if (!v.empty()) memcpy(at, v.data(), 4 * v.size());
-            at += 4 * v.size();
-        }
-    }
+    if (lplan.count()) memcpy(m + o_items, lplan.items.data(), 4 * lplan.items.size());
     if (!codes.empty()) memcpy(m + o_codes, codes.data(), codes.size());
     SW_CUDA(ctx, cudaEventRecord(s->start_ev[buf], st));
     SW_CUDA(ctx, cudaMemcpyAsync(s->d_meta, m, total, cudaMemcpyHostToDevice, st));
@@ -452,8 +447,8 @@ sw_status enqueue_round(sw_ctx* ctx, sw_serve_state* s, int chunk, int buf,
             SW_CUDA(ctx, cudaMemsetAsync(s->d_scores + (size_t)sl * n_rec, 0,
                                          (size_t)n_rec * sizeof(int), st));
     // counters: stack i at [i], the overflow count at [ns], paired entry j at
-    // [ns + 1 + j], then the long items' per row count
-    const size_t n_counters = ns + 1 + ne + kLongBuckets;
+    // [ns + 1 + j], then the long items'
+    const size_t n_counters = ns + 1 + ne + 1;
     if (n_counters > s->counters_cap)
         SW_SET(ctx, SW_ERR_UNSUPPORTED, "%zu paired launch entries exceed the counters (%zu)", ne,
                s->counters_cap);
@@ -993,7 +988,7 @@ extern "C" sw_status sw_serve_start(sw_ctx* ctx, const sw_serve_options* opt) {
                           ctx->pair_ncols.begin();
         if (n > 0 && n < npairs && n <= 4096) {
             s->n_long = n;
-            s->max_stack_rows = std::min(s->max_stack_rows, kLongItemRows);
+            s->max_stack_rows = std::min(s->max_stack_rows, (uint32_t)kLongItemRows);
         }
     }
     s->n_chunks = (int)std::max<int64_t>(1, std::min<int64_t>(o.chunks, std::max<int64_t>(npairs, 1)));
@@ -1034,7 +1029,7 @@ extern "C" sw_status sw_serve_start(sw_ctx* ctx, const sw_serve_options* opt) {
          cudaMemcpy(s->d_pair_ids, ids.data(), ids.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess))
         return fail("pair ring");
     if (dev_alloc(&s->d_scores, (size_t)s->n_slots * std::max(n_rec, 1)) != cudaSuccess ||
-        dev_alloc(&s->d_counters, 6 * (size_t)s->n_slots + 16 + kLongBuckets) != cudaSuccess)
+        dev_alloc(&s->d_counters, 6 * (size_t)s->n_slots + 17) != cudaSuccess)
         return fail("slots");
     // overflow entries: one per (request, record) at worst, bounded
     s->ovf_cap = std::min<size_t>((size_t)s->n_slots * std::max(n_rec, 1),
@@ -1082,7 +1077,7 @@ extern "C" sw_status sw_serve_start(sw_ctx* ctx, const sw_serve_options* opt) {
     // stacks (at most one per slot), the overflow count, and paired entries
     // (a lane of at most max_stack_rows rows has at most that / pair_seg
     // segments; two lanes per double stack)
-    s->counters_cap = 6 * (size_t)s->n_slots + 16 + kLongBuckets;
+    s->counters_cap = 6 * (size_t)s->n_slots + 17;
     s->slots.assign((size_t)s->n_slots, Slot());
     s->stats.slots = (uint32_t)s->n_slots;
     s->stats.chunks = (uint32_t)s->n_chunks;
