@@ -294,8 +294,7 @@ sw_status enqueue_batch(sw_ctx* ctx, sw_batch_state* b, uint32_t nq, size_t qbyt
             q.nstacks = L.scount;
             q.counters = b->d_counters + L.counter_base;
             q.mat = ctx->d_mat;
-            q.gap_oe = ctx->params.gap_open + ctx->params.gap_extend;
-            q.gap_e = ctx->params.gap_extend;
+            q.gap = gap_args(ctx->params.gap_open, ctx->params.gap_extend);
             q.bnd = b->d_bnd + b->bnd_cap / 2;
             q.bnd_group = L.bnd_group;
             q.scores = b->d_scores;

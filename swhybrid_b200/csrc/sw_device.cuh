@@ -22,6 +22,23 @@ constexpr uint32_t kPadPair = (kZeroCode << 8) | kZeroCode;
 // (H grows by at most max(matrix) per cell, so a lane can only wrap after
 // holding a value above 32767 - max(matrix); the host passes that bound.)
 
+// Gap costs of the paired-query kernel, also as both 16-bit lanes of a word.  As
+// kernel arguments the words can be read from the constant bank where they are
+// used; derived in the kernel they take registers it does not have (16x64 at gap
+// costs 8/2: 234.6 ms, 229.9 with the words; the batch of qp_table's comment).
+// The plain kernel has the registers: with the words it measured up to 6 % slower
+// or 4 % faster by shape, so it derives them.
+struct GapArgs {
+    int oe, e;                  // open + extend, extend
+    uint32_t oe2, e2, ne2;      // (oe, oe), (e, e), (-e, -e)
+};
+
+inline GapArgs gap_args(int open, int extend) {
+    const int oe = open + extend;
+    const uint32_t ne = (uint16_t)(int16_t)-extend;
+    return GapArgs{oe, extend, (uint32_t)oe * 0x10001u, (uint32_t)extend * 0x10001u, ne * 0x10001u};
+}
+
 struct Pair2 {          // per DB record pair, 8 bytes
     uint32_t off16;     // start of the pair's column stream, in 16-byte units
     uint32_t ncols;     // columns (length of the longer record)

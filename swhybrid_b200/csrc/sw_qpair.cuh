@@ -47,7 +47,7 @@ struct QpArgs {
     int nstacks;
     int* counters;              // one unit counter per double stack (zero before)
     const int8_t* mat;
-    int gap_oe, gap_e;          // open + extend, extend
+    GapArgs gap;
     uint2* bnd;                 // per-group boundary rows
     size_t bnd_group;
     int* scores;                // [query][sorted position], zero before (atomicMax)
@@ -541,10 +541,13 @@ __device__ __forceinline__ void run_qpairs(const QpArgs& a, const uint4* prof, c
             const uint32_t keep = ~reset, zr = HZ & reset, zf = FZ & reset;
             const uint8_t* colb = reinterpret_cast<const uint8_t*>(col) + half;
             // thread 0 takes the row above from bq0 (the zero row where there
-            // is none): a branch in this loop costs more than the selects
+            // is none): a branch in this loop costs more than the selects.  One
+            // step per iteration: with two, the kernels with run-time gap costs
+            // spill up to 136 bytes and 32x32 is 6 % slower (237 ms, 223 with one;
+            // 16x64 the same, 16x48 2 % faster; the batch of qp_table's comment)
             auto plain_steps = [&](auto with_bnd) {
                 constexpr bool BND = decltype(with_bnd)::value;
-#pragma unroll 2
+#pragma unroll 1
                 for (; k > 0; --k) {
                     if (BND) __syncwarp();
                     uint32_t h_in = __shfl_up_sync(FULL, out_h, 1, T);
@@ -589,7 +592,7 @@ template <int T, int R, int BLOCK, class CELL>
 __global__ void __launch_bounds__(BLOCK, 1) sw_qpbatch(const QpArgs a) {
     extern __shared__ uint4 prof4[];
     constexpr int G = BLOCK / T;
-    const CELL K(a.gap_oe, a.gap_e);
+    const CELL K(a.gap);
     const int units = 2 * a.pair_count;
     const int n_long = min(a.long_units, units);
     int cur = -1;               // the double stack whose profile is in shared memory

@@ -499,8 +499,7 @@ sw_status enqueue_round(sw_ctx* ctx, sw_serve_state* s, int chunk, int buf,
         q.nstacks = (int)L.count;
         q.counters = s->d_counters + ns + 1 + L.first;
         q.mat = ctx->d_mat;
-        q.gap_oe = ctx->params.gap_open + ctx->params.gap_extend;
-        q.gap_e = ctx->params.gap_extend;
+        q.gap = gap_args(ctx->params.gap_open, ctx->params.gap_extend);
         q.bnd = s->d_bnd;
         q.bnd_group = s->bnd_group;
         q.scores = s->d_scores;

@@ -145,6 +145,10 @@ struct CellNarrow {
     uint32_t ne16;          // (-e, -e)
     int q;
     static constexpr uint32_t Z = (uint32_t)kNarrowZero * 0x10001u;
+    // costs as kernel arguments, for kernels short of registers (see GapArgs)
+    __device__ __forceinline__ explicit CellNarrow(const GapArgs& g)
+        : q2(Q > 0 ? (uint32_t)Q * 0x10001u : g.oe2), e2(Q > 0 ? (uint32_t)E * 0x10001u : g.e2),
+          ne16(Q > 0 ? dup16(-E) : g.ne2), q(Q > 0 ? Q : g.oe) {}
     __device__ __forceinline__ CellNarrow(int q_, int e_) {
         q = Q > 0 ? Q : q_;
         const int e = Q > 0 ? E : e_;

@@ -51,3 +51,20 @@ def test_served_with_every_paired_shape(case, shape, rows, chunks):
         finally:
             c.serve_stop()
     assert [got[i] for i in range(len(queries))] == want
+
+
+@pytest.mark.parametrize("gap_open,gap_extend", [(8, 2), (12, 3), (1, 1), (300, 300)])
+@pytest.mark.parametrize("shape,rows", SHAPES)
+def test_batch_at_run_time_gap_costs(case, shape, rows, gap_open, gap_extend):
+    """Gap costs without a kernel of their own, also where the matrix is too wide
+    for the plain kernel's narrow cell (1/1) and past any score's reach (300/300)."""
+    db, queries = case
+    with capi.Context(0, capi.default_params(gap_open=gap_open, gap_extend=gap_extend)) as c:
+        c.load_db(db.residues, db.offsets)
+        c.set_batch_options(pair_shape=shape, pair_rows=rows)
+        hits, scores = c.search_batch(queries, want_scores=True)
+    for q, sc, h, w in zip(queries, scores, hits,
+                           wanted(db, queries, gap_open + gap_extend, gap_extend)):
+        want = oracle.search(q, db.residues, db.offsets, M, gap_open + gap_extend, gap_extend, mode=0)
+        np.testing.assert_array_equal(sc, want, err_msg=f"query of {len(q)}")
+        assert h == w
