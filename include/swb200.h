@@ -530,8 +530,9 @@ sw_status sw_serve_stop(struct sw_ctx *ctx);
  * residues (a longer one scores 0 and the call returns SW_ERR_UNSUPPORTED
  * after scoring the others), at most 2^31 - 1 records and 2^24 query
  * residues (SW_ERR_UNSUPPORTED, nothing scored).  The first call on a device
- * looks up the array's device address; make that first call before any
- * stream capture.  The call waits for its own work on cuda_stream (NULL =
+ * looks up the array's device address and loads the kernels of every query
+ * length; make that first call (n_records 0 will do) before any stream
+ * capture.  The call waits for its own work on cuda_stream (NULL =
  * the default stream) before it returns.  All calls share the array and
  * each starts by clearing its counter: calls that overlap on the GPU race. */
 sw_status sw_score_noalloc(int device, const sw_params *params, const uint8_t *d_query,

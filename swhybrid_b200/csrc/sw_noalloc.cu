@@ -425,9 +425,35 @@ const NaKernel kNaKernels[] = {
     na_inst<48, true, 256, 1>(),  na_inst<64, true, 256, 1>(),
 };
 
-// Device address of the static scratch, looked up once per device.
+// What the first call on a device looks up.  It also loads every kernel a later
+// call may take (the runtime otherwise loads each one when it is first used,
+// which can allocate device memory and block) and allows it its shared memory.
+struct NaDevice {
+    void* scratch = nullptr;     // device address of the static array
+    int sms = 0, max_smem = 0;
+};
 std::mutex g_na_mutex;
-void* g_na_addr[64] = {nullptr};
+NaDevice g_na_device[64];
+
+bool na_first_call(int device, NaDevice* d) {
+    NaDevice x;
+    if (cudaDeviceGetAttribute(&x.sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&x.max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) !=
+            cudaSuccess ||
+        cudaGetSymbolAddress(&x.scratch, g_noalloc_scratch) != cudaSuccess)
+        return false;
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, (const void*)sw_noalloc_prepare) != cudaSuccess ||
+        cudaFuncGetAttributes(&fa, (const void*)sw_score_noalloc_lookup) != cudaSuccess)
+        return false;
+    for (const NaKernel& k : kNaKernels)
+        if (cudaFuncGetAttributes(&fa, k.fn) != cudaSuccess ||
+            cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 x.max_smem - (int)fa.sharedSizeBytes) != cudaSuccess)
+            return false;
+    *d = x;
+    return true;
+}
 
 }  // namespace
 
@@ -450,18 +476,17 @@ extern "C" sw_status sw_score_noalloc(int device, const sw_params* params, const
     cudaStream_t st = (cudaStream_t)cuda_stream;
     sw_status rc = SW_OK;
     do {
-        void* addr = nullptr;
+        NaDevice dev;
         {
             std::lock_guard<std::mutex> lock(g_na_mutex);
-            if (!g_na_addr[device]) {
-                if (cudaGetSymbolAddress(&g_na_addr[device], g_noalloc_scratch) != cudaSuccess) {
-                    g_na_addr[device] = nullptr;
-                    rc = SW_ERR_CUDA;
-                    break;
-                }
+            if (!g_na_device[device].scratch && !na_first_call(device, &g_na_device[device])) {
+                cudaGetLastError();
+                rc = SW_ERR_CUDA;
+                break;
             }
-            addr = g_na_addr[device];
+            dev = g_na_device[device];
         }
+        void* const addr = dev.scratch;
         if (n_records == 0) break;
         if (qlen == 0) {
             if (cudaMemsetAsync(d_scores, 0, (size_t)n_records * sizeof(int32_t), st) != cudaSuccess)
@@ -487,25 +512,13 @@ extern "C" sw_status sw_score_noalloc(int device, const sw_params* params, const
             a.row_best[i] = 0;
             for (int j = 0; j < 32; ++j) a.row_best[i] = std::max(a.row_best[i], a.mat[i * 32 + j]);
         }
-        int sms = 0, max_smem = 0;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
         const NaKernel* k = nullptr;
         for (const NaKernel& x : kNaKernels)
             if (!k && (x.rows >= (int)qlen || &x == std::end(kNaKernels) - 1)) k = &x;
-        const bool looked_up = k->smem((int)qlen) > (size_t)max_smem;
+        const bool looked_up = k->smem((int)qlen) > (size_t)dev.max_smem;
         const void* fn = looked_up ? (const void*)&sw_score_noalloc_lookup : k->fn;
         const size_t smem = looked_up ? 0 : k->smem((int)qlen);
         const int threads = looked_up ? kNaLookupThreads : k->threads;
-        int occ = 0;
-        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-                cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, threads, smem) !=
-                cudaSuccess || occ < 1 || sms < 1) {
-            cudaGetLastError();
-            rc = SW_ERR_CUDA;
-            break;
-        }
         // the header and the scores (merged by maximum) start at zero
         if (cudaMemsetAsync(addr, 0, sizeof(NaHeader), st) != cudaSuccess ||
             cudaMemsetAsync(d_scores, 0, (size_t)n_records * sizeof(int32_t), st) != cudaSuccess) {
@@ -514,11 +527,10 @@ extern "C" sw_status sw_score_noalloc(int device, const sw_params* params, const
         }
         void* args[] = {&a};
         const unsigned prep = std::min<unsigned>(
-            (unsigned)sms, (std::max(n_records, qlen) + kNaThreads - 1) / kNaThreads);
+            (unsigned)dev.sms, (std::max(n_records, qlen) + kNaThreads - 1) / kNaThreads);
         const unsigned grid =
             looked_up ? (unsigned)(kNaSlices / (kNaLookupThreads / 32))
-                      : std::min<unsigned>((unsigned)(std::min(occ, k->blocks) * sms),
-                                           std::max(n_records, 1u));
+                      : std::min<unsigned>((unsigned)(k->blocks * dev.sms), std::max(n_records, 1u));
         if (cudaLaunchKernel((const void*)sw_noalloc_prepare, dim3(prep), dim3(kNaThreads), args, 0,
                              st) != cudaSuccess ||
             cudaLaunchKernel(fn, dim3(grid), dim3(threads), args, smem, st) != cudaSuccess) {
