@@ -257,12 +257,7 @@ extern "C" sw_status sw_ctx_create(int device, const sw_params* params, sw_ctx**
     return SW_OK;
 }
 
-static void free_db(sw_ctx* ctx) {
-    swb::free_batch(ctx);
-    swb::free_traceback(ctx);
-    swb::free_image(ctx);
-    ctx->rec_pos.clear();
-    ctx->rec_len.clear();
+static void free_db_buffers(sw_ctx* ctx) {
     dev_free(ctx->d_rs_scratch);
     dev_free(ctx->d_db);
     dev_free(ctx->d_pairs);
@@ -276,6 +271,15 @@ static void free_db(sw_ctx* ctx) {
     dev_free(ctx->d_ovf);
     dev_free(ctx->d_keys[0]);
     dev_free(ctx->d_keys[1]);
+}
+
+static void free_db(sw_ctx* ctx) {
+    swb::free_batch(ctx);
+    swb::free_traceback(ctx);
+    swb::free_image(ctx);
+    ctx->rec_pos.clear();
+    ctx->rec_len.clear();
+    free_db_buffers(ctx);
     ctx->n_records = 0;
     ctx->n_pairs = 0;
     ctx->pair_ncols.clear();
@@ -413,36 +417,58 @@ sw_status swb::db_load(sw_ctx* ctx, const uint8_t* residues, const uint64_t* off
         ctx->pair_cols_total += pairs[p].ncols;
         ctx->pair_prefix[p + 1] = ctx->pair_cols_total;
     }
-    auto nomem = [&](const char* what) {
-        free_db(ctx);
-        ctx->err = std::string("device allocation failed: ") + what;
-        return SW_ERR_NOMEM;
-    };
+    ctx->db_units = (uint64_t)units;
+    ctx->max_cols = max_cols;
     // room for windows of long pairs: an eighth of the DB's columns (half a
     // million for a small DB, never more than the DB itself)
     ctx->win_units = std::min<uint64_t>(units, std::max<uint64_t>(units / 8, 65536));
     // (the long-pair kernel's windows need no boundary rows, eight times as
     // much memory: twice the room)
     ctx->long_win_units = std::min<uint64_t>(units, std::max<uint64_t>(units / 4, 131072));
-    if (units + ctx->long_win_units >= (1ull << 32)) ctx->win_units = ctx->long_win_units = 0;
-    ctx->win_cap = (int)(ctx->long_win_units / (kMinWindow / 8) + 1);
-    if (dev_alloc(&ctx->d_db, units + ctx->long_win_units) != cudaSuccess) return nomem("db");
-    if (dev_alloc(&ctx->d_win_pairs, ctx->win_cap) != cudaSuccess) return nomem("windows");
-    if (dev_alloc(&ctx->d_win_ids, ctx->win_cap) != cudaSuccess) return nomem("windows");
-    if (dev_alloc(&ctx->d_pairs, npairs_all) != cudaSuccess) return nomem("pairs");
-    if (dev_alloc(&ctx->d_perm, n) != cudaSuccess) return nomem("perm");
-    if (dev_alloc(&ctx->d_bnd, (units + ctx->win_units) * 16) != cudaSuccess) return nomem("boundary rows");
-    ctx->db_units = (uint64_t)units;
-    if (dev_alloc(&ctx->d_counters, kCounters + n + 1) != cudaSuccess) return nomem("scores");
-    ctx->d_scores = ctx->d_counters + kCounters;
-    if (dev_alloc(&ctx->d_scores_rec, n + 1) != cudaSuccess) return nomem("scores");
-    if (dev_alloc(&ctx->d_ovf, n + 1) != cudaSuccess) return nomem("overflow list");
-    ctx->max_cols = max_cols;
-    if (dev_alloc(&ctx->d_rs_scratch, (size_t)kRescoreWarps * max_cols) != cudaSuccess)
-        return nomem("re-score rows");
+    // Searches do without windows where they do not fit, so a DB that nearly
+    // fills the device gets no room: where it would take over half of what the
+    // DB leaves free, or the buffers do not all fit beside it.
+    size_t free_b = 0, total_b = 0;
+    SW_CUDA(ctx, cudaMemGetInfo(&free_b, &total_b));
     const size_t nblk = (n + kTopkKeys - 1) / kTopkKeys + 1;
-    if (dev_alloc(&ctx->d_keys[0], nblk * kMaxTopK) != cudaSuccess) return nomem("keys");
-    if (dev_alloc(&ctx->d_keys[1], nblk * kMaxTopK) != cudaSuccess) return nomem("keys");
+    const uint64_t db_need = units * 144 + npairs_all * sizeof(Pair2) + n * 16 +
+                             (uint64_t)kRescoreWarps * max_cols * sizeof(uint2) +
+                             2 * nblk * kMaxTopK * sizeof(unsigned long long);
+    const uint64_t win_need = ctx->long_win_units * 16 + ctx->win_units * 128;
+    if (units + ctx->long_win_units >= (1ull << 32) || db_need + 2 * win_need > free_b)
+        ctx->win_units = ctx->long_win_units = 0;
+    auto alloc = [&]() -> const char* {       // null, or what did not fit
+        ctx->win_cap = (int)(ctx->long_win_units / (kMinWindow / 8) + 1);
+        if (dev_alloc(&ctx->d_db, units + ctx->long_win_units) != cudaSuccess) return "db";
+        if (dev_alloc(&ctx->d_win_pairs, ctx->win_cap) != cudaSuccess) return "windows";
+        if (dev_alloc(&ctx->d_win_ids, ctx->win_cap) != cudaSuccess) return "windows";
+        if (dev_alloc(&ctx->d_pairs, npairs_all) != cudaSuccess) return "pairs";
+        if (dev_alloc(&ctx->d_perm, n) != cudaSuccess) return "perm";
+        if (dev_alloc(&ctx->d_bnd, (units + ctx->win_units) * 16) != cudaSuccess)
+            return "boundary rows";
+        if (dev_alloc(&ctx->d_counters, kCounters + n + 1) != cudaSuccess) return "scores";
+        ctx->d_scores = ctx->d_counters + kCounters;
+        if (dev_alloc(&ctx->d_scores_rec, n + 1) != cudaSuccess) return "scores";
+        if (dev_alloc(&ctx->d_ovf, n + 1) != cudaSuccess) return "overflow list";
+        if (dev_alloc(&ctx->d_rs_scratch, (size_t)kRescoreWarps * max_cols) != cudaSuccess)
+            return "re-score rows";
+        if (dev_alloc(&ctx->d_keys[0], nblk * kMaxTopK) != cudaSuccess) return "keys";
+        if (dev_alloc(&ctx->d_keys[1], nblk * kMaxTopK) != cudaSuccess) return "keys";
+        return nullptr;
+    };
+    const char* failed = alloc();
+    if (failed && ctx->long_win_units > 0) {
+        cudaGetLastError();
+        free_db_buffers(ctx);
+        ctx->win_units = ctx->long_win_units = 0;
+        failed = alloc();
+    }
+    if (failed) {
+        free_db(ctx);
+        cudaGetLastError();
+        ctx->err = std::string("device allocation failed: ") + failed;
+        return SW_ERR_NOMEM;
+    }
     if (!stream.empty())
         SW_CUDA(ctx, cudaMemcpy(ctx->d_db, stream.data(), stream.size(), cudaMemcpyHostToDevice));
     if (npairs_all)
