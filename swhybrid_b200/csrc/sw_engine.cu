@@ -1311,17 +1311,20 @@ struct SearchLayout {
 };
 
 // Without a configured shape or cut-over: the layout the time model prefers.
-// Returns false when it keeps one bulk shape for every pair.
+// Returns false when it keeps one bulk shape, the configuration's long one, for
+// every pair (windows and splits take the short one; they are the same but in a
+// caller's table).
 bool model_layout(sw_ctx* ctx, int qlen, int64_t span, SearchLayout* L) {
     const sw_kernel_config& cfg = L->cfg;
     const WfKernel* kb = find_kernel(cfg.short_group_width, cfg.short_rows_per_thread);
-    if (!kb || ctx->n_pairs == 0) return false;
+    const WfKernel* k1 = find_kernel(cfg.long_group_width, cfg.long_rows_per_thread);
+    if (!kb || !k1 || ctx->n_pairs == 0) return false;
     const int rows = std::min(qlen, launch_rows(ctx, *kb, qlen));
     const double share = group_share(ctx, *kb, rows);
     if ((double)ctx->pair_ncols[0] <= 0.9 * share) return false;
     const double np = (double)ctx->n_pairs, total = (double)ctx->pair_cols_total;
     auto passes = [qlen](const WfKernel& k) { return (double)((qlen + k.T * k.R - 1) / (k.T * k.R)); };
-    const double whole = bulk_clocks(*kb, plain_block(ctx, *kb), passes(*kb), np, total,
+    const double whole = bulk_clocks(*k1, plain_block(ctx, *k1), passes(*k1), np, total,
                                      ctx->pair_ncols[0], ctx->num_sms);
     const WfKernel* shapes[kModelShapes];
     const int n_shapes = model_shapes(ctx, qlen, kb, shapes);
@@ -1376,8 +1379,8 @@ void layout_search(sw_ctx* ctx, int qlen, int64_t span, SearchLayout* L) {
     const bool callers_cut = cfg.cutover > 0 && !ctx->tuning_builtin;
     if (!ctx->has_override && !callers_cut) {
         if (model_layout(ctx, qlen, span, L)) return;
-        L->bulk_T = cfg.short_group_width;
-        L->bulk_R = cfg.short_rows_per_thread;
+        L->bulk_T = cfg.long_group_width;
+        L->bulk_R = cfg.long_rows_per_thread;
         L->bulk_b = 0;
         L->bulk_e = ctx->n_pairs;
         L->longest = ctx->n_pairs > 0 ? (double)ctx->pair_ncols[0] : 0.0;
