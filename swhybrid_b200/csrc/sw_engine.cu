@@ -1213,6 +1213,7 @@ LongItemPlan plan_long_items(sw_ctx* ctx, const std::vector<uint32_t>& qlen,
             if (n > 16384) break;
             const double cols = (double)ctx->pair_prefix[n];
             for (const int x : {2, 4, 8, 12, 16, 24, 32, 48, 64, 80, 96}) {
+                if (x >= sms) break;
                 const double tl = std::max(slow * longest, per_col * cols / x) +
                                   0.3 * std::min(slow * longest, per_col * cols / x);
                 const double tb = qp_clocks(loads, total - cols / chunks, ctx->pair_ncols[n],

@@ -155,9 +155,11 @@ struct LongItemPlan {
     size_t smem = 0;
     size_t count() const { return items.size() / 2; }
 };
-// The split of the pairs for queries of the given lengths (0: none), or of
-// `n_long` pairs when that is >= 0.  cols, units: columns and pairs of the
-// paired launches without a split (a serving round sees one chunk of them).
+// The pairs that leave the paired launches (0: none) for queries of the given
+// lengths (0: a query that takes no part), or the items of the first `n_long`
+// pairs when that is >= 0.  loads: the paired launches, each run by groups_per_sm
+// groups an SM whose passes are rows_per_pass rows of both lanes; they score
+// 1 / chunks of the DB's columns.
 LongItemPlan plan_long_items(sw_ctx* ctx, const std::vector<uint32_t>& qlen,
                              const std::vector<QpLoad>& loads, int groups_per_sm, int rows_per_pass,
                              double chunks, int64_t n_long);
