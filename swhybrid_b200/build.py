@@ -32,7 +32,8 @@ def default_header_text(table_path: str = TABLE) -> str:
         "namespace swb {",
         "",
         "// {max_qlen, {long T, long R, short T, short R, cut-over}[, row-segment plan:",
-        "//  {{T, R, passes}, ...}, passes 0 = the rest of the query]}",
+        "//  {{T, R, passes}, ...}, passes 0 = the rest of the query]}.  The cut-overs count",
+        "// where a caller sets the same table; in its place here the time model decides.",
         "constexpr sw_tuning_entry kDefaultTuning[] = {",
     ]
     for row in doc["table"]:

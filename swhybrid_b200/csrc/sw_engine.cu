@@ -663,6 +663,8 @@ extern "C" sw_status sw_get_kernel_config(sw_ctx* ctx, uint32_t qlen, sw_kernel_
     if (!ctx || !cfg) return SW_ERR_INVALID;
     if (!ctx->db_loaded) SW_SET(ctx, SW_ERR_STATE, "no DB loaded");
     *cfg = choose_config(ctx, (int)std::max<uint32_t>(qlen, 1));
+    // the time model takes the place of the built-in table's cut-overs
+    if (!ctx->has_override && ctx->tuning_builtin) cfg->cutover = 0;
     return SW_OK;
 }
 
