@@ -799,6 +799,19 @@ int build_plan(sw_ctx* ctx, int qlen, const WfKernel* ks, double longest, RowSeg
     return n;
 }
 
+// Pipelines of P warps one block of a long kernel holds (0: none fits).
+int long_pipelines(sw_ctx* ctx, const LongKernel& k, int P, size_t* smem) {
+    if (P > kLongMaxPasses) return 0;
+    int n = 0;
+    const sw_ctx::LongFit& f = ctx->long_fit[&k - long_kernels(&n)];
+    const size_t dyn = (size_t)f.max_dyn;
+    const int warp_regs = (f.regs + 7) / 8 * 8 * 32;
+    int G = std::min(k.max_threads / 32, ctx->regs_per_sm / std::max(warp_regs, 1)) / P;
+    while (G > 0 && k.smem(P, G) > dyn) --G;
+    *smem = dyn;
+    return G;
+}
+
 // The long-pair kernel for a query: the configured long shape when the
 // configuration names one apart from the bulk shape (a shape table names one
 // shape for both) and it is a compiled sw_long row count (group width 32)
@@ -813,25 +826,8 @@ const LongKernel* choose_long(sw_ctx* ctx, const sw_kernel_config& cfg, int qlen
     const LongKernel* lk = long_kernels(&n);
     auto fits = [&](const LongKernel& k) {
         const int P = (qlen + 32 * k.R - 1) / (32 * k.R);
-        if (P > kLongMaxPasses) return false;
-        cudaFuncAttributes fa;
-        if (cudaFuncGetAttributes(&fa, k.fn[ctx->cell]) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
-        const size_t dyn = (size_t)ctx->max_smem - fa.sharedSizeBytes;
-        const int warp_regs = (fa.numRegs + 7) / 8 * 8 * 32;
-        int G = std::min(k.max_threads / 32, ctx->regs_per_sm / std::max(warp_regs, 1)) / P;
-        while (G > 0 && k.smem(P, G) > dyn) --G;
-        while (G > 0) {
-            int nb = 0;
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k.fn[ctx->cell], G * P * 32,
-                                                              dyn) ==
-                    cudaSuccess && nb >= 1)
-                break;
-            cudaGetLastError();
-            --G;
-        }
+        size_t dyn = 0;
+        const int G = long_pipelines(ctx, k, P, &dyn);
         if (G == 0) return false;
         *passes = P;
         *pipelines = G;
@@ -986,19 +982,6 @@ struct Split {
     double clocks = 1e300;
 };
 
-// Pipelines of P warps one block of a long kernel holds (0: none fits).
-int long_pipelines(sw_ctx* ctx, const LongKernel& k, int P, size_t* smem) {
-    if (P > kLongMaxPasses) return 0;
-    int n = 0;
-    const sw_ctx::LongFit& f = ctx->long_fit[&k - long_kernels(&n)];
-    const size_t dyn = (size_t)f.max_dyn;
-    const int warp_regs = (f.regs + 7) / 8 * 8 * 32;
-    int G = std::min(k.max_threads / 32, ctx->regs_per_sm / std::max(warp_regs, 1)) / P;
-    while (G > 0 && k.smem(P, G) > dyn) --G;
-    *smem = dyn;
-    return G;
-}
-
 // Bulk shapes the model chooses from: `given`, and (unless they are fixed) the
 // two of each group width that suit the query's rows best.  A table's shape is
 // tuned for a large DB; a small one, or one with long records, wants wider
@@ -1050,7 +1033,7 @@ Split plan_split(sw_ctx* ctx, int qlen, int64_t span, const WfKernel* const* sha
                  int n_shapes) {
     Split best;
     const int64_t np = ctx->n_pairs;
-    if (np == 0) return best;
+    if (np == 0 || n_shapes == 0) return best;    // (no bulk shape: a query of row segments)
     struct Long {
         const LongKernel* k;
         int P, G;
