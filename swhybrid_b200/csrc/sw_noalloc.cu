@@ -316,8 +316,8 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) sw_score_noalloc_kernel(c
     }
 }
 
-// Queries whose byte profile does not fit a block's shared memory (over ~9,000
-// residues): passes of 512 rows, scores looked up in a shared copy of the
+// Queries whose byte profile does not fit a block's shared memory (over 8,192
+// residues, four passes of 51,200 bytes): passes of 512 rows, scores looked up in a shared copy of the
 // matrix, one boundary row of kNaMaxLen per warp.
 __global__ void __launch_bounds__(kNaLookupThreads) sw_score_noalloc_lookup(const NaArgs a) {
     constexpr int kRows = 16;

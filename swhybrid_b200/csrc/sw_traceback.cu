@@ -45,9 +45,9 @@ constexpr int kTbWarpRows = 32 * kTbRows;      // rows per warp
 constexpr int kTbMaxWarps = 32;                // warps (row blocks in flight) per record
 constexpr int kTbK = 32;                       // column steps between block barriers
 // Step lag of warp w behind warp w-1: its last lane writes column c at its
-// step c + 31, the next warp's first lane reads it at step c, K + 1 block steps
-// later, so a barrier lies between; the ring's 128 >= 2K + 1 columns put
-// another between that read and the entry's next write.
+// step c + 31, the next warp's first lane reads it a step ahead of its own, at
+// c - 1, which is K block steps later, so a barrier lies between; the entry's next
+// write (column c + 128) comes 96 >= K steps after that read, past another.
 constexpr int kTbLag = kTbK + 32;
 constexpr int kTbRing = 128;
 constexpr int kTbLimitRows = 512;              // row granularity of the size limit
