@@ -214,8 +214,11 @@ def probe_rates(device: int):
         # functions, and the same cell built by hand from 32-bit operations
         "cell8_intrinsics_gcups": out[14] / 1e9,
         "cell8_swar_gcups": out[15] / 1e9,
-        # the batched kernel's paired-query cell (no per-row byte unpacking)
+        # the wide cell without its per-row byte unpacking
         "cell_pair_mix_gcups": out[16] / 1e9,
+        # the cells that run here: plain, and the paired-query kernel's
+        "cell_narrow_mix_gcups": out[17] / 1e9,
+        "cell_narrow_pair_mix_gcups": out[18] / 1e9,
         "sms": int(sms), "attr_clock_mhz": mhz,
     }
 
@@ -689,7 +692,8 @@ def run_ours(args, rank, world, local_rank):
         peaks, peak_kind = measured_peaks()
         rates = probe_rates(local_rank)
         fp_gcups = tot.cells / (tot.first_pass_ms * 1e-3) / 1e9 if tot.first_pass_ms else None
-        st = ctx.db_stats()
+        # the pairs' column streams: neighbours of the length order side by side
+        column_bytes = int(((np.sort(db.lengths())[::-1][::2] + 7) // 8).sum()) * 16
         lens = [L for (L, _, _) in per_query]
         lat = np.array([t for (_, t, _) in per_query])
         kernel_lat = np.array([k for (_, _, k) in per_query])
@@ -706,7 +710,7 @@ def run_ours(args, rank, world, local_rank):
                        "n_residues": int(db.total), "query_lengths": [len(q) for q in queries],
                        "top_k": 10, "gaps": "open 10 / extend 2", "matrix": "BLOSUM62",
                        "l2": "inputs larger than L2 (DB column streams ~%d MB)" %
-                             (st.device_bytes // 9 // 2**20),
+                             (column_bytes // 2**20),
                        "tuning_table": "swhybrid_b200/tuned/b200.json" if tuned else "cost model",
                        "kernel_config_q144": list(ctx.kernel_config(144)),
                        "kernel_config_q5478": list(ctx.kernel_config(5478)),
@@ -726,19 +730,20 @@ def run_ours(args, rank, world, local_rank):
             "roofline": {
                 "bound": "int_alu (packed int16x2 DPX)",
                 "achieved": round(fp_gcups, 1) if fp_gcups else None,
-                "peak": round(rates["cell_mix_gcups"], 1),
+                "peak": round(rates["cell_narrow_mix_gcups"], 1),
                 "unit": "GCUPS",
-                "frac": round(fp_gcups / rates["cell_mix_gcups"], 4) if fp_gcups else None,
+                "frac": round(fp_gcups / rates["cell_narrow_mix_gcups"], 4) if fp_gcups else None,
                 # DRAM bytes (read + write) of one bulk first-pass launch, from the ncu
-                # capture of sw_wavefront<16,48,256> on this DB with the 1,434-residue
-                # query (dram__bytes_read.sum 1.87 GB + dram__bytes_write.sum 1.61 GB):
-                # the 194 MB column stream once per pass plus the pass-boundary rows
-                # (16 B per column written by pass 0, read by pass 1).  At 3.5 TCUPS
-                # that is ~43 GB/s, far below HBM: the kernel is ALU-bound.
-                "traffic": 3.48e9,
-                "traffic_unit": "bytes per launch (query 1,434, 2 passes)",
+                # capture of sw_wavefront<4,40,384> on this DB with the 1,434-residue
+                # query (dram__bytes_read.sum 7.61 GB + dram__bytes_write.sum 8.42 GB):
+                # the 194 MB column stream once per pass and the boundary rows of eight
+                # hand-offs between nine passes (16 B per column each, written and read;
+                # L2 holds few of them).  44.1 ms: 364 GB/s, far below HBM: the kernel
+                # is ALU-bound.
+                "traffic": 1.603e10,
+                "traffic_unit": "bytes per launch (query 1,434, 9 passes)",
                 "algorithmic_bytes_per_launch": 194_000_000,   # the DB column stream, read once
-                "peak_source": "measured live: libswprobe cell-mix kernel (first-pass "
+                "peak_source": "measured live: libswprobe narrow-cell kernel (first-pass "
                                "instruction mix from registers, full occupancy)",
                 "first_pass_launches": int(tot.first_pass_launches),
                 "first_pass_ms": round(tot.first_pass_ms, 3),
@@ -752,7 +757,7 @@ def run_ours(args, rank, world, local_rank):
         if batched is not None:
             # most of the batch runs two queries per register (no per-row byte
             # unpacking): its roofline is that cell's measured mix
-            pm = rates.get("cell_pair_mix_gcups")
+            pm = rates.get("cell_narrow_pair_mix_gcups")
             batched["roofline"] = {
                 "bound": "int_alu (packed int16x2 DPX, paired queries)",
                 "achieved": batched["value"], "peak": round(pm, 1) if pm else None,
@@ -762,7 +767,7 @@ def run_ours(args, rank, world, local_rank):
         if served is not None:
             # the rounds run the same paired kernel: rate over the rounds'
             # device time against the same measured mix
-            pm = rates.get("cell_pair_mix_gcups")
+            pm = rates.get("cell_narrow_pair_mix_gcups")
             dg = served["saturated"].get("device_gcups")
             served["roofline"] = {
                 "bound": "int_alu (packed int16x2 DPX, paired queries)",

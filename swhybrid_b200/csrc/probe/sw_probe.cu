@@ -13,9 +13,9 @@
 //   op 5  __viaddmax_s16x2 and IMAD interleaved 1:1 (do they co-issue?)
 //   op 6  three-input integer add (IADD3)
 //   op 7  three-input logic op (LOP3)
-//   op 8  the first pass's per-row cell recurrence as sw_wavefront.cuh runs
-//         it (4 DPX + 1 32-bit add + 1 PRMT per row, 1 three-way max per two rows),
-//         without its shared-memory loads and shuffles
+//   op 8  the first pass's per-row cell recurrence for any matrix (CellWide of
+//         sw_wavefront.cuh: 4 DPX + 1 32-bit add + 1 PRMT per row, 1 three-way max
+//         per two rows), without its shared-memory loads and shuffles
 //   op 9  __hmax2 (half2 max), op 10 __hadd2, op 11 __hmax2 and
 //         __viaddmax_s16x2 interleaved 1:1 (does half2 max use another pipe?)
 //   op 12 an 8-bit first pass, four records per register, with CUDA's
@@ -26,10 +26,15 @@
 //   op 13 the same 8-bit cell built by hand: 7-bit lanes under a guard bit,
 //         a byte-wise maximum as a 32-bit subtract (IADD3), a sign-byte
 //         broadcast (PRMT) and a select (LOP3), adds as plain 32-bit adds
-//   op 14 the paired-query cell of the batched kernel (sw_qpair.cuh): the
-//         first pass's mix without the PRMT (profile words arrive packed)
+//   op 14 op 8 without the PRMT (two queries per register: profile words arrive
+//         packed)
+//   op 15 the per-row cell recurrence that ordinary matrices run (CellNarrow of
+//         sw_wavefront.cuh with the costs 12/2 as immediates: 3 DPX + 3 32-bit adds
+//         + 1 PRMT per row, 1 three-way max per two rows), two chains side by side as
+//         in the kernel
+//   op 16 op 15 without the PRMT: the paired-query kernel's cell (sw_qpair.cuh)
 // Rates are returned in lane-operations per second (ops 0-2, 4-7; a 16x2
-// operation counts as two) and in cell updates per second (ops 3, 8, 14: two
+// operation counts as two) and in cell updates per second (ops 3, 8, 14-16: two
 // cells per row and register; ops 12, 13: four).
 #include <cstdint>
 #include <cuda_fp16.h>
@@ -298,6 +303,62 @@ __global__ void __launch_bounds__(512) cell_pair_kernel(uint32_t* sink, int iter
     if (r == 0x9e3779b9u) sink[0] = r;
 }
 
+// CellNarrow's recurrence, two F chains (a thread's two half-columns); PAIR: the
+// profile words arrive packed.
+template <bool PAIR>
+__global__ void __launch_bounds__(512) cell_narrow_kernel(uint32_t* sink, int iters, uint32_t seed) {
+    constexpr int R = 32, HALF = R / 2;
+    constexpr uint32_t Z = 0x04000400u, Q = 0x000c000cu, X = 0x00020002u, NX = 0xfffefffeu;
+    uint32_t H[R], E[R];
+    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        H[k] = Z - Q + ((tid + k) & 0x000f000fu);
+        E[k] = Z;
+    }
+    uint32_t S0 = Z - Q, S1 = Z - Q, f0 = Z, f1 = Z, d0 = Z - Q, d1 = Z - Q;
+    uint32_t A0 = (seed ^ tid) & 0x0f0f0f0fu, A1 = (seed * 3u) & 0x0f0f0f0fu;
+    uint32_t B0 = (seed + tid) & 0x0f0f0f0fu, B1 = ~seed & 0x0f0f0f0fu;
+    uint32_t W[4] = {A0 & 0x000f000fu, A1 & 0x000f000fu, B0 & 0x000f000fu, B1 & 0x000f000fu};
+    auto word = [&](int k) {
+        if (PAIR) return W[k & 3];
+        const uint32_t sel = (uint32_t)(k & 3) | ((uint32_t)((k & 3) | 8) << 4) |
+                             ((uint32_t)(4 + (k & 3)) << 8) | ((uint32_t)((4 + (k & 3)) | 8) << 12);
+        return prmt((k & 4) ? A1 : A0, (k & 4) ? B1 : B0, sel);
+    };
+    for (int i = 0; i < iters; ++i) {
+#pragma unroll
+        for (int k = HALF - 1; k >= 0; --k) {
+            H[HALF + k] = (k ? H[HALF + (k ? k - 1 : 0)] : d1) + word(HALF + k);
+            H[k] = (k ? H[k ? k - 1 : 0] : d0) + word(k);
+        }
+#pragma unroll
+        for (int k = 0; k < HALF; ++k) {
+            const uint32_t h0 = __vimax3_s16x2(H[k], E[k], f0) - Q;
+            const uint32_t h1 = __vimax3_s16x2(H[HALF + k], E[HALF + k], f1) - Q;
+            H[k] = h0;
+            H[HALF + k] = h1;
+            E[k] = __viaddmax_s16x2(E[k], NX, h0);
+            E[HALF + k] = __viaddmax_s16x2(E[HALF + k], NX, h1);
+            f0 = __vimax3_s16x2(f0 - X, h0, Z);
+            f1 = __vimax3_s16x2(f1 - X, h1, Z);
+            if (k & 1) {
+                S0 = __vimax3_s16x2(S0, H[k - 1], h0);
+                S1 = __vimax3_s16x2(S1, H[HALF + k - 1], h1);
+            }
+        }
+        A0 = (A0 * 1664525u + 1013904223u) & 0x0f0f0f0fu;
+        B0 ^= A0;
+        if (PAIR) W[0] = A0 & 0x000f000fu;
+        d0 = (S0 & 0x000f000fu) + (Z - Q);
+        d1 = (S1 & 0x000f000fu) + (Z - Q);
+    }
+    uint32_t r = S0 ^ S1;
+#pragma unroll
+    for (int k = 0; k < R; ++k) r ^= H[k] ^ E[k];
+    if (r == 0x9e3779b9u) sink[0] = r;
+}
+
 template <typename K>
 double time_kernel(K kern, int sms, int iters, uint32_t* sink, double work_per_thread) {
     const int blocks = sms * 4, threads = 512;
@@ -321,8 +382,8 @@ double time_kernel(K kern, int sms, int iters, uint32_t* sink, double work_per_t
 
 // out[0..8] = rates of ops 0..8 (see the file comment); out[9] = SM count;
 // out[10] = SM clock in MHz reported by the device attribute; out[11..13] =
-// rates of ops 9..11; out[14..16] = rates of ops 12..14 (out holds at least
-// 17 entries).  Returns 0 on success.
+// rates of ops 9..11; out[14..18] = rates of ops 12..16 (out holds at least
+// 19 entries).  Returns 0 on success.
 extern "C" int swprobe_rates(int device, double* out, int iters) {
     if (cudaSetDevice(device) != cudaSuccess) return 1;
     int sms = 0, clk = 0;
@@ -348,6 +409,8 @@ extern "C" int swprobe_rates(int device, double* out, int iters) {
     out[14] = time_kernel(cell8_intrin_kernel, sms, iters / 4, sink, 16.0 * 4);
     out[15] = time_kernel(cell8_swar_kernel, sms, iters / 4, sink, 16.0 * 4);
     out[16] = time_kernel(cell_pair_kernel, sms, iters / 4, sink, 16.0 * 2);
+    out[17] = time_kernel(cell_narrow_kernel<false>, sms, iters / 4, sink, 32.0 * 2);
+    out[18] = time_kernel(cell_narrow_kernel<true>, sms, iters / 4, sink, 32.0 * 2);
     cudaFree(sink);
     return cudaGetLastError() == cudaSuccess ? 0 : 3;
 }
