@@ -541,13 +541,16 @@ __device__ __forceinline__ void run_qpairs(const QpArgs& a, const uint4* prof, c
             const uint32_t keep = ~reset, zr = HZ & reset, zf = FZ & reset;
             const uint8_t* colb = reinterpret_cast<const uint8_t*>(col) + half;
             // thread 0 takes the row above from bq0 (the zero row where there
-            // is none): a branch in this loop costs more than the selects.  One
-            // step per iteration: with two, the kernels with run-time gap costs
-            // spill up to 136 bytes and 32x32 is 6 % slower (237 ms, 223 with one;
-            // 16x64 the same, 16x48 2 % faster; the batch of qp_table's comment)
+            // is none): a branch in this loop costs more than the selects.  Two
+            // steps per iteration where the costs are immediates (0.8 % at 16x64 with
+            // 128 served requests, 2 % at 16x48), one where that takes registers the
+            // kernel does not have: with run-time costs (up to 136 bytes spilled)
+            // and at 32x32 (237 ms with two, 223 with one; the batch of qp_table's
+            // comment)
+            constexpr int kUnroll = CELL::kRunTime || T == 32 ? 1 : 2;
             auto plain_steps = [&](auto with_bnd) {
                 constexpr bool BND = decltype(with_bnd)::value;
-#pragma unroll 1
+#pragma unroll kUnroll
                 for (; k > 0; --k) {
                     if (BND) __syncwarp();
                     uint32_t h_in = __shfl_up_sync(FULL, out_h, 1, T);

@@ -145,6 +145,7 @@ struct CellNarrow {
     uint32_t ne16;          // (-e, -e)
     int q;
     static constexpr uint32_t Z = (uint32_t)kNarrowZero * 0x10001u;
+    static constexpr bool kRunTime = Q == 0;
     // costs as kernel arguments, for kernels short of registers (see GapArgs)
     __device__ __forceinline__ explicit CellNarrow(const GapArgs& g)
         : q2(Q > 0 ? (uint32_t)Q * 0x10001u : g.oe2), e2(Q > 0 ? (uint32_t)E * 0x10001u : g.e2),
