@@ -958,7 +958,7 @@ __global__ void __launch_bounds__(BLOCK, 1) sw_batch(const BatchArgs a) {
         r.win_ids = nullptr;
         r.n_win = 0;
         r.counter = a.counters + i;
-        r.first_blocks = (int)gridDim.x;
+        r.first_blocks = 0;     // a block that comes late to a stack must not hold its longest pairs
         r.block0 = 0;
         r.P = P;
         r.pass0 = 0;
