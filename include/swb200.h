@@ -346,8 +346,9 @@ sw_status sw_get_totals(const struct sw_ctx *ctx, sw_totals *out);
  * Options of sw_search_batch.  Queries shorter than stack_rows residues are
  * packed several to a "stack" (rows_per_thread-aligned blocks of one virtual
  * query) and scored by one launch of shape group_width x rows_per_thread;
- * longer queries form stacks of their own, grouped by the shape the tuning
- * table gives their length.  Pairs of records longer than cutover columns run
+ * longer queries form stacks of their own, grouped by the shape a caller's
+ * table or override gives their length, else the one with the least time on
+ * this DB by the time model.  Pairs of records longer than cutover columns run
  * in a concurrent launch with the long shape (0: those too long for the paired
  * launches run beside them in the long-pair kernel).  use_graph != 0
  * captures each batch signature (query count and lengths) as a CUDA graph and

@@ -513,7 +513,7 @@ extern "C" sw_status sw_search_batch(sw_ctx* ctx, uint32_t nq, const uint8_t* qu
     const bool pair_all = qk && b->opt.pair_long;
     uint32_t i0 = 0;
     while (!pair_all && i0 < nz && qlen[order[i0]] >= cap_rows) {
-        const sw_kernel_config c = choose_config(ctx, (int)qlen[order[i0]]);
+        const sw_kernel_config c = choose_stack_config(ctx, (int)qlen[order[i0]], n_long);
         if (buckets.empty() || buckets.back().T != c.short_group_width ||
             buckets.back().R != c.short_rows_per_thread || buckets.back().stacks.size() >= 1024)
             buckets.push_back(Bucket{c.short_group_width, c.short_rows_per_thread, {}});

@@ -953,6 +953,37 @@ double bulk_clocks(const WfKernel& k, int block, double P, double units, double 
     return P * step * (std::max(avg, 1.18 * longest) + tail) + 15e3;
 }
 
+// The shape of a tall query's stack in a batch, whose pairs are [first, n_pairs).
+// The built-in table and the cost model are for the plain kernel with its windows
+// and long-pair split, which the stacked kernel has not; here the shape with the
+// least time is taken, its longest pair's serial columns included (24 queries of
+// 50..3,000 residues in 8x32 stacks of 1,024 rows against 60,000 records, 20 of
+// them of 10,000..35,000 residues: 1,049 ms with the table's shapes, 213 with
+// these; counting the chain of only one stack in full: 42 against 34 ms for 8
+// queries of 2,000..3,000 and 20,000 records).
+sw_kernel_config choose_stack_config(sw_ctx* ctx, int qlen, int64_t first) {
+    if (ctx->has_override || first >= ctx->n_pairs ||
+        (!ctx->tuning_builtin && find_entry(ctx, qlen)))
+        return choose_config(ctx, qlen);      // the caller's shape
+    const double cols = (double)(ctx->pair_cols_total - ctx->pair_prefix[first]);
+    double best = 1e300;
+    sw_kernel_config cfg = choose_config(ctx, qlen);
+    int n = 0;
+    const WfKernel* ks = wf_kernels(&n);
+    for (int i = 0; i < n; ++i) {
+        const WfKernel& k = ks[i];
+        if (shape_occupancy(ctx, k, qlen) == 0) continue;
+        const double t = bulk_clocks(k, k.block, (qlen + k.T * k.R - 1) / (k.T * k.R),
+                                     (double)(ctx->n_pairs - first), cols,
+                                     (double)ctx->pair_ncols[first], ctx->num_sms);
+        if (t < best) {
+            best = t;
+            cfg = sw_kernel_config{k.T, k.R, k.T, k.R, 0};
+        }
+    }
+    return cfg;
+}
+
 // One column step of the long-pair kernel with `warps` warps per SM.
 double long_step_clocks(int R, int warps) {
     const int n = (warps + 3) / 4;      // warps per scheduler

@@ -178,6 +178,7 @@ int launch_rows(sw_ctx* ctx, const WfKernel& k, int qlen);
 sw_status search_host(sw_ctx* ctx, const uint8_t* query, uint32_t qlen, sw_hit* hits,
                       uint32_t* n_hits, int32_t* scores);
 sw_kernel_config choose_config(sw_ctx* ctx, int qlen);
+sw_kernel_config choose_stack_config(sw_ctx* ctx, int qlen, int64_t first);
 sw_status take_marks(sw_ctx* ctx, sw_ctx::Marks* m);
 sw_status drain(sw_ctx* ctx, float* last_ms, float* last_fp_ms);
 void free_batch(sw_ctx* ctx);
