@@ -269,8 +269,9 @@ typedef struct sw_plan_step {
  * library (swhybrid_b200/tuned/b200.json); this call replaces it, and n = 0
  * clears it (the cost model alone chooses).  With the built-in table a time
  * model may take another bulk shape, windows or a long-pair split where the
- * DB's longest pairs ask for one; this call's entries keep their shapes and
- * their cut-overs.
+ * DB's longest pairs ask for one; this call's entries keep their shapes, and
+ * their cut-overs where a pair of that many columns is within a group's even
+ * share of the DB (else windows or a split by the time model).
  *
  * plan (optional, plan[0].group_width = 0 for none): the query's rows in
  * consecutive row segments of different shapes, so that only the last

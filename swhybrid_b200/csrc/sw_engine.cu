@@ -1393,7 +1393,15 @@ bool model_layout(sw_ctx* ctx, int qlen, int64_t span, SearchLayout* L) {
 
 void layout_search(sw_ctx* ctx, int qlen, int64_t span, SearchLayout* L) {
     const sw_kernel_config& cfg = L->cfg = choose_config(ctx, qlen);
-    const bool callers_cut = cfg.cutover > 0 && !ctx->tuning_builtin;
+    // A cut-over of a caller's table counts where the pairs it leaves to the bulk
+    // launch fit a group's even share (the rule of a plan's steps): measured on a
+    // large DB, it has a small one wait for them (4x40 with a cut-over of 4,096,
+    // query 1,434: 44.2 ms against 44.5 without on 570,200 records, but 20.3
+    // against 6.2 on 60,020 and 11.6 against 1.0 on 6,000).
+    const WfKernel* ks = find_kernel(cfg.short_group_width, cfg.short_rows_per_thread);
+    const bool callers_cut =
+        cfg.cutover > 0 && !ctx->tuning_builtin && ks &&
+        (double)cfg.cutover <= plan_share(ctx, *ks, std::min(qlen, launch_rows(ctx, *ks, qlen)));
     if (!ctx->has_override && !callers_cut) {
         if (model_layout(ctx, qlen, span, L)) return;
         L->bulk_T = cfg.long_group_width;
