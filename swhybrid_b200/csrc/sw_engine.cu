@@ -1452,23 +1452,35 @@ void layout_search(sw_ctx* ctx, int qlen, int64_t span, SearchLayout* L) {
     L->bulk_e = ctx->n_pairs;
     L->n_long = L->split ? n_long : 0;
     if (L->split) {
-        // SMs for the long launch: the best of the model for its pairs and
-        // row count beside this bulk shape
+        // SMs and pipelines a block for the long launch: the best of the model for
+        // its pairs and row count beside this bulk shape.  Few pipelines step faster,
+        // which a few much longer pairs want; when only more SMs could make them
+        // few, the launch took 100 SMs and the bulk one waited (query 500 against
+        // 60,020 records, first pass at 8x40 6.3 ms, 2.9 now; at 4x40 6.4, 3.2).
         double best = 1e300;
         const double cols = (double)ctx->pair_prefix[n_long];
         const int G0 = L->lpipes;
         for (int x = 1; x < ctx->num_sms; x += 1 + x / 8) {
-            const int G = (int)std::min<int64_t>(G0, (n_long + x - 1) / x);
-            const double tl = long_clocks(L->lk->R, L->lpasses, G, (double)n_long, cols,
-                                          ctx->pair_ncols[0], x);
+            const int most = (int)std::min<int64_t>(G0, (n_long + x - 1) / x);
+            double tl = 1e300;
+            int G = 0;
+            for (int g = 1; g <= most; g = g < most ? std::min(2 * g, most) : g + 1) {
+                const double t = long_clocks(L->lk->R, L->lpasses, g, (double)n_long, cols,
+                                             ctx->pair_ncols[0], x);
+                if (t < tl) {
+                    tl = t;
+                    G = g;
+                }
+            }
             const WfKernel* k = find_kernel(L->bulk_T, L->bulk_R);
             const double P = k ? (qlen + k->T * k->R - 1) / (k->T * k->R) : 1;
             const double tb = k ? bulk_clocks(*k, plain_block(ctx, *k), P,
                                               (double)(ctx->n_pairs - n_long),
                                               (double)ctx->pair_cols_total - cols,
                                               ctx->pair_ncols[n_long], ctx->num_sms - x) : 0.0;
-            if (std::max(tl, tb) < best) {
-                best = std::max(tl, tb);
+            const double t = std::max(tl, tb) + 0.1 * std::min(tl, tb);
+            if (t < best) {
+                best = t;
                 L->lsms = x;
                 L->lpipes = G;
             }
