@@ -715,7 +715,7 @@ extern "C" sw_status sw_search_batch(sw_ctx* ctx, uint32_t nq, const uint8_t* qu
         }
         std::vector<uint32_t> lq(nq, 0);
         for (uint32_t i = ip; i < nz; ++i) lq[order[i]] = qlen[order[i]];
-        lplan = plan_long_items(ctx, lq, loads, qk->block / qk->T, (int)pass_rows, 1.0, -1);
+        lplan = plan_long_items(ctx, lq, loads, *qk, 1.0, -1);
         bool first_launch = true;
         for (const auto& grp : groups) {
             if (grp.empty()) continue;

@@ -1182,20 +1182,32 @@ Split plan_split(sw_ctx* ctx, int qlen, int64_t span, const WfKernel* const* sha
 // records with 20 of 10,000..35,000 residues: 100 ms a round, 25 of them work).
 // The pairs above a cut-over go to sw_long_items instead, beside the launches.
 
-// Clocks of the paired launches on `sms` SMs, longest record `longest`: a
-// group's step takes as long as the SM's groups at 23.5 cells per clock.
-static double qp_clocks(const std::vector<QpLoad>& loads, double cols, double longest, double groups,
-                        int rows_per_pass, double sms) {
-    const double step = groups * rows_per_pass * 2.0 / 23.5;
+// Clocks of the paired launches on `sms` SMs, longest record `longest`.  While
+// every group has work a group's step takes as long as the SM's groups at 22.5
+// cells per clock; what is left of the longest record's chain then runs beside
+// few others, nearer to a step's own latency.  The chains start with the launch
+// where the long units are dealt first (dealt), else with each double stack, so
+// that the last one's overlaps its own stack only.  (Over 40 batches of 2..64
+// queries against 2,000..57,000 records, four shapes: 0.8..1.2 of the measured
+// time for 8 of 10; with the whole chain at full-load steps 0.92..1.54, and batches
+// of short queries lost up to 26 % to items they did not need.)
+static double qp_clocks(const std::vector<QpLoad>& loads, double cols, double longest,
+                        const QpKernel& k, double sms, bool dealt) {
+    const double groups = (double)k.block / k.T;
+    const double step = groups * k.T * k.R * 2.0 / 22.5;
+    const double few = std::min(step, 0.3 * step + 0.7 * (60.0 + 11.7 * k.R));
     double t = 0;
-    for (const QpLoad& l : loads)
-        t += std::max(l.sum_passes * 2.0 * cols / (groups * sms), l.max_passes * longest) * step + 20e3;
+    for (const QpLoad& l : loads) {
+        const double even = l.sum_passes * 2.0 * cols / (groups * sms);
+        const double beside = dealt ? even : even * l.max_passes / std::max(l.sum_passes, 1.0);
+        t += even * step + std::max(0.0, l.max_passes * longest - beside) * few + 20e3;
+    }
     return t;
 }
 
 LongItemPlan plan_long_items(sw_ctx* ctx, const std::vector<uint32_t>& qlen,
-                             const std::vector<QpLoad>& loads, int groups_per_sm, int rows_per_pass,
-                             double chunks, int64_t given) {
+                             const std::vector<QpLoad>& loads, const QpKernel& k, double chunks,
+                             int64_t given) {
     LongItemPlan plan;
     const int64_t np = ctx->n_pairs;
     if (np == 0) return plan;
@@ -1218,7 +1230,8 @@ LongItemPlan plan_long_items(sw_ctx* ctx, const std::vector<uint32_t>& qlen,
     const double total = (double)ctx->pair_cols_total / chunks, longest = ctx->pair_ncols[0];
     const int sms = ctx->num_sms;
     if (given < 0) {
-        double best = 0.95 * qp_clocks(loads, total, longest, groups_per_sm, rows_per_pass, sms);
+        // (the estimates are good to 20 %: less than that is not worth the split)
+        double best = 0.8 * qp_clocks(loads, total, longest, k, sms, true);
         int64_t prev = 0;
         for (double cut = longest * 0.95; cut >= 256.0; cut /= 1.4) {
             const int64_t n = std::partition_point(ctx->pair_ncols.begin(), ctx->pair_ncols.end(),
@@ -1232,8 +1245,8 @@ LongItemPlan plan_long_items(sw_ctx* ctx, const std::vector<uint32_t>& qlen,
                 if (x >= sms) break;
                 const double tl = std::max(slow * longest, per_col * cols / x) +
                                   0.3 * std::min(slow * longest, per_col * cols / x);
-                const double tb = qp_clocks(loads, total - cols / chunks, ctx->pair_ncols[n],
-                                            groups_per_sm, rows_per_pass, sms - x);
+                const double tb =
+                    qp_clocks(loads, total - cols / chunks, ctx->pair_ncols[n], k, sms - x, false);
                 if (std::max(tl, tb) < best) {
                     best = std::max(tl, tb);
                     plan.n_long = n;
@@ -1245,7 +1258,7 @@ LongItemPlan plan_long_items(sw_ctx* ctx, const std::vector<uint32_t>& qlen,
         // the pairs are given: SMs in proportion to the work
         plan.n_long = given;
         const double wl = per_col * (double)ctx->pair_prefix[given];
-        const double wb = qp_clocks(loads, total, 0.0, groups_per_sm, rows_per_pass, 1.0);
+        const double wb = qp_clocks(loads, total, 0.0, k, 1.0, true);
         plan.sms = std::max(1, std::min(sms * 2 / 3, (int)std::lround(sms * wl / (wl + wb))));
     }
     if (plan.n_long == 0) return plan;

@@ -157,12 +157,12 @@ struct LongItemPlan {
 };
 // The pairs that leave the paired launches (0: none) for queries of the given
 // lengths (0: a query that takes no part), or the items of the first `n_long`
-// pairs when that is >= 0.  loads: the paired launches, each run by groups_per_sm
-// groups an SM whose passes are rows_per_pass rows of both lanes; they score
+// pairs when that is >= 0.  loads: the paired launches, of kernel k, each over
 // 1 / chunks of the DB's columns.
+struct QpKernel;
 LongItemPlan plan_long_items(sw_ctx* ctx, const std::vector<uint32_t>& qlen,
-                             const std::vector<QpLoad>& loads, int groups_per_sm, int rows_per_pass,
-                             double chunks, int64_t n_long);
+                             const std::vector<QpLoad>& loads, const QpKernel& k, double chunks,
+                             int64_t n_long);
 sw_status launch_long_items(sw_ctx* ctx, cudaStream_t stream, const LongItemPlan& plan,
                             const uint2* d_items, int* d_counter, const uint8_t* d_queries,
                             const uint32_t* d_qoff, const uint32_t* d_qlens, int* d_scores,

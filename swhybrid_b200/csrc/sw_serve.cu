@@ -374,8 +374,7 @@ sw_status enqueue_round(sw_ctx* ctx, sw_serve_state* s, int chunk, int buf,
             loads.push_back(load);
         }
         if (any) {
-            lplan = plan_long_items(ctx, lq, loads, qk->block / qk->T, (int)(qT * qR),
-                                    (double)s->n_chunks, s->n_long);
+            lplan = plan_long_items(ctx, lq, loads, *qk, (double)s->n_chunks, s->n_long);
             if (lplan.n_long == 0)
                 SW_SET(ctx, SW_ERR_UNSUPPORTED, "long pairs of a round do not fit shared memory");
         }

@@ -14,6 +14,7 @@ SOURCE = r"""
 #include <cstdio>
 #include <cstdlib>
 #include "csrc/sw_engine.h"
+#include "csrc/sw_registry.h"
 int main(int argc, char** argv) {
     sw_ctx c;
     c.num_sms = atoi(argv[1]);
@@ -29,7 +30,7 @@ int main(int argc, char** argv) {
     std::vector<swb::QpLoad> loads(3);
     for (auto& l : loads) { l.sum_passes = 8; l.max_passes = 2; }
     const swb::LongItemPlan plan =
-        swb::plan_long_items(&c, qlen, loads, 16, 1024, 1.0, argc > 2 ? atoi(argv[2]) : -1);
+        swb::plan_long_items(&c, qlen, loads, *swb::find_qp(16, 64), 1.0, argc > 2 ? atoi(argv[2]) : -1);
     printf("%lld %d %zu\n", (long long)plan.n_long, plan.sms, plan.count());
 }
 """
