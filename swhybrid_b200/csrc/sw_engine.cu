@@ -1183,19 +1183,23 @@ Split plan_split(sw_ctx* ctx, int qlen, int64_t span, const WfKernel* const* sha
 // The pairs above a cut-over go to sw_long_items instead, beside the launches.
 
 // Clocks of the paired launches on `sms` SMs, longest record `longest`.  While
-// every group has work a group's step takes as long as the SM's groups at 22.5
+// every group has work a group's step takes as long as the SM's groups at 21.5
 // cells per clock; what is left of the longest record's chain then runs beside
 // few others, nearer to a step's own latency.  The chains start with the launch
 // where the long units are dealt first (dealt), else with each double stack, so
-// that the last one's overlaps its own stack only.  (Over 40 batches of 2..64
-// queries against 2,000..57,000 records, four shapes: 0.8..1.2 of the measured
-// time for 8 of 10; with the whole chain at full-load steps 0.92..1.54, and batches
-// of short queries lost up to 26 % to items they did not need.)
+// that the last one's overlaps its own stack only.  Over 110 batches of 2..64
+// queries against 2,000..57,000 records in four shapes, without items: 0.81..1.21
+// of the measured time for 8 of 10.  With plan_long_items' choice by it (and what
+// it weighs the items at) a batch took 1.036 of the best choice's time in the
+// geometric mean and in 3 of the 110 over 1.02 of the time without items, 1.06
+// at most.  (With the whole chain at full-load steps, as it was, 45 queries of
+// 81..478 residues against 32,360 records took 28.0 ms at 32x32, 22 without items.)
 static double qp_clocks(const std::vector<QpLoad>& loads, double cols, double longest,
                         const QpKernel& k, double sms, bool dealt) {
     const double groups = (double)k.block / k.T;
-    const double step = groups * k.T * k.R * 2.0 / 22.5;
-    const double few = std::min(step, 0.3 * step + 0.7 * (60.0 + 11.7 * k.R));
+    const double step = groups * k.T * k.R * 2.0 / 21.5;
+    const double full = dealt ? 0.3 : 0.6;
+    const double few = std::min(step, full * step + (1.0 - full) * (60.0 + 11.7 * k.R));
     double t = 0;
     for (const QpLoad& l : loads) {
         const double even = l.sum_passes * 2.0 * cols / (groups * sms);
@@ -1211,27 +1215,27 @@ LongItemPlan plan_long_items(sw_ctx* ctx, const std::vector<uint32_t>& qlen,
     LongItemPlan plan;
     const int64_t np = ctx->n_pairs;
     if (np == 0) return plan;
-    auto step_of = [](uint32_t q, int* pipes) {
-        const int R = long_item_rows((int)q), P = (int)((q + 32 * R - 1) / (32 * R));
-        *pipes = kLongItemWarps / P;
-        return long_step_clocks(R, P * *pipes);
+    // a query's items: pipelines, clocks a step, steps besides the columns' (half
+    // the pipeline's fill, whose steps have fewer warps)
+    struct Query {
+        uint32_t q;
+        int G;
+        double step, fill;
     };
-    // per pair column: SM clocks of all queries, and the slowest query's step
-    double per_col = 0, slow = 0;
-    for (const uint32_t q : qlen) {
-        if (q == 0) continue;
-        if (q > (uint32_t)kLongItemRows) return plan;     // too long for a block's warps
-        int G = 0;
-        const double step = step_of(q, &G);
-        per_col += step / G;
-        slow = std::max(slow, step);
+    std::vector<Query> queries;
+    for (uint32_t q = 0; q < (uint32_t)qlen.size(); ++q) {
+        if (qlen[q] == 0) continue;
+        if (qlen[q] > (uint32_t)kLongItemRows) return plan;     // too long for a block's warps
+        const int R = long_item_rows((int)qlen[q]);
+        const int P = (int)((qlen[q] + 32 * R - 1) / (32 * R)), G = kLongItemWarps / P;
+        queries.push_back(Query{q, G, 1.04 * long_step_clocks(R, P * G), (P - 1) * 32.0 + 48.0});
     }
-    if (per_col == 0) return plan;
+    if (queries.empty()) return plan;
     const double total = (double)ctx->pair_cols_total / chunks, longest = ctx->pair_ncols[0];
     const int sms = ctx->num_sms;
     if (given < 0) {
-        // (the estimates are good to 20 %: less than that is not worth the split)
-        double best = 0.8 * qp_clocks(loads, total, longest, k, sms, true);
+        // (less than a tenth is within the estimates' error)
+        double best = 0.9 * qp_clocks(loads, total, longest, k, sms, true);
         int64_t prev = 0;
         for (double cut = longest * 0.95; cut >= 256.0; cut /= 1.4) {
             const int64_t n = std::partition_point(ctx->pair_ncols.begin(), ctx->pair_ncols.end(),
@@ -1241,10 +1245,16 @@ LongItemPlan plan_long_items(sw_ctx* ctx, const std::vector<uint32_t>& qlen,
             prev = n;
             if (n > 16384) break;
             const double cols = (double)ctx->pair_prefix[n];
+            double work = 0, chain = 0;         // of all items, of the longest
+            for (const Query& q : queries) {
+                const double G = (double)std::min<int64_t>(q.G, n);
+                work += q.step * (cols / G + q.fill * std::ceil(n / G));
+                chain = std::max(chain, q.step * (longest + q.fill));
+            }
             for (const int x : {2, 4, 8, 12, 16, 24, 32, 48, 64, 80, 96}) {
                 if (x >= sms) break;
-                const double tl = std::max(slow * longest, per_col * cols / x) +
-                                  0.3 * std::min(slow * longest, per_col * cols / x);
+                const double tl =
+                    std::max(chain, work / x) + 0.1 * std::min(chain, work / x);
                 const double tb =
                     qp_clocks(loads, total - cols / chunks, ctx->pair_ncols[n], k, sms - x, false);
                 if (std::max(tl, tb) < best) {
@@ -1254,12 +1264,8 @@ LongItemPlan plan_long_items(sw_ctx* ctx, const std::vector<uint32_t>& qlen,
                 }
             }
         }
-    } else if (given > 0) {
-        // the pairs are given: SMs in proportion to the work
+    } else {
         plan.n_long = given;
-        const double wl = per_col * (double)ctx->pair_prefix[given];
-        const double wb = qp_clocks(loads, total, 0.0, k, 1.0, true);
-        plan.sms = std::max(1, std::min(sms * 2 / 3, (int)std::lround(sms * wl / (wl + wb))));
     }
     if (plan.n_long == 0) return plan;
     struct Item {
@@ -1267,15 +1273,22 @@ LongItemPlan plan_long_items(sw_ctx* ctx, const std::vector<uint32_t>& qlen,
         double t;
     };
     std::vector<Item> list;
-    for (uint32_t q = 0; q < (uint32_t)qlen.size(); ++q) {
-        if (qlen[q] == 0) continue;
-        int G = 0;
-        const double step = step_of(qlen[q], &G);
-        plan.smem = std::max(plan.smem, long_item_smem((int)qlen[q]));
-        for (int64_t p = 0; p < plan.n_long; p += G)
-            list.push_back(Item{q, (uint32_t)p, ctx->pair_ncols[p] * step});
+    for (const Query& q : queries) {
+        plan.smem = std::max(plan.smem, long_item_smem((int)qlen[q.q]));
+        for (int64_t p = 0; p < plan.n_long; p += q.G)
+            list.push_back(Item{q.q, (uint32_t)p, (ctx->pair_ncols[p] + q.fill) * q.step});
     }
     if (plan.smem > (size_t)ctx->max_smem - 1024) return LongItemPlan{};
+    if (given > 0) {
+        // the pairs are given: SMs in proportion to the work, the items' as their
+        // blocks hold it (an item lasts as long as its first pair, however many of
+        // its pipelines have one: by the pairs' columns alone 52 requests of 309..7,284
+        // residues waited 16 ms for their items after 59 ms of a round's launches)
+        double wl = 0;
+        for (const Item& i : list) wl += i.t;
+        const double wb = qp_clocks(loads, total, 0.0, k, 1.0, true);
+        plan.sms = std::max(1, std::min(sms * 2 / 3, (int)std::lround(sms * wl / (wl + wb))));
+    }
     std::stable_sort(list.begin(), list.end(),
                      [](const Item& x, const Item& y) { return x.t > y.t; });
     for (const Item& i : list) {
