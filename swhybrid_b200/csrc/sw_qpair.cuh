@@ -430,13 +430,11 @@ __device__ __forceinline__ void run_qpairs(const QpArgs& a, const uint4* prof, c
             const uint32_t cont = (t > 0) ? ~f_reset : 0u;
             m = __vimax3_s16x2(m, (acc_in & cont) | (HZ & ~cont), HZ);
             acc_out = m;
-            // (a unit past the end has no entry in pair_ids: its number decides first)
-            int pos = a.n_records;
-            if (f_unit < units) {
-                const int at = a.pair_begin + (f_unit >> 1);
-                pos = 2 * (a.pair_ids ? (int)a.pair_ids[at] : at) + (f_unit & 1);
-            }
-            if (pos < a.n_records) {
+            // (a unit past the end has no entry in pair_ids: the last one's is read)
+            const int at = a.pair_begin + (min(f_unit, units - 1) >> 1);
+            const int gp = a.pair_ids ? (int)a.pair_ids[at] : at;
+            const int pos = 2 * gp + (f_unit & 1);
+            if (pos < a.n_records && f_unit < units) {
                 if (fq_lo >= 0 && (f_last & 0xffffu)) {
                     const int s0 = lo16(m);
                     const int qb = fq_lo * a.n_records;
