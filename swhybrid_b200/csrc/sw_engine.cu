@@ -1504,7 +1504,7 @@ void layout_search(sw_ctx* ctx, int qlen, int64_t span, SearchLayout* L) {
                                               (double)(ctx->n_pairs - n_long),
                                               (double)ctx->pair_cols_total - cols,
                                               ctx->pair_ncols[n_long], ctx->num_sms - x) : 0.0;
-            const double t = std::max(tl, tb) + 0.1 * std::min(tl, tb);
+            const double t = std::max(tl, tb) + 0.01 * std::min(tl, tb);
             if (t < best) {
                 best = t;
                 L->lsms = x;
