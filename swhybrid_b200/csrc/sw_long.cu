@@ -38,7 +38,7 @@
 // (sw_windows) that are units of their own and merge by maximum.
 // Query 1,900 against 20,200 records of which 200 hold 43 % of the residues:
 // 17.5 ms before (two half-columns per thread, guarded steps, 3 warps of 24 rows
-// per pair, pipelines crowded on few SMs), 5.2 now.
+// per pair, pipelines crowded on few SMs), 5.5 now.
 #include <cstdint>
 
 #include <cuda_runtime.h>

@@ -24,7 +24,7 @@
 // one), 5.5 with the byte profile's extraction.  The profile is read from shared memory,
 // one conflict-free 16- or 4-byte word per 4 rows; looking each cell up in the
 // matrix cost a bank-conflicted load per cell.  10,000 records, query 375:
-// 4,400 us a call before (256 warps, 512-row passes, matrix lookups), 559 now.
+// 4,400 us a call before (256 warps, 512-row passes, matrix lookups), 527 now.
 //
 // A record is a serial chain of columns, so records longer than an even share
 // of the columns are cut into windows that overlap by the longest span an

@@ -520,7 +520,9 @@ sw_status enqueue_round(sw_ctx* ctx, sw_serve_state* s, int chunk, int buf,
         // Every launch of the round leaves the long items their SMs: units are
         // dealt to blocks, and one that waited for such an SM held its launch to
         // the end of the long items (384 requests queued at once against 570,200
-        // records: 6.03 TCUPS with only the first launch leaving them, 6.52 now).
+        // records: 6.03 TCUPS with only the first launch leaving them, 6.50 now;
+        // 6.51 with the long records in the ring, where one held a light load's
+        // rounds: 1,000 requests at half that rate p50 0.70 s, 0.34 now).
         const int sms = ctx->num_sms - lplan.sms;
         q.long_units = qp_long_units([&](int p) { return (uint64_t)s->ring_ncols[(size_t)(cb + p)]; },
                                      pair_count, s->chunk_cols[(size_t)chunk],

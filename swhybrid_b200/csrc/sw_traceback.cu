@@ -23,7 +23,7 @@
 // branch: columns outside the record run on zero-score residues.  The walk is a
 // chain of loads, one per run.  Ten alignments of 1,000 x 1,000: 2,340 us a call before (one
 // warp per record, 16 rows a lane in two passes, matrix lookups per cell, one
-// dependent load per walked cell), TB1 now.
+// dependent load per walked cell), 481 now.
 // The direction bits take qlen x record length / 2 bytes per record, in a
 // scratch buffer the context keeps (grown on demand, bounded per call).
 #include <algorithm>

@@ -16,8 +16,9 @@ constexpr WfKernel inst() {
 }  // namespace
 
 // rows per thread R (any even number; the two half-columns hold R/2 rows
-// each) and the block size that leaves every shape register room without
-// spilling (block sizes are multiples of 128 threads); 48 rows run 12 warps
+// each) and the block size that leaves every shape register room with next
+// to no spilling (16 rows: up to 16 bytes, 8 stacked: 6, 48 with run-time gap costs:
+// 8; block sizes are multiples of 128 threads); 48 rows run 12 warps
 // per SM with CellNarrow (6.05 against 5.65 TCUPS at 8) and 8 with CellWide
 extern const WfKernel wf_table_t32[] = {
     inst<4, 768>(),  inst<6, 768>(),  inst<8, 768>(),  inst<10, 640>(), inst<12, 640>(),
